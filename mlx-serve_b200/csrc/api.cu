@@ -885,6 +885,7 @@ QB200_API int qb200_kv_decode_attention(qb200_tensor* res, const qb200_tensor* q
   a.B = B; a.Hq = Hq; a.Hkv = Hkv; a.T = T; a.D = D; a.Dv = Dv;
   a.q_str[0] = q->stride[0]; a.q_str[1] = q->stride[1];
   a.o_str[0] = res->stride[0]; a.o_str[1] = res->stride[1];
+  a.Tq = (int)Tq; a.q_tq = q->stride[2]; a.o_tq = res->stride[2];
   for (int d = 0; d < 3; ++d) {
     a.kq_str[d] = k_q->stride[d]; a.ksb_str[d] = k_scales->stride[d];
     a.vq_str[d] = v_q->stride[d]; a.vsb_str[d] = v_scales->stride[d];
@@ -904,9 +905,15 @@ QB200_API int qb200_kv_decode_attention(qb200_tensor* res, const qb200_tensor* q
     return fail(QB200_ERR_WORKSPACE, "kv_decode_attention: workspace of %zu bytes needed, %zu given", need, workspace_bytes);
   if (Tq > 1) {
     // Verify widths: query position tq of sequence b attends to the first T - T_q + 1 + tq cache positions (the
-    // end-aligned causal tail, src/transformer.zig:5314-5318).  Every (b, tq) runs as a sequence of its own over the
-    // same cache view, with that length; the cache is read T_q times, the repeats out of L2.
+    // end-aligned causal tail, src/transformer.zig:5314-5318).
     if (T < Tq) return fail(QB200_ERR_BAD_SHAPE, "kv_decode_attention: the cache view must hold at least T_q tokens");
+    if (kv_f16_supported(a)) {   // the query positions are rows of the kernel's query tiles
+      const cudaError_t ev = launch_kv_attn(a, (cudaStream_t)s);
+      if (ev != cudaSuccess) return cuda_fail(ev, "kv_decode_attention");
+      return QB200_OK;
+    }
+    // Other geometries: every (b, tq) runs as a sequence of its own over the same cache view, with that length; the
+    // cache is read T_q times, the repeats out of L2.
     const int esz = dtype_size(q->dtype);
     for (int64_t b = 0; b < B; ++b) {   // one launch per sequence: its T_q query positions as T_q "sequences"
       KvSeqTable tab;
@@ -923,7 +930,7 @@ QB200_API int qb200_kv_decode_attention(qb200_tensor* res, const qb200_tensor* q
         e.T = T - Tq + 1 + tq;
       }
       KvAttnArgs c = a;
-      c.B = Tq;
+      c.B = Tq; c.Tq = 1;
       c.q = (const char*)q->data + b * q->stride[0] * esz;
       c.out = (char*)res->data + b * res->stride[0] * esz;
       c.q_str[0] = q->stride[2];
@@ -1008,6 +1015,7 @@ QB200_API int qb200_kv_decode_attention_ptrs(qb200_tensor* res, const qb200_tens
   a.Hq = Hq; a.Hkv = Hkv; a.T = T_max; a.D = D; a.Dv = Dv;
   a.q_str[0] = q->stride[0]; a.q_str[1] = q->stride[1];
   a.o_str[0] = res->stride[0]; a.o_str[1] = res->stride[1];
+  a.Tq = 1; a.q_tq = 0; a.o_tq = 0;
   a.gs = gs; a.bits = nb; a.scale = scale;
   if ((st = parse_kv_mask(a, q, mask_mode, mask_arr, kv_lens, B, T_max))) return st;
   a.B = B < kMaxSeqPtrs ? B : kMaxSeqPtrs;

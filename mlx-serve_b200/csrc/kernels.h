@@ -193,6 +193,7 @@ struct KvAttnArgs {
   const uint32_t* vq; const void* vs; const void* vb;
   int64_t B, Hq, Hkv, T, D, Dv;
   int64_t q_str[2], o_str[2];          // (batch, head) strides in elements; last dim contiguous
+  int Tq; int64_t q_tq, o_tq;          // query positions (causal tail when > 1) and their strides
   int64_t kq_str[3], ksb_str[3];       // (batch, head, token)
   int64_t vq_str[3], vsb_str[3];
   int gs, bits;
@@ -215,7 +216,8 @@ struct KvSeqTable { KvSeq s[kMaxSeqPtrs]; };
 struct KvNoTable {};
 size_t kv_attn_workspace_bytes(int64_t B, int64_t Hq, int64_t Hkv, int64_t T, int64_t Dv);
 bool kv_attn_supported(const KvAttnArgs& a);
-bool kv_fast_supported(const KvAttnArgs& a, const KvSeqTable* seqs = nullptr);
+bool kv_fast_supported(const KvAttnArgs& a, const KvSeqTable* seqs = nullptr);   // kv_attn_fast.cu: integer MMA, D = 128, GQA <= 4, T_q = 1
+bool kv_f16_supported(const KvAttnArgs& a, const KvSeqTable* seqs = nullptr);    // kv_attn_f16.cu: fp16 MMA, D = 64 / 128, GQA <= 8, T_q <= 8
 cudaError_t launch_kv_attn(const KvAttnArgs& a, cudaStream_t st, const KvSeqTable* seqs = nullptr);  // seqs: a.B <= kMaxSeqPtrs views, a.T their longest
 
 }  // namespace qb

@@ -26,11 +26,9 @@ struct SplitPlan {
   int64_t tokens_per_split;  // multiple of 128
 };
 
-// Deterministic in (B, Hkv, T) so that the workspace query and the launch agree.
-// A split is served by one CTA of 8 warps that take its 128-token blocks round-robin.  The plan minimises
-//   waves of CTAs over the GPU x (blocks per warp + a fixed per-CTA cost of ~0.7 block times)
-// summed over the two residencies the fast kernel has (one CTA per SM at 8 bits, two at 4 bits; the bit
-// width is not an input here because the workspace query does not know it).
+// Deterministic in (B, Hkv, T): sizes the workspace, and is the plan of the CUDA-core kernel.  It minimises waves of CTAs
+// over the GPU x (128-token blocks per warp of 8 + a fixed per-CTA cost of ~0.7 block times), summed over one and two CTAs
+// per SM.
 __host__ SplitPlan plan_splits(int64_t B, int64_t Hkv, int64_t T) {
   SplitPlan p;
   const int nsm = sm_count();   // CTA slots: one CTA per SM at 8 bits, two at 4 bits
@@ -53,6 +51,30 @@ __host__ SplitPlan plan_splits(int64_t B, int64_t Hkv, int64_t T) {
   p.nsplit = (int)best_ns;
   p.tokens_per_split = best_tps;
   return p;
+}
+
+// Splits of the fp16 tensor-core kernel.  Three CTAs of 4 warps live on an SM; a CTA's warps take the 64-token blocks of its
+// split in turn, so a round of a CTA is 256 tokens.  A round costs about 0.9 us in a CTA that has its SM to itself and
+// 0.6 us of SM time when three share it; a CTA's start and end cost about one round; beyond 8 splits the partial results
+// go through memory and a merge launch (about 2.5 us).  The partials have to fit the workspace the caller was told to
+// bring, which plan_splits sized.
+__host__ int plan_f16(const KvAttnArgs& a, int64_t qtiles, int max_fused) {
+  const int64_t pairs = a.B * a.Hkv * qtiles, nsm = sm_count();
+  const int64_t rows = a.B * a.Hq * a.Tq;
+  const int64_t fit = (int64_t)(a.workspace_bytes / sizeof(float)) / (rows * (2 + a.Dv));
+  int64_t max_ns = (a.T + 127) / 128;
+  if (max_ns > 1024) max_ns = 1024;
+  int64_t best = 1;
+  double best_cost = -1.0;
+  for (int64_t ns = 1; ns <= max_ns && (ns <= max_fused || ns <= fit); ++ns) {
+    const double rounds = (double)((((a.T + ns - 1) / ns + 63) / 64 + 3) / 4) + 1.0;
+    const int64_t per_sm = (pairs * ns + nsm - 1) / nsm, full = per_sm / 3, rest = per_sm % 3;
+    double cost = (double)full * rounds * 1.8;
+    if (rest) cost += rounds * (rest == 1 ? 0.9 : 1.3);
+    if (ns > max_fused) cost += 2.5;
+    if (best_cost < 0.0 || cost < best_cost - 1e-9) { best_cost = cost; best = ns; }
+  }
+  return (int)best;
 }
 
 struct KvK {
@@ -221,21 +243,34 @@ __global__ void __launch_bounds__(128) kv_split_generic(KvK p, const __grid_cons
   }
 }
 
-// out = (sum_b o_b w_b) / (sum_b l_b w_b), w_b = exp(m_b - max m)  (src/transformer.zig:5194-5203)
-__global__ void kv_merge(KvK p) {
+// out = (sum_b o_b w_b) / (sum_b l_b w_b), w_b = exp(m_b - max m)  (src/transformer.zig:5194-5203).  A CTA per output
+// row; launched as a programmatic dependent of the split kernel.
+__global__ void __launch_bounds__(128) kv_merge(KvK p) {
   const KvAttnArgs& a = p.a;
-  const int h = blockIdx.x;
+  __shared__ float wgt[1024];   // plan_splits and plan_f16 cap the splits at 1024
+  const int h = blockIdx.x, tq = blockIdx.z;
   const int64_t b = blockIdx.y;
-  const int64_t base = (b * a.Hq + h) * p.nsplit;
+  const int64_t base = ((b * a.Hq + h) * a.Tq + tq) * p.nsplit;
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   float M = kNegBig;
-  for (int s = 0; s < p.nsplit; ++s) M = fmaxf(M, p.part_m[base + s]);
+  for (int s = threadIdx.x & 31; s < p.nsplit; s += 32) M = fmaxf(M, p.part_m[base + s]);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, o));
   float L = 0.f;
-  for (int s = 0; s < p.nsplit; ++s) L += p.part_l[base + s] * __expf(p.part_m[base + s] - M);
+  for (int s = threadIdx.x & 31; s < p.nsplit; s += 32) {
+    const float w = __expf(p.part_m[base + s] - M);
+    if (threadIdx.x < 32) wgt[s] = w;
+    L += p.part_l[base + s] * w;
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) L += __shfl_xor_sync(0xffffffffu, L, o);
   const float inv = L > 0.f ? 1.f / L : 0.f;
+  __syncthreads();
   for (int e = threadIdx.x; e < a.Dv; e += blockDim.x) {
     float O = 0.f;
-    for (int s = 0; s < p.nsplit; ++s) O += p.part_o[(base + s) * a.Dv + e] * __expf(p.part_m[base + s] - M);
-    const int64_t off = b * a.o_str[0] + (int64_t)h * a.o_str[1] + e;
+#pragma unroll 4
+    for (int s = 0; s < p.nsplit; ++s) O += p.part_o[(base + s) * a.Dv + e] * wgt[s];
+    const int64_t off = b * a.o_str[0] + (int64_t)h * a.o_str[1] + tq * a.o_tq + e;
     const float v = O * inv;
     if (a.q_dtype == QB200_FLOAT32) ((float*)a.out)[off] = v;
     else ((uint16_t*)a.out)[off] = f32_to_bf16_bits(v);
@@ -244,8 +279,10 @@ __global__ void kv_merge(KvK p) {
 
 }  // namespace
 
-cudaError_t launch_kv_fast(const KvAttnArgs& a, int nsplit, int64_t tps, float* pm, float* pl, float* po,
-                           cudaStream_t st, const KvSeqTable* seqs, bool fused);
+cudaError_t launch_kv_fast(const KvAttnArgs& a, int nsplit, float* pm, float* pl, float* po, cudaStream_t st, const KvSeqTable* seqs,
+                           bool fused);
+cudaError_t launch_kv_f16(const KvAttnArgs& a, int nsplit, float* pm, float* pl, float* po, cudaStream_t st, const KvSeqTable* seqs,
+                          bool fused);
 constexpr int kMaxFusedSplits = 8;   // the portable cluster size
 
 size_t kv_attn_workspace_bytes(int64_t B, int64_t Hq, int64_t Hkv, int64_t T, int64_t Dv) {
@@ -262,16 +299,6 @@ bool kv_attn_supported(const KvAttnArgs& a) {
   if (gqa < 1 || gqa > kMaxGqa) return false;
   if (a.Hkv > 65535 || a.B > 65535) return false;
   return true;
-}
-
-// QB200_KV_FUSED_MERGE=0 in the environment keeps the partials-plus-merge-kernel path for every split count (a
-// diagnostic for measuring the two against each other on one GPU; read once).
-static bool fused_merge_enabled() {
-  static const bool v = [] {
-    const char* e = getenv("QB200_KV_FUSED_MERGE");
-    return !(e && e[0] == '0');
-  }();
-  return v;
 }
 
 cudaError_t launch_kv_attn(const KvAttnArgs& a, cudaStream_t st, const KvSeqTable* seqs) {
@@ -293,12 +320,23 @@ cudaError_t launch_kv_attn(const KvAttnArgs& a, cudaStream_t st, const KvSeqTabl
     // Measured against the merge kernel on one GPU (16 sequences, 8 kv heads): 4-bit caches 23.4 against 24.0 us at
     // 4096 tokens and 132.8 against 134.0 us at 32768; 8-bit caches, whose CTAs fill an SM alone, 33.0 against 31.8 us
     // at 4096 tokens -- so only the 4-bit kernel takes the cluster form.
-    if (sp.nsplit <= kMaxFusedSplits && a.bits == 4 && fused_merge_enabled()) {
-      e = launch_kv_fast(a, sp.nsplit, sp.tokens_per_split, p.part_m, p.part_l, p.part_o, st, seqs, true);
+    if (sp.nsplit <= kMaxFusedSplits && a.bits == 4) {
+      e = launch_kv_fast(a, sp.nsplit, p.part_m, p.part_l, p.part_o, st, seqs, true);
       if (e == cudaSuccess) return e;
       (void)cudaGetLastError();   // a cluster this launch could not place: fall back to partials and the merge kernel
     }
-    e = launch_kv_fast(a, sp.nsplit, sp.tokens_per_split, p.part_m, p.part_l, p.part_o, st, seqs, false);
+    e = launch_kv_fast(a, sp.nsplit, p.part_m, p.part_l, p.part_o, st, seqs, false);
+  } else if (kv_f16_supported(a, seqs)) {
+    // Head dim 64, GQA 5..8 and the verify widths.  They ran on the CUDA-core kernel before: 2 sequences x 28 query heads x 4
+    // verify positions over 4099 tokens at 8 bits 858 -> 20 us, 7 x 14 heads over 22k tokens 1775 -> 38 us, head dim 64
+    // 346 -> 10 us.  For GQA <= 4 at head dim 128 the integer kernel above spends fewer instructions per token (two planes
+    // of 4 heads fill its MMA columns) and is faster: 133 against 203 us for 16 x 32k tokens.
+    // Up to 8 splits per (sequence, kv head, query tile) merge inside a cluster here too, at both code widths.
+    p.nsplit = plan_f16(a, (p.gqa * a.Tq + 7) / 8, kMaxFusedSplits);
+    if (p.nsplit <= kMaxFusedSplits) return launch_kv_f16(a, p.nsplit, nullptr, nullptr, nullptr, st, seqs, true);
+    const int64_t parts = a.B * a.Hq * a.Tq * p.nsplit;
+    p.part_m = ws; p.part_l = ws + parts; p.part_o = ws + 2 * parts;
+    e = launch_kv_f16(a, p.nsplit, p.part_m, p.part_l, p.part_o, st, seqs, false);
   } else {
     const int nwarp = 4;
     const size_t smem = (size_t)(p.gqa * a.D + 2 * nwarp * p.gqa + nwarp * p.gqa * a.Dv) * sizeof(float);
@@ -313,8 +351,16 @@ cudaError_t launch_kv_attn(const KvAttnArgs& a, cudaStream_t st, const KvSeqTabl
     }
   }
   if (e != cudaSuccess) return e;
-  dim3 mgrid((unsigned)a.Hq, (unsigned)a.B, 1);
-  return launch_kernel(kv_merge, mgrid, dim3(128), 0, st, p);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)a.Hq, (unsigned)a.B, (unsigned)a.Tq);
+  cfg.blockDim = dim3(128);
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kv_merge, p);
 }
 
 }  // namespace qb

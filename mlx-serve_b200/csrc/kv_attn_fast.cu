@@ -54,7 +54,6 @@ template <int BITS> struct Geo {
 struct FastK {
   KvAttnArgs a;
   int nsplit;
-  int64_t tps;  // tokens per split, multiple of 128
   int gqa;
   int fused;    // the splits of a (sequence, kv head) are the CTAs of one cluster: rank 0 merges them and writes the output
   float* part_m; float* part_l; float* part_o;
@@ -180,8 +179,11 @@ __global__ void __launch_bounds__(kWarps * 32, BITS == 4 ? 2 : 1) kv_fast_kernel
   }
   int64_t len = a.kv_lens ? (int64_t)a.kv_lens[b] : T_seq;
   len = len > T_seq ? T_seq : (len < 0 ? 0 : len);
-  const int64_t t_begin = (int64_t)split * p.tps;
-  int64_t t_end = t_begin + p.tps;
+  // every sequence is cut by its own length, so that the CTAs of a ragged batch carry even shares (16 sequences of 16k to
+  // 32k tokens at 4 bits took as long as 16 of 32k when the cut was made for the longest)
+  const int64_t tps = ((len + p.nsplit - 1) / p.nsplit + kBlockTok - 1) / kBlockTok * kBlockTok;
+  const int64_t t_begin = (int64_t)split * tps;
+  int64_t t_end = t_begin + tps;
   t_end = t_end > len ? len : t_end;
   const int nblocks = t_end > t_begin ? (int)((t_end - t_begin + kBlockTok - 1) / kBlockTok) : 0;
   const int my_blocks = warp < nblocks ? (nblocks - warp + kWarps - 1) / kWarps : 0;
@@ -537,7 +539,7 @@ __global__ void __launch_bounds__(kWarps * 32, BITS == 4 ? 2 : 1) kv_fast_kernel
 
 bool kv_fast_supported(const KvAttnArgs& a, const KvSeqTable* seqs) {
   if (a.bits != 4 && a.bits != 8) return false;
-  if (a.D != kD || a.Dv != kD || a.gs != 64) return false;
+  if (a.D != kD || a.Dv != kD || a.gs != 64 || a.Tq != 1) return false;
   const int64_t gqa = a.Hq / a.Hkv;
   if (gqa < 1 || gqa > 4) return false;
   if (a.q_dtype != QB200_BFLOAT16 && a.q_dtype != QB200_FLOAT32) return false;
@@ -598,10 +600,10 @@ cudaError_t launch_fast_inst(const FastK& p, const TAB& tab, dim3 grid, cudaStre
 }
 }  // namespace
 
-cudaError_t launch_kv_fast(const KvAttnArgs& a, int nsplit, int64_t tps, float* pm, float* pl, float* po,
+cudaError_t launch_kv_fast(const KvAttnArgs& a, int nsplit, float* pm, float* pl, float* po,
                            cudaStream_t st, const KvSeqTable* seqs, bool fused) {
   FastK p;
-  p.a = a; p.nsplit = nsplit; p.tps = tps; p.gqa = (int)(a.Hq / a.Hkv);
+  p.a = a; p.nsplit = nsplit; p.gqa = (int)(a.Hq / a.Hkv);
   p.fused = fused ? 1 : 0;
   p.part_m = pm; p.part_l = pl; p.part_o = po;
   const dim3 grid((unsigned)nsplit, (unsigned)a.Hkv, (unsigned)a.B);

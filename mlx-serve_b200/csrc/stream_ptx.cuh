@@ -10,6 +10,10 @@ namespace qb {
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src));
 }
+// the same with the last 16 - `bytes` of the destination zeroed and not read
+__device__ __forceinline__ void cp_async16_z(uint32_t dst, const void* src, uint32_t bytes) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes));
+}
 __device__ __forceinline__ void cp_async8(uint32_t dst, const void* src) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst), "l"(src));
 }
@@ -37,7 +41,7 @@ __device__ __forceinline__ void mma_u8s8_z(int (&d)[4], uint32_t a0, uint32_t a1
       : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3])
       : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
-// Kept in program order (the attention kernel interleaves it with ldmatrix reads of the same stage).
+// Kept in program order (for use beside ldmatrix reads of the same stage).
 __device__ __forceinline__ void mma_u8s8_ordered(int (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
                                                  uint32_t b0, uint32_t b1) {
   asm volatile(
