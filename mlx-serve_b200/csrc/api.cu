@@ -223,12 +223,13 @@ QB200_API void qb200_set_error_handler(qb200_error_handler_func handler, void* d
 QB200_API const char* qb200_last_error(void) { return g_last_error.c_str(); }
 QB200_API const char* qb200_version(void) { return "qb200 0.1 (sm_100a)"; }
 QB200_API int qb200_debug_tc_status(void) {
-  const int tc = qmm_tc_error_code();
-  return tc ? tc : qmv_wide_error_code();
+  const int tc = qmm_tc_error_code(), f16 = qmv_f16_error_code();
+  return tc ? tc : (f16 ? f16 : qmv_wide_error_code());
 }
 QB200_API void qb200_debug_tc_reset(void) {
   qmm_tc_error_reset();
   qmv_wide_error_reset();
+  qmv_f16_error_reset();
 }
 
 QB200_API int qb200_quantized_matmul_shape(const qb200_tensor* x, const qb200_tensor* w, const qb200_tensor* scales,
@@ -319,6 +320,15 @@ static int64_t wide_max_tokens() {
 }
 static bool takes_wide(const QmmArgs& a) { return a.M > 8 && a.M <= wide_max_tokens() && qmv_wide_supported(a); }
 
+// What the tuned kernels decline -- K no multiple of 256, group size 32, group size 128 at 8 bits -- goes to the fp16 kernel,
+// which takes any multiple of the group size (in blocks of 32 tokens).  It is the slower one where both serve a shape
+// (C2 layer at 1 / 8 / 27 tokens: 60 / 88 / 192 us against 34 / 55 / 110), and two orders of magnitude faster than the CUDA-core
+// kernel that served these shapes before.
+static bool takes_f16(const QmmArgs& a) {
+  if (takes_wide(a) || (a.M > 8 && qmm_tc_supported(a)) || qmv_stream_supported(a)) return false;
+  return qmv_f16_supported(a);
+}
+
 static cudaError_t dispatch_qmm(const QmmArgs& a, cudaStream_t s) {
   if (!a.transpose) return qmv_rows_supported(a) ? launch_qmv_rows(a, s) : launch_qmm_generic(a, s);
   if (a.nbatch > 1 && qmv_shortk_supported(a)) return launch_qmv_shortk(a, s);   // one W per batch element, short K: q @ K^T
@@ -326,6 +336,7 @@ static cudaError_t dispatch_qmm(const QmmArgs& a, cudaStream_t s) {
   if (a.M > wide_max_tokens() && a.M > 8 && qmm_tc_supported(a)) return launch_qmm_tc(a, s);
   if (a.M > 8 && !qmv_stream_supported(a) && qmm_tc_supported(a)) return launch_qmm_tc(a, s);
   if (qmv_stream_supported(a)) return launch_qmv_stream(a, s);
+  if (qmv_f16_supported(a)) return launch_qmv_f16(a, s);
   if (qmv_mma_supported(a)) return launch_qmv_mma(a, s);
   return launch_qmm_generic(a, s);
 }
@@ -356,21 +367,24 @@ QB200_API int qb200_quantized_matmul_batch(qb200_tensor* const* res, const qb200
     const int n = count - i0 < kChunk ? count - i0 : kChunk;
     QmmArgs a[kChunk];
     bool empty[kChunk];
-    bool fuse = n > 1, wide = n > 1;
+    bool fuse = n > 1, wide = n > 1, f16 = n > 1;
     for (int i = 0; i < n; ++i) {
       int st = prepare_qmm(res[i0 + i], x, w[i0 + i], scales[i0 + i], biases[i0 + i], transpose_w, group_size, bits,
                            mode, &a[i], &empty[i]);
       if (st) return st;
       // the matrices share a launch where the single call would take a streaming kernel (same rule as dispatch_qmm)
+      f16 = f16 && !empty[i] && takes_f16(a[i]) && a[i].K == a[0].K;
       wide = wide && !empty[i] && takes_wide(a[i]) && a[i].K == a[0].K;
       fuse = fuse && !empty[i] && a[i].M <= 8 && qmv_stream_supported(a[i]) && a[i].K == a[0].K;
     }
     // beyond the streaming kernels' widths, up to 256 tokens: one launch of the tensor-core kernel over all matrices
-    bool tc = n > 1 && !wide && !fuse;
+    bool tc = n > 1 && !wide && !fuse && !f16;
     for (int i = 0; i < n && tc; ++i) tc = !empty[i] && a[i].M > wide_max_tokens() && a[i].M > 8;
     tc = tc && qmm_tc_multi_supported(a, n);
     cudaError_t e = cudaSuccess;
-    if (wide) {
+    if (f16) {
+      e = launch_qmv_f16_multi(a, n, (cudaStream_t)s);
+    } else if (wide) {
       e = launch_qmv_wide_multi(a, n, (cudaStream_t)s);
     } else if (tc) {
       e = launch_qmm_tc_multi(a, n, (cudaStream_t)s);

@@ -112,6 +112,13 @@ cudaError_t launch_qmv_shortk(const QmmArgs& a, cudaStream_t st);
 bool qmv_mma_supported(const QmmArgs& a);
 cudaError_t launch_qmv_mma(const QmmArgs& a, cudaStream_t st);
 
+// ---- qmv_f16.cu : weight-streaming kernel on the fp16 tensor cores, up to 32 tokens per launch, any multiple of the group size ----
+bool qmv_f16_supported(const QmmArgs& a);
+cudaError_t launch_qmv_f16(const QmmArgs& a, cudaStream_t st);
+cudaError_t launch_qmv_f16_multi(const QmmArgs* a, int count, cudaStream_t st);   // same x, <= 4 matrices
+int qmv_f16_error_code();     // 0, or the code of a bounded wait that expired
+void qmv_f16_error_reset();
+
 // ---- qmv_stream.cu : persistent cp.async-ring weight-streaming kernel (decode widths) ----
 bool qmv_stream_supported(const QmmArgs& a);
 cudaError_t launch_qmv_stream(const QmmArgs& a, cudaStream_t st);

@@ -1,0 +1,43 @@
+"""The fp16 streaming kernel: contraction widths that are only multiples of the group size, every group size, row counts and
+token counts around its tiles, against the CPU oracle (fp32 weight term)."""
+import numpy as np
+import pytest
+import torch
+
+from oracle import qoracle as qo
+from test_gpu_qmm import _run
+from util import dev_triple, gate_f32, make_weight, rand_bf16, to_dev_bf16
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("bits,gs,M,N,K", [
+    (4, 64, 1, 16, 64), (4, 64, 8, 7211, 2880), (8, 64, 5, 65, 576), (4, 64, 3, 1, 14272),         # one group; odd pitches of scales
+    (4, 32, 1, 300, 32), (4, 32, 8, 129, 1056), (8, 32, 7, 300, 2016), (8, 128, 4, 63, 1152), (4, 128, 2, 700, 640),
+    (4, 64, 9, 515, 2880), (8, 64, 16, 130, 192), (4, 32, 17, 257, 992), (8, 128, 32, 64, 1664),   # two and four token tiles
+    (4, 64, 33, 200, 704), (4, 32, 70, 65, 288)])                                                  # more than one pass
+def test_any_width(bits, gs, M, N, K):
+    rng = np.random.default_rng(bits * 1000 + gs + M + N + K)
+    q, s, b = make_weight(rng, (N, K), gs, bits)
+    r32, _ = _run(rand_bf16(rng, (M, K)), q, s, b, gs, bits)
+    assert r32 < 1e-4
+
+
+def test_several_matrices_and_wide_ranges():
+    """Three matrices in one call (row shares cross their borders); activations over 40 octaves; rows of a larger matrix."""
+    import qb200
+    rng = np.random.default_rng(3)
+    K, M = 1344, 6
+    ws = [make_weight(rng, (n, K), 64, 4) for n in (700, 33, 250)]
+    x = qo.bf16_round((rng.standard_normal((M, K)) * np.exp2(rng.integers(-20, 20, (M, K)))).astype(np.float32))
+    dev = [dev_triple(*w) for w in ws]
+    dev[1] = [t[4:28] for t in dev[1]]
+    outs = [torch.empty((M, n), dtype=torch.float32, device="cuda") for n in (700, 24, 250)]
+    qb200.quantized_matmul_batch(torch.from_numpy(x).cuda(), dev, outs, True, 64, 4)
+    for y, w, sl in zip(outs, ws, (slice(None), slice(4, 28), slice(None))):
+        gate_f32(y.cpu().numpy(), qo.qmm(x, *[a[sl] for a in w], 64, 4), "several matrices")
+    xn = x.copy()
+    xn[2, 77] = np.inf
+    y = qb200.quantized_matmul(to_dev_bf16(qo.f32_to_bf16(xn)), *dev[0], True, 64, 4)
+    assert torch.isnan(y[2]).all() and torch.isfinite(y[[0, 1, 3, 4, 5]]).all()
+    assert qb200.lib().qb200_debug_tc_status() == 0
