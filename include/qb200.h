@@ -333,8 +333,7 @@ QB200_API int qb200_add_rms_norm(qb200_tensor* sum_res, qb200_tensor* norm_res, 
 QB200_API int qb200_rope(qb200_tensor* res, const qb200_tensor* x, int dims, bool traditional, qb200_optional_float base,
                          float scale, const qb200_tensor* offsets, const qb200_tensor* freqs, qb200_stream s);
 /* fusedSwiGLU of the dense MLP (computeGeglu, src/transformer.zig:8220-8243): silu(gate) * up with the rounding points
- * of the reference's kernel (src/transformer.zig:19842-19851).  The first call on a device uploads the 128 KiB sigmoid
- * table (call once before capturing a graph). */
+ * of the reference's kernel (src/transformer.zig:19842-19851). */
 QB200_API int qb200_swiglu(qb200_tensor* res, const qb200_tensor* gate, const qb200_tensor* up, qb200_stream s);
 /* The rotation of the TurboQuant cache schemes (src/kv_quant.zig:164-403; quantizeTurbo = rotate then mlx_quantize,
  * dequantizeTurbo = mlx_dequantize then rotate): res = x @ R along the last axis, R = diag(sg) H diag(sg) / sqrt(D) with H

@@ -64,6 +64,19 @@ __device__ __forceinline__ uint32_t pack2(float lo, float hi) {
   return *(const uint32_t*)&h;
 }
 
+// sigmoid of a bf16 value, rounded to bf16: the two-sided form of MLX's Sigmoid as the reference quotes it
+// (src/transformer.zig:17566-17570).  The approximate exponential and reciprocal give the same bf16 as fp32 libm for every
+// one of the 65536 patterns with |x| <= 80 (the elementwise tests go through all of them); beyond, where the result is
+// subnormal, the exact functions do.
+__device__ __forceinline__ float sigmoid_bf16(float x) {
+  const float ax = fabsf(x);
+  float e, r;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(ax * 1.4426950408889634f));
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(1.f + e));
+  if (ax > 80.f) r = 1.f / (1.f + expf(ax));
+  return bf16_bits_to_f32(f32_to_bf16_bits(x < 0.f ? r : 1.f - r));
+}
+
 template <typename T> struct IO;
 template <> struct IO<float> {
   __device__ static __forceinline__ float load(const void* p, int64_t i) { return ((const float*)p)[i]; }
@@ -103,7 +116,7 @@ __device__ __forceinline__ uint32_t ldg_stream_u32(const void* p) {
 
 // D(16x8,f32) += A(16x16,bf16,row) * B(16x8,bf16,col)
 __device__ __forceinline__ void mma_bf16_16816(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-  asm volatile(
+  asm(
       "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
       : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
@@ -117,6 +130,19 @@ __device__ __forceinline__ void mma_f16_16816(float (&d)[4], uint32_t a0, uint32
       : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
       : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
+// The same with a zero C operand.
+__device__ __forceinline__ void mma_f16_16816_z(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+      : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.f));
+}
+// D(16x8,f32) += A(16x8,bf16) * B(8x8,bf16)
+__device__ __forceinline__ void mma_bf16_1688(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t b) {
+  asm("mma.sync.aligned.m16n8k8.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%0,%1,%2,%3};"
+      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+      : "r"(a0), "r"(a1), "r"(b));
+}
+__device__ __forceinline__ float pow2i(int e) { return __uint_as_float((uint32_t)(e + 127) << 23); }   // 2^e, e in [-126, 127]
 // two fp32 -> packed fp16 (round to nearest even), `lo` in the low half
 __device__ __forceinline__ uint32_t pack_f16x2(float lo, float hi) {
   uint32_t r;

@@ -120,18 +120,26 @@ __global__ void __launch_bounds__(256) rope_kernel(const uint16_t* x, uint16_t* 
 
 // silu(gate) * up with the rounding points of the reference's fused kernel (src/transformer.zig:19842-19851): the
 // sigmoid of the bf16 gate from a table over all bf16 patterns, g * sig rounded, then * up rounded.
-__global__ void __launch_bounds__(256) swiglu_kernel(const uint16_t* gate, const uint16_t* up, uint16_t* out, const uint16_t* sigtab,
-                                                     int64_t rows, int d, int64_t ldg, int64_t ldu, int64_t ldo) {
-  const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const int per_row = d / 2;
-  if (idx >= rows * per_row) return;
-  const int64_t r = idx / per_row;
-  const int i = (int)(idx - r * per_row) * 2;
-  const uint32_t gv = *(const uint32_t*)(gate + r * ldg + i), uv = *(const uint32_t*)(up + r * ldu + i);
+__device__ __forceinline__ uint32_t swiglu2(uint32_t gv, uint32_t uv) {
   const float g0 = bf16lo(gv), g1 = bf16hi(gv);
-  const float s0 = bf16_bits_to_f32(sigtab[gv & 0xFFFFu]), s1 = bf16_bits_to_f32(sigtab[gv >> 16]);
-  const float y0 = rbf16(g0 * s0) * bf16lo(uv), y1 = rbf16(g1 * s1) * bf16hi(uv);
-  *(uint32_t*)(out + r * ldo + i) = pack_bf16x2(y0, y1);
+  return pack2(rbf16(g0 * sigmoid_bf16(g0)) * bf16lo(uv), rbf16(g1 * sigmoid_bf16(g1)) * bf16hi(uv));
+}
+// VEC values per thread: 8 where rows allow 16-byte accesses (32768 rows of 768: 65 us with a table of sigmoids, whose
+// 32-way gathers were the bound), 2 otherwise.
+template <int VEC>
+__global__ void __launch_bounds__(256) swiglu_kernel(const uint16_t* gate, const uint16_t* up, uint16_t* out, int64_t rows, int d, int64_t ldg, int64_t ldu,
+                                                     int64_t ldo) {
+  const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const int per_row = d / VEC;
+  if (idx >= rows * per_row) return;
+  const int64_t r = idx <= 0x7fffffff ? (int64_t)((uint32_t)idx / (uint32_t)per_row) : idx / per_row;
+  const int i = (int)(idx - r * per_row) * VEC;
+  if constexpr (VEC == 8) {
+    const uint4 g = *(const uint4*)(gate + r * ldg + i), u = *(const uint4*)(up + r * ldu + i);
+    *(uint4*)(out + r * ldo + i) = make_uint4(swiglu2(g.x, u.x), swiglu2(g.y, u.y), swiglu2(g.z, u.z), swiglu2(g.w, u.w));
+  } else {
+    *(uint32_t*)(out + r * ldo + i) = swiglu2(*(const uint32_t*)(gate + r * ldg + i), *(const uint32_t*)(up + r * ldu + i));
+  }
 }
 
 // ---- one new token per sequence into per-sequence packed caches (KVCache.updateAffine per slot,
@@ -331,12 +339,10 @@ cudaError_t launch_rope(const uint16_t* x, uint16_t* out, const int32_t* offsets
 
 cudaError_t launch_swiglu(const uint16_t* gate, const uint16_t* up, uint16_t* out, int64_t rows, int d, int64_t ldg, int64_t ldu,
                           int64_t ldo, cudaStream_t st) {
-  const int64_t total = rows * (d / 2);
+  const bool vec = d % 8 == 0 && ((((uintptr_t)gate | (uintptr_t)up | (uintptr_t)out | (uintptr_t)((ldg | ldu | ldo) * 2)) & 15) == 0);
+  const int64_t total = rows * (d / (vec ? 8 : 2));
   if (total <= 0) return cudaSuccess;
-  cudaError_t te;
-  const uint16_t* tab = sigmoid_table(st, &te);
-  if (!tab) return te;
-  return launch_kernel(swiglu_kernel, dim3((unsigned)((total + 255) / 256)), dim3(256), 0, st, gate, up, out, tab, rows, d, ldg, ldu, ldo);
+  return launch_kernel(vec ? swiglu_kernel<8> : swiglu_kernel<2>, dim3((unsigned)((total + 255) / 256)), dim3(256), 0, st, gate, up, out, rows, d, ldg, ldu, ldo);
 }
 
 cudaError_t launch_kv_append_seqs(const KvAppendSeqsArgs& h, cudaStream_t st) {

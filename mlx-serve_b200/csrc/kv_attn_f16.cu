@@ -91,16 +91,6 @@ __device__ __forceinline__ float ex2(float x) {
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
-__device__ __forceinline__ float pow2i(int e) {   // 2^e, e clamped to the normal range
-  e = e < -126 ? -126 : (e > 127 ? 127 : e);
-  return __uint_as_float((uint32_t)(e + 127) << 23);
-}
-// D(16x8,f32) += A(16x8,bf16) * B(8x8,bf16)
-__device__ __forceinline__ void mma_bf16_1688(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t b) {
-  asm("mma.sync.aligned.m16n8k8.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%0,%1,%2,%3};"
-               : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-               : "r"(a0), "r"(a1), "r"(b));
-}
 // x = hi + lo: hi is x with the mantissa cut to fp16's, lo the exact rest; both packed in pairs (a in the low half)
 __device__ __forceinline__ void split2(float a, float b, uint32_t& hi, uint32_t& lo) {
   const float ah = __uint_as_float(__float_as_uint(a) & 0xFFFFE000u), bh = __uint_as_float(__float_as_uint(b) & 0xFFFFE000u);

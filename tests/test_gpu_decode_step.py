@@ -225,3 +225,18 @@ def test_one_layer_tick_against_the_oracle_chain():
     # the caches received exactly the oracle's new triples
     for n in range(N):
         assert np.array_equal(from_dev_u32(dk[n][0][0, :, lens[n]]), caches[n][0][0][0, :, lens[n]])
+
+
+def test_swiglu_over_every_gate_pattern():
+    """The computed sigmoid: all 65536 bf16 patterns of the gate, in rows of 8-value and of 2-value accesses."""
+    import qb200
+    gate = torch.arange(65536, dtype=torch.int32).to(torch.int16).view(torch.bfloat16)
+    gate = gate[~torch.isnan(gate.float())]
+    n = gate.numel() // 64 * 64
+    g32, up = gate[:n].float(), torch.full((n,), 1.5)
+    sy = 1.0 / (1.0 + torch.exp(g32.abs()))
+    sig = torch.where(g32 < 0, sy, 1.0 - sy).to(torch.bfloat16).float()
+    ref = ((g32 * sig).to(torch.bfloat16).float() * up).to(torch.bfloat16)
+    for shape in ((n // 64, 64), (n // 2, 2)):
+        y = qb200.swiglu(gate[:n].view(shape).cuda(), up.to(torch.bfloat16).view(shape).cuda())
+        assert torch.equal(y.cpu().view(-1).view(torch.int16)[~torch.isnan(ref.float())], ref.view(torch.int16)[~torch.isnan(ref.float())])

@@ -116,3 +116,22 @@ def test_kv_append_matches_oracle_and_leaves_neighbours(bits):
     assert bool((cs[:, :, :off] == 7.0).all()) and bool((cb[:, :, off + S:] == -7.0).all())
     with pytest.raises(qb200.Qb200Error):
         qb200.kv_append(cq, cs, cb, to_dev_bf16(qo.f32_to_bf16(x)), cap - 1, bits, 64)
+
+
+@pytest.mark.parametrize("bits,gs,shape", [(4, 64, (3, 5, 64)), (8, 32, (2, 3, 7, 96)), (4, 128, (1, 128)), (8, 64, (2, 130, 192))])
+def test_codes_on_rounding_ties(bits, gs, shape):
+    """Values half way between two codes (where the division's rounding decides), over strided rows of odd counts."""
+    import qb200
+    rng = np.random.default_rng(bits + gs)
+    bins = 2 ** bits - 1
+    x = (rng.integers(0, 2 * bins + 1, shape) * 0.5).astype(np.float32) * np.float32(0.125) - np.float32(bins / 16)
+    x.reshape(-1, gs)[:, 0] = -bins / 16.0       # every group spans the whole range: scale 1/8
+    x.reshape(-1, gs)[:, 1] = bins / 16.0
+    x = qo.bf16_round(x)
+    q, s, b = qo.quantize(x, gs, bits)
+    pad = np.zeros(shape[:-2] + (shape[-2] + 3, shape[-1]), np.float32)
+    pad[..., 2:2 + shape[-2], :] = x
+    xd = to_dev_bf16(qo.f32_to_bf16(pad))[..., 2:2 + shape[-2], :]
+    dq, ds, db = qb200.quantize(xd, gs, bits)
+    assert np.array_equal(from_dev_u32(dq), q) and np.array_equal(from_dev_bf16(ds), s) and np.array_equal(from_dev_bf16(db), b)
+    assert np.array_equal(from_dev_bf16(qb200.dequantize(dq, ds, db, gs, bits)), qo.dequantize(q, s, b, gs, bits, out_bf16=True))
