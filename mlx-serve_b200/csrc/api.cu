@@ -320,13 +320,27 @@ static int64_t wide_max_tokens() {
 }
 static bool takes_wide(const QmmArgs& a) { return a.M > 8 && a.M <= wide_max_tokens() && qmv_wide_supported(a); }
 
-// What the tuned kernels decline -- K no multiple of 256, group size 32, group size 128 at 8 bits -- goes to the fp16 kernel,
-// which takes any multiple of the group size (in blocks of 32 tokens).  It is the slower one where both serve a shape
-// (C2 layer at 1 / 8 / 27 tokens: 60 / 88 / 192 us against 34 / 55 / 110), and two orders of magnitude faster than the CUDA-core
-// kernel that served these shapes before.
-static bool takes_f16(const QmmArgs& a) {
-  if (takes_wide(a) || (a.M > 8 && qmm_tc_supported(a)) || qmv_stream_supported(a)) return false;
-  return qmv_f16_supported(a);
+// What the tuned kernels decline -- K no multiple of 256, group size 32, group size 128 at 8 bits -- goes to one of four kernels,
+// by times of each over M 1 - 64, N 100 - 12000, K 128 - 4416 (us):
+//  * tiny products to the CUDA-core kernel, whose launch is the shortest (300 x 704, 8 tokens: 3.1 against 3.9);
+//  * 8 bits, K a multiple of 128, few weights and tokens to the integer MMA kernel (1137 x 640, 8 tokens: 3.1 against 4.3);
+//  * more than 8 tokens to the tiled kernel (4000 x 4416, 16 tokens: 10.9 against 18), up to 16 tokens only while the weights are
+//    few -- it reads them at half the streaming kernel's rate (12000 x 4416, 16 tokens: 31 against 24) --, and from 5 tokens where
+//    K is long and the rows of W are too few to occupy the streaming kernel (1137 x 4416, 8 tokens: 7.6 against 10.9);
+//  * the rest to the fp16 streaming kernel.  (Where qmv_stream and qmv_wide serve a shape they are faster than either.)
+enum class Ragged { none, generic, mma, f16, tile };
+static Ragged ragged_kernel(const QmmArgs& a) {
+  if (takes_wide(a) || (a.M > 8 && qmm_tc_supported(a)) || qmv_stream_supported(a)) return Ragged::none;
+  const bool mma = qmv_mma_supported(a), f16 = qmv_f16_supported(a), tile = qmm_tile_supported(a);
+  if ((double)a.M * a.N * a.K * a.nbatch <= 3.6e6 && !mma) return Ragged::generic;
+  if (mma) {
+    const bool few = a.M <= 2 ? a.K <= 1024 : (a.M <= 4 ? a.K <= 2048 : (a.M <= 8 ? true : (a.M <= 16 ? a.K <= 2304 : false)));
+    if ((few && a.N <= 4096) || (a.M > 16 && a.M <= 32 && a.K <= (a.N > 2048 ? 640 : 512) && a.N <= 8192)) return Ragged::mma;
+  }
+  if (tile && (a.M > 16 || (a.M > 8 && (a.N <= 6144 || a.K <= 256)) || (a.M > 4 && a.K >= 1536 && a.N <= a.K && a.N <= 6144))) return Ragged::tile;
+  if (f16) return Ragged::f16;
+  if (tile && a.M > 8) return Ragged::tile;
+  return mma ? Ragged::mma : Ragged::generic;
 }
 
 static cudaError_t dispatch_qmm(const QmmArgs& a, cudaStream_t s) {
@@ -336,8 +350,12 @@ static cudaError_t dispatch_qmm(const QmmArgs& a, cudaStream_t s) {
   if (a.M > wide_max_tokens() && a.M > 8 && qmm_tc_supported(a)) return launch_qmm_tc(a, s);
   if (a.M > 8 && !qmv_stream_supported(a) && qmm_tc_supported(a)) return launch_qmm_tc(a, s);
   if (qmv_stream_supported(a)) return launch_qmv_stream(a, s);
-  if (qmv_f16_supported(a)) return launch_qmv_f16(a, s);
-  if (qmv_mma_supported(a)) return launch_qmv_mma(a, s);
+  switch (ragged_kernel(a)) {
+    case Ragged::mma: return launch_qmv_mma(a, s);
+    case Ragged::f16: return launch_qmv_f16(a, s);
+    case Ragged::tile: return launch_qmm_tile(a, s);
+    default: break;
+  }
   return launch_qmm_generic(a, s);
 }
 
@@ -373,7 +391,7 @@ QB200_API int qb200_quantized_matmul_batch(qb200_tensor* const* res, const qb200
                            mode, &a[i], &empty[i]);
       if (st) return st;
       // the matrices share a launch where the single call would take a streaming kernel (same rule as dispatch_qmm)
-      f16 = f16 && !empty[i] && takes_f16(a[i]) && a[i].K == a[0].K;
+      f16 = f16 && !empty[i] && a[i].K == a[0].K && ragged_kernel(a[i]) == Ragged::f16;
       wide = wide && !empty[i] && takes_wide(a[i]) && a[i].K == a[0].K;
       fuse = fuse && !empty[i] && a[i].M <= 8 && qmv_stream_supported(a[i]) && a[i].K == a[0].K;
     }
@@ -513,6 +531,7 @@ QB200_API int qb200_gather_qmm(qb200_tensor* res, const qb200_tensor* x, const q
   else if (many && gather_tc_supported(a)) e = launch_gather_tc(a, (cudaStream_t)s);
   else if (gather_stream_supported(a)) e = launch_gather_stream(a, (cudaStream_t)s);
   else if (gather_tc_supported(a) && a.I >= 1024) e = launch_gather_tc(a, (cudaStream_t)s);
+  else if (gather_tile_supported(a)) e = launch_gather_tile(a, (cudaStream_t)s);
   else if (gather_mma_supported(a)) e = launch_gather_mma(a, (cudaStream_t)s);
   else e = launch_gather_generic(a, (cudaStream_t)s);
   if (e != cudaSuccess) return cuda_fail(e, "gather_qmm");

@@ -119,6 +119,13 @@ cudaError_t launch_qmv_f16_multi(const QmmArgs* a, int count, cudaStream_t st); 
 int qmv_f16_error_code();     // 0, or the code of a bounded wait that expired
 void qmv_f16_error_reset();
 
+// ---- qmm_tile.cu : tiled form with the fp32 weight term, any multiple of the group size, more than 32 tokens; rows sorted by expert ----
+bool qmm_tile_supported(const QmmArgs& a);
+cudaError_t launch_qmm_tile(const QmmArgs& a, cudaStream_t st);
+struct GatherArgs;
+bool gather_tile_supported(const GatherArgs& a);
+cudaError_t launch_gather_tile(const GatherArgs& a, cudaStream_t st);
+
 // ---- qmv_stream.cu : persistent cp.async-ring weight-streaming kernel (decode widths) ----
 bool qmv_stream_supported(const QmmArgs& a);
 cudaError_t launch_qmv_stream(const QmmArgs& a, cudaStream_t st);
