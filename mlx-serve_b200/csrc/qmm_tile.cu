@@ -17,6 +17,8 @@
 //    bf16 parts, so both terms are a few small MMAs per eight groups (and X itself a product with ones).  (fp32 sums of 64 products of magnitude 128 |x|: their
 //    rounding stays below 1e-5 of the result.)
 //  * Sorted rows: a CTA owns TM consecutive rows of the sorted list and runs one pass over K per expert it finds there; no tables.
+//    With few rows per expert these passes would follow one another in a few CTAs: then a CTA owns one piece, up to TM rows of one
+//    expert (cut where the expert changes and at multiples of TM), which it finds by counting the cuts of the list.
 #include <type_traits>
 
 #include "kernels.h"
@@ -35,6 +37,7 @@ struct TileK {
   const void* rhs; int rhs_i64;
   int64_t wes, ses;
   int E;
+  int pieces;                    // a CTA per piece of up to TM rows of one expert, instead of per TM rows of the list
 };
 
 template <int BITS, int GS, int TM, int WN>
@@ -74,8 +77,7 @@ __global__ void __launch_bounds__(kThreads, 2) qmm_tile_kernel(const __grid_cons
   extern __shared__ __align__(128) unsigned char smem[];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
   const int wn = warp % WN, wm = warp / WN;
-  const int n0 = blockIdx.x * TN, m0 = blockIdx.y * TM;
-  const int mtile = p.M - m0 < TM ? p.M - m0 : TM;
+  const int n0 = blockIdx.x * TN;
   const uint32_t s0 = (uint32_t)__cvta_generic_to_shared(smem);
   unsigned char* raw_p = smem;
   unsigned char* w_p = raw_p + kRing * GE::RAW;
@@ -90,6 +92,33 @@ __global__ void __launch_bounds__(kThreads, 2) qmm_tile_kernel(const __grid_cons
     return p.rhs_i64 ? (int)((const long long*)p.rhs)[row] : ((const int*)p.rhs)[row];
   };
 
+  int m0 = blockIdx.y * TM, mtile = p.M - m0 < TM ? p.M - m0 : TM;
+  if (GROUPED && p.pieces) {
+    // this CTA's piece is number blockIdx.y: every thread counts the cuts among its share of the rows, whoever owns it finds it
+    int* cnt = (int*)smem;
+    const int R = (p.M + kThreads - 1) / kThreads, r0 = tid * R < p.M ? tid * R : p.M, r1 = r0 + R < p.M ? r0 + R : p.M;
+    int n = 0, prev = r0 > 0 && r0 < r1 ? expert_of(r0 - 1) : -1;
+    for (int r = r0; r < r1; ++r) { const int e = expert_of(r); n += r % TM == 0 || e != prev; prev = e; }
+    int sum = n;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) { const int v = __shfl_up_sync(0xffffffffu, sum, o); if (lane >= o) sum += v; }
+    if (lane == 31) cnt[warp] = sum;
+    if (tid == 0) cnt[kThreads / 32] = -1;
+    __syncthreads();
+    for (int w = 0; w < warp; ++w) sum += cnt[w];
+    int left = (int)blockIdx.y - (sum - n);     // cuts of this thread before the piece
+    if (left >= 0 && left < n) {
+      int r = r0;
+      prev = r0 > 0 ? expert_of(r0 - 1) : -1;
+      for (; r < r1; ++r) { const int e = expert_of(r); if (r % TM == 0 || e != prev) { if (left == 0) break; --left; } prev = e; }
+      cnt[kThreads / 32] = r;
+    }
+    __syncthreads();
+    m0 = cnt[kThreads / 32];
+    if (m0 < 0) return;                         // fewer pieces than CTAs
+    const int end = m0 - m0 % TM + TM;          // (an expert's end before it ends the segment below)
+    mtile = (end < p.M ? end : p.M) - m0;
+  }
   for (int lo = 0; lo < mtile;) {
     // the tokens [lo, hi) of this tile share one weight matrix
     int hi = mtile, ex = 0;
@@ -99,7 +128,7 @@ __global__ void __launch_bounds__(kThreads, 2) qmm_tile_kernel(const __grid_cons
       while (a < b) { const int m = (a + b) >> 1; if (expert_of(m0 + m) > ex) b = m; else a = m + 1; }
       hi = a;
     }
-    if (GROUPED && (ex < 0 || ex >= p.E)) { lo = hi; continue; }   // padding rows are left untouched, as in every other form
+    if (GROUPED && (ex < 0 || ex >= p.E)) { if (p.pieces) return; lo = hi; continue; }   // padding rows are left untouched, as in every other form
     const uint32_t* wq = p.w + (int64_t)ex * p.wes;
     const uint16_t* sp = p.s + (int64_t)ex * p.ses;
     const uint16_t* bp = p.b + (int64_t)ex * p.ses;
@@ -378,6 +407,7 @@ __global__ void __launch_bounds__(kThreads, 2) qmm_tile_kernel(const __grid_cons
         for (int k = 0; k < 8; ++k)
           if (c + k < nv) yr[k] = sr[k];
     }
+    if (GROUPED && p.pieces) return;
     lo = hi;
   }
 }
@@ -398,7 +428,7 @@ cudaError_t launch_inst(const TileK& p, int nsplit, cudaStream_t st) {
       if (dev >= 0 && dev < 64) done[dev] = true;
     }
   }
-  const dim3 grid((unsigned)((p.N + GE::TN - 1) / GE::TN), (unsigned)((p.M + TM - 1) / TM), (unsigned)nsplit);
+  const dim3 grid((unsigned)((p.N + GE::TN - 1) / GE::TN), (unsigned)(p.pieces ? p.pieces : (p.M + TM - 1) / TM), (unsigned)nsplit);
   if (nsplit == 1) return launch_kernel(kern, grid, dim3(kThreads), GE::kSmem, st, p);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
@@ -477,9 +507,11 @@ cudaError_t launch_gather_tile(const GatherArgs& a, cudaStream_t st) {
   p.gshift = a.gs == 128 ? 1 : 0;
   p.M = (int)a.I; p.N = (int)a.N; p.K = (int)a.K; p.ldx = a.K; p.ldw = a.K * a.bits / 32; p.lds = a.K / a.gs; p.ldy = a.N;
   p.rhs = a.rhs; p.rhs_i64 = a.rhs_dtype == QB200_INT64; p.wes = a.w_expert_stride; p.ses = a.s_expert_stride; p.E = (int)a.E;
-  // tokens per tile by the rows an expert has on average: a tile runs one pass over K per expert in it
-  const int64_t per = a.I / a.E;
-  const int tm = per > 16 ? 64 : 32;
+  // Tokens per tile by the rows an expert has on average.  A CTA per piece while finding it is quick and tiles hold several
+  // experts (us, per tile -> per piece: 96 rows, 64 experts, 2048 x 896 163 -> 41; 200 rows, 8 experts, 1024 x 640, 8 bits
+  // 23 -> 14; 968 rows, 64 experts, 1792 x 896 83 -> 73; but 4800 rows, 64 experts, 1024 x 640 74 -> 84).
+  const int tm = a.I / a.E > 32 ? 64 : 32;
+  if (a.I <= 4096) p.pieces = (int)((a.I + tm - 1) / tm + (a.E < a.I ? a.E : a.I) - 1);
   return a.bits == 4 ? launch_gs<4>(p, a.gs, tm, 1, st) : launch_gs<8>(p, a.gs, tm, 1, st);
 }
 

@@ -24,7 +24,8 @@ def test_dense(bits, gs, M, N, K):
 
 @pytest.mark.parametrize("bits,gs,E,N,K,counts", [
     (4, 64, 5, 130, 192, (3, 0, 17, 1, 40)), (8, 64, 3, 257, 704, (100, 33, 64)), (4, 32, 4, 65, 352, (0, 9, 0, 70)),
-    (8, 128, 2, 128, 640, (1, 200))])
+    (8, 128, 2, 128, 640, (1, 200)),
+    (4, 64, 3, 60, 64, (2500, 1, 1600))])                                    # too many rows for a CTA per piece
 def test_sorted_rows(bits, gs, E, N, K, counts):
     import qb200
     rng = np.random.default_rng(E + N + K)
