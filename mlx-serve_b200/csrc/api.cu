@@ -223,13 +223,15 @@ QB200_API void qb200_set_error_handler(qb200_error_handler_func handler, void* d
 QB200_API const char* qb200_last_error(void) { return g_last_error.c_str(); }
 QB200_API const char* qb200_version(void) { return "qb200 0.1 (sm_100a)"; }
 QB200_API int qb200_debug_tc_status(void) {
-  const int tc = qmm_tc_error_code(), f16 = qmv_f16_error_code();
-  return tc ? tc : (f16 ? f16 : qmv_wide_error_code());
+  for (int code : {qmm_tc_error_code(), qmm_pair_error_code(), qmv_f16_error_code()})
+    if (code) return code;
+  return qmv_wide_error_code();
 }
 QB200_API void qb200_debug_tc_reset(void) {
   qmm_tc_error_reset();
   qmv_wide_error_reset();
   qmv_f16_error_reset();
+  qmm_pair_error_reset();
 }
 
 QB200_API int qb200_quantized_matmul_shape(const qb200_tensor* x, const qb200_tensor* w, const qb200_tensor* scales,
@@ -347,6 +349,7 @@ static cudaError_t dispatch_qmm(const QmmArgs& a, cudaStream_t s) {
   if (!a.transpose) return qmv_rows_supported(a) ? launch_qmv_rows(a, s) : launch_qmm_generic(a, s);
   if (a.nbatch > 1 && qmv_shortk_supported(a)) return launch_qmv_shortk(a, s);   // one W per batch element, short K: q @ K^T
   if (takes_wide(a)) return launch_qmv_wide(a, s);
+  if (qmm_pair_supported(a)) return launch_qmm_pair(a, s);
   if (a.M > wide_max_tokens() && a.M > 8 && qmm_tc_supported(a)) return launch_qmm_tc(a, s);
   if (a.M > 8 && !qmv_stream_supported(a) && qmm_tc_supported(a)) return launch_qmm_tc(a, s);
   if (qmv_stream_supported(a)) return launch_qmv_stream(a, s);
@@ -397,7 +400,7 @@ QB200_API int qb200_quantized_matmul_batch(qb200_tensor* const* res, const qb200
     }
     // beyond the streaming kernels' widths, up to 256 tokens: one launch of the tensor-core kernel over all matrices
     bool tc = n > 1 && !wide && !fuse && !f16;
-    for (int i = 0; i < n && tc; ++i) tc = !empty[i] && a[i].M > wide_max_tokens() && a[i].M > 8;
+    for (int i = 0; i < n && tc; ++i) tc = !empty[i] && a[i].M > wide_max_tokens() && a[i].M > 8 && !qmm_pair_supported(a[i]);
     tc = tc && qmm_tc_multi_supported(a, n);
     cudaError_t e = cudaSuccess;
     if (f16) {
@@ -528,6 +531,7 @@ QB200_API int qb200_gather_qmm(qb200_tensor* res, const qb200_tensor* x, const q
   const bool many = a.I >= 32 * a.E && a.I >= 1024;
   // Up to 16 rows (single-token decode: every row its own expert): a CTA per (row, 16 output rows).
   if (gather_small_supported(a)) e = launch_gather_small(a, (cudaStream_t)s);
+  else if (many && gather_pair_supported(a)) e = launch_gather_pair(a, (cudaStream_t)s);
   else if (many && gather_tc_supported(a)) e = launch_gather_tc(a, (cudaStream_t)s);
   else if (gather_stream_supported(a)) e = launch_gather_stream(a, (cudaStream_t)s);
   else if (gather_tc_supported(a) && a.I >= 1024) e = launch_gather_tc(a, (cudaStream_t)s);

@@ -149,6 +149,14 @@ struct GatherArgs;
 bool gather_tc_supported(const GatherArgs& a);   // rows sorted by expert, many rows: grouped GEMM on the same kernel
 cudaError_t launch_gather_tc(const GatherArgs& a, cudaStream_t st);
 
+// ---- qmm_pair.cu : the same on CTA pairs (cta_group::2), many tokens ----
+bool qmm_pair_supported(const QmmArgs& a);
+cudaError_t launch_qmm_pair(const QmmArgs& a, cudaStream_t st);
+bool gather_pair_supported(const GatherArgs& a);
+cudaError_t launch_gather_pair(const GatherArgs& a, cudaStream_t st);
+int qmm_pair_error_code();    // 0, or the code of a bounded wait that expired
+void qmm_pair_error_reset();
+
 struct GatherArgs {
   const void* x; const uint32_t* w; const void* s; const void* b; void* y;
   int x_dtype;

@@ -12,14 +12,10 @@
 //
 // Persistent, warp-specialised CTAs (one per SM) walk the output tiles of
 // 256 tokens x BN weight rows (BN chosen per problem so that the last wave of
-// tiles is full), K in steps of 64 through a 3- or 4-stage ring (and a ring of packed codes beside it).  Two tile
-// forms: BN <= 128 with two accumulator sets in tensor memory (the epilogue of
-// tile i overlaps the main loop of tile i+1; used below 257 tokens and by the
-// grouped form), and BN <= 208 with one set (fewer shared-memory operand bytes
-// per MAC -- the resource that bounds this kernel -- at the price of an
-// epilogue that is not overlapped; used for wide prefill).  Roles:
-//   warps 0-15 : dequantisers in groups that take k-blocks in turn (four groups of four warps
-//                for tiles of up to 128 weight rows, two of eight for the wide form): a group's
+// tiles is full), K in steps of 64 through a 3- or 4-stage ring (and a ring of packed codes beside it), two
+// accumulator sets in tensor memory (the epilogue of tile i overlaps the main loop of tile i+1).  The kernel of a few
+// to 256 tokens, of few weight rows, and of the grouped forms the CTA-pair kernel (qmm_pair.cu) declines.  Roles:
+//   warps 0-15 : dequantisers in groups that take k-blocks in turn (four groups of four warps; two of eight in the grouped form): a group's
 //                per-k-block latency -- two barrier polls, scale selection, proxy fence, arrival
 //                -- is several times its arithmetic, so several k-blocks are always being
 //                converted side by side.  One thread per weight row: packed codes -> exact bf16
@@ -47,11 +43,7 @@
 //                two meet at a named barrier, which costs the issuer a few cycles.
 // Every mbarrier wait is bounded: on expiry the kernel records an error code,
 // every role leaves its loops, the CTA frees its tensor memory and returns.
-#include <cuda.h>
-
-#include <mutex>
-
-#include "kernels.h"
+#include "tc_ptx.cuh"
 
 namespace qb {
 namespace {
@@ -62,27 +54,21 @@ constexpr int BM = 256, BN_MAX = 128, BK = 64;
 // next 64 columns of K instead of the next 128 tokens, and B has two sub-tiles, one per dequant group: what a
 // k-block costs there is the hand-over of a stage between the roles (~800 cycles with nothing to compute), not any
 // role's work, so it is paid half as often.
-__host__ __device__ constexpr int stages_of(bool grouped, bool wide = false, bool half = false) { return half ? 3 : ((grouped || wide) ? 3 : 4); }
+__host__ __device__ constexpr int stages_of(bool grouped, bool half = false) { return half || grouped ? 3 : 4; }
 __host__ __device__ constexpr int kb_per_stage_of(bool half) { return half ? 2 : 1; }
 // Buffers of the packed-code ring (each holds 128 bytes of every weight row of the tile: four k-blocks at 4 bits,
 // two at 8).  Two are enough: trading pipeline stages for a ring of five or six buffers was measured and changed
 // nothing at few tokens (the refills are not what the k-loop waits for).
-__host__ __device__ constexpr int raw_bufs_of(bool grouped, bool wide = false, bool half = false) { return 2; }
-// The wide form multiplies one B tile of up to 208 weight rows per stage against both token halves: fewer
-// operand bytes per MAC through shared memory (the resource that bounds this kernel), at the price of a
-// single accumulator set in tensor memory (2 x 256 columns), i.e. an epilogue that is not overlapped.
-constexpr int BN_WIDE = 208, BN_WIDE_GROUPED = 192;   // the grouped form keeps 8 KiB for its tables
-__host__ __device__ constexpr int bn_max_of(bool wide, bool grouped = false) { return wide ? (grouped ? BN_WIDE_GROUPED : BN_WIDE) : BN_MAX; }
+constexpr int RAW_BUFS = 2;
 constexpr int kMaxGroupExperts = 1024;
 // The sixteen dequant warps work in groups; group g converts the k-blocks with (index % groups) == g, one thread per
 // weight row (both halves of the row's 64 codes).  What a group spends per k-block is mostly not arithmetic -- two
 // barrier polls of ~130 cycles each, the scale selection, the proxy fence, the arrival: ~1500 cycles around ~400 of
-// conversion -- and the k-loop of a few-token tile ran at exactly (that sum) / groups.  Tiles of up to 128 weight
-// rows therefore use four groups of four warps; the wide form needs eight warps to cover its 208 rows.  A group must
-// not step further than the stage ring holds (groups <= stages x k-blocks per stage): its wait on a stage's "empty"
+// conversion -- and the k-loop of a few-token tile ran at exactly (that sum) / groups.  The dense forms
+// therefore use four groups of four warps.  A group must not step further than the stage ring holds (groups <= stages x k-blocks per stage): its wait on a stage's "empty"
 // barrier names a phase by parity, and a group that is two completions ahead of the barrier reads the previous
 // round's completion as its own.  The grouped form has three one-k-block stages and so keeps two groups.
-__host__ __device__ constexpr int dq_groups_of(bool wide, bool grouped) { return (wide || grouped) ? 2 : 4; }
+__host__ __device__ constexpr int dq_groups_of(bool grouped) { return grouped ? 2 : 4; }
 constexpr int kDequantWarps = 16, kEpiWarps = 4;
 constexpr int kEpiWarp0 = kDequantWarps;            // warps 16..19: warp % 4 = TMEM lane quarter
 constexpr int kTmaWarp = kEpiWarp0 + kEpiWarps, kWTmaWarp = kTmaWarp + 1, kMmaWarp = kWTmaWarp + 1;
@@ -91,7 +77,6 @@ constexpr int kThreads = (kScoutWarp + 1) * 32;
 constexpr int A_STAGE_BYTES = BM * BK * 2;   // two 128-row boxes
 constexpr int B_STAGE_BYTES = BN_MAX * BK * 2;
 constexpr int RAW_BYTES = BN_MAX * 128;      // one super-block of packed codes: 128 bytes of every weight row
-constexpr uint32_t kSpinLimit = 1u << 24;
 
 __device__ int g_tc_error = 0;   // 0 = ok; otherwise the code of the wait that expired
 
@@ -127,92 +112,10 @@ struct TileCoord {
   int wrow0, wrow_last;  // first weight row of the tile in the (stacked) weight matrix; last row that may be read
 };
 
-__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count));
-}
-__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-__device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
-}
-// Bounded wait; returns false when the limit expired.
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
-  const uint32_t addr = smem_u32(bar);
-  for (uint32_t it = 0; it < kSpinLimit; ++it) {
-    uint32_t done;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(done)
-        : "r"(addr), "r"(parity)
-        : "memory");
-    if (done) return true;
-  }
-  return false;
-}
-// The same for waits that are off the critical path (producers running ahead, the epilogue waiting for a
-// whole tile): after a few polls the thread sleeps between polls, so that it does not take issue slots
-// from the warps that convert weights.  Still bounded: 2^22 polls of at least 100 ns.
-__device__ __forceinline__ bool mbar_wait_relaxed(uint64_t* bar, uint32_t parity) {
-  const uint32_t addr = smem_u32(bar);
-  for (uint32_t it = 0; it < (kSpinLimit >> 2); ++it) {
-    uint32_t done;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(done)
-        : "r"(addr), "r"(parity)
-        : "memory");
-    if (done) return true;
-    if (it >= 4) __nanosleep(100);
-  }
-  return false;
-}
-// Wait of the dequant warps: they run several stages ahead of the tensor core, so a poll that fails is followed
-// by a short sleep -- sixteen warps polling in a tight loop take issue slots from the one thread that issues MMAs.
-__device__ __forceinline__ bool mbar_wait_backoff(uint64_t* bar, uint32_t parity) {
-  const uint32_t addr = smem_u32(bar);
-  for (uint32_t it = 0; it < kSpinLimit; ++it) {
-    uint32_t done;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(done)
-        : "r"(addr), "r"(parity)
-        : "memory");
-    if (done) return true;
-    __nanosleep(40);
-  }
-  return false;
-}
-__device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, uint64_t* bar, int x, int y) {
-  asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
-               ::"r"(dst), "l"(map), "r"(smem_u32(bar)), "r"(x), "r"(y)
-               : "memory");
-}
-__device__ __forceinline__ uint32_t cluster_rank_tc() { uint32_t r; asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r)); return r; }
-__device__ __forceinline__ void cluster_sync_tc() {   // all threads of all CTAs of the cluster (hardware barrier)
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
 __device__ __forceinline__ void st_cluster_v4(uint32_t addr, uint32_t rank, float4 v) {
   uint32_t ra;
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"(addr), "r"(rank));
   asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(ra), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w) : "memory");
-}
-// K-major, SWIZZLE_128B operand descriptor: rows of 128 bytes, 8-row atoms 1024 bytes apart.
-__device__ __forceinline__ uint64_t make_desc(uint32_t saddr) {
-  uint64_t d = 0;
-  d |= (uint64_t)((saddr & 0x3FFFF) >> 4);   // start address
-  d |= (uint64_t)1 << 16;                    // leading byte offset (unused for swizzled K-major)
-  d |= (uint64_t)(1024 >> 4) << 32;          // stride byte offset
-  d |= (uint64_t)1 << 46;                    // descriptor version (Blackwell)
-  d |= (uint64_t)2 << 61;                    // SWIZZLE_128B
-  return d;
 }
 // bf16 x bf16 -> f32, A and B K-major, M = 128, N = bn
 __device__ __forceinline__ uint32_t make_idesc(int bn) {
@@ -250,70 +153,6 @@ __device__ __forceinline__ void umma_commit_addr(uint32_t bar_smem, uint32_t iss
       "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}"
       ::"r"(bar_smem), "r"(issue) : "memory");
 }
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,"
-      "%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]),
-        "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]),
-        "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-      : "r"(taddr));
-}
-
-// 32 codes (half of a k-block) of one weight row -> 32 bf16 values q*s+b (one rounding), written as
-// chunks 4h..4h+3 of the 128-byte row `r` of a K-major SWIZZLE_128B tile (16-byte chunk c lands at
-// chunk c ^ (r & 7)).
-template <int BITS>
-__device__ __forceinline__ void dequant_half(const uint32_t* codes, uint32_t sb2, uint32_t bb2, unsigned char* tile, int r,
-                                             int h) {
-  // sb2 / bb2: the group's scale / bias replicated in both bf16 lanes
-  const __nv_bfloat162 s2 = *(const __nv_bfloat162*)&sb2, b2 = *(const __nv_bfloat162*)&bb2;
-  unsigned char* row = tile + r * 128;
-  const int xr = ((4 * h) ^ (r & 7)) << 4;   // chunk (4h + c) ^ (r & 7) = ((4h) ^ (r & 7)) ^ c for c < 4
-  if constexpr (BITS == 4) {
-    const __nv_bfloat162 c128 = __float2bfloat162_rn(128.f);
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {  // one packed word = 8 values = one 16-byte chunk of bf16
-      const uint32_t w = codes[c];
-      // bytes (q1q0, q3q2, q5q4, q7q6) -> bytes q0,q1,q2,q3 and q4,q5,q6,q7 in order
-      const uint32_t lo = __byte_perm(w, 0, 0x4140), hi = __byte_perm(w, 0, 0x4342);
-      const uint32_t nl = (lo | (lo << 4)) & 0x0F0F0F0Fu, nh = (hi | (hi << 4)) & 0x0F0F0F0Fu;
-      uint32_t o[4];
-      // 0x43 in the high byte of a bf16 lane: 128 + q, exact
-      o[0] = __byte_perm(nl, 0x43434343u, 0x5140);
-      o[1] = __byte_perm(nl, 0x43434343u, 0x5342);
-      o[2] = __byte_perm(nh, 0x43434343u, 0x5140);
-      o[3] = __byte_perm(nh, 0x43434343u, 0x5342);
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        __nv_bfloat162 v = *(__nv_bfloat162*)&o[j];
-        v = __hsub2(v, c128);         // exact q
-        v = __hfma2(v, s2, b2);       // q*s + b, rounded once
-        o[j] = *(uint32_t*)&v;
-      }
-      *(uint4*)(row + (xr ^ (c << 4))) = make_uint4(o[0], o[1], o[2], o[3]);
-    }
-  } else {
-    const float sf = bf16lo(sb2), bf = bf16lo(bb2);
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {  // two packed words = 8 values
-      uint32_t o[4];
-#pragma unroll
-      for (int q = 0; q < 2; ++q) {
-        const uint32_t w = codes[2 * c + q];
-        const float f0 = __uint_as_float(__byte_perm(w, 0x4B000000u, 0x7540)) - 8388608.f;
-        const float f1 = __uint_as_float(__byte_perm(w, 0x4B000000u, 0x7541)) - 8388608.f;
-        const float f2 = __uint_as_float(__byte_perm(w, 0x4B000000u, 0x7542)) - 8388608.f;
-        const float f3 = __uint_as_float(__byte_perm(w, 0x4B000000u, 0x7543)) - 8388608.f;
-        o[2 * q] = pack_bf16x2(fmaf(f0, sf, bf), fmaf(f1, sf, bf));
-        o[2 * q + 1] = pack_bf16x2(fmaf(f2, sf, bf), fmaf(f3, sf, bf));
-      }
-      *(uint4*)(row + (xr ^ (c << 4))) = make_uint4(o[0], o[1], o[2], o[3]);
-    }
-  }
-}
-
 // Tile t -> coordinates.  Dense: token block t % tiles_m (fastest, so that CTAs running side by side share
 // a weight tile through L2), weight block t / tiles_m.  Grouped: the expert whose tile range holds t, then
 // the same order inside the expert (s_off: first routed row of every expert, s_tcum: prefix of their tile counts).
@@ -361,22 +200,22 @@ struct IssuerArgs {
   int tile0, ntiles, tstride, nkb, BN;
   const int* s_off; const int* s_tcum;
 };
-template <bool GROUPED, bool WIDE, bool HALF>
+template <bool GROUPED, bool HALF>
 __device__ __noinline__ void issuer_walk(const TcK& p, const IssuerArgs a, uint32_t lead) {
-  constexpr int STAGES = stages_of(GROUPED, WIDE, HALF);
+  constexpr int STAGES = stages_of(GROUPED, HALF);
   constexpr int KPST = kb_per_stage_of(HALF);          // k-blocks per stage
   constexpr int A_STAGE = A_STAGE_BYTES;               // two x boxes: two token halves, or (few-token form) two k-blocks
-  constexpr int B_SUB = bn_max_of(WIDE, GROUPED) * BK * 2, B_STAGE = KPST * B_SUB;
-  constexpr int HALF_COLS = WIDE ? 256 : 128;
+  constexpr int B_SUB = BN_MAX * BK * 2, B_STAGE = KPST * B_SUB;
+  constexpr int HALF_COLS = 128;
   const uint32_t idesc = make_idesc(a.BN);
   const uint64_t adesc0 = make_desc(a.a_smem), bdesc0 = make_desc(a.b_smem);
   int it = 0, ti = 0;
   for (int tile = a.tile0; tile < a.ntiles; tile += a.tstride, ++ti) {
     const TileCoord tc = tile_coords<GROUPED>(p, a.BN, a.s_off, a.s_tcum, tile);
     const bool two_halves = tc.row0 + 128 < tc.row_end;  // the second 128 token rows hold real tokens
-    // dense form: two accumulator sets used alternately; wide form: one set, reused by every tile
-    const int buf = WIDE ? 0 : ti & 1;
-    const uint32_t d0 = a.tmem_base + buf * 256;   // (buf is 0 in the wide form)
+    // two accumulator sets, used alternately
+    const int buf = ti & 1;
+    const uint32_t d0 = a.tmem_base + buf * 256;
     for (int kb = 0; kb < a.nkb; kb += KPST, ++it) {   // `it` counts stages
       const int st = it % STAGES;
       // the scout has seen both "full" barriers of this stage (and, before a tile's first k-block, that the
@@ -409,22 +248,20 @@ __device__ __noinline__ void issuer_walk(const TcK& p, const IssuerArgs a, uint3
   }
 }
 
-template <int BITS, bool GROUPED, bool WIDE, bool HALF = false>
+template <int BITS, bool GROUPED, bool HALF = false>
 __global__ void __launch_bounds__(kThreads, 1) qmm_tc_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ TcMaps wmaps, TcK p) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
-  // 1024-byte alignment for the swizzled tiles.  The wide form has no room for the slack: the kernel has no
-  // static shared memory, so its dynamic window starts aligned; that is verified below.
-  unsigned char* smem = WIDE ? smem_raw : (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-  constexpr int STAGES = stages_of(GROUPED, WIDE, HALF);
+  // 1024-byte alignment for the swizzled tiles
+  unsigned char* smem = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+  constexpr int STAGES = stages_of(GROUPED, HALF);
   constexpr int KPST = kb_per_stage_of(HALF);          // k-blocks per stage (2 in the few-token form)
-  constexpr int DQG = dq_groups_of(WIDE, GROUPED);     // dequant groups, kDequantWarps / DQG warps each
+  constexpr int DQG = dq_groups_of(GROUPED);     // dequant groups, kDequantWarps / DQG warps each
   static_assert(DQG <= STAGES * KPST, "a dequant group would run more than one ring round ahead of its barrier");
   constexpr int A_STAGE = A_STAGE_BYTES;               // two x boxes: two token halves, or (few-token form) two k-blocks
-  constexpr int B_SUB = bn_max_of(WIDE, GROUPED) * BK * 2, B_STAGE = KPST * B_SUB, RAW_B = bn_max_of(WIDE, GROUPED) * 128;
-  constexpr int HALF_COLS = WIDE ? 256 : 128;      // tensor-memory columns between the two token halves
+  constexpr int B_SUB = BN_MAX * BK * 2, B_STAGE = KPST * B_SUB, RAW_B = BN_MAX * 128;
+  constexpr int HALF_COLS = 128;      // tensor-memory columns between the two token halves
   unsigned char* a_tiles = smem;                                   // [STAGES][2][128 x 64 bf16]
   unsigned char* b_tiles = smem + STAGES * A_STAGE;                // [STAGES][BN x 64 bf16]
-  constexpr int RAW_BUFS = raw_bufs_of(GROUPED, WIDE, HALF);
   unsigned char* raw = b_tiles + STAGES * B_STAGE;                 // [RAW_BUFS][BN x 128 B of packed codes]
   uint64_t* bars = (uint64_t*)(raw + RAW_BUFS * RAW_B);
   uint64_t* full_a = bars, *full_b = bars + STAGES, *empty = bars + 2 * STAGES;
@@ -437,7 +274,7 @@ __global__ void __launch_bounds__(kThreads, 1) qmm_tc_kernel(const __grid_consta
   int* s_tcum = s_off + (kMaxGroupExperts + 1);     // [E + 1]
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  constexpr bool CAN_SPLIT = !GROUPED && !WIDE;
+  constexpr bool CAN_SPLIT = !GROUPED;
   const int S = CAN_SPLIT ? p.ksplit : 1;                  // CTAs per tile (cluster size)
   const int crank = S > 1 ? (int)cluster_rank_tc() : 0;
   const int nkb = p.K / BK / S;                            // k-blocks of this CTA
@@ -451,8 +288,7 @@ __global__ void __launch_bounds__(kThreads, 1) qmm_tc_kernel(const __grid_consta
     for (int i = 0; i < STAGES; ++i) { mbar_init(&full_a[i], 1); mbar_init(&full_b[i], KPST * kDequantWarps / DQG); mbar_init(&empty[i], 1); }
     for (int i = 0; i < 2; ++i) { mbar_init(&acc_full[i], 1); mbar_init(&acc_empty[i], kEpiWarps * 32); }
     for (int i = 0; i < RAW_BUFS; ++i) { mbar_init(&raw_full[i], 1); mbar_init(&raw_empty[i], (kDequantWarps / DQG) * (DQG < KPS ? DQG : KPS)); }
-    s_fail = (WIDE && (smem_u32(smem) & 1023u) != 0) ? 8 : 0;   // misaligned window: every role leaves at once
-    if (s_fail) atomicCAS(&g_tc_error, 0, 8);
+    s_fail = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == kMmaWarp) {  // tensor memory: 512 columns = two sets of two 128x128 fp32 accumulators
@@ -558,14 +394,14 @@ __global__ void __launch_bounds__(kThreads, 1) qmm_tc_kernel(const __grid_consta
       ia.empty_smem = smem_u32(empty); ia.acc_full_smem = smem_u32(acc_full);
       ia.tile0 = tile0; ia.ntiles = ntiles; ia.tstride = tstride; ia.nkb = nkb; ia.BN = BN;
       ia.s_off = s_off; ia.s_tcum = s_tcum;
-      issuer_walk<GROUPED, WIDE, HALF>(p, ia, lane == 0 ? 1u : 0u);
+      issuer_walk<GROUPED, HALF>(p, ia, lane == 0 ? 1u : 0u);
     }
   } else if (warp == kScoutWarp) {
     // ---------------- the issuer's scout: the same walk, one meeting per k-block ----------------
     int it = 0, ti = 0, fail = 0;
     for (int tile = tile0; tile < ntiles; tile += tstride, ++ti) {
-      const int buf = WIDE ? 0 : ti & 1;
-      const int use = WIDE ? ti : ti >> 1;     // how many times this accumulator set was used before
+      const int buf = ti & 1;
+      const int use = ti >> 1;     // how many times this accumulator set was used before
       if (!fail && s_fail) fail = 9;           // another role gave up
       if (!fail && use >= 1 && !mbar_wait_relaxed(&acc_empty[buf], (use - 1) & 1)) fail = 6;
       for (int kb = 0; kb < nkb; kb += KPST, ++it) {   // `it` counts stages
@@ -581,7 +417,7 @@ __global__ void __launch_bounds__(kThreads, 1) qmm_tc_kernel(const __grid_consta
   } else if (warp < kDequantWarps) {
     // ---------------- dequant producers: DQG groups, one thread per weight row ----------------
     constexpr int WPG = kDequantWarps / DQG;   // warps per group
-    constexpr int TPR = (WPG * 32) / bn_max_of(WIDE, GROUPED);   // threads per weight row: 1, or 2 (a half of the k-block each)
+    constexpr int TPR = (WPG * 32) / BN_MAX;   // threads per weight row: 1, or 2 (a half of the k-block each)
     static_assert(TPR == 1 || TPR == 2, "dequant thread layout");
     const int grp = warp / WPG, wg = warp % WPG;
     const int r = (wg % (WPG / TPR)) * 32 + lane, h = wg / (WPG / TPR);
@@ -696,8 +532,8 @@ __global__ void __launch_bounds__(kThreads, 1) qmm_tc_kernel(const __grid_consta
       const TileCoord tc = coords(tile);
       const int m0 = tc.row0, n0 = tc.n0, nend = tc.nend, mend = tc.row_end;
       const bool ksum = m0 + 128 >= mend;   // (same test as the MMA issuer's two_halves)
-      const int buf = WIDE ? 0 : ti & 1;
-      ok = mbar_wait_relaxed(&acc_full[buf], (WIDE ? ti : ti >> 1) & 1);
+      const int buf = ti & 1;
+      ok = mbar_wait_relaxed(&acc_full[buf], (ti >> 1) & 1);
       if (!ok || s_fail) { ok = false; break; }
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       if (S > 1) break;   // split-K: one tile per cluster; the partial accumulators are exchanged below
@@ -841,39 +677,19 @@ __global__ void __launch_bounds__(kThreads, 1) qmm_tc_kernel(const __grid_consta
   }
 }
 
-typedef CUresult (*EncodeFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
-                             const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
-                             CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-EncodeFn get_encode() {
-  static EncodeFn fn = nullptr;
-  static bool tried = false;
-  std::lock_guard<std::mutex> setup_lk(setup_mutex());
-  if (!tried) {
-    tried = true;
-    void* sym = nullptr;
-    cudaDriverEntryPointQueryResult qres;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &sym, cudaEnableDefault, &qres) == cudaSuccess &&
-        qres == cudaDriverEntryPointSuccess)
-      fn = (EncodeFn)sym;
-  }
-  return fn;
+constexpr size_t pipe_bytes_tc(bool grouped, bool half = false) {   // stages + code ring
+  return (size_t)stages_of(grouped, half) * (A_STAGE_BYTES + kb_per_stage_of(half) * BN_MAX * BK * 2) +
+         (size_t)RAW_BUFS * BN_MAX * 128;
 }
-
-constexpr size_t pipe_bytes_tc(bool grouped, bool wide, bool half = false) {   // stages + code ring
-  return (size_t)stages_of(grouped, wide, half) * (A_STAGE_BYTES + kb_per_stage_of(half) * bn_max_of(wide, grouped) * BK * 2) +
-         (size_t)raw_bufs_of(grouped, wide, half) * bn_max_of(wide, grouped) * 128;
+constexpr size_t smem_bytes_tc(bool grouped, bool half = false) {
+  return pipe_bytes_tc(grouped, half) + (3 * stages_of(grouped, half) + 4 + 2 * RAW_BUFS) * 8 + 16 +
+         (grouped ? (size_t)2 * (kMaxGroupExperts + 1) * 4 : 0) + 1024;
 }
-constexpr size_t smem_bytes_tc(bool grouped, bool wide, bool half = false) {
-  return pipe_bytes_tc(grouped, wide, half) + (3 * stages_of(grouped, wide, half) + 4 + 2 * raw_bufs_of(grouped, wide, half)) * 8 + 16 +
-         (grouped ? (size_t)2 * (kMaxGroupExperts + 1) * 4 : 0) + (wide ? 0 : 1024);
-}
-static_assert(smem_bytes_tc(false, true) <= 227 * 1024 && smem_bytes_tc(true, true) <= 227 * 1024, "wide form does not fit in shared memory");
-static_assert(smem_bytes_tc(false, false) <= 227 * 1024 && smem_bytes_tc(true, false) <= 227 * 1024, "shared memory");
-static_assert(smem_bytes_tc(false, false, true) <= 227 * 1024, "few-token form does not fit in shared memory");
+static_assert(smem_bytes_tc(false) <= 227 * 1024 && smem_bytes_tc(true) <= 227 * 1024, "shared memory");
+static_assert(smem_bytes_tc(false, true) <= 227 * 1024, "few-token form does not fit in shared memory");
 
 // pipeline buffers reused by the split-K exchange (either few-token form)
-constexpr size_t STAGES_DENSE_BYTES = pipe_bytes_tc(false, false) < pipe_bytes_tc(false, false, true) ? pipe_bytes_tc(false, false) : pipe_bytes_tc(false, false, true);
+constexpr size_t STAGES_DENSE_BYTES = pipe_bytes_tc(false) < pipe_bytes_tc(false, true) ? pipe_bytes_tc(false) : pipe_bytes_tc(false, true);
 
 
 // Weight rows per tile: the candidate whose tile count fills the last wave best.  Time per tile ~ rows + 40:
@@ -884,11 +700,11 @@ int64_t count_tiles(const int64_t* N, int nmat, int bn) {   // weight-row blocks
   for (int i = 0; i < nmat; ++i) t += (N[i] + bn - 1) / bn;
   return t;
 }
-int pick_bn(int64_t M, const int64_t* N, int nmat, int nsm, int bn_max = BN_MAX) {
+int pick_bn(int64_t M, const int64_t* N, int nmat, int nsm) {
   const int64_t tiles_m = (M + BM - 1) / BM;
-  int best = bn_max;
+  int best = BN_MAX;
   int64_t best_cost = -1;
-  for (int bn = bn_max; bn >= 32; bn -= 16) {
+  for (int bn = BN_MAX; bn >= 32; bn -= 16) {
     const int64_t tiles = tiles_m * count_tiles(N, nmat, bn);
     const int64_t waves = (tiles + nsm - 1) / nsm;
     const int64_t cost = waves * (bn + 40);
@@ -924,17 +740,17 @@ struct TcLaunch {
   const void* rhs; int rhs_i64; int E;   // grouped form only
 };
 
-template <int BITS, bool GROUPED, bool WIDE, bool HALF = false>
+template <int BITS, bool GROUPED, bool HALF = false>
 cudaError_t launch_tc_inst(const CUtensorMap& xmap, const TcMaps& wmap, const TcK& p, dim3 grid, cudaStream_t st,
                            int cluster = 1) {
   static bool done[64] = {};
   int dev = 0;
   cudaGetDevice(&dev);
-  constexpr size_t smem = smem_bytes_tc(GROUPED, WIDE, HALF);
+  constexpr size_t smem = smem_bytes_tc(GROUPED, HALF);
   {
   std::lock_guard<std::mutex> setup_lk(setup_mutex());   // first use on a device, from any thread
   if (dev < 0 || dev >= 64 || !done[dev]) {
-    cudaError_t e = cudaFuncSetAttribute(qmm_tc_kernel<BITS, GROUPED, WIDE, HALF>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = cudaFuncSetAttribute(qmm_tc_kernel<BITS, GROUPED, HALF>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     if (dev >= 0 && dev < 64) done[dev] = true;
   }
@@ -950,9 +766,9 @@ cudaError_t launch_tc_inst(const CUtensorMap& xmap, const TcMaps& wmap, const Tc
     attr[0].val.clusterDim.x = cluster; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, qmm_tc_kernel<BITS, GROUPED, WIDE, HALF>, xmap, wmap, p);
+    return cudaLaunchKernelEx(&cfg, qmm_tc_kernel<BITS, GROUPED, HALF>, xmap, wmap, p);
   }
-  qmm_tc_kernel<BITS, GROUPED, WIDE, HALF><<<grid, kThreads, smem, st>>>(xmap, wmap, p);
+  qmm_tc_kernel<BITS, GROUPED, HALF><<<grid, kThreads, smem, st>>>(xmap, wmap, p);
   return cudaGetLastError();
 }
 
@@ -966,7 +782,7 @@ int split_capacity(int cluster) {
   if (dev < 0 || dev >= 64) dev = 0;
   std::lock_guard<std::mutex> setup_lk(setup_mutex());
   if (cached[dev][cluster] == 0) {
-    constexpr size_t smem = smem_bytes_tc(false, false);
+    constexpr size_t smem = smem_bytes_tc(false);
     int n = 0;
     cudaLaunchConfig_t q = {};
     q.gridDim = dim3((unsigned)(sm_count() / cluster * cluster));
@@ -977,8 +793,8 @@ int split_capacity(int cluster) {
     qa[0].val.clusterDim.x = cluster; qa[0].val.clusterDim.y = 1; qa[0].val.clusterDim.z = 1;
     q.attrs = qa;
     q.numAttrs = 1;
-    if (cudaFuncSetAttribute(qmm_tc_kernel<BITS, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
-        cudaOccupancyMaxActiveClusters(&n, qmm_tc_kernel<BITS, false, false>, &q) != cudaSuccess) {
+    if (cudaFuncSetAttribute(qmm_tc_kernel<BITS, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&n, qmm_tc_kernel<BITS, false>, &q) != cudaSuccess) {
       (void)cudaGetLastError();
       n = 0;
     }
@@ -993,8 +809,8 @@ cudaError_t launch_tc(const TcLaunch* av, int nmat, bool grouped, cudaStream_t s
   const TcLaunch& a = av[0];
   int64_t Nv[kMaxTcMat];
   for (int i = 0; i < nmat; ++i) Nv[i] = av[i].N;
-  int64_t Ntot = 0, Nmin = a.N;
-  for (int i = 0; i < nmat; ++i) { Ntot += Nv[i]; Nmin = Nv[i] < Nmin ? Nv[i] : Nmin; }
+  int64_t Ntot = 0;
+  for (int i = 0; i < nmat; ++i) Ntot += Nv[i];
   EncodeFn enc = get_encode();
   if (!enc) return cudaErrorNotSupported;
   CUtensorMap map;
@@ -1008,14 +824,10 @@ cudaError_t launch_tc(const TcLaunch* av, int nmat, bool grouped, cudaStream_t s
   if (r != CUDA_SUCCESS) return cudaErrorInvalidValue;
   TcK p;
   const int nsm = sm_count();
-  // Wide tiles when both 128-token halves of a tile are in use and there are enough weight rows to fill the GPU
-  // with them; the grouped form does not know its tile count on the host and takes full-width dense tiles.
-  // (grouped: many rows per expert on average, so that most tiles have both halves)
-  const bool wide = grouped ? (a.M >= 192 * (int64_t)a.E && a.N >= 256) : (a.M > 256 && Nmin >= 1024);
   if (grouped) {
     // tile width with the best product of (rows used / rows multiplied) and the width's own efficiency
     // (time per tile ~ width + 40, as in pick_bn)
-    const int cap = bn_max_of(wide, true);
+    const int cap = BN_MAX;
     int best = cap;
     double best_score = -1.0;
     for (int bn = cap; bn >= 64; bn -= 16) {
@@ -1025,14 +837,14 @@ cudaError_t launch_tc(const TcLaunch* av, int nmat, bool grouped, cudaStream_t s
     }
     p.BN = a.N >= 64 ? best : (int)((a.N + 15) / 16 * 16);
   } else {
-    p.BN = pick_bn(a.M, Nv, nmat, nsm, bn_max_of(wide));
+    p.BN = pick_bn(a.M, Nv, nmat, nsm);
   }
   // Split-K over a cluster when a few-token problem has too few tiles to occupy the GPU: with one tile per CTA
   // the time is the number of k-blocks a CTA walks (plus ~6 k-block times for the exchange), whatever the tile
   // width, so K is cut in 4 or 2 and the tile is made just wide enough for tiles x ranks to fit the SMs.
   p.ksplit = 1;
-  const bool half = !grouped && !wide && a.M <= 128;   // no tile has a second token half: stages of one x box
-  if (!grouped && !wide && a.M <= 256) {
+  const bool half = !grouped && a.M <= 128;   // no tile has a second token half: stages of one x box
+  if (!grouped && a.M <= 256) {
     const int gshift = a.gs == 128 ? 1 : 0;
     const int nkb_all = (int)(a.K / BK);
     const int64_t plain_tiles = count_tiles(Nv, nmat, p.BN);
@@ -1081,16 +893,14 @@ cudaError_t launch_tc(const TcLaunch* av, int nmat, bool grouped, cudaStream_t s
   dim3 grid((unsigned)((!grouped && p.ntiles < nsm) ? p.ntiles : nsm), 1, 1);
   if (p.ksplit > 1) {
     grid = dim3((unsigned)(p.ntiles * p.ksplit), 1, 1);   // one tile per cluster
-    if (half) return a.bits == 4 ? launch_tc_inst<4, false, false, true>(map, wmap, p, grid, st, p.ksplit)
-                                 : launch_tc_inst<8, false, false, true>(map, wmap, p, grid, st, p.ksplit);
-    return a.bits == 4 ? launch_tc_inst<4, false, false>(map, wmap, p, grid, st, p.ksplit)
-                       : launch_tc_inst<8, false, false>(map, wmap, p, grid, st, p.ksplit);
+    if (half) return a.bits == 4 ? launch_tc_inst<4, false, true>(map, wmap, p, grid, st, p.ksplit)
+                                 : launch_tc_inst<8, false, true>(map, wmap, p, grid, st, p.ksplit);
+    return a.bits == 4 ? launch_tc_inst<4, false>(map, wmap, p, grid, st, p.ksplit)
+                       : launch_tc_inst<8, false>(map, wmap, p, grid, st, p.ksplit);
   }
-  if (grouped && wide) return a.bits == 4 ? launch_tc_inst<4, true, true>(map, wmap, p, grid, st) : launch_tc_inst<8, true, true>(map, wmap, p, grid, st);
-  if (grouped) return a.bits == 4 ? launch_tc_inst<4, true, false>(map, wmap, p, grid, st) : launch_tc_inst<8, true, false>(map, wmap, p, grid, st);
-  if (wide) return a.bits == 4 ? launch_tc_inst<4, false, true>(map, wmap, p, grid, st) : launch_tc_inst<8, false, true>(map, wmap, p, grid, st);
-  if (half) return a.bits == 4 ? launch_tc_inst<4, false, false, true>(map, wmap, p, grid, st) : launch_tc_inst<8, false, false, true>(map, wmap, p, grid, st);
-  return a.bits == 4 ? launch_tc_inst<4, false, false>(map, wmap, p, grid, st) : launch_tc_inst<8, false, false>(map, wmap, p, grid, st);
+  if (grouped) return a.bits == 4 ? launch_tc_inst<4, true>(map, wmap, p, grid, st) : launch_tc_inst<8, true>(map, wmap, p, grid, st);
+  if (half) return a.bits == 4 ? launch_tc_inst<4, false, true>(map, wmap, p, grid, st) : launch_tc_inst<8, false, true>(map, wmap, p, grid, st);
+  return a.bits == 4 ? launch_tc_inst<4, false>(map, wmap, p, grid, st) : launch_tc_inst<8, false>(map, wmap, p, grid, st);
 }
 
 }  // namespace

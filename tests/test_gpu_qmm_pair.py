@@ -1,0 +1,46 @@
+"""The CTA-pair tensor-core kernel: edges of its token and weight-row tiles, one and two units a tile, several waves, and rows sorted
+by expert, against the CPU oracle (weight term rounded to bf16 once)."""
+import numpy as np
+import pytest
+import torch
+
+from oracle import qoracle as qo
+from test_gpu_qmm import _run
+from util import dev_triple, gate_bf16, make_weight, rand_bf16, to_dev_bf16
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("bits,gs,M,N,K", [
+    (4, 64, 257, 512, 256), (8, 64, 289, 769, 512), (4, 128, 513, 1023, 768), (4, 64, 129, 6144, 256),   # edges of units and row blocks
+    (4, 64, 1000, 600, 1280), (8, 128, 1100, 2304, 256), (4, 64, 2500, 5000, 256)])                      # several waves, one unit and two
+def test_dense(bits, gs, M, N, K):
+    import qb200
+    rng = np.random.default_rng(bits * 100 + gs + M + N + K)
+    q, s, b = make_weight(rng, (N, K), gs, bits)
+    x = rand_bf16(rng, (M, K))
+    if M * N < 1 << 20:
+        _run(x, q, s, b, gs, bits)
+    else:   # the oracle takes sampled rows
+        y = qb200.quantized_matmul(to_dev_bf16(qo.f32_to_bf16(x)), *dev_triple(q, s, b), True, gs, bits).float().cpu().numpy()
+        rows = rng.choice(M, 48, replace=False)
+        gate_bf16(y[rows], qo.qmm(x[rows], q, s, b, gs, bits, bf16_weights=True), "sampled rows")
+    assert qb200.lib().qb200_debug_tc_status() == 0
+
+
+@pytest.mark.parametrize("bits,gs,N,K,counts", [
+    (4, 64, 300, 256, (600, 0, 33, 1, 513, 70)), (8, 64, 256, 512, (0, 257, 900, 31)), (4, 128, 513, 256, (5, 2000)),
+    (4, 64, 256, 256, tuple(32 + (i * 7) % 5 for i in range(300)))])                                     # more experts than fit beside six stages
+def test_sorted_rows(bits, gs, N, K, counts):
+    import qb200
+    rng = np.random.default_rng(len(counts) + N + K)
+    E = len(counts)
+    q, s, b = make_weight(rng, (E, N, K), gs, bits)
+    x = rand_bf16(rng, (sum(counts), 1, K))
+    idx = np.repeat(np.arange(E), counts).astype(np.int32)
+    y = qb200.gather_qmm(to_dev_bf16(qo.f32_to_bf16(x)), *dev_triple(q, s, b), None, torch.from_numpy(idx).cuda(), True, gs, bits, sorted_indices=True)
+    x, y = x[:, 0], y.float().cpu().numpy()[:, 0]
+    for e in range(0, E, 1 + E // 20):
+        if counts[e]:
+            gate_bf16(y[idx == e], qo.qmm(x[idx == e], q[e], s[e], b[e], gs, bits, bf16_weights=True), f"expert {e}")
+    assert qb200.lib().qb200_debug_tc_status() == 0
