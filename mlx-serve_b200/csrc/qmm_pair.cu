@@ -11,24 +11,26 @@
 //
 //  * Cluster of two CTAs, persistent, one pair per two SMs.  A tile is one or two units of up to 256 tokens.  Accumulators: two
 //    slots of 256 columns of tensor memory that units take in turn: the epilogue of one-unit tiles runs beside the next tile.
-//  * Roles per CTA: warps 0-15 convert weights (four groups of four warps that take k-blocks in turn, a thread per weight row),
-//    16-19 epilogue, 20 TMA of x, 21 TMA of packed codes, 22 the MMA issuer (CTA 0 only: its instructions read both CTAs' operands),
-//    23 the issuer's scout (CTA 0).  Copies and converters of CTA 1 arrive at CTA 0's barrier of the stage; one commit frees the
-//    stage in both.
+//  * Roles per CTA: twelve warps convert weights (three groups of four that take k-blocks in turn, a thread per weight row), four
+//    are the epilogue, and one each loads x, loads packed codes, issues the MMAs (CTA 0 only: its instructions read both CTAs'
+//    operands) and scouts for the issuer (CTA 0).  These four share a scheduler without any converting warp: beside one, the
+//    issuer took 450 cycles for four MMAs, its few instructions refetched each time.  Copies and converters of CTA 1 arrive at
+//    CTA 0's barrier of the stage; one commit frees the stage in both.
 //  * What a k-block costs beside its MMAs is synchronisation (measured with the work left out), so: one lane polls for a group of
 //    warps and the others follow at a named barrier (polls by all lanes are served one after another and delay the copies'
 //    arrivals); no cluster-scope release or acquire on the barriers (each was a fence of about 2000 cycles); the scout runs ahead of
 //    the issuer through a named barrier per stage; the issuer's operands are warp-uniform.
-// us, before -> after: 2048 tokens, 14336 x 4096 224 -> 172, 4096 x 14336 284 -> 159, 4096 x 4096 98 -> 52, 4096^3 at 8 bits
-// 194 -> 97 (1.4 - 1.5 PFLOP/s); 4096 tokens x 8 of 128 experts 768 x 2048 180 -> 129, 2048 x 768 199 -> 136.
+// us, before -> after: 2048 tokens, 14336 x 4096 224 -> 162, 4096 x 14336 284 -> 157, 4096 x 4096 98 -> 52, 4096^3 at 8 bits
+// 194 -> 95 (1.3 - 1.5 PFLOP/s); 4096 tokens x 8 of 128 experts 768 x 2048 180 -> 125, 2048 x 768 199 -> 137.
 // Every mbarrier wait is bounded: on expiry the kernel records a code, the role leaves its loops, tensor memory is freed.
 #include "tc_ptx.cuh"
 
 namespace qb {
 namespace {
 
-constexpr int BK = 64, RAWB = 2, DQG = 4, WPG = 4, SMAX = 6;
-constexpr int kDqWarps = 16, kEpi0 = 16, kXWarp = 20, kWWarp = 21, kMmaWarp = 22, kScoutWarp = 23, kThreads = 24 * 32;
+constexpr int BK = 64, RAWB = 2, DQG = 3, WPG = 4, SMAX = 6;
+// warps with warp % 4 == 3 share a scheduler, and leave it to the roles that the others wait for
+constexpr int kMmaWarp = 3, kScoutWarp = 7, kXWarp = 11, kWWarp = 15, kEpi0 = 16, kThreads = 20 * 32;
 constexpr int TILE = 128 * BK * 2, RAW = 128 * 128;   // 128 rows of one k-block as bf16; of one piece of packed codes
 constexpr int kMaxE = 256;                            // experts whose tables fit beside the rings; more take the room of a sixth stage
 // two units a tile: 4 stages of weights and two boxes of x; one unit: 6 stages of weights and one
@@ -334,8 +336,8 @@ __global__ void __launch_bounds__(kThreads, 1) qmm_pair_kernel(const __grid_cons
         }
       }
     }
-  } else if (warp < kDqWarps) {
-    const int grp = warp / WPG, r = (warp % WPG) * 32 + lane;
+  } else if (warp < kEpi0) {
+    const int dq = (warp >> 2) * 3 + (warp & 3), grp = dq / WPG, r = (dq % WPG) * 32 + lane;
     const int ntl = ntiles > tile0 ? (ntiles - tile0 + tstride - 1) / tstride : 0, total = ntl * nkb;
     // scales and biases of this thread's row: windows of 8 values (8 << gshift k-blocks), one window ahead
     const int WL = 8 << p.gshift;
@@ -360,14 +362,14 @@ __global__ void __launch_bounds__(kThreads, 1) qmm_pair_kernel(const __grid_cons
     };
     if (p.sb_vec) prefetch();
     bool ok = true;
-    int tl = 0, kb = grp - DQG, st = grp, round = 0;     // (four groups, at least four stages)
+    int tl = 0, kb = grp - DQG, st = grp, round = 0, window = -1, turn = 0;     // (three groups, at least four stages)
     for (int it = grp; it < total; it += DQG) {
       kb += DQG;
       if (kb >= nkb) { kb -= nkb; ++tl; if (!p.sb_vec) row_ptrs(tl, c_sp, c_bp); }
       const int sb = it / KPS, kbl = it % KPS, buf = sb % RAWB;   // nkb is a multiple of KPS
       uint32_t sv2, bv2;
       if (p.sb_vec) {
-        if ((kb & (WL - 1)) == grp) { s_cur = s_nxt; b_cur = b_nxt; prefetch(); }
+        if (it >> (3 + p.gshift) != window) { window = it >> (3 + p.gshift); s_cur = s_nxt; b_cur = b_nxt; prefetch(); }
         const int e = (kb >> p.gshift) & 7;
         const uint32_t sw = e < 4 ? (e < 2 ? s_cur.x : s_cur.y) : (e < 6 ? s_cur.z : s_cur.w);
         const uint32_t bw = e < 4 ? (e < 2 ? b_cur.x : b_cur.y) : (e < 6 ? b_cur.z : b_cur.w);
@@ -379,13 +381,13 @@ __global__ void __launch_bounds__(kThreads, 1) qmm_pair_kernel(const __grid_cons
         bv2 = bv | (bv << 16);
       }
       // one lane of the group polls for the codes and for the stage, the group follows at a named barrier
-      if (warp % WPG == 0 && lane == 0) {
+      if (dq % WPG == 0 && lane == 0) {
         bool go = wait_cta(&raw_full[buf], (sb / RAWB) & 1);
         if (go && round > 0) go = wait_cta(&empty[st], (round - 1) & 1);
-        s_go[grp * 2 + ((it / DQG) & 1)] = go && !s_fail;
+        s_go[grp * 2 + turn] = go && !s_fail;
       }
       asm volatile("bar.sync %0, 128;" ::"r"(1 + SMAX + grp) : "memory");
-      ok = s_go[grp * 2 + ((it / DQG) & 1)] != 0;   // (two slots in turn: the next write comes after everybody's read)
+      ok = s_go[grp * 2 + turn] != 0;   // (two slots in turn: the next write comes after everybody's read)
       if (!ok) break;
       constexpr int WPH = 32 * BITS / 32;
       uint32_t c[2][WPH];
@@ -406,6 +408,7 @@ __global__ void __launch_bounds__(kThreads, 1) qmm_pair_kernel(const __grid_cons
         arrive_addr(full0 + (uint32_t)st * 8u);
         mbar_arrive(&raw_empty[buf]);   // (only now that the words have been consumed)
       }
+      turn ^= 1;
       st += DQG;
       if (st >= S) { st -= S; ++round; }
     }
@@ -512,7 +515,7 @@ cudaError_t launch_qmm_pair(const QmmArgs& a, cudaStream_t st) {
   double best = -1.0;
   for (int h = 512; h >= 64; h -= 32) {
     const int64_t tiles = ((a.M + h - 1) / h) * nb;
-    const double kb = h <= 256 ? 0.43 : 0.52 + (h > 352 ? (h - 352) * 0.0007 : 0.0), epi = h <= 256 ? 0.5 : h * 0.012;
+    const double kb = h <= 256 ? 0.39 : 0.52 + (h > 352 ? (h - 352) * 0.0007 : 0.0), epi = h <= 256 ? 0.5 : h * 0.012;
     const double cost = (double)((tiles + pairs - 1) / pairs) * ((double)(a.K / BK) * kb + epi);
     if (best < 0 || cost < best - 1e-9) { best = cost; p.h = h; }
   }

@@ -138,19 +138,17 @@ __device__ __forceinline__ void dequant_half(const uint32_t* codes, uint32_t sb2
       *(uint4*)(row + (xr ^ (c << 4))) = make_uint4(o[0], o[1], o[2], o[3]);
     }
   } else {
-    const float sf = bf16lo(sb2), bf = bf16lo(bb2);
 #pragma unroll
     for (int c = 0; c < 4; ++c) {  // two packed words = 8 values
       uint32_t o[4];
 #pragma unroll
-      for (int q = 0; q < 2; ++q) {
-        const uint32_t w = codes[2 * c + q];
-        const float f0 = __uint_as_float(__byte_perm(w, 0x4B000000u, 0x7540)) - 8388608.f;
-        const float f1 = __uint_as_float(__byte_perm(w, 0x4B000000u, 0x7541)) - 8388608.f;
-        const float f2 = __uint_as_float(__byte_perm(w, 0x4B000000u, 0x7542)) - 8388608.f;
-        const float f3 = __uint_as_float(__byte_perm(w, 0x4B000000u, 0x7543)) - 8388608.f;
-        o[2 * q] = pack_bf16x2(fmaf(f0, sf, bf), fmaf(f1, sf, bf));
-        o[2 * q + 1] = pack_bf16x2(fmaf(f2, sf, bf), fmaf(f3, sf, bf));
+      for (int j = 0; j < 4; ++j) {
+        const uint32_t w = codes[2 * c + (j >> 1)], v = __byte_perm(w, 0, j & 1 ? 0x4342 : 0x4140);   // two codes in 16-bit halves
+        // exact bf16 integers: 128 + the low seven bits, minus 128 where the top bit is clear (0x80 * 0x186 = 0xC300 = -128)
+        const uint32_t lo = (v & 0x007F007Fu) | 0x43004300u, hi = ((v & 0x00800080u) ^ 0x00800080u) * 0x186u;
+        __nv_bfloat162 q = __hadd2(*(const __nv_bfloat162*)&lo, *(const __nv_bfloat162*)&hi);
+        q = __hfma2(q, s2, b2);       // q*s + b, rounded once
+        o[j] = *(uint32_t*)&q;
       }
       *(uint4*)(row + (xr ^ (c << 4))) = make_uint4(o[0], o[1], o[2], o[3]);
     }
