@@ -129,10 +129,16 @@ __device__ __forceinline__ void mma_bf16(float (&d)[4], uint32_t a0, uint32_t a1
 
 // A lane owns 16 consecutive K values of a 64-group (k = 16 t + o) of the rows g and g + 8.  Which of them
 // sit in MMA step m (0..3), operand register r (0: a0/a1 with b0, 1: a2/a3 with b1), element e (0, 1) is a
-// free permutation of K as long as the activations are staged alike.  4 bits: the pairs one LOP3 cuts out
-// of a packed word, (w >> 4i) & 0x000F000F = codes (i, i + 4) of that word.  8 bits: in order.
+// free permutation of K as long as the activations are staged alike: the pairs one LOP3 cuts out of a packed
+// word.  4 bits: (w >> 4i) & 0x000F000F = codes (i, i + 4); 8 bits: bytes (r, r + 2).
 template <int BITS> __host__ __device__ constexpr int kofs(int m, int r, int e) {
-  return BITS == 4 ? 8 * (m >> 1) + 2 * (m & 1) + r + 4 * e : 4 * m + 2 * r + e;
+  return BITS == 4 ? 8 * (m >> 1) + 2 * (m & 1) + r + 4 * e : 4 * m + r + 2 * e;
+}
+// bytes 0 and 2 as exact bf16 integers: 128 + the low seven bits, minus 128 where the top bit is clear
+// (0x80 * 0x186 = 0xC300 = -128)
+__device__ __forceinline__ __nv_bfloat162 bf16_bytes(uint32_t v) {
+  const uint32_t lo = lop3_and_or(v, 0x007F007Fu, 0x43004300u), hi = ((v & 0x00800080u) ^ 0x00800080u) * 0x186u;
+  return __hadd2(*(const __nv_bfloat162*)&lo, *(const __nv_bfloat162*)&hi);
 }
 
 // ---- activations -> bf16 B fragments in slices, one thread per (token slot, 16 K values) ----
@@ -387,22 +393,18 @@ __global__ void __launch_bounds__(kThreads, 1) qmv_wide_kernel(const __grid_cons
         } else {
           const uint4 wl = *(const uint4*)(st + frag_off[j]);
           const uint4 wh = *(const uint4*)(st + frag_off[j] + 1024);
-          const float sfl = bf16lo(s_lo), bfl = bf16lo(b_lo), sfh = bf16lo(s_hi), bfh = bf16lo(b_hi);
           const uint32_t wlv[4] = {wl.x, wl.y, wl.z, wl.w}, whv[4] = {wh.x, wh.y, wh.z, wh.w};
+          const __nv_bfloat162 s2l = *(const __nv_bfloat162*)&s_lo, b2l = *(const __nv_bfloat162*)&b_lo;
+          const __nv_bfloat162 s2h = *(const __nv_bfloat162*)&s_hi, b2h = *(const __nv_bfloat162*)&b_hi;
 #pragma unroll
-          for (int m = 0; m < 4; ++m) {   // word m holds codes 4m .. 4m + 3: (a0: 4m, 4m+1), (a2: 4m+2, 4m+3)
-            const float l0 = __uint_as_float(__byte_perm(wlv[m], 0x4B000000u, 0x7540)) - 8388608.f;
-            const float l1 = __uint_as_float(__byte_perm(wlv[m], 0x4B000000u, 0x7541)) - 8388608.f;
-            const float l2 = __uint_as_float(__byte_perm(wlv[m], 0x4B000000u, 0x7542)) - 8388608.f;
-            const float l3 = __uint_as_float(__byte_perm(wlv[m], 0x4B000000u, 0x7543)) - 8388608.f;
-            const float h0 = __uint_as_float(__byte_perm(whv[m], 0x4B000000u, 0x7540)) - 8388608.f;
-            const float h1 = __uint_as_float(__byte_perm(whv[m], 0x4B000000u, 0x7541)) - 8388608.f;
-            const float h2 = __uint_as_float(__byte_perm(whv[m], 0x4B000000u, 0x7542)) - 8388608.f;
-            const float h3 = __uint_as_float(__byte_perm(whv[m], 0x4B000000u, 0x7543)) - 8388608.f;
-            A[m][0] = pack_bf16x2(fmaf(l0, sfl, bfl), fmaf(l1, sfl, bfl));
-            A[m][2] = pack_bf16x2(fmaf(l2, sfl, bfl), fmaf(l3, sfl, bfl));
-            A[m][1] = pack_bf16x2(fmaf(h0, sfh, bfh), fmaf(h1, sfh, bfh));
-            A[m][3] = pack_bf16x2(fmaf(h2, sfh, bfh), fmaf(h3, sfh, bfh));
+          for (int m = 0; m < 4; ++m) {   // word m holds codes 4m .. 4m + 3: pairs (4m, 4m + 2) and (4m + 1, 4m + 3)
+#pragma unroll
+            for (int r = 0; r < 2; ++r) {
+              const __nv_bfloat162 vl = __hfma2(bf16_bytes(r ? wlv[m] >> 8 : wlv[m]), s2l, b2l);
+              const __nv_bfloat162 vh = __hfma2(bf16_bytes(r ? whv[m] >> 8 : whv[m]), s2h, b2h);
+              A[m][2 * r] = *(const uint32_t*)&vl;
+              A[m][2 * r + 1] = *(const uint32_t*)&vh;
+            }
           }
         }
         // Four token tiles at a time: their B fragments first, then the MMA steps with the tiles innermost, so
