@@ -79,11 +79,12 @@ __host__ int plan_f16(const KvAttnArgs& a, int64_t qtiles, int max_fused) {
 
 // Splits of the 4-bit integer kernel where they merge inside a cluster (no partials in memory).  A CTA reads a token of one kv head
 // in 4.3 ns alone on its SM and in 7.6 ns beside a second one, plus about 6 us of start and end and 0.8 us of merge per split.  While all CTAs are resident the
-// longest sequence decides, in rounds of 512 tokens a CTA; beyond, sequences of ragged lengths (three quarters of the longest
-// on average) follow one another on the places that clusters of that size can take, and half a CTA is left over at the end.
+// longest sequence decides, in rounds of 512 tokens a CTA; beyond, CTAs follow one another on the places that clusters of that size can take: whole waves when all sequences are as
+// long, else one after another with half a CTA left over at the end.  `mean`: mean length / T; lengths that only the device
+// knows are taken as three quarters of the longest.
 // (Within 10 % of the times of 1 - 8 splits at 16 x 8 pairs of 32768 tokens, 5 x 8 of 9000, 32 x 8 of 3000, 12 x 2 of 16000 and
 // 40 x 8 of 16000, where the plan by whole waves gave 128 / 21 / 29 / 29 / 144 us and this one 122 / 21 / 29 / 24 / 134.)
-__host__ int plan_clusters(int64_t pairs, int64_t T) {
+__host__ int plan_clusters(int64_t pairs, int64_t T, double mean) {
   static const double place[8] = {1.0, 1.0, 0.943, 0.959, 0.946, 0.912, 0.875, 0.892};   // of two CTAs per SM, by cluster size
   int best = 1;
   double best_cost = -1.0;
@@ -92,7 +93,8 @@ __host__ int plan_clusters(int64_t pairs, int64_t T) {
     double cost;
     if (2.0 * n <= slots) cost = 0.0043 * up + 6.0 + 0.8 * ns;
     else if (n <= slots) cost = 0.0076 * up + 6.0 + 0.8 * ns;
-    else cost = (0.0076 * 0.75 * tok + 6.0) * (n / slots + 0.5) + 0.8 * ns;
+    else if (mean > 0.95) cost = (0.0076 * up + 6.0) * (double)(int64_t)(n / slots + 0.999) + 0.8 * ns;
+    else cost = (0.0076 * mean * tok + 6.0) * (n / slots + 0.5) + 0.8 * ns;
     if (best_cost < 0.0 || cost < best_cost - 1e-9) { best_cost = cost; best = ns; }
   }
   return best;
@@ -342,7 +344,12 @@ cudaError_t launch_kv_attn(const KvAttnArgs& a, cudaStream_t st, const KvSeqTabl
     // 4096 tokens and 132.8 against 134.0 us at 32768; 8-bit caches, whose CTAs fill an SM alone, 33.0 against 31.8 us
     // at 4096 tokens -- so only the 4-bit kernel takes the cluster form.
     if (sp.nsplit <= kMaxFusedSplits && a.bits == 4) {
-      e = launch_kv_fast(a, plan_clusters(a.B * a.Hkv, a.T), p.part_m, p.part_l, p.part_o, st, seqs, true);
+      double mean = a.kv_lens ? 0.75 : 1.0;
+      if (seqs) {
+        mean = 0.0;
+        for (int64_t b = 0; b < a.B; ++b) mean += (double)seqs->s[b].T / (double)(a.B * a.T);
+      }
+      e = launch_kv_fast(a, plan_clusters(a.B * a.Hkv, a.T, mean), p.part_m, p.part_l, p.part_o, st, seqs, true);
       if (e == cudaSuccess) return e;
       (void)cudaGetLastError();   // a cluster this launch could not place: fall back to partials and the merge kernel
     }
