@@ -38,7 +38,9 @@ constexpr size_t kTiles = (size_t)12 * TILE + RAWB * RAW;
 constexpr int kBars = 2 * SMAX + 2 * RAWB + 4;
 constexpr size_t smem_of(bool grouped) { return kTiles + kBars * 8 + 48 + (grouped ? 2 * (kMaxE + 1) * 4 : 0); }
 static_assert(smem_of(true) <= 227 * 1024, "shared memory");
-constexpr uint32_t kSpin = 1u << 12, kNap = 1000000;   // polls, and how long the hardware may hold one (ns)
+// Polls of a bounded wait, and how long the hardware may hold one (ns).  With 1 ms, waits of more than a millisecond (an epilogue's at
+// K = 196608) never ended; with 20 us they do, and shorter waits cost the same.
+constexpr uint32_t kSpin = 1u << 18, kNap = 20000;
 
 __device__ int g_pair_error = 0;                 // 0, or the code of a wait that expired
 
@@ -215,7 +217,7 @@ __global__ void __launch_bounds__(kThreads, 1) qmm_pair_kernel(const __grid_cons
 
   if (tid == 0) {
     for (int i = 0; i < SMAX; ++i) { mbar_init(&full[i], 1 + 2 * WPG); mbar_init(&empty[i], 1); }
-    for (int i = 0; i < RAWB; ++i) { mbar_init(&raw_full[i], 1); mbar_init(&raw_empty[i], WPG * KPS); }
+    for (int i = 0; i < RAWB; ++i) { mbar_init(&raw_full[i], 1); mbar_init(&raw_empty[i], WPG * KPS + (KPS < DQG ? DQG - KPS : 0)); }
     for (int i = 0; i < 2; ++i) { mbar_init(&acc_full[i], 1); mbar_init(&acc_empty[i], 8); }
     s_fail = (smem_u32(smem) & 1023u) ? 308 : 0;           // misaligned window: every role leaves at once
     if (s_fail) atomicCAS(&g_pair_error, 0, 308);
@@ -362,7 +364,7 @@ __global__ void __launch_bounds__(kThreads, 1) qmm_pair_kernel(const __grid_cons
     };
     if (p.sb_vec) prefetch();
     bool ok = true;
-    int tl = 0, kb = grp - DQG, st = grp, round = 0, window = -1, turn = 0;     // (three groups, at least four stages)
+    int tl = 0, kb = grp - DQG, st = grp, round = 0, window = -1, turn = 0, seen = 0;     // (three groups, at least four stages)
     for (int it = grp; it < total; it += DQG) {
       kb += DQG;
       if (kb >= nkb) { kb -= nkb; ++tl; if (!p.sb_vec) row_ptrs(tl, c_sp, c_bp); }
@@ -382,7 +384,14 @@ __global__ void __launch_bounds__(kThreads, 1) qmm_pair_kernel(const __grid_cons
       }
       // one lane of the group polls for the codes and for the stage, the group follows at a named barrier
       if (dq % WPG == 0 && lane == 0) {
-        bool go = wait_cta(&raw_full[buf], (sb / RAWB) & 1);
+        // Pieces without a k-block of this group are seen and released too: a parity names a phase only to who follows every one.
+        bool go = true;
+        for (; KPS < DQG && seen < sb; ++seen) {
+          go = go && wait_cta(&raw_full[seen % RAWB], (seen / RAWB) & 1);
+          mbar_arrive(&raw_empty[seen % RAWB]);
+        }
+        seen = sb + 1;
+        go = go && wait_cta(&raw_full[buf], (sb / RAWB) & 1);
         if (go && round > 0) go = wait_cta(&empty[st], (round - 1) & 1);
         s_go[grp * 2 + turn] = go && !s_fail;
       }

@@ -44,3 +44,15 @@ def test_sorted_rows(bits, gs, N, K, counts):
         if counts[e]:
             gate_bf16(y[idx == e], qo.qmm(x[idx == e], q[e], s[e], b[e], gs, bits, bf16_weights=True), f"expert {e}")
     assert qb200.lib().qb200_debug_tc_status() == 0
+
+
+def test_tile_of_more_than_a_millisecond():
+    """One tile over a contraction so long that the epilogue's wait outlives any single poll; checked against the exact sum."""
+    import qb200
+    M, N, K = 257, 512, 196608
+    w = qb200.quantize(torch.randn(N, K, device="cuda", dtype=torch.bfloat16) * 0.02, 64, 4)
+    x = torch.randn(M, K, device="cuda", dtype=torch.bfloat16)
+    y = qb200.quantized_matmul(x, *w, True, 64, 4)
+    assert qb200.lib().qb200_debug_tc_status() == 0
+    ref = x[:64].double() @ qb200.dequantize(*w, 64, 4, dtype=torch.bfloat16).double().t()
+    assert float((y[:64].double() - ref).norm() / ref.norm()) < 3e-3
