@@ -103,8 +103,20 @@ qb200_optional_int opt(PyObject* o) {
   if (o == Py_None) return {0, false};
   return {(int)as_long(o), true};
 }
-int bits_or_4(PyObject* o) { return o == Py_None ? 4 : (int)as_long(o); }
-int gs_or_64(PyObject* o) { return o == Py_None ? 64 : (int)as_long(o); }
+// Sizes of outputs follow Python's rules, as the callers see Python functions: whole numbers only, // rounds down, and a
+// division by zero is an exception.  (The library checks bits and group size too, but after the output exists.)
+int64_t as_index(PyObject* o) {
+  const Py_ssize_t v = PyNumber_AsSsize_t(o, PyExc_OverflowError);
+  if (v == -1 && PyErr_Occurred()) throw PyFail();
+  return (int64_t)v;
+}
+int64_t floor_div(int64_t a, int64_t b) {
+  if (b == 0) { PyErr_SetString(PyExc_ZeroDivisionError, "integer division or modulo by zero"); throw PyFail(); }
+  const int64_t q = a / b;
+  return a % b != 0 && (a < 0) != (b < 0) ? q - 1 : q;
+}
+int64_t bits_or_4(PyObject* o) { return o == Py_None ? 4 : as_index(o); }
+int64_t gs_or_64(PyObject* o) { return o == Py_None ? 64 : as_index(o); }
 
 void* stream() { return (void*)c10::cuda::getCurrentCUDAStream().stream(); }
 
@@ -340,7 +352,7 @@ PyObject* dequantize(Args a) {
   at::Tensor out;
   if (a[7] == Py_None) {
     Shape shp = lead(w, 1);
-    shp.push_back(w.size(-1) * 32 / bits_or_4(a[4]));
+    shp.push_back(floor_div(w.size(-1) * 32, bits_or_4(a[4])));
     out = empty(shp, w, odt);
   } else {
     out = tensor(a[7]);
@@ -357,11 +369,10 @@ PyObject* dequantize(Args a) {
 // w, group_size, bits, mode
 PyObject* quantize(Args a) {
   const at::Tensor& w = tensor(a[0]);
-  const int gs = gs_or_64(a[1]), nb = bits_or_4(a[2]);
-  const int64_t D = w.size(-1);
+  const int64_t gs = gs_or_64(a[1]), nb = bits_or_4(a[2]), D = w.size(-1);
   Shape sq = lead(w, 1), ss = sq;
-  sq.push_back(D * nb / 32);
-  ss.push_back(gs ? D / gs : 0);
+  sq.push_back(floor_div(D * nb, 32));
+  ss.push_back(floor_div(D, gs));
   at::Tensor q = empty(sq, w, at::kInt), s = empty(ss, w, at::kBFloat16), b = empty(ss, w, at::kBFloat16);
   T dq = packed(q), ds = plain(s), db = plain(b), dw = plain(w), none;
   none.none();
@@ -382,9 +393,9 @@ PyObject* kv_append(Args a) {
   return ret(Py_None);
 }
 
-at::Tensor attn_out(PyObject* out, const at::Tensor& q, int64_t Tq, const at::Tensor& vq, int bits) {
+at::Tensor attn_out(PyObject* out, const at::Tensor& q, int64_t Tq, int64_t Dv) {
   if (out != Py_None) return tensor(out);
-  return empty({q.size(0), q.size(1), Tq, vq.size(3) * 32 / bits}, q);
+  return empty({q.size(0), q.size(1), Tq, Dv}, q);
 }
 
 // q, k_triple, v_triple, bits, group_size, scale, mask_mode, mask, kv_lens, workspace, out
@@ -395,8 +406,8 @@ PyObject* kv_decode_attention(Args a) {
   const int nb = (int)as_long(a[3]), gs = (int)as_long(a[4]);
   const float scale = (float)as_double(a[5]);
   const char* mm = as_str(a[6]);
-  const int64_t B = q.size(0), Hq = q.size(1), Tq = q.size(2), Dv = vq.size(3) * 32 / nb;
-  at::Tensor out = attn_out(a[10], q, Tq, vq, nb), ws;
+  const int64_t B = q.size(0), Hq = q.size(1), Tq = q.size(2), Dv = floor_div(vq.size(3) * 32, as_index(a[3]));
+  at::Tensor out = attn_out(a[10], q, Tq, Dv), ws;
   if (a[9] == Py_None) {
     const size_t need = qb200_kv_decode_attention_workspace_size(Tq > 1 ? Tq : B, Hq, kq.size(1), kq.size(2), Dv);
     ws = empty({(int64_t)(need > 16 ? need : 16)}, q, at::kByte);
@@ -443,9 +454,10 @@ PyObject* kv_decode_attention_ptrs(Args a) {
   for (int64_t i = 0; i < B; ++i) tmax = std::max(tmax, k[0][i]->ndim > 2 ? k[0][i]->shape[2] : (int64_t)0);
   Seq v0(vl[0]);
   const at::Tensor& vq = tensor(v0[0]);
-  at::Tensor out = attn_out(a[10], q, 1, vq, nb), ws;
+  const int64_t Dv = floor_div(vq.size(3) * 32, as_index(a[3]));
+  at::Tensor out = attn_out(a[10], q, 1, Dv), ws;
   if (a[9] == Py_None) {
-    const size_t need = qb200_kv_decode_attention_ptrs_workspace_size(B, Hq, k[0][0]->shape[1], tmax, vq.size(3) * 32 / nb);
+    const size_t need = qb200_kv_decode_attention_ptrs_workspace_size(B, Hq, k[0][0]->shape[1], tmax, Dv);
     ws = empty({(int64_t)(need > 16 ? need : 16)}, q, at::kByte);
   } else {
     ws = tensor(a[9]);
