@@ -160,6 +160,10 @@ struct Seq {
     if (i >= size()) { PyErr_SetString(PyExc_IndexError, "qb200: the list is too short"); throw PyFail(); }
     return PySequence_Fast_GET_ITEM(o, i);
   }
+  // one entry for each of n sequences or matrices (a shorter list fails where its missing entry is asked for)
+  void at_most(Py_ssize_t n) const {
+    if (size() > n) { PyErr_SetString(PyExc_IndexError, "qb200: the list is too long"); throw PyFail(); }
+  }
 };
 
 // (codes, scales, biases) of every sequence as the ABI's three pointer lists.
@@ -221,6 +225,7 @@ PyObject* quantized_matmul_batch(Args a) {
   T x = plain(a[0]);
   Seq tl(a[1]), ol(a[2]);
   const Py_ssize_t n = tl.size();
+  ol.at_most(n);
   Triples w(tl, n);
   std::vector<T> y(n);
   std::vector<qb200_tensor*> yp(n);
@@ -295,7 +300,7 @@ PyObject* pack(std::initializer_list<PyObject*> items) {   // takes the referenc
 // logits, k
 PyObject* moe_route(Args a) {
   const at::Tensor& l = tensor(a[0]);
-  const long k = as_long(a[1]);
+  const int64_t k = as_index(a[1]);
   Shape s = lead(l, 1);
   s.push_back(k);
   at::Tensor inds = empty(s, l, at::kInt), scores = empty(s, l);
@@ -402,6 +407,8 @@ at::Tensor attn_out(PyObject* out, const at::Tensor& q, int64_t Tq, int64_t Dv) 
 PyObject* kv_decode_attention(Args a) {
   const at::Tensor& q = tensor(a[0]);
   Seq k(a[1]), v(a[2]);
+  for (const Seq* s : {&k, &v})
+    if (s->size() != 3) { PyErr_SetString(PyExc_ValueError, "qb200: (codes, scales, biases) were expected"); throw PyFail(); }
   const at::Tensor &kq = tensor(k[0]), &vq = tensor(v[0]);
   const int nb = (int)as_long(a[3]), gs = (int)as_long(a[4]);
   const float scale = (float)as_double(a[5]);
@@ -448,16 +455,21 @@ PyObject* kv_decode_attention_ptrs(Args a) {
   const float scale = (float)as_double(a[5]);
   const char* mm = as_str(a[6]);
   const int64_t B = q.size(0), Hq = q.size(1);
-  if (B > 0 && (kl.size() == 0 || vl.size() == 0)) { PyErr_SetString(PyExc_IndexError, "qb200: the list is too short"); throw PyFail(); }
+  kl.at_most(B);
+  vl.at_most(B);
+  Seq k0(kl[0]), v0(vl[0]);
+  const int64_t Hkv = tensor(k0[0]).size(1);
+  const at::Tensor& vq = tensor(v0[0]);
   Triples k(kl, B), v(vl, B);
   int64_t tmax = 0;
-  for (int64_t i = 0; i < B; ++i) tmax = std::max(tmax, k[0][i]->ndim > 2 ? k[0][i]->shape[2] : (int64_t)0);
-  Seq v0(vl[0]);
-  const at::Tensor& vq = tensor(v0[0]);
+  for (int64_t i = 0; i < B; ++i) {
+    if (k[0][i]->ndim < 3) { PyErr_SetString(PyExc_IndexError, "qb200: a cache view of four dimensions was expected"); throw PyFail(); }
+    tmax = std::max(tmax, k[0][i]->shape[2]);
+  }
   const int64_t Dv = floor_div(vq.size(3) * 32, as_index(a[3]));
   at::Tensor out = attn_out(a[10], q, 1, Dv), ws;
   if (a[9] == Py_None) {
-    const size_t need = qb200_kv_decode_attention_ptrs_workspace_size(B, Hq, k[0][0]->shape[1], tmax, Dv);
+    const size_t need = qb200_kv_decode_attention_ptrs_workspace_size(B, Hq, Hkv, tmax, Dv);
     ws = empty({(int64_t)(need > 16 ? need : 16)}, q, at::kByte);
   } else {
     ws = tensor(a[9]);
@@ -535,6 +547,8 @@ PyObject* swiglu(Args a) {
 PyObject* kv_append_seqs(Args a) {
   Seq kl(a[0]), vl(a[1]), ol(a[4]);
   const Py_ssize_t n = kl.size();
+  vl.at_most(n);
+  ol.at_most(n);
   Triples k(kl, n), v(vl, n);
   std::vector<int64_t> off((size_t)n);
   for (Py_ssize_t i = 0; i < n; ++i) off[i] = as_long(ol[i]);
