@@ -38,9 +38,12 @@ constexpr size_t kTiles = (size_t)12 * TILE + RAWB * RAW;
 constexpr int kBars = 2 * SMAX + 2 * RAWB + 4;
 constexpr size_t smem_of(bool grouped) { return kTiles + kBars * 8 + 48 + (grouped ? 2 * (kMaxE + 1) * 4 : 0); }
 static_assert(smem_of(true) <= 227 * 1024, "shared memory");
-// Polls of a bounded wait, and how long the hardware may hold one (ns).  With 1 ms, waits of more than a millisecond (an epilogue's at
-// K = 196608) never ended; with 20 us they do, and shorter waits cost the same.
-constexpr uint32_t kSpin = 1u << 18, kNap = 20000;
+// Limits of a bounded wait.  The time decides: how long the hardware holds a poll is its own choice below kNap, and in this kernel, where
+// other barriers of the CTA change all the time, it is 0.36 us whatever kNap says (20 us to 1 ms: 6300 polls in the 2.3 ms an epilogue
+// waits at K = 196608; a lone waiter is held for the whole of kNap).  A number of polls therefore was a limit of 1.5 ms (2^12), then of
+// 95 ms (2^18), which longer contractions outlive.
+constexpr uint32_t kPolls = 1u << 24, kNap = 20000;
+constexpr uint64_t kLimitNs = 4000000000ull;
 
 __device__ int g_pair_error = 0;                 // 0, or the code of a wait that expired
 
@@ -56,15 +59,28 @@ struct Tile {
   int row0, row_end, units, nn0, nn1;            // tokens [row0, row_end), in units of nn0 and nn1 (multiples of 32, up to 256)
   int n0, nend, wrow0, wlast;                    // output columns; first weight row of the tile, last one of the matrix
 };
-__device__ __forceinline__ bool wait_cta(uint64_t* bar, uint32_t parity) {
-  const uint32_t addr = smem_u32(bar);
-  for (uint32_t it = 0; it < kSpin; ++it) {
-    uint32_t done;
-    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-                 : "=r"(done) : "r"(addr), "r"(parity), "r"(kNap) : "memory");
-    if (done) return true;
+__device__ __forceinline__ bool poll_cta(uint32_t addr, uint32_t parity) {
+  uint32_t done;
+  asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+               : "=r"(done) : "r"(addr), "r"(parity), "r"(kNap) : "memory");
+  return done != 0;
+}
+// (out of line: the waits of the running kernel end in the loop below)
+__device__ __noinline__ bool wait_long(uint32_t addr, uint32_t parity) {
+  uint64_t t0, now;
+  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t0));
+  for (uint32_t it = 0; it < kPolls; ++it) {
+    if (poll_cta(addr, parity)) return true;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
+    if (now - t0 > kLimitNs) break;
   }
   return false;
+}
+__device__ __forceinline__ bool wait_cta(uint64_t* bar, uint32_t parity) {
+  const uint32_t addr = smem_u32(bar);
+  for (int it = 0; it < 4096; ++it)
+    if (poll_cta(addr, parity)) return true;
+  return wait_long(addr, parity);
 }
 // (a shared::cluster address)
 __device__ __forceinline__ void arrive_addr(uint32_t bar) {

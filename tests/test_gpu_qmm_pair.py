@@ -46,13 +46,33 @@ def test_sorted_rows(bits, gs, N, K, counts):
     assert qb200.lib().qb200_debug_tc_status() == 0
 
 
-def test_tile_of_more_than_a_millisecond():
-    """One tile over a contraction so long that the epilogue's wait outlives any single poll; checked against the exact sum."""
+@pytest.mark.parametrize("bits", [4, 8])
+def test_tile_of_more_than_a_millisecond(bits):
+    """One tile over a long contraction: the epilogue waits 2.3 ms.  Checked against the exact sum."""
     import qb200
     M, N, K = 257, 512, 196608
-    w = qb200.quantize(torch.randn(N, K, device="cuda", dtype=torch.bfloat16) * 0.02, 64, 4)
+    w = qb200.quantize(torch.randn(N, K, device="cuda", dtype=torch.bfloat16) * 0.02, 64, bits)
     x = torch.randn(M, K, device="cuda", dtype=torch.bfloat16)
-    y = qb200.quantized_matmul(x, *w, True, 64, 4)
+    y = qb200.quantized_matmul(x, *w, True, 64, bits)
     assert qb200.lib().qb200_debug_tc_status() == 0
-    ref = x[:64].double() @ qb200.dequantize(*w, 64, 4, dtype=torch.bfloat16).double().t()
+    ref = x[:64].double() @ qb200.dequantize(*w, 64, bits, dtype=torch.bfloat16).double().t()
     assert float((y[:64].double() - ref).norm() / ref.norm()) < 3e-3
+
+
+@pytest.mark.parametrize("bits", [4, 8])
+def test_tile_of_a_tenth_of_a_second(bits):
+    """The epilogue waits for more than 2^18 polls.  x is zero but for 96 places over the whole of K, and every product a multiple of 1/2, so
+    that the sum is exact: the result differs by its rounding to bf16 alone (2^-8 of the value)."""
+    import qb200
+    M, N, K = 257, 512, 10485760
+    g = torch.Generator(device="cuda").manual_seed(bits)
+    codes = torch.randint(-2 ** 31, 2 ** 31 - 1, (N, K * bits // 32), device="cuda", generator=g, dtype=torch.int32)
+    scales = 0.5 * torch.randint(1, 3, (N, K // 64), device="cuda", generator=g).to(torch.bfloat16)
+    x = torch.zeros(M, K, device="cuda", dtype=torch.bfloat16)
+    at = torch.linspace(0, K - 1, 96, device="cuda").long()
+    x[:, at] = torch.randint(-8, 9, (M, 96), device="cuda", generator=g).to(torch.bfloat16)
+    y = qb200.quantized_matmul(x, codes, scales, torch.zeros_like(scales), True, 64, bits)
+    assert qb200.lib().qb200_debug_tc_status() == 0
+    q = (codes[:, at * bits // 32] >> (at * bits % 32)) & (2 ** bits - 1)
+    ref = x[:, at].double() @ (q * scales[:, at // 64].float()).to(torch.bfloat16).double().t()
+    assert bool(((y.double() - ref).abs() <= 2.0 ** -8 * ref.abs()).all())
