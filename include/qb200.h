@@ -108,6 +108,9 @@ QB200_API int qb200_debug_tc_status(void);
 /* Clears that code (it is sticky: once set it stays until cleared).  A host should read the status once per step
  * after its stream synchronisation -- a non-zero code means a result of that step is incomplete -- and clear it. */
 QB200_API void qb200_debug_tc_reset(void);
+/* For tests of that: how many polls a wait of the fp16 streaming kernel takes before it gives up, in the launches of the calling
+ * thread from now on (below 0: none, so that the kernel gives up at its first wait; 0: the kernel's own limit). */
+QB200_API void qb200_debug_wait_polls(int polls);
 
 /* ---- mlx_quantized_matmul (src/mlx.zig:262) ----
  * transpose_w = true : y[..., m, n] = sum_k x[..., m, k] * What[..., n, k]

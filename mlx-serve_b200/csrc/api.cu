@@ -234,6 +234,8 @@ QB200_API void qb200_debug_tc_reset(void) {
   qmm_pair_error_reset();
 }
 
+QB200_API void qb200_debug_wait_polls(int polls) { wait_polls() = polls; }
+
 QB200_API int qb200_quantized_matmul_shape(const qb200_tensor* x, const qb200_tensor* w, const qb200_tensor* scales,
                                            bool transpose_w, qb200_optional_int group_size, qb200_optional_int bits,
                                            int64_t* out_shape, int32_t* out_ndim) {

@@ -10,6 +10,11 @@ std::mutex& setup_mutex() {
   return mu;
 }
 
+int& wait_polls() {
+  static thread_local int polls = 0;
+  return polls;
+}
+
 // Streaming multiprocessors of the current device (148 on B200).  A failed query (no device, as in a
 // host-only check of the library) answers 148 so that size queries stay deterministic.
 int sm_count() {

@@ -24,6 +24,7 @@ inline cudaError_t launch_kernel(void (*kern)(KArgs...), dim3 grid, dim3 block, 
 int report_error(int status, const char* msg);  // api.cu: last-error string + handler
 int sm_count();                                 // device.cu: SMs of the current device
 std::mutex& setup_mutex();                      // device.cu: guards every first-use-per-device set-up
+int& wait_polls();                              // device.cu: this thread's limit for the waits of the kernels that take one (0: theirs, below: none)
 
 // ---- elementwise.cu ----
 struct DequantArgs {

@@ -66,6 +66,7 @@ struct F16K {
   int gc;                  // 64-groups per CTA (the last may have fewer)
   int ct;                  // activation columns stored per n8 tile (1, 2, 4, 8)
   int stages;
+  int polls;               // of a wait, before it gives up
 };
 
 #define QB_SEL4(arr, i) ((i) == 0 ? (arr)[0] : ((i) == 1 ? (arr)[1] : ((i) == 2 ? (arr)[2] : (arr)[3])))
@@ -81,21 +82,32 @@ __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
 __device__ __forceinline__ void mbar_arrive_cp_async(uint32_t bar) {
   asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bar) : "memory");
 }
-// Bounded: after kPolls unsuccessful polls (each of them suspends for a while) the wait records `code` and gives up.
-constexpr int kPolls = 1 << 20;
+template <bool CLUSTER>
+__device__ __forceinline__ bool mbar_poll(uint32_t bar, uint32_t parity) {
+  uint32_t ok;
+  if constexpr (CLUSTER)
+    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2, %3;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                 : "=r"(ok) : "r"(bar), "r"(parity), "r"(2000u) : "memory");
+  else
+    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                 : "=r"(ok) : "r"(bar), "r"(parity), "r"(2000u) : "memory");
+  return ok != 0;
+}
+// Bounded: a wait gives up after the polls that the word `polls` in shared memory allows (the hardware holds one for 0.4 to 2 us, so the
+// default is a second or more), records `code` if it is the launch's first, and leaves 0 in the word: no wait of the CTA is long after
+// that.  The producers then leave their loops, and the consumers leave theirs together at the end of the block of rows, storing
+// nothing of it.  (A word and no register: the wider instantiations have none to spare.)
+constexpr int kPolls = 1 << 21;
 template <bool CLUSTER = false>
-__device__ __forceinline__ void mbar_wait(uint32_t bar, uint32_t parity, int code) {
-  for (int i = 0; i < kPolls; ++i) {
-    uint32_t ok;
-    if constexpr (CLUSTER)
-      asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2, %3;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-                   : "=r"(ok) : "r"(bar), "r"(parity), "r"(2000u) : "memory");
-    else
-      asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-                   : "=r"(ok) : "r"(bar), "r"(parity), "r"(2000u) : "memory");
-    if (ok) return;
-  }
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, uint32_t polls, int code) {
+  if (mbar_poll<CLUSTER>(bar, parity)) return true;
+  int n;
+  asm volatile("ld.volatile.shared.u32 %0, [%1];" : "=r"(n) : "r"(polls) : "memory");
+  for (; n > 0; --n)
+    if (mbar_poll<CLUSTER>(bar, parity)) return true;
   atomicCAS(&g_f16_error, 0, code);
+  asm volatile("st.volatile.shared.u32 [%0], %1;" ::"r"(polls), "r"(0u) : "memory");
+  return false;
 }
 __device__ __forceinline__ void consumers_sync() { asm volatile("bar.sync 1, %0;" ::"n"(kCW * 32) : "memory"); }
 __device__ __forceinline__ uint32_t lds_u16(uint32_t a) {
@@ -163,7 +175,11 @@ __global__ void __launch_bounds__(kThreads, 1) qmv_f16_kernel(const __grid_const
   uint32_t* s_max = (uint32_t*)sp; sp += 32 * 4;
   float* s_ts = (float*)sp; sp += 8 * NT * 4;
   const uint32_t full = smem_u32(sp), empty = full + 8 * NS, rx = empty + 8 * NS;
+  const uint32_t polls = rx + 16;                                       // what is left of a wait: 0 once one has run out
+  volatile int* pw = (volatile int*)(sp + 16 * NS + 16);                // (that word), and [2]: the consumers leave, by block in turn
   if (tid == 0) {
+    pw[0] = p.polls;
+    pw[1] = pw[2] = 0;
     for (int i = 0; i < NS; ++i) { mbar_init(full + 8 * i, kPW * 32); mbar_init(empty + 8 * i, kCW); }
     mbar_init(rx, kCW * cs);
     mbar_init(rx + 8, kCW * cs);
@@ -182,8 +198,9 @@ __global__ void __launch_bounds__(kThreads, 1) qmv_f16_kernel(const __grid_const
     int v = v0;
     uint32_t st = 0, ph = 1;    // stage index; parity of the wait for its previous readers (the first round passes at once)
     auto advance = [&]() { if (++st == (uint32_t)NS) { st = 0; ph ^= 1; } };
+    bool ok = true;
     Block b;
-    while (next_block(p, v, v1, b)) {
+    while (ok && next_block(p, v, v1, b)) {
       const int64_t ldw = QB_SEL4(p.ldw, b.mi) * 4, lds = QB_SEL4(p.lds, b.mi) * 2;
       const unsigned char* wsrc = (const unsigned char*)QB_SEL4(p.w, b.mi) + (size_t)k0 * BITS / 8 + (int64_t)(b.row + lr) * ldw + lc;
       const unsigned char* sbase = (const unsigned char*)QB_SEL4(p.s, b.mi);
@@ -192,7 +209,8 @@ __global__ void __launch_bounds__(kThreads, 1) qmv_f16_kernel(const __grid_const
       int64_t soff = (int64_t)(b.row + r0 + lane) * lds + (int64_t)(k0 / GS) * 2;               // of this lane's row
       const int n = b.n;
       for (int ch = 0; ch < nch; ++ch) {
-        mbar_wait(empty + 8 * st, ph, 1);
+        ok = mbar_wait(empty + 8 * st, ph, polls, 1);
+        if (!ok) break;
         const uint32_t dst = ring + st * GE::STAGE, fb = full + 8 * st;
         const int left = klen - ch * kKC;
         if (lc < left * BITS / 8) {
@@ -223,11 +241,13 @@ __global__ void __launch_bounds__(kThreads, 1) qmv_f16_kernel(const __grid_const
         advance();
       }
       // one stage slot per block is the consumers' scratch for the sums over their K shares
-      mbar_wait(empty + 8 * st, ph, 2);
+      ok = ok && mbar_wait(empty + 8 * st, ph, polls, 2);
+      if (!ok) break;
       mbar_arrive(full + 8 * st);
       advance();
     }
     asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncwarp();
     if (cs > 1) {
       asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
       cluster_sync_all();   // nobody's shared memory goes away while a peer may still write to it
@@ -389,7 +409,7 @@ __global__ void __launch_bounds__(kThreads, 1) qmv_f16_kernel(const __grid_const
   const uint32_t wlane = (uint32_t)((wr * 16 + g) * GE::PITCH + wk * GE::GB) + (GS == 32 ? (BITS == 4 ? 4 : 8) * t : (BITS == 4 ? 8 : 16) * t);
   uint32_t st = 0, ph = 0;
   auto advance = [&]() { if (++st == (uint32_t)NS) { st = 0; ph ^= 1; } };
-  int v = v0, rxn = 0;
+  int v = v0, rxn = 0;                                                // (rxn: blocks finished)
   Block b;
   while (next_block(p, v, v1, b)) {
     float acc[kTPW][NT][4];
@@ -400,7 +420,7 @@ __global__ void __launch_bounds__(kThreads, 1) qmv_f16_kernel(const __grid_const
     // scales of row g start this many bytes into the 16-byte window of the first stage (the same for rows g + 8 k)
     const uint32_t sh0 = (uint32_t)((((int64_t)(b.row + g) * QB_SEL4(p.lds, b.mi) + k0 / GS) * 2) & 15);
     for (int ch = 0; ch < nch; ++ch) {
-      mbar_wait(full + 8 * st, ph, 3);
+      mbar_wait(full + 8 * st, ph, polls, 3);
       const uint32_t sb = ring + st * GE::STAGE;
       const uint32_t sh = CB % 16 == 0 ? sh0 : ((sh0 + (uint32_t)(ch * CB)) & 15u);
       const uint32_t sa = sb + GE::W + (uint32_t)((wr * 16 + g) * kSBP) + sh;
@@ -508,7 +528,8 @@ __global__ void __launch_bounds__(kThreads, 1) qmv_f16_kernel(const __grid_const
     }
 
     // ---- the block's sums: over the warps of a tile in shared memory, over the cluster through distributed shared memory ----
-    mbar_wait(full + 8 * st, ph, 4);
+    mbar_wait(full + 8 * st, ph, polls, 4);
+    if (pw[0] == 0) pw[1 + (rxn & 1)] = 1;                    // seen by all consumers behind the barrier that they meet at next
     unsigned char* red = smem + (size_t)st * GE::STAGE;       // [wk][tile][lane] float4, one token tile at a time
     const int oc = 512 / cs;                                  // outputs of a token tile that one CTA finishes
     if (cs > 1 && rxn == 0) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
@@ -532,6 +553,7 @@ __global__ void __launch_bounds__(kThreads, 1) qmv_f16_kernel(const __grid_const
         st_cluster_f32(map_to_rank(smem_u32(slot), owner), vout[nt]);
       }
     }
+    const int out = pw[1 + (rxn & 1)];                        // (the same for all: the next block writes the other word)
     __syncwarp();
     if (lane == 0) mbar_arrive(empty + 8 * st);
     advance();
@@ -539,11 +561,11 @@ __global__ void __launch_bounds__(kThreads, 1) qmv_f16_kernel(const __grid_const
     bool mine = true;
     if (cs > 1) {
       // every warp tells every CTA of the cluster that its part has been written
-      if (lane < cs) {
+      if (lane < cs && !out) {                                // (no arrival: the peers' waits run out too)
         const uint32_t rb = map_to_rank(rx + 8 * (rxn & 1), (uint32_t)lane);
         asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(rb) : "memory");
       }
-      mbar_wait<true>(rx + 8 * (rxn & 1), (uint32_t)((rxn >> 1) & 1), 5);
+      if (!out) mbar_wait<true>(rx + 8 * (rxn & 1), (uint32_t)((rxn >> 1) & 1), polls, 5);
       mine = tid < oc;
       o = crank * oc + tid;
       if (mine) {
@@ -554,9 +576,9 @@ __global__ void __launch_bounds__(kThreads, 1) qmv_f16_kernel(const __grid_const
           vout[nt] = s;
         }
       }
-      ++rxn;
     }
     // oc is a multiple of 32 lanes and of a lane's 4 components: a warp stores or does not
+    const bool good = !out && (cs == 1 || pw[0] != 0);
     if (mine) {
       const int row = (o >> 7) * 16 + ((o & 127) >> 4) + 8 * ((o >> 1) & 1);
       void* ym = QB_SEL4(p.y, b.mi);
@@ -566,12 +588,14 @@ __global__ void __launch_bounds__(kThreads, 1) qmv_f16_kernel(const __grid_const
         const int col = nt * 8 + 2 * ((o >> 2) & 3) + (o & 1);
         if (p.x_f32) {
           const float s = vout[nt] + __shfl_xor_sync(0xffffffffu, vout[nt], 1);   // high and low part of one token
-          if (!(o & 1) && (col >> 1) < p.M && row < b.n) ((float*)ym)[(int64_t)(col >> 1) * ldy + b.row + row] = s;
-        } else if (col < p.M && row < b.n) {
+          if (!(o & 1) && (col >> 1) < p.M && row < b.n && good) ((float*)ym)[(int64_t)(col >> 1) * ldy + b.row + row] = s;
+        } else if (col < p.M && row < b.n && good) {
           ((uint16_t*)ym)[(int64_t)col * ldy + b.row + row] = f32_to_bf16_bits(vout[nt]);
         }
       }
     }
+    ++rxn;
+    if (out) break;
   }
   if (cs > 1) {
     if (rxn == 0) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
@@ -581,7 +605,7 @@ __global__ void __launch_bounds__(kThreads, 1) qmv_f16_kernel(const __grid_const
 
 size_t smem_bytes(int stage, int ns, int gc, int nt, int ct, int cs, int gs) {
   return (size_t)ns * stage + (size_t)gc * 128 * nt * ct + (size_t)((gc + kGC - 1) / kGC) * (gs == 32 ? 2 : 1) * 3 * nt * 128 +
-         (cs > 1 ? (size_t)nt * 4096 : 0) + 128 + 32 * nt + 16 * ns + 16;
+         (cs > 1 ? (size_t)nt * 4096 : 0) + 128 + 32 * nt + 16 * ns + 32;
 }
 
 // Cluster size, stages and shared memory of a launch with `cols` activation columns; false when the activations do not fit.
@@ -722,6 +746,7 @@ cudaError_t launch_qmv_f16_multi(const QmmArgs* a, int count, cudaStream_t st) {
   p.K = (int)a[0].K;
   p.ldx = a[0].ldx;
   p.x_f32 = a[0].x_dtype == QB200_FLOAT32;
+  p.polls = wait_polls() == 0 ? kPolls : (wait_polls() > 0 ? wait_polls() : 0);
   const int esz = p.x_f32 ? 4 : 2;
   const int64_t per = p.x_f32 ? 16 : 32;
   for (int64_t m0 = 0; m0 < a[0].M; m0 += per) {

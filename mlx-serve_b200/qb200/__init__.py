@@ -113,6 +113,8 @@ def lib():
         L.qb200_moe_sort_by_expert.argtypes = [TP] * 6 + [C.c_int, C.c_void_p]
         L.qb200_moe_sort_by_expert.restype = C.c_int
         L.qb200_debug_tc_reset.restype = None
+        L.qb200_debug_wait_polls.argtypes = [C.c_int]
+        L.qb200_debug_wait_polls.restype = None
         L.qb200_kv_chunk_save.argtypes = [C.c_char_p, C.c_void_p, C.c_int, C.c_int64, C.c_int64, C.c_void_p]
         L.qb200_kv_chunk_restore.argtypes = [C.c_char_p, C.c_void_p, C.c_int, C.c_int64, C.c_int64, C.c_void_p]
         L.qb200_checkpoint_open.argtypes = [C.POINTER(C.c_void_p), C.c_char_p]

@@ -41,3 +41,30 @@ def test_several_matrices_and_wide_ranges():
     y = qb200.quantized_matmul(to_dev_bf16(qo.f32_to_bf16(xn)), *dev[0], True, 64, 4)
     assert torch.isnan(y[2]).all() and torch.isfinite(y[[0, 1, 3, 4, 5]]).all()
     assert qb200.lib().qb200_debug_tc_status() == 0
+
+
+@pytest.mark.parametrize("M,N,K", [(5, 40000, 704), (16, 12000, 8896)])   # several blocks a CTA; a cluster over K, two token tiles
+def test_waits_that_run_out(M, N, K):
+    """A wait that gives up ends the launch: its status is set, nothing is stored behind it, and the next launch is as ever."""
+    import qb200
+    L = qb200.lib()
+    w = qb200.quantize(torch.randn(N, K, device="cuda", dtype=torch.bfloat16) * 0.02, 64, 4)
+    x = torch.randn(M, K, device="cuda", dtype=torch.bfloat16)
+    good = qb200.quantized_matmul(x, *w, True, 64, 4)
+    assert L.qb200_debug_tc_status() == 0
+    try:
+        for polls in (-1, 1, 2):
+            y = torch.full_like(good, float("nan"))
+            L.qb200_debug_wait_polls(polls)
+            qb200.quantized_matmul(x, *w, True, 64, 4, out=y)
+            status, done = L.qb200_debug_tc_status(), ~torch.isnan(y)
+            assert status in (201, 202, 203, 204, 205) or (polls > 0 and status == 0)
+            assert bool((y[done] == good[done]).all())
+            assert (status == 0) == bool(done.all())
+            assert polls > 0 or not bool(done.any())
+            L.qb200_debug_tc_reset()
+    finally:
+        L.qb200_debug_wait_polls(0)
+        L.qb200_debug_tc_reset()
+    assert torch.equal(qb200.quantized_matmul(x, *w, True, 64, 4), good)
+    assert L.qb200_debug_tc_status() == 0
