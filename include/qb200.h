@@ -111,6 +111,9 @@ QB200_API void qb200_debug_tc_reset(void);
 /* For tests of that: how many polls a wait of the fp16 streaming kernel takes before it gives up, in the launches of the calling
  * thread from now on (below 0: none, so that the kernel gives up at its first wait; 0: the kernel's own limit). */
 QB200_API void qb200_debug_wait_polls(int polls);
+/* For tests: launches of thread-block clusters by the calling thread are treated as refused by the device, so that the forms without
+ * clusters take their place. */
+QB200_API void qb200_debug_refuse_clusters(bool refuse);
 
 /* ---- mlx_quantized_matmul (src/mlx.zig:262) ----
  * transpose_w = true : y[..., m, n] = sum_k x[..., m, k] * What[..., n, k]

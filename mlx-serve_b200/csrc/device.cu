@@ -15,6 +15,11 @@ int& wait_polls() {
   return polls;
 }
 
+bool& refuse_clusters() {
+  static thread_local bool refuse = false;
+  return refuse;
+}
+
 // Streaming multiprocessors of the current device (148 on B200).  A failed query (no device, as in a
 // host-only check of the library) answers 148 so that size queries stay deterministic.
 int sm_count() {

@@ -24,6 +24,13 @@ inline cudaError_t launch_kernel(void (*kern)(KArgs...), dim3 grid, dim3 block, 
 int report_error(int status, const char* msg);  // api.cu: last-error string + handler
 int sm_count();                                 // device.cu: SMs of the current device
 std::mutex& setup_mutex();                      // device.cu: guards every first-use-per-device set-up
+bool& refuse_clusters();                        // device.cu: this thread's launches of clusters are refused
+// A launch with a cluster dimension, which the device may refuse where it cannot place one (a slice of a GPU, other limits).
+template <typename... KArgs, typename... Args>
+inline cudaError_t launch_clusters(const cudaLaunchConfig_t& cfg, void (*kern)(KArgs...), Args&&... args) {
+  if (refuse_clusters()) return cudaErrorLaunchOutOfResources;
+  return cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...);
+}
 int& wait_polls();                              // device.cu: this thread's limit for the waits of the kernels that take one (0: theirs, below: none)
 
 // ---- elementwise.cu ----

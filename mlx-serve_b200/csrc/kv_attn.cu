@@ -58,10 +58,10 @@ __host__ SplitPlan plan_splits(int64_t B, int64_t Hkv, int64_t T) {
 // 0.6 us of SM time when three share it; a CTA's start and end cost about one round; beyond 8 splits the partial results
 // go through memory and a merge launch (about 2.5 us).  The partials have to fit the workspace the caller was told to
 // bring, which plan_splits sized.
+__host__ int64_t f16_fit(const KvAttnArgs& a) { return (int64_t)(a.workspace_bytes / sizeof(float)) / (a.B * a.Hq * a.Tq * (2 + a.Dv)); }
 __host__ int plan_f16(const KvAttnArgs& a, int64_t qtiles, int max_fused) {
   const int64_t pairs = a.B * a.Hkv * qtiles, nsm = sm_count();
-  const int64_t rows = a.B * a.Hq * a.Tq;
-  const int64_t fit = (int64_t)(a.workspace_bytes / sizeof(float)) / (rows * (2 + a.Dv));
+  const int64_t fit = f16_fit(a);
   int64_t max_ns = (a.T + 127) / 128;
   if (max_ns > 1024) max_ns = 1024;
   int64_t best = 1;
@@ -361,7 +361,13 @@ cudaError_t launch_kv_attn(const KvAttnArgs& a, cudaStream_t st, const KvSeqTabl
     // of 4 heads fill its MMA columns) and is faster: 133 against 203 us for 16 x 32k tokens.
     // Up to 8 splits per (sequence, kv head, query tile) merge inside a cluster here too, at both code widths.
     p.nsplit = plan_f16(a, (p.gqa * a.Tq + 7) / 8, kMaxFusedSplits);
-    if (p.nsplit <= kMaxFusedSplits) return launch_kv_f16(a, p.nsplit, nullptr, nullptr, nullptr, st, seqs, true);
+    if (p.nsplit <= kMaxFusedSplits) {
+      e = launch_kv_f16(a, p.nsplit, nullptr, nullptr, nullptr, st, seqs, true);
+      if (e == cudaSuccess || p.nsplit == 1) return e;
+      (void)cudaGetLastError();   // a cluster this launch could not place: partials and the merge kernel, for as many splits as fit
+      if (p.nsplit > f16_fit(a)) p.nsplit = (int)f16_fit(a);
+      if (p.nsplit <= 1) return launch_kv_f16(a, 1, nullptr, nullptr, nullptr, st, seqs, true);   // (one split: no cluster)
+    }
     const int64_t parts = a.B * a.Hq * a.Tq * p.nsplit;
     p.part_m = ws; p.part_l = ws + parts; p.part_o = ws + 2 * parts;
     e = launch_kv_f16(a, p.nsplit, p.part_m, p.part_l, p.part_o, st, seqs, false);

@@ -609,7 +609,7 @@ cudaError_t launch_f16_inst(const F16K& p, const TAB& tab, dim3 grid, cudaStream
     attr[0].val.clusterDim.x = (unsigned)p.nsplit; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kern, p, tab);
+    return launch_clusters(cfg, kern, p, tab);
   }
   return launch_kernel(kern, grid, dim3(kWarps * 32), smem, st, p, tab);
 }

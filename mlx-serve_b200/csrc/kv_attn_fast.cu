@@ -594,7 +594,7 @@ cudaError_t launch_fast_inst(const FastK& p, const TAB& tab, dim3 grid, cudaStre
     attr[0].val.clusterDim.x = (unsigned)p.nsplit; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kv_fast_kernel<BITS, TAB>, p, tab);
+    return launch_clusters(cfg, kv_fast_kernel<BITS, TAB>, p, tab);
   }
   return launch_kernel(kv_fast_kernel<BITS, TAB>, grid, dim3(kWarps * 32), smem, st, p, tab);
 }

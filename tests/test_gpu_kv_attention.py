@@ -218,3 +218,26 @@ def test_verify_widths_with_the_causal_tail(Tq, bits, B, Hq, Hkv, T):
         gate_f32(got[:, :, tq], ref, f"verify width {Tq}, position {tq}")
     with pytest.raises(qb200.Qb200Error):
         qb200.kv_decode_attention(torch.from_numpy(q).cuda(), dk, dv, bits, 64, D ** -0.5)   # no mask mode: declined
+
+
+@pytest.fixture
+def no_clusters():
+    import qb200
+    qb200.lib().qb200_debug_refuse_clusters(True)
+    yield
+    qb200.lib().qb200_debug_refuse_clusters(False)
+
+
+@pytest.mark.parametrize("Tq,bits,B,Hq,Hkv,T", [(1, 4, 2, 14, 2, 900), (1, 8, 1, 8, 2, 700), (4, 8, 2, 28, 4, 1100), (2, 4, 1, 12, 2, 500)])
+def test_where_no_cluster_can_be_placed(no_clusters, Tq, bits, B, Hq, Hkv, T):
+    """Splits that would merge inside a cluster go through the workspace and the merge kernel: both split kernels, one token and verify
+    widths, head dims 128 and 64."""
+    if Tq > 1:
+        test_verify_widths_with_the_causal_tail(Tq, bits, B, Hq, Hkv, T)
+    else:
+        _run(np.random.default_rng(T), B, Hq, Hkv, T, 128, bits)
+        _run(np.random.default_rng(T), B, Hq, Hkv, T, 64, bits)
+
+
+def test_pointer_form_where_no_cluster_can_be_placed(no_clusters):
+    test_pointer_form_other_head_dims_and_more_than_32_sequences()
