@@ -348,17 +348,26 @@ static Ragged ragged_kernel(const QmmArgs& a) {
   return mma ? Ragged::mma : Ragged::generic;
 }
 
+// Kernels whose launch is a cluster give way to the ones that served their shapes before where the device places none.
+static bool launched(cudaError_t e) {
+  if (e == cudaSuccess) return true;
+  (void)cudaGetLastError();
+  return false;
+}
 static cudaError_t dispatch_qmm(const QmmArgs& a, cudaStream_t s) {
   if (!a.transpose) return qmv_rows_supported(a) ? launch_qmv_rows(a, s) : launch_qmm_generic(a, s);
   if (a.nbatch > 1 && qmv_shortk_supported(a)) return launch_qmv_shortk(a, s);   // one W per batch element, short K: q @ K^T
   if (takes_wide(a)) return launch_qmv_wide(a, s);
-  if (qmm_pair_supported(a)) return launch_qmm_pair(a, s);
+  if (qmm_pair_supported(a) && launched(launch_qmm_pair(a, s))) return cudaSuccess;
   if (a.M > wide_max_tokens() && a.M > 8 && qmm_tc_supported(a)) return launch_qmm_tc(a, s);
   if (a.M > 8 && !qmv_stream_supported(a) && qmm_tc_supported(a)) return launch_qmm_tc(a, s);
   if (qmv_stream_supported(a)) return launch_qmv_stream(a, s);
   switch (ragged_kernel(a)) {
     case Ragged::mma: return launch_qmv_mma(a, s);
-    case Ragged::f16: return launch_qmv_f16(a, s);
+    case Ragged::f16:
+      if (launched(launch_qmv_f16(a, s))) return cudaSuccess;
+      if (qmv_mma_supported(a)) return launch_qmv_mma(a, s);
+      break;
     case Ragged::tile: return launch_qmm_tile(a, s);
     default: break;
   }
@@ -406,8 +415,8 @@ QB200_API int qb200_quantized_matmul_batch(qb200_tensor* const* res, const qb200
     for (int i = 0; i < n && tc; ++i) tc = !empty[i] && a[i].M > wide_max_tokens() && a[i].M > 8 && !qmm_pair_supported(a[i]);
     tc = tc && qmm_tc_multi_supported(a, n);
     cudaError_t e = cudaSuccess;
-    if (f16) {
-      e = launch_qmv_f16_multi(a, n, (cudaStream_t)s);
+    if (f16 && launched(launch_qmv_f16_multi(a, n, (cudaStream_t)s))) {
+      // one launch has taken all of them
     } else if (wide) {
       e = launch_qmv_wide_multi(a, n, (cudaStream_t)s);
     } else if (tc) {
@@ -534,7 +543,7 @@ QB200_API int qb200_gather_qmm(qb200_tensor* res, const qb200_tensor* x, const q
   const bool many = a.I >= 32 * a.E && a.I >= 1024;
   // Up to 16 rows (single-token decode: every row its own expert): a CTA per (row, 16 output rows).
   if (gather_small_supported(a)) e = launch_gather_small(a, (cudaStream_t)s);
-  else if (many && gather_pair_supported(a)) e = launch_gather_pair(a, (cudaStream_t)s);
+  else if (many && gather_pair_supported(a) && launched(launch_gather_pair(a, (cudaStream_t)s))) e = cudaSuccess;
   else if (many && gather_tc_supported(a)) e = launch_gather_tc(a, (cudaStream_t)s);
   else if (gather_stream_supported(a)) e = launch_gather_stream(a, (cudaStream_t)s);
   else if (gather_tc_supported(a) && a.I >= 1024) e = launch_gather_tc(a, (cudaStream_t)s);

@@ -499,7 +499,7 @@ cudaError_t launch_inst(const CUtensorMap& xmap, const CUtensorMap& wmap, const 
   attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kern, xmap, wmap, p);
+  return launch_clusters(cfg, kern, xmap, wmap, p);
 }
 bool make_map(CUtensorMap* m, CUtensorMapDataType t, const void* base, int64_t cols, int64_t rows, int64_t pitch, int bc, int br) {
   const EncodeFn enc = get_encode();

@@ -440,7 +440,10 @@ cudaError_t launch_inst(const TileK& p, int nsplit, cudaStream_t st) {
   attr[0].val.clusterDim.x = 1; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = (unsigned)nsplit;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kern, p);
+  const cudaError_t e = launch_clusters(cfg, kern, p);
+  if (e == cudaSuccess) return e;
+  (void)cudaGetLastError();   // a cluster this launch could not place: a CTA takes the whole of K
+  return launch_kernel(kern, dim3(grid.x, grid.y), dim3(kThreads), GE::kSmem, st, p);
 }
 template <int BITS, int GS>
 cudaError_t launch_shape(const TileK& p, int tm, int nsplit, cudaStream_t st) {

@@ -680,7 +680,7 @@ cudaError_t launch_inst(const F16K& p, size_t smem, cudaStream_t st) {
   attr[1].val.clusterDim.x = p.cluster;
   cfg.attrs = attr;
   cfg.numAttrs = p.cluster > 1 ? 2 : 1;
-  return cudaLaunchKernelEx(&cfg, kern, p);
+  return p.cluster > 1 ? launch_clusters(cfg, kern, p) : cudaLaunchKernelEx(&cfg, kern, p);
 }
 template <int BITS, int NT>
 cudaError_t launch_gs(const F16K& p, int gs, size_t smem, cudaStream_t st) {

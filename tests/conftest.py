@@ -35,3 +35,11 @@ def pytest_collection_modifyitems(config, items):
     for item in items:
         if "gpu" in item.keywords:
             item.add_marker(skip)
+
+
+@pytest.fixture
+def no_clusters():
+    import qb200
+    qb200.lib().qb200_debug_refuse_clusters(True)
+    yield
+    qb200.lib().qb200_debug_refuse_clusters(False)

@@ -220,14 +220,6 @@ def test_verify_widths_with_the_causal_tail(Tq, bits, B, Hq, Hkv, T):
         qb200.kv_decode_attention(torch.from_numpy(q).cuda(), dk, dv, bits, 64, D ** -0.5)   # no mask mode: declined
 
 
-@pytest.fixture
-def no_clusters():
-    import qb200
-    qb200.lib().qb200_debug_refuse_clusters(True)
-    yield
-    qb200.lib().qb200_debug_refuse_clusters(False)
-
-
 @pytest.mark.parametrize("Tq,bits,B,Hq,Hkv,T", [(1, 4, 2, 14, 2, 900), (1, 8, 1, 8, 2, 700), (4, 8, 2, 28, 4, 1100), (2, 4, 1, 12, 2, 500)])
 def test_where_no_cluster_can_be_placed(no_clusters, Tq, bits, B, Hq, Hkv, T):
     """Splits that would merge inside a cluster go through the workspace and the merge kernel: both split kernels, one token and verify

@@ -68,3 +68,22 @@ def test_waits_that_run_out(M, N, K):
         L.qb200_debug_tc_reset()
     assert torch.equal(qb200.quantized_matmul(x, *w, True, 64, 4), good)
     assert L.qb200_debug_tc_status() == 0
+
+
+@pytest.mark.parametrize("bits,gs,M,N,K", [(4, 64, 4, 600, 20096), (8, 128, 4, 300, 19968), (4, 32, 4, 130, 19232)])
+def test_a_cluster_over_k_and_where_none_can_be_placed(bits, gs, M, N, K):
+    """Activations of that length are split over a cluster; without one the kernels before this one serve them."""
+    import qb200
+    test_any_width(bits, gs, M, N, K)
+    qb200.lib().qb200_debug_refuse_clusters(True)
+    try:
+        test_any_width(bits, gs, M, N, K)
+        rng = np.random.default_rng(K)
+        w = [make_weight(rng, (n, K), gs, bits) for n in (N, 33)]
+        x = rand_bf16(rng, (M, K))
+        y = [torch.empty((M, n), dtype=torch.float32, device="cuda") for n in (N, 33)]
+        qb200.quantized_matmul_batch(torch.from_numpy(x).cuda(), [dev_triple(*t) for t in w], y, True, gs, bits)
+        for r, t in zip(y, w):
+            gate_f32(r.cpu().numpy(), qo.qmm(x, *t, gs, bits), "several matrices")
+    finally:
+        qb200.lib().qb200_debug_refuse_clusters(False)

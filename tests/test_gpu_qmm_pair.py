@@ -76,3 +76,9 @@ def test_tile_of_a_tenth_of_a_second(bits):
     q = (codes[:, at * bits // 32] >> (at * bits % 32)) & (2 ** bits - 1)
     ref = x[:, at].double() @ (q * scales[:, at // 64].float()).to(torch.bfloat16).double().t()
     assert bool(((y.double() - ref).abs() <= 2.0 ** -8 * ref.abs()).all())
+
+
+def test_where_no_cluster_can_be_placed(no_clusters):
+    """The one-CTA kernel takes the pairs' place."""
+    test_dense(4, 64, 257, 512, 256)
+    test_sorted_rows(8, 64, 256, 512, (0, 257, 900, 31))

@@ -38,3 +38,9 @@ def test_sorted_rows(bits, gs, E, N, K, counts):
         r = qo.qmm(xf[idx == e], q[e], s[e], b[e], gs, bits)
         rms = np.sqrt(np.mean(r * r, axis=-1, keepdims=True)) + 1e-30
         assert (np.abs(y[idx == e] - r) <= np.abs(r) * 2.0 ** -8 + 1e-4 * rms).all()
+
+
+@pytest.mark.parametrize("bits,gs,M,N,K", [(4, 64, 9, 300, 4416), (8, 64, 65, 127, 704), (4, 32, 40, 260, 1056)])
+def test_where_no_cluster_can_be_placed(no_clusters, bits, gs, M, N, K):
+    """A CTA takes the whole of K."""
+    test_dense(bits, gs, M, N, K)
