@@ -111,6 +111,10 @@ QB200_API void qb200_debug_tc_reset(void);
 /* For tests of that: how many polls a wait of the fp16 streaming kernel takes before it gives up, in the launches of the calling
  * thread from now on (below 0: none, so that the kernel gives up at its first wait; 0: the kernel's own limit). */
 QB200_API void qb200_debug_wait_polls(int polls);
+/* For tests: whether a linear launched on this stream now would read its weights before the kernels ahead of it are complete.  It does
+ * only under stream capture, behind kernels of this library that write no weights; weights may come from earlier work in the stream
+ * like every other operand. */
+QB200_API bool qb200_debug_weights_settled(qb200_stream s);
 /* For tests: launches of thread-block clusters by the calling thread are treated as refused by the device, so that the forms without
  * clusters take their place. */
 QB200_API void qb200_debug_refuse_clusters(bool refuse);

@@ -79,6 +79,7 @@ pub extern "c" fn qb200_config_quantization(json_text: [*:0]const u8, bits: *c_i
 pub extern "c" fn qb200_debug_tc_status() c_int;
 pub extern "c" fn qb200_debug_tc_reset() void;
 pub extern "c" fn qb200_debug_wait_polls(polls: c_int) void;
+pub extern "c" fn qb200_debug_weights_settled(s: Stream) bool;
 pub extern "c" fn qb200_debug_refuse_clusters(refuse: bool) void;
 // expert-parallel routed-expert block (include/qb200_ep.h, libqb200_ep.so: links NCCL)
 pub extern "c" fn qb200_moe_block_ep(res: *Tensor, x: *const Tensor, inds: *const Tensor, scores: *const Tensor, w_gate: *const Tensor, s_gate: *const Tensor, b_gate: *const Tensor, w_up: *const Tensor, s_up: *const Tensor, b_up: *const Tensor, w_down: *const Tensor, s_down: *const Tensor, b_down: *const Tensor, num_experts: c_int, world: c_int, rank: c_int, comm: ?*anyopaque, capacity: i64, group_size: c_int, bits: c_int, overflow: ?*c_int, workspace: ?*anyopaque, workspace_bytes: usize, s: Stream) c_int;

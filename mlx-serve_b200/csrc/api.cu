@@ -235,6 +235,7 @@ QB200_API void qb200_debug_tc_reset(void) {
 }
 
 QB200_API void qb200_debug_wait_polls(int polls) { wait_polls() = polls; }
+QB200_API bool qb200_debug_weights_settled(qb200_stream s) { return weights_settled((cudaStream_t)s); }
 QB200_API void qb200_debug_refuse_clusters(bool refuse) { refuse_clusters() = refuse; }
 
 QB200_API int qb200_quantized_matmul_shape(const qb200_tensor* x, const qb200_tensor* w, const qb200_tensor* scales,

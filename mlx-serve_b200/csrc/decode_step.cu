@@ -302,6 +302,9 @@ __global__ void __launch_bounds__(256) turbo_rotate_kernel(const uint16_t* x, ui
 
 }  // namespace
 
+static const Reader kReaders[] = {Reader((const void*)rms_norm_kernel<true>), Reader((const void*)rms_norm_kernel<false>), Reader((const void*)rope_kernel),
+                                  Reader((const void*)swiglu_kernel<8>), Reader((const void*)swiglu_kernel<2>)};
+
 cudaError_t launch_rms_norm(const uint16_t* a, const uint16_t* b, const uint16_t* w, uint16_t* sum_out, uint16_t* norm_out,
                             int64_t rows, int d, int64_t lda, int64_t ldb, int64_t lds, int64_t ldn, float eps, cudaStream_t st) {
   if (rows <= 0 || d <= 0) return cudaSuccess;

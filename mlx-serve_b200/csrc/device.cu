@@ -1,5 +1,6 @@
 // Per-device facts the launch planners need, looked up once per device under a lock.
 #include <mutex>
+#include <set>
 
 #include "kernels.h"
 
@@ -8,6 +9,46 @@ namespace qb {
 std::mutex& setup_mutex() {
   static std::mutex mu;
   return mu;
+}
+
+namespace {
+std::mutex g_reader_mu;
+std::set<const void*>& readers() {
+  static std::set<const void*>* s = new std::set<const void*>;
+  return *s;
+}
+}  // namespace
+
+void note_reader(const void* kernel) {
+  std::lock_guard<std::mutex> lk(g_reader_mu);
+  readers().insert(kernel);
+}
+
+bool weights_settled(cudaStream_t st) {
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(st, &status) != cudaSuccess) { (void)cudaGetLastError(); return false; }
+  if (status != cudaStreamCaptureStatusActive) return false;
+  const cudaGraphNode_t* before = nullptr;
+  const cudaGraphEdgeData* edges = nullptr;
+  size_t n = 0;
+  unsigned long long id;
+  cudaGraph_t graph;
+  if (cudaStreamGetCaptureInfo_v3(st, &status, &id, &graph, &before, &edges, &n) != cudaSuccess || status != cudaStreamCaptureStatusActive) {
+    (void)cudaGetLastError();
+    return false;
+  }
+  for (size_t i = 0; i < n; ++i) {   // (none: the graph starts here, and a graph starts when all work before it is complete)
+    cudaGraphNodeType type;
+    cudaKernelNodeParams kp;
+    if (cudaGraphNodeGetType(before[i], &type) != cudaSuccess || type != cudaGraphNodeTypeKernel ||
+        cudaGraphKernelNodeGetParams(before[i], &kp) != cudaSuccess) {   // (another library's kernel may have no name here)
+      (void)cudaGetLastError();
+      return false;
+    }
+    std::lock_guard<std::mutex> lk(g_reader_mu);
+    if (!readers().count(kp.func)) return false;
+  }
+  return true;
 }
 
 int& wait_polls() {

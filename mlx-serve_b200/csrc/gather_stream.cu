@@ -87,9 +87,9 @@ __global__ void __launch_bounds__(kThreads, 1) gather_stream_kernel(GK p) {
   const uint32_t my_ring = (uint32_t)__cvta_generic_to_shared(ring + (size_t)warp * kStages * kStageBytes);
   const unsigned char* my_ring_p = ring + (size_t)warp * kStages * kStageBytes;
 
-  // The indices (and activations) may come from the previous kernel in the stream.
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  // The indices, activations and weights may come from the previous kernel in the stream.
   asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
   // ---- every CTA derives the same per-expert row counts and the prefix of their cost in tiles ----
   const int E = (int)p.E, I = (int)p.I;
@@ -622,6 +622,7 @@ cudaError_t launch_gather_stream(const GatherArgs& a, cudaStream_t st) {
   if (dev < 0 || dev >= 64 || !done[bi][dev]) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(227 * 1024 - kStaticSmem));
     if (e != cudaSuccess) return e;
+    note_reader(kern);
     if (dev >= 0 && dev < 64) done[bi][dev] = true;
   }
   }

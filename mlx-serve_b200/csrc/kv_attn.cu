@@ -302,6 +302,8 @@ __global__ void __launch_bounds__(128) kv_merge(KvK p) {
 
 }  // namespace
 
+static const Reader kMergeReader((const void*)kv_merge);
+
 cudaError_t launch_kv_fast(const KvAttnArgs& a, int nsplit, float* pm, float* pl, float* po, cudaStream_t st, const KvSeqTable* seqs,
                            bool fused);
 cudaError_t launch_kv_f16(const KvAttnArgs& a, int nsplit, float* pm, float* pl, float* po, cudaStream_t st, const KvSeqTable* seqs,

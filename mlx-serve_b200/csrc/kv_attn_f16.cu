@@ -595,6 +595,7 @@ cudaError_t launch_f16_inst(const F16K& p, const TAB& tab, dim3 grid, cudaStream
     if (dev < 0 || dev >= 64 || !done[dev]) {
       const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
       if (e != cudaSuccess) return e;
+      note_reader((const void*)kern);
       if (dev >= 0 && dev < 64) done[dev] = true;
     }
   }

@@ -580,6 +580,7 @@ cudaError_t launch_fast_inst(const FastK& p, const TAB& tab, dim3 grid, cudaStre
     if (dev < 0 || dev >= 64 || !done[dev]) {
       const cudaError_t e = cudaFuncSetAttribute(kv_fast_kernel<BITS, TAB>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
       if (e != cudaSuccess) return e;
+      note_reader((const void*)kv_fast_kernel<BITS, TAB>);
       if (dev >= 0 && dev < 64) done[dev] = true;
     }
   }

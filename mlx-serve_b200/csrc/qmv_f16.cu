@@ -19,7 +19,8 @@
 //  * The CTAs of a cluster split K over the same rows when the activations are many (they would not fit, and every CTA
 //    would convert all of them); partial sums meet through distributed shared memory, each CTA finishing its share.
 //  * Rows are dealt to the clusters evenly, to the row, across all matrices of the call: no last wave.
-//  * Programmatic dependent launch: the ring fills with weights before the wait for the previous kernel.
+//  * Programmatic dependent launch; where the host knows that the kernels before write no weights (weights_settled), the ring fills
+//    with them before the wait.
 // Measured: 5 tokens x 7211 x 2880 (4-bit) 59 us on the CUDA-core kernel before, see the dispatch rule in api.cu.  The rows
 // of a 64-row block end in a sum over eight warps (and the cluster) that stops the consumers, which is what keeps it behind
 // the ring-per-warp kernel of qmv_stream.cu at the widths both serve.
@@ -66,6 +67,7 @@ struct F16K {
   int gc;                  // 64-groups per CTA (the last may have fewer)
   int ct;                  // activation columns stored per n8 tile (1, 2, 4, 8)
   int stages;
+  int early;               // the weights may be read before the previous grid is complete
   int polls;               // of a wait, before it gives up
 };
 
@@ -191,8 +193,8 @@ __global__ void __launch_bounds__(kThreads, 1) qmv_f16_kernel(const __grid_const
 
   if (warp >= kCW) {
     // =========================== producer warps: half of a stage's rows each ===========================
-    // the next grid in the stream may be scheduled now; weights, scales and biases are no kernel's output
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    // the kernel before may have written the weights, unless the host knows better
+    if (!p.early) asm volatile("griddepcontrol.wait;" ::: "memory");
     constexpr int LPR = GE::ROWB / 16, RPI = 32 / LPR, HR = kRB / kPW;   // lanes per row, rows per copy instruction, rows per warp
     const int r0 = (warp - kCW) * HR, lr = r0 + lane / LPR, lc = (lane % LPR) * 16;
     int v = v0;
@@ -258,6 +260,7 @@ __global__ void __launch_bounds__(kThreads, 1) qmv_f16_kernel(const __grid_const
   // =========================== consumer warps ===========================
   for (int i = tid; i < ((p.gc + kGC - 1) / kGC) * SUBS * 3 * NT * 32; i += kCW * 32) ((uint32_t*)xb)[i] = 0u;
   asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
   // ---- stage the activations: one thread per 8 consecutive values of a token ----
   {
@@ -667,6 +670,7 @@ cudaError_t launch_inst(const F16K& p, size_t smem, cudaStream_t st) {
         }
         clusters_of[di][i] = n;
       }
+      note_reader((const void*)kern);
       attr_done[di] = true;
     }
   }
@@ -756,6 +760,7 @@ cudaError_t launch_qmv_f16_multi(const QmmArgs* a, int count, cudaStream_t st) {
       p.y[i] = (char*)q.y + (q.yb.offset(0) + m0 * q.ldy) * esz;
     }
     p.M = (int)((a[0].M - m0) < per ? (a[0].M - m0) : per);
+    p.early = m0 > 0 || weights_settled(st);   // (behind the first block: that block's launch is what comes before)
     int nt;
     size_t smem;
     if (!plan(p, p.M * (p.x_f32 ? 2 : 1), a[0].bits, a[0].gs, &nt, &smem)) return cudaErrorInvalidConfiguration;

@@ -78,6 +78,7 @@ struct StreamK {
   int ntl_max;        // max tiles per group (sizes the multi-pass accumulator)
   int ksplit;         // > 1: the CTAs of a cluster share their tiles and split K (partial sums meet in rank 0)
   int upc;            // K units per CTA in that mode
+  int early;          // the weights may be read before the previous grid is complete
 };
 
 __device__ __forceinline__ void group_barrier(int grp) {
@@ -214,16 +215,16 @@ __global__ void __launch_bounds__(kWarpsPerGroup * groups_for(M1) * 32, M1 ? 2 :
   }
 
   setup();
+  // Before anything is read or written, the previous grid has completed and its writes are visible; the weights of the first stages
+  // come earlier where the host knows that they are none of its writes.  Then let the next grid in the stream begin launching.
+  if (!p.early) asm volatile("griddepcontrol.wait;" ::: "memory");
 #pragma unroll
   for (int i = 0; i < kStages - 1; ++i) {
     if (prod_valid()) issue();
     cp_async_commit();
   }
-
-  // Let the next grid in the stream begin launching, then wait for the previous grid to complete (and
-  // its writes to be visible) before reading activations or writing outputs.
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   if constexpr (!M1) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 
   uint32_t c_off = 0;   // byte offset of the stage the next unit is read from
@@ -651,6 +652,7 @@ cudaError_t launch_inst(StreamK p, cudaStream_t st) {
         if (cs == 1 && covered * 100 >= sm_count() * 97) { cs = c; ctas = covered; }
       }
     }
+    note_reader((const void*)kern);
     cluster_of[di] = cs; max_ctas_of[di] = ctas; split_cluster_of[di] = scs; split_ctas_of[di] = sctas;
     attr_done[di] = true;
   }
@@ -662,8 +664,8 @@ cudaError_t launch_inst(StreamK p, cudaStream_t st) {
   size_t smem = 0;
   if (!plan_stream(p, NT, M1, &grid, &smem, &cs, cs, M1 ? 0 : max_ctas, BITS == 4 ? 256 : 128, split_cluster, split_ctas))
     return cudaErrorInvalidConfiguration;
-  // Programmatic dependent launch: this grid may start (and prefetch weights, which no kernel writes)
-  // before the previous grid in the stream has finished; it waits for that grid before touching x or y.
+  // Programmatic dependent launch: this grid may start (and, where it is known to be safe, fetch its first weights) before the
+  // previous grid in the stream has finished; it waits for that grid before touching x or y.
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid);
   cfg.blockDim = dim3(kWarpsPerGroup * groups_for(M1) * 32);
@@ -736,6 +738,7 @@ cudaError_t launch_qmv_stream_multi(const QmmArgs* a, int count, cudaStream_t st
       p.y[i] = (char*)q.y + (q.yb.offset(0) + m0 * q.ldy) * esz;
     }
     p.M = (int)((a[0].M - m0) < kMaxTok ? (a[0].M - m0) : kMaxTok);
+    p.early = m0 > 0 || weights_settled(st);   // (behind the first block: that block's launch is what comes before)
     cudaError_t e = a[0].bits == 4 ? launch_bits<4>(p, st) : launch_bits<8>(p, st);
     if (e != cudaSuccess) return e;
   }

@@ -66,6 +66,7 @@ static __device__ __align__(256) unsigned char g_wide_scratch[kScratchBytes];   
 struct PrepK {
   const uint16_t* x; unsigned char* out;
   int M, K, NT;
+  int early;   // the kernels before this one wrote no weights
   int64_t ldx;
 };
 
@@ -145,8 +146,11 @@ __device__ __forceinline__ __nv_bfloat162 bf16_bytes(uint32_t v) {
 // Token slots beyond M and K values beyond K (the last slice is padded) are written as zeros.
 template <int BITS>
 __global__ void __launch_bounds__(256) wide_prep_kernel(PrepK p) {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  // The main kernel reads weights as soon as it is let in: now, where the host knows that the kernels before this one wrote none,
+  // else when they are complete.
+  if (p.early) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const int NT = p.NT, SK = slice_k(NT), kpad = (p.K + SK - 1) / SK * SK;
   const int ppt = kpad >> 4;                                   // 16-value pieces per token
   const int idx = blockIdx.x * 256 + threadIdx.x;
@@ -284,10 +288,10 @@ __global__ void __launch_bounds__(kThreads, 1) qmv_wide_kernel(const __grid_cons
 #pragma unroll
   for (int i = 0; i < kStages - 1; ++i) { issue(); cp_async_commit(); }
 
-  // Let the next grid in the stream begin launching; wait for the previous one (the activation fragments,
-  // and whatever wrote y last) before touching anything but the weights.
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  // Wait for the previous grid (the activation fragments, and whatever wrote y last) before touching anything but the weights -- it
+  // let this one in when they could be read --, then let the next grid in the stream begin launching.
   asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   __syncthreads();   // the mbarriers are initialised
 
   // ---- activation slices: slice i of this CTA's range lives in buffer i & 1 ----
@@ -542,6 +546,7 @@ cudaError_t launch_wide_inst(const WideK& p, int grid, cudaStream_t st) {
     if (dev < 0 || dev >= 64 || !done[dev]) {
       const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_wide(NT));
       if (e != cudaSuccess) return e;
+      note_reader((const void*)kern);
       if (dev >= 0 && dev < 64) done[dev] = true;
     }
   }
@@ -613,6 +618,7 @@ cudaError_t launch_qmv_wide_multi(const QmmArgs* a, int count, cudaStream_t st) 
     pk.x = (const uint16_t*)a[0].x + (a[0].xb.offset(0) + m0 * a[0].ldx);
     pk.out = scratch;
     pk.M = M; pk.K = p.K; pk.NT = NT; pk.ldx = a[0].ldx;
+    pk.early = m0 > 0 || weights_settled(st);   // (behind the first pass: that pass's launch is what comes before)
     const int sk = slice_k(NT), kpad = (p.K + sk - 1) / sk * sk;
     const int pblocks = (NT * 8 * (kpad / 16) + 255) / 256;
     cudaLaunchConfig_t cfg = {};

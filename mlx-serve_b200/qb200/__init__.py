@@ -115,6 +115,8 @@ def lib():
         L.qb200_debug_tc_reset.restype = None
         L.qb200_debug_wait_polls.argtypes = [C.c_int]
         L.qb200_debug_wait_polls.restype = None
+        L.qb200_debug_weights_settled.argtypes = [C.c_void_p]
+        L.qb200_debug_weights_settled.restype = C.c_bool
         L.qb200_debug_refuse_clusters.argtypes = [C.c_bool]
         L.qb200_debug_refuse_clusters.restype = None
         L.qb200_kv_chunk_save.argtypes = [C.c_char_p, C.c_void_p, C.c_int, C.c_int64, C.c_int64, C.c_void_p]
