@@ -253,6 +253,9 @@ struct KvSeq {
 };
 struct KvSeqTable { KvSeq s[kMaxSeqPtrs]; };
 struct KvNoTable {};
+// How the integer kernel cuts a sequence: `cluster` CTAs hold the `ns` splits of cluster / ns (sequence, kv head) pairs.  Where ns_even
+// differs (lengths that only the device knows), the kernel takes ns_even splits from a mean length of even_from times the longest on.
+struct KvSplits { int cluster, ns, ns_even; float even_from; };
 size_t kv_attn_workspace_bytes(int64_t B, int64_t Hq, int64_t Hkv, int64_t T, int64_t Dv);
 bool kv_attn_supported(const KvAttnArgs& a);
 bool kv_fast_supported(const KvAttnArgs& a, const KvSeqTable* seqs = nullptr);   // kv_attn_fast.cu: integer MMA, D = 128, GQA <= 4, T_q = 1

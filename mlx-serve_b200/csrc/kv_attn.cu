@@ -78,26 +78,55 @@ __host__ int plan_f16(const KvAttnArgs& a, int64_t qtiles, int max_fused) {
 }
 
 // Splits of the 4-bit integer kernel where they merge inside a cluster (no partials in memory).  A CTA reads a token of one kv head
-// in 4.3 ns alone on its SM and in 7.6 ns beside a second one, plus about 6 us of start and end and 0.8 us of merge per split.  While all CTAs are resident the
-// longest sequence decides, in rounds of 512 tokens a CTA; beyond, CTAs follow one another on the places that clusters of that size can take: whole waves when all sequences are as
-// long, else one after another with half a CTA left over at the end.  `mean`: mean length / T; lengths that only the device
-// knows are taken as three quarters of the longest.
-// (Within 10 % of the times of 1 - 8 splits at 16 x 8 pairs of 32768 tokens, 5 x 8 of 9000, 32 x 8 of 3000, 12 x 2 of 16000 and
-// 40 x 8 of 16000, where the plan by whole waves gave 128 / 21 / 29 / 29 / 144 us and this one 122 / 21 / 29 / 24 / 134.)
-__host__ int plan_clusters(int64_t pairs, int64_t T, double mean) {
+// in 4.3 ns alone on its SM and in 7.6 ns beside a second one, plus about 6 us of start and end and 0.8 us of merge per split.  While
+// all CTAs are resident the longest sequence decides, in rounds of 512 tokens a CTA; beyond, CTAs follow one another on the places
+// that clusters of that size can take.  A last wave that is nearly empty costs less than half a wave, as its CTAs have their SMs to
+// themselves (27 x 8 pairs of 20992 tokens: 1.46 waves of two splits take 134 us, 0.73 of one split 164); lengths that differ
+// (`mean`: mean length / T) blur the waves.  Within 8 % (geometric mean over 1 - 8 splits) of what 15 shapes took, 16 to 320 pairs
+// of 3000 to 33280 tokens, equal or spread down to a half; its choice is within 5 % of the best of them in all.  (Counting whole
+// waves for equal lengths chose up to 23 % worse.)
+__host__ double cost_clusters(int64_t pairs, int64_t T, double mean, int cluster, int ns) {
   static const double place[8] = {1.0, 1.0, 0.943, 0.959, 0.946, 0.912, 0.875, 0.892};   // of two CTAs per SM, by cluster size
-  int best = 1;
-  double best_cost = -1.0;
-  for (int ns = 1; ns <= 8 && (ns == 1 || T / ns >= 256); ++ns) {
-    const double n = (double)pairs * ns, slots = 2.0 * sm_count() * place[ns - 1], tok = (double)T / ns, up = (double)((T + 512 * ns - 1) / (512 * ns) * 512);
-    double cost;
-    if (2.0 * n <= slots) cost = 0.0043 * up + 6.0 + 0.8 * ns;
-    else if (n <= slots) cost = 0.0076 * up + 6.0 + 0.8 * ns;
-    else if (mean > 0.95) cost = (0.0076 * up + 6.0) * (double)(int64_t)(n / slots + 0.999) + 0.8 * ns;
-    else cost = (0.0076 * mean * tok + 6.0) * (n / slots + 0.5) + 0.8 * ns;
-    if (best_cost < 0.0 || cost < best_cost - 1e-9) { best_cost = cost; best = ns; }
+  const double n = (double)pairs * ns, slots = 2.0 * sm_count() * place[cluster - 1], up = (double)((T + 512 * ns - 1) / (512 * ns) * 512);
+  if (2.0 * n <= slots) return 0.0043 * up + 6.0 + 0.8 * ns;
+  if (n <= slots) return 0.0076 * up + 6.0 + 0.8 * ns;
+  double waves = n / slots;
+  if (mean > 0.95) waves = waves + 0.15 > floor(waves) + 0.4 ? waves + 0.15 : floor(waves) + 0.4;
+  else waves += 0.4;
+  return (0.0076 * mean * (double)T / ns + 6.0) * waves + 0.8 * ns;
+}
+// `mean` 0: lengths that only the device knows.  The splits are those that lose least over lengths all alike and lengths spread evenly
+// down to half of the longest.  Equal lengths may still want fewer: the kernel then takes those when it finds the lengths alike,
+// several pairs to a cluster.  (16 x 8 pairs of 32768 tokens: 4 splits take 106 us spread and 137 equal, 2 splits 116 and 131; the
+// kernel that chooses 106 and 133.)  Finding out costs the start of every CTA a reduction over the lengths, up to 2 us of a small
+// call, so it is left out where the model gives it less than 3 % or the call takes less than 60 us.
+__host__ KvSplits plan_clusters(int64_t pairs, int64_t T, double mean) {
+  const double m_spread = mean > 0.0 ? mean : 0.75, m_even = mean > 0.0 ? mean : 1.0;
+  const bool choose = mean <= 0.0 && pairs < (1 << 24);   // (the kernel counts pairs in 32 bits)
+  double spread[9], even[9], least_spread = 1e30, least_even = 1e30;
+  int ns_even[9], count = 0;
+  for (int c = 1; c <= 8 && (c == 1 || T / c >= 256); count = c++) {
+    spread[c] = cost_clusters(pairs, T, m_spread, c, c);
+    even[c] = cost_clusters(pairs, T, m_even, c, c);
+    ns_even[c] = c;
+    if (choose && even[c] >= 60.0) {
+      const double enough = 0.97 * even[c];
+      for (int ns = 1; ns < c; ++ns) {
+        const double cost = c % ns == 0 ? cost_clusters(pairs, T, m_even, c, ns) : 1e30;
+        if (cost < enough && cost < even[c]) { even[c] = cost; ns_even[c] = ns; }
+      }
+    }
+    least_spread = spread[c] < least_spread ? spread[c] : least_spread;
+    least_even = even[c] < least_even ? even[c] : least_even;
   }
-  return best;
+  int best = 1;
+  for (int c = 2; c <= count; ++c)
+    if (spread[c] / least_spread + even[c] / least_even < spread[best] / least_spread + even[best] / least_even - 1e-9) best = c;
+  KvSplits s = {best, best, ns_even[best], 0.75f};
+  while (s.ns_even != best && s.even_from < 1.f &&
+         cost_clusters(pairs, T, s.even_from, best, best) < cost_clusters(pairs, T, s.even_from, best, s.ns_even))
+    s.even_from += 0.03125f;
+  return s;
 }
 
 struct KvK {
@@ -304,7 +333,7 @@ __global__ void __launch_bounds__(128) kv_merge(KvK p) {
 
 static const Reader kMergeReader((const void*)kv_merge);
 
-cudaError_t launch_kv_fast(const KvAttnArgs& a, int nsplit, float* pm, float* pl, float* po, cudaStream_t st, const KvSeqTable* seqs,
+cudaError_t launch_kv_fast(const KvAttnArgs& a, KvSplits splits, float* pm, float* pl, float* po, cudaStream_t st, const KvSeqTable* seqs,
                            bool fused);
 cudaError_t launch_kv_f16(const KvAttnArgs& a, int nsplit, float* pm, float* pl, float* po, cudaStream_t st, const KvSeqTable* seqs,
                           bool fused);
@@ -346,7 +375,7 @@ cudaError_t launch_kv_attn(const KvAttnArgs& a, cudaStream_t st, const KvSeqTabl
     // 4096 tokens and 132.8 against 134.0 us at 32768; 8-bit caches, whose CTAs fill an SM alone, 33.0 against 31.8 us
     // at 4096 tokens -- so only the 4-bit kernel takes the cluster form.
     if (sp.nsplit <= kMaxFusedSplits && a.bits == 4) {
-      double mean = a.kv_lens ? 0.75 : 1.0;
+      double mean = a.kv_lens ? 0.0 : 1.0;
       if (seqs) {
         mean = 0.0;
         for (int64_t b = 0; b < a.B; ++b) mean += (double)seqs->s[b].T / (double)(a.B * a.T);
@@ -355,7 +384,7 @@ cudaError_t launch_kv_attn(const KvAttnArgs& a, cudaStream_t st, const KvSeqTabl
       if (e == cudaSuccess) return e;
       (void)cudaGetLastError();   // a cluster this launch could not place: fall back to partials and the merge kernel
     }
-    e = launch_kv_fast(a, sp.nsplit, p.part_m, p.part_l, p.part_o, st, seqs, false);
+    e = launch_kv_fast(a, KvSplits{sp.nsplit, sp.nsplit, sp.nsplit, 2.f}, p.part_m, p.part_l, p.part_o, st, seqs, false);
   } else if (kv_f16_supported(a, seqs)) {
     // Head dim 64, GQA 5..8 and the verify widths.  They ran on the CUDA-core kernel before: 2 sequences x 28 query heads x 4
     // verify positions over 4099 tokens at 8 bits 858 -> 20 us, 7 x 14 heads over 22k tokens 1775 -> 38 us, head dim 64

@@ -9,7 +9,7 @@
 //
 // Organisation (HBM-bound: the packed bytes are read once, straight from the
 // strided cache views):
-//  * grid (split, kv head, sequence); 8 warps per CTA, each warp walks blocks
+//  * grid (split, kv head, sequence) -- or, where the kernel chooses the splits, (place in the cluster, cluster); 8 warps per CTA, each warp walks blocks
 //    of 128 tokens with its own online softmax and its own cp.async ring of
 //    32-token K and V stages (codes + scales + biases), so no warp waits on
 //    another for data and nothing can dead-lock.
@@ -53,9 +53,9 @@ template <int BITS> struct Geo {
 
 struct FastK {
   KvAttnArgs a;
-  int nsplit;
+  KvSplits s;
   int gqa;
-  int fused;    // the splits of a (sequence, kv head) are the CTAs of one cluster: rank 0 merges them and writes the output
+  int fused;    // the splits of a (sequence, kv head) are in one cluster: the CTA of the first merges them and writes the output
   float* part_m; float* part_l; float* part_o;
 };
 
@@ -89,15 +89,24 @@ __device__ __forceinline__ float ex2(float x) {
 }
 
 // TAB = KvSeqTable: sequence b reads its own cache view from the table; KvNoTable: one strided [B, Hkv, T, .] tensor.
-template <int BITS, class TAB>
+// CHOOSE: the kernel finds out whether the lengths are alike and takes ns_even or ns splits (a kernel of its own: its start is longer).
+template <int BITS, class TAB, bool CHOOSE>
 __global__ void __launch_bounds__(kWarps * 32, BITS == 4 ? 2 : 1) kv_fast_kernel(FastK p, const __grid_constant__ TAB tab) {
   constexpr bool PTRS = std::is_same<TAB, KvSeqTable>::value;
   using G = Geo<BITS>;
   extern __shared__ __align__(128) unsigned char smem[];
   const KvAttnArgs& a = p.a;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
-  const int split = blockIdx.x, hk = blockIdx.y;
-  const int64_t b = blockIdx.z;
+  int nsplit = p.s.ns, split = blockIdx.x, rank0 = 0, hk = blockIdx.y;   // rank0: the cluster's rank with this pair's first split
+  int64_t b = blockIdx.z;
+  bool live = true;
+  float len_sum = 0.f, len_max = 0.f;
+  if constexpr (CHOOSE) {
+    for (int i = lane; i < (int)a.B; i += 32) {
+      const float l = fminf(fmaxf((float)a.kv_lens[i], 0.f), (float)a.T);
+      len_sum += l; len_max = fmaxf(len_max, l);
+    }
+  }
 
   unsigned char* sp = smem;
   unsigned char* ring = sp;     sp += (size_t)kWarps * G::STAGES * G::STAGE_BYTES;
@@ -107,7 +116,7 @@ __global__ void __launch_bounds__(kWarps * 32, BITS == 4 ? 2 : 1) kv_fast_kernel
   // after the main loop the ring is reused for the cross-warp merge
 
   // ---- stage q * scale * log2(e) as two s8 planes per head (one warp; tiny) ----
-  if (warp == 0) {
+  auto stage_queries = [&]() {
     // item = (head h, 8-value chunk c of the 128-wide row): 4 x 16 = 64 items, two per lane
 #pragma unroll
     for (int rep = 0; rep < 2; ++rep) {
@@ -152,6 +161,29 @@ __global__ void __launch_bounds__(kWarps * 32, BITS == 4 ? 2 : 1) kv_fast_kernel
         qfrag[(grp * 2 + jm) * 32 + (2 * h + pl) * 4 + tt] = o;
       }
     }
+  };
+  if (warp == 0) stage_queries();
+  if constexpr (CHOOSE) {
+    // Lengths all alike, or nearly: fewer splits, so several pairs to a cluster.  Every warp of the grid finds the same mean; the
+    // queries above are staged for the other case meanwhile (waiting for the mean first took 2 us more, 108 against 106).
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      len_sum += __shfl_xor_sync(0xffffffffu, len_sum, o);
+      len_max = fmaxf(len_max, __shfl_xor_sync(0xffffffffu, len_max, o));
+    }
+    if (__all_sync(0xffffffffu, len_sum >= p.s.even_from * len_max * (float)a.B)) {   // (a vote, so what follows stays in uniform registers)
+      nsplit = p.s.ns_even;
+      const unsigned per = (unsigned)(p.s.cluster / nsplit), sub = (unsigned)split / (unsigned)nsplit, pairs = (unsigned)a.B * gridDim.y;
+      const unsigned first = (blockIdx.z * gridDim.y + blockIdx.y) * per;
+      if (first >= pairs) return;      // no pair is left for this cluster
+      rank0 = (int)sub * nsplit;
+      split -= rank0;
+      live = first + sub < pairs;      // a place behind the last pair: no tokens, no output
+      const unsigned pair = live ? first + sub : 0;
+      b = pair / gridDim.y; hk = (int)(pair % gridDim.y);
+      __syncwarp();
+      if (warp == 0) stage_queries();
+    }
   }
   __syncthreads();
 
@@ -178,10 +210,10 @@ __global__ void __launch_bounds__(kWarps * 32, BITS == 4 ? 2 : 1) kv_fast_kernel
     T_seq = a.T;
   }
   int64_t len = a.kv_lens ? (int64_t)a.kv_lens[b] : T_seq;
-  len = len > T_seq ? T_seq : (len < 0 ? 0 : len);
+  len = len > T_seq ? T_seq : (len < 0 || !live ? 0 : len);
   // every sequence is cut by its own length, so that the CTAs of a ragged batch carry even shares (16 sequences of 16k to
   // 32k tokens at 4 bits took as long as 16 of 32k when the cut was made for the longest)
-  const int64_t tps = ((len + p.nsplit - 1) / p.nsplit + kBlockTok - 1) / kBlockTok * kBlockTok;
+  const int64_t tps = ((len + nsplit - 1) / nsplit + kBlockTok - 1) / kBlockTok * kBlockTok;
   const int64_t t_begin = (int64_t)split * tps;
   int64_t t_end = t_begin + tps;
   t_end = t_end > len ? len : t_end;
@@ -504,23 +536,23 @@ __global__ void __launch_bounds__(kWarps * 32, BITS == 4 ? 2 : 1) kv_fast_kernel
       co[i] = Ov;
       if (e == 0) { cm[h] = M; cl[h] = L; }
     } else {
-      const int64_t pi = (b * a.Hq + hk * p.gqa + h) * p.nsplit + split;
+      const int64_t pi = (b * a.Hq + hk * p.gqa + h) * nsplit + split;
       p.part_o[pi * kD + e] = Ov;
       if (e == 0) { p.part_m[pi] = M * 0.6931471805599453f; p.part_l[pi] = L; }  // natural-log domain for the merge
     }
   }
   if (p.fused) {
     // out = (sum_r o_r w_r) / (sum_r l_r w_r), w_r = 2^(m_r - max m)  (src/transformer.zig:5194-5203), r over the cluster
-    if (p.nsplit > 1) cluster_sync_all(); else __syncthreads();
-    if (split == 0) {   // the cluster spans the grid's x dimension: its rank is the split index
+    if (p.s.cluster > 1) cluster_sync_all(); else __syncthreads();
+    if (split == 0 && live) {   // the cluster spans the grid's x dimension
       const uint32_t cm_s = (uint32_t)__cvta_generic_to_shared(cm), cl_s = (uint32_t)__cvta_generic_to_shared(cl),
                      co_s = (uint32_t)__cvta_generic_to_shared(co);
       for (int i = tid; i < p.gqa * kD; i += kWarps * 32) {
         const int h = i / kD, e = i - h * kD;
         float M = kNegBig;
-        for (int r = 0; r < p.nsplit; ++r) M = fmaxf(M, ld_cluster_f32(map_to_rank(cm_s + 4u * h, (uint32_t)r)));
+        for (int r = rank0; r < rank0 + nsplit; ++r) M = fmaxf(M, ld_cluster_f32(map_to_rank(cm_s + 4u * h, (uint32_t)r)));
         float L = 0.f, Ov = 0.f;
-        for (int r = 0; r < p.nsplit; ++r) {
+        for (int r = rank0; r < rank0 + nsplit; ++r) {
           const float wgt = ex2(ld_cluster_f32(map_to_rank(cm_s + 4u * h, (uint32_t)r)) - M);
           L += ld_cluster_f32(map_to_rank(cl_s + 4u * h, (uint32_t)r)) * wgt;
           Ov += ld_cluster_f32(map_to_rank(co_s + 4u * i, (uint32_t)r)) * wgt;
@@ -531,7 +563,7 @@ __global__ void __launch_bounds__(kWarps * 32, BITS == 4 ? 2 : 1) kv_fast_kernel
         else ((uint16_t*)a.out)[off] = f32_to_bf16_bits(v);
       }
     }
-    if (p.nsplit > 1) cluster_sync_all();   // the other ranks' shared memory stays alive until rank 0 has read it
+    if (p.s.cluster > 1) cluster_sync_all();   // the other ranks' shared memory stays alive until rank 0 has read it
   }
 }
 
@@ -569,7 +601,7 @@ bool kv_fast_supported(const KvAttnArgs& a, const KvSeqTable* seqs) {
 }
 
 namespace {
-template <int BITS, class TAB>
+template <int BITS, class TAB, bool CHOOSE = false>
 cudaError_t launch_fast_inst(const FastK& p, const TAB& tab, dim3 grid, cudaStream_t st) {
   const size_t smem = (size_t)kWarps * (Geo<BITS>::STAGES * Geo<BITS>::STAGE_BYTES + Geo<BITS>::SB_BYTES) + 4 * 32 * 8 + 64;
   static bool done[64] = {};
@@ -578,13 +610,13 @@ cudaError_t launch_fast_inst(const FastK& p, const TAB& tab, dim3 grid, cudaStre
   {
     std::lock_guard<std::mutex> setup_lk(setup_mutex());   // first use on a device, from any thread
     if (dev < 0 || dev >= 64 || !done[dev]) {
-      const cudaError_t e = cudaFuncSetAttribute(kv_fast_kernel<BITS, TAB>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+      const cudaError_t e = cudaFuncSetAttribute(kv_fast_kernel<BITS, TAB, CHOOSE>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
       if (e != cudaSuccess) return e;
-      note_reader((const void*)kv_fast_kernel<BITS, TAB>);
+      note_reader((const void*)kv_fast_kernel<BITS, TAB, CHOOSE>);
       if (dev >= 0 && dev < 64) done[dev] = true;
     }
   }
-  if (p.fused && p.nsplit > 1) {
+  if (p.fused && p.s.cluster > 1) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = dim3(kWarps * 32);
@@ -592,22 +624,23 @@ cudaError_t launch_fast_inst(const FastK& p, const TAB& tab, dim3 grid, cudaStre
     cfg.stream = st;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = (unsigned)p.nsplit; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+    attr[0].val.clusterDim.x = (unsigned)p.s.cluster; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return launch_clusters(cfg, kv_fast_kernel<BITS, TAB>, p, tab);
+    return launch_clusters(cfg, kv_fast_kernel<BITS, TAB, CHOOSE>, p, tab);
   }
-  return launch_kernel(kv_fast_kernel<BITS, TAB>, grid, dim3(kWarps * 32), smem, st, p, tab);
+  return launch_kernel(kv_fast_kernel<BITS, TAB, CHOOSE>, grid, dim3(kWarps * 32), smem, st, p, tab);
 }
 }  // namespace
 
-cudaError_t launch_kv_fast(const KvAttnArgs& a, int nsplit, float* pm, float* pl, float* po,
+cudaError_t launch_kv_fast(const KvAttnArgs& a, KvSplits splits, float* pm, float* pl, float* po,
                            cudaStream_t st, const KvSeqTable* seqs, bool fused) {
   FastK p;
-  p.a = a; p.nsplit = nsplit; p.gqa = (int)(a.Hq / a.Hkv);
+  p.a = a; p.s = splits; p.gqa = (int)(a.Hq / a.Hkv);
   p.fused = fused ? 1 : 0;
   p.part_m = pm; p.part_l = pl; p.part_o = po;
-  const dim3 grid((unsigned)nsplit, (unsigned)a.Hkv, (unsigned)a.B);
+  const dim3 grid((unsigned)splits.cluster, (unsigned)a.Hkv, (unsigned)a.B);
+  if (splits.ns != splits.ns_even) return launch_fast_inst<4, KvNoTable, true>(p, KvNoTable{}, grid, st);
   if (seqs) return a.bits == 4 ? launch_fast_inst<4, KvSeqTable>(p, *seqs, grid, st) : launch_fast_inst<8, KvSeqTable>(p, *seqs, grid, st);
   return a.bits == 4 ? launch_fast_inst<4, KvNoTable>(p, KvNoTable{}, grid, st) : launch_fast_inst<8, KvNoTable>(p, KvNoTable{}, grid, st);
 }

@@ -233,3 +233,30 @@ def test_where_no_cluster_can_be_placed(no_clusters, Tq, bits, B, Hq, Hkv, T):
 
 def test_pointer_form_where_no_cluster_can_be_placed(no_clusters):
     test_pointer_form_other_head_dims_and_more_than_32_sequences()
+
+
+@pytest.mark.parametrize("B,Hkv,T", [(255, 1, 6656), (125, 1, 12800), (83, 1, 26112), (63, 1, 33280)])
+def test_splits_follow_the_lengths_on_the_device(B, Hkv, T):
+    """4-bit integer kernel, shapes where lengths all alike and spread lengths want other splits (odd numbers of pairs: a cluster of
+    several pairs is not always full).  Equal lengths on the device run as if no lengths were given; all others as each sequence alone."""
+    import qb200
+    g = torch.Generator(device="cuda").manual_seed(B + T)
+    D, Hq = 128, 4 * Hkv
+    kt, vt = _device_cache(g, B, Hkv, T, D, 4)
+    q = torch.randn((B, Hq, 1, D), device="cuda", generator=g)
+    run = lambda lens: qb200.kv_decode_attention(q, kt, vt, 4, 64, D ** -0.5, kv_lens=lens)  # noqa: E731
+    assert torch.equal(run(torch.full((B,), T, dtype=torch.int32, device="cuda")), run(None))
+    ragged = torch.randint(T // 2, T + 1, (B,), device="cuda", generator=g).to(torch.int32)
+    ragged[0] = T
+    skewed = torch.randint(0, 90, (B,), device="cuda", generator=g).to(torch.int32)
+    skewed[B // 2] = T
+    for lens in (ragged, skewed, torch.zeros_like(ragged)):
+        got = run(lens)
+        assert not torch.isnan(got).any()
+        for b, n in enumerate(lens.tolist()):
+            if n == 0:
+                assert not got[b].any()
+                continue
+            one = qb200.kv_decode_attention(q[b:b + 1], [t[b:b + 1, :, :n] for t in kt], [t[b:b + 1, :, :n] for t in vt], 4, 64, D ** -0.5)
+            # p * v_scale enters the integer tensor cores as 15-bit fixed point per 128-token block
+            assert float((got[b] - one[0]).abs().max()) <= 5e-3 * float(one.pow(2).mean().sqrt())
