@@ -54,10 +54,13 @@ __host__ SplitPlan plan_splits(int64_t B, int64_t Hkv, int64_t T) {
 }
 
 // Splits of the fp16 tensor-core kernel.  Three CTAs of 4 warps live on an SM; a CTA's warps take the 64-token blocks of its
-// split in turn, so a round of a CTA is 256 tokens.  A round costs about 0.9 us in a CTA that has its SM to itself and
-// 0.6 us of SM time when three share it; a CTA's start and end cost about one round; beyond 8 splits the partial results
-// go through memory and a merge launch (about 2.5 us).  The partials have to fit the workspace the caller was told to
-// bring, which plan_splits sized.
+// split in turn, so a round of a CTA is 256 tokens, and one with fewer blocks than warps counts half for what it lacks.  At head dim 128 and 4 bits a round
+// takes 2.4 us in a CTA that has its SM to itself, 3.2 beside a second one and 4.2 among three (0.55 of that at head dim 64, 1.1 at 8 bits); a CTA's start and end
+// take 5 us, the merge of a cluster 0.6 and 0.2 for each split.  Beyond 8 splits the partial results go through memory and a merge launch (1.5 us).  The partials have to fit the workspace the caller was told to
+// bring, which plan_splits sized.  Within 8 % (geometric mean) of what 28 shapes take at 1 - 20 splits, 4 to 256 pairs of 500 to
+// 32768 tokens; the choice is the best of them or within 1 % for all but the longest verify batch (16 x 16 pairs of 32768: 390 us
+// against 351) and 500 tokens at head dim 64 (6.5 against 5.9).  2 sequences x 28 heads x 4 verify positions over 4099 tokens:
+// 20.5 us at 6 splits, 19.1 at 8.
 __host__ int64_t f16_fit(const KvAttnArgs& a) { return (int64_t)(a.workspace_bytes / sizeof(float)) / (a.B * a.Hq * a.Tq * (2 + a.Dv)); }
 __host__ int plan_f16(const KvAttnArgs& a, int64_t qtiles, int max_fused) {
   const int64_t pairs = a.B * a.Hkv * qtiles, nsm = sm_count();
@@ -67,11 +70,11 @@ __host__ int plan_f16(const KvAttnArgs& a, int64_t qtiles, int max_fused) {
   int64_t best = 1;
   double best_cost = -1.0;
   for (int64_t ns = 1; ns <= max_ns && (ns <= max_fused || ns <= fit); ++ns) {
-    const double rounds = (double)((((a.T + ns - 1) / ns + 63) / 64 + 3) / 4) + 1.0;
-    const int64_t per_sm = (pairs * ns + nsm - 1) / nsm, full = per_sm / 3, rest = per_sm % 3;
-    double cost = (double)full * rounds * 1.8;
-    if (rest) cost += rounds * (rest == 1 ? 0.9 : 1.3);
-    if (ns > max_fused) cost += 2.5;
+    const int64_t blocks = ((a.T + ns - 1) / ns + 63) / 64, per_sm = (pairs * ns + nsm - 1) / nsm, full = per_sm / 3, rest = per_sm % 3;
+    const double rounds = (0.5 * (double)((blocks + 3) / 4) + 0.125 * (double)blocks) * (a.D == 64 ? 0.55 : 1.0) * (a.bits == 8 ? 1.1 : 1.0);
+    double cost = (double)full * (4.2 * rounds + 5.0) + (ns > 1 ? 0.6 : 0.0) + 0.2 * (double)(ns < max_fused ? ns : max_fused);
+    if (rest) cost += (rest == 1 ? 2.4 : 3.2) * rounds + 5.0;
+    if (ns > max_fused) cost += 1.5;
     if (best_cost < 0.0 || cost < best_cost - 1e-9) { best_cost = cost; best = ns; }
   }
   return (int)best;
