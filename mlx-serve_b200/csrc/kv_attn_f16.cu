@@ -70,14 +70,6 @@ struct F16K {
   float* part_m; float* part_l; float* part_o;
 };
 
-// Two 16x16 byte matrices, transposed: lanes 0-15 give the row addresses of the first, 16-31 of the
-// second.  Lane (g, t) receives for each matrix: r0 = rows 4t..4t+3 of byte column g, r1 = of column g+8.
-__device__ __forceinline__ void ldmatrix_b8_trans_x2(uint32_t (&r)[4], uint32_t addr) {
-  asm volatile("ldmatrix.sync.aligned.m16n16.x2.trans.shared.b8 {%0,%1,%2,%3}, [%4];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
-               : "r"(addr));
-}
-
 // 16-byte chunk swizzle of a stage row: the score phase reads 8 consecutive rows, the value phase rows {0,8,1,9,..}; with
 // this both take the fewest shared-memory wavefronts at every row size.
 template <int CH> __device__ __forceinline__ int swz(int row) {
@@ -85,11 +77,6 @@ template <int CH> __device__ __forceinline__ int swz(int row) {
   if (CH >= 4) f |= ((row >> 1) & 1) << 1;
   if (CH >= 8) f |= (row & 1) << 2;
   return f;
-}
-__device__ __forceinline__ float ex2(float x) {
-  float y;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
 }
 // x = hi + lo: hi is x with the mantissa cut to fp16's, lo the exact rest; both packed in pairs (a in the low half)
 __device__ __forceinline__ void split2(float a, float b, uint32_t& hi, uint32_t& lo) {

@@ -59,14 +59,6 @@ struct FastK {
   float* part_m; float* part_l; float* part_o;
 };
 
-// Two 16x16 byte matrices, transposed: lanes 0-15 give the row addresses of the first, 16-31 of the
-// second.  Lane (g, t) receives for each matrix: r0 = rows 4t..4t+3 of byte column g, r1 = of column g+8.
-__device__ __forceinline__ void ldmatrix_b8_trans_x2(uint32_t (&r)[4], uint32_t addr) {
-  asm volatile("ldmatrix.sync.aligned.m16n16.x2.trans.shared.b8 {%0,%1,%2,%3}, [%4];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
-               : "r"(addr));
-}
-
 // 16-byte chunk swizzle of a stage row; keeps both the 64/128-bit fragment reads of the score phase and
 // the ldmatrix row reads of the value phase at the minimum number of shared-memory wavefronts.
 template <int BITS> __device__ __forceinline__ int swz(int row) {
@@ -81,11 +73,6 @@ __device__ __forceinline__ int fix15(float x, float up) {
 }
 __device__ __forceinline__ uint32_t plane_byte(int v, int plane) {
   return plane == 0 ? (uint32_t)((v >> 7) & 0xFF) : (uint32_t)(v & 127);
-}
-__device__ __forceinline__ float ex2(float x) {
-  float y;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
 }
 
 // TAB = KvSeqTable: sequence b reads its own cache view from the table; KvNoTable: one strided [B, Hkv, T, .] tensor.

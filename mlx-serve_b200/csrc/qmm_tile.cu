@@ -61,11 +61,10 @@ __device__ __forceinline__ void expand4(uint32_t w, uint32_t (&o)[4]) {
 #pragma unroll
   for (int i = 0; i < 4; ++i) o[i] = lop3_and_or(w >> (4 * i), 0x000F000Fu, 0x43004300u);
 }
-// 8 bits: the pairs (0, 2) and (1, 3) of the word as integers 0..255, exact in bf16: 128 + the low seven bits, minus 128 where
-// the top bit is clear (0x80 * 0x186 = 0xC300 = -128)
-__device__ __forceinline__ uint32_t bf16_of_bytes(uint32_t v) {
-  const uint32_t a = lop3_and_or(v, 0x007F007Fu, 0x43004300u), b = ((v & 0x00800080u) ^ 0x00800080u) * 0x186u;
-  const __nv_bfloat162 r = __hadd2(*(const __nv_bfloat162*)&a, *(const __nv_bfloat162*)&b);
+
+// 8 bits: the pairs (0, 2) and (1, 3) of the word as integers 0..255
+__device__ __forceinline__ uint32_t byte_pair(uint32_t v) {
+  const __nv_bfloat162 r = bf16_of_bytes(v);
   return *(const uint32_t*)&r;
 }
 
@@ -296,7 +295,7 @@ __global__ void __launch_bounds__(kThreads, 2) qmm_tile_kernel(const __grid_cons
             }
           } else {
 #pragma unroll
-            for (int k = 0; k < 4; ++k) { A[m][k][h] = bf16_of_bytes(w[k] & 0x00FF00FFu); A[m][k][2 + h] = bf16_of_bytes((w[k] >> 8) & 0x00FF00FFu); }
+            for (int k = 0; k < 4; ++k) { A[m][k][h] = byte_pair(w[k] & 0x00FF00FFu); A[m][k][2 + h] = byte_pair((w[k] >> 8) & 0x00FF00FFu); }
           }
           const uint16_t* sq = (const uint16_t*)(sb_p + (blk & 1) * 2 * GE::SB) + row * 8 + in * H;
 #pragma unroll

@@ -91,13 +91,6 @@ __device__ __forceinline__ int mat_of_tile(const WideK& p, int tile) {
   return mi;
 }
 
-__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count));
-}
-__device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
-}
 // Bounded wait; false when the limit expired.
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
   const uint32_t addr = smem_u32(bar);
@@ -134,12 +127,6 @@ __device__ __forceinline__ void mma_bf16(float (&d)[4], uint32_t a0, uint32_t a1
 // word.  4 bits: (w >> 4i) & 0x000F000F = codes (i, i + 4); 8 bits: bytes (r, r + 2).
 template <int BITS> __host__ __device__ constexpr int kofs(int m, int r, int e) {
   return BITS == 4 ? 8 * (m >> 1) + 2 * (m & 1) + r + 4 * e : 4 * m + r + 2 * e;
-}
-// bytes 0 and 2 as exact bf16 integers: 128 + the low seven bits, minus 128 where the top bit is clear
-// (0x80 * 0x186 = 0xC300 = -128)
-__device__ __forceinline__ __nv_bfloat162 bf16_bytes(uint32_t v) {
-  const uint32_t lo = lop3_and_or(v, 0x007F007Fu, 0x43004300u), hi = ((v & 0x00800080u) ^ 0x00800080u) * 0x186u;
-  return __hadd2(*(const __nv_bfloat162*)&lo, *(const __nv_bfloat162*)&hi);
 }
 
 // ---- activations -> bf16 B fragments in slices, one thread per (token slot, 16 K values) ----
@@ -404,8 +391,8 @@ __global__ void __launch_bounds__(kThreads, 1) qmv_wide_kernel(const __grid_cons
           for (int m = 0; m < 4; ++m) {   // word m holds codes 4m .. 4m + 3: pairs (4m, 4m + 2) and (4m + 1, 4m + 3)
 #pragma unroll
             for (int r = 0; r < 2; ++r) {
-              const __nv_bfloat162 vl = __hfma2(bf16_bytes(r ? wlv[m] >> 8 : wlv[m]), s2l, b2l);
-              const __nv_bfloat162 vh = __hfma2(bf16_bytes(r ? whv[m] >> 8 : whv[m]), s2h, b2h);
+              const __nv_bfloat162 vl = __hfma2(bf16_of_bytes(r ? wlv[m] >> 8 : wlv[m]), s2l, b2l);
+              const __nv_bfloat162 vh = __hfma2(bf16_of_bytes(r ? whv[m] >> 8 : whv[m]), s2h, b2h);
               A[m][2 * r] = *(const uint32_t*)&vl;
               A[m][2 * r + 1] = *(const uint32_t*)&vh;
             }

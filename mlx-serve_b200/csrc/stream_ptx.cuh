@@ -102,4 +102,18 @@ __device__ __forceinline__ float fmax_nan(float a, float b) {
 __device__ __forceinline__ bool nonfinite(float mx) { return ((__float_as_uint(mx) >> 23) & 0xFF) == 0xFF; }
 __device__ __forceinline__ float poison_if(bool bad, float v) { return bad ? __uint_as_float(0x7FC00000u) : v; }
 
+// ---- attention: transposed byte matrices, the exponential of the softmax ----
+// Two 16x16 byte matrices, transposed: lanes 0-15 give the row addresses of the first, 16-31 of the
+// second.  Lane (g, t) receives for each matrix: r0 = rows 4t..4t+3 of byte column g, r1 = of column g+8.
+__device__ __forceinline__ void ldmatrix_b8_trans_x2(uint32_t (&r)[4], uint32_t addr) {
+  asm volatile("ldmatrix.sync.aligned.m16n16.x2.trans.shared.b8 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(addr));
+}
+__device__ __forceinline__ float ex2(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+
 }  // namespace qb

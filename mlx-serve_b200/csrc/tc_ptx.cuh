@@ -11,16 +11,6 @@ namespace qb {
 
 constexpr uint32_t kSpinLimit = 1u << 24;
 
-__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count));
-}
-__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-__device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
-}
 // Bounded wait; returns false when the limit expired.
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
   const uint32_t addr = smem_u32(bar);
@@ -144,10 +134,7 @@ __device__ __forceinline__ void dequant_half(const uint32_t* codes, uint32_t sb2
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         const uint32_t w = codes[2 * c + (j >> 1)], v = __byte_perm(w, 0, j & 1 ? 0x4342 : 0x4140);   // two codes in 16-bit halves
-        // exact bf16 integers: 128 + the low seven bits, minus 128 where the top bit is clear (0x80 * 0x186 = 0xC300 = -128)
-        const uint32_t lo = (v & 0x007F007Fu) | 0x43004300u, hi = ((v & 0x00800080u) ^ 0x00800080u) * 0x186u;
-        __nv_bfloat162 q = __hadd2(*(const __nv_bfloat162*)&lo, *(const __nv_bfloat162*)&hi);
-        q = __hfma2(q, s2, b2);       // q*s + b, rounded once
+        const __nv_bfloat162 q = __hfma2(bf16_of_bytes(v), s2, b2);       // q*s + b, rounded once
         o[j] = *(uint32_t*)&q;
       }
       *(uint4*)(row + (xr ^ (c << 4))) = make_uint4(o[0], o[1], o[2], o[3]);
