@@ -119,7 +119,7 @@ __global__ void __launch_bounds__(256) rope_kernel(const uint16_t* x, uint16_t* 
 }
 
 // silu(gate) * up with the rounding points of the reference's fused kernel (src/transformer.zig:19842-19851): the
-// sigmoid of the bf16 gate from a table over all bf16 patterns, g * sig rounded, then * up rounded.
+// sigmoid of the bf16 gate rounded to bf16 (computed: sigmoid_bf16), g * sig rounded, then * up rounded.
 __device__ __forceinline__ uint32_t swiglu2(uint32_t gv, uint32_t uv) {
   const float g0 = bf16lo(gv), g1 = bf16hi(gv);
   return pack2(rbf16(g0 * sigmoid_bf16(g0)) * bf16lo(uv), rbf16(g1 * sigmoid_bf16(g1)) * bf16hi(uv));

@@ -452,7 +452,7 @@ __global__ void __launch_bounds__(128) moe_route_kernel(MoeRouteArgs a) {
 
 template <bool F32>
 cudaError_t route_dispatch(const MoeRouteArgs& a, cudaStream_t st) {
-  const int warps = a.T >= 4 * 148 ? 4 : 1;   // few rows: a CTA each, so that every one has an SM to itself
+  const int warps = a.T >= 4 * sm_count() ? 4 : 1;   // few rows: a CTA each, so that every one has an SM to itself
   const unsigned blocks = (unsigned)((a.T + warps - 1) / warps);
   if (a.E <= 128) moe_route_kernel<F32, 4><<<blocks, warps * 32, 0, st>>>(a);
   else if (a.E <= 256) moe_route_kernel<F32, 8><<<blocks, warps * 32, 0, st>>>(a);

@@ -136,7 +136,7 @@ cudaError_t launch_qmv_f16_multi(const QmmArgs* a, int count, cudaStream_t st); 
 int qmv_f16_error_code();     // 0, or the code of a bounded wait that expired
 void qmv_f16_error_reset();
 
-// ---- qmm_tile.cu : tiled form with the fp32 weight term, any multiple of the group size, more than 32 tokens; rows sorted by expert ----
+// ---- qmm_tile.cu : tiled form with the fp32 weight term, any multiple of the group size, more than 4 tokens; rows sorted by expert ----
 bool qmm_tile_supported(const QmmArgs& a);
 cudaError_t launch_qmm_tile(const QmmArgs& a, cudaStream_t st);
 struct GatherArgs;
@@ -256,6 +256,8 @@ struct KvNoTable {};
 // How the integer kernel cuts a sequence: `cluster` CTAs hold the `ns` splits of cluster / ns (sequence, kv head) pairs.  Where ns_even
 // differs (lengths that only the device knows), the kernel takes ns_even splits from a mean length of even_from times the longest on.
 struct KvSplits { int cluster, ns, ns_even; float even_from; };
+struct KvPlaces { int n[9]; };
+KvPlaces kv_fast_places();   // kv_attn_fast.cu: CTAs of the 4-bit kernel that the device holds at once, by cluster size (1 - 8)
 size_t kv_attn_workspace_bytes(int64_t B, int64_t Hq, int64_t Hkv, int64_t T, int64_t Dv);
 bool kv_attn_supported(const KvAttnArgs& a);
 bool kv_fast_supported(const KvAttnArgs& a, const KvSeqTable* seqs = nullptr);   // kv_attn_fast.cu: integer MMA, D = 128, GQA <= 4, T_q = 1

@@ -88,9 +88,8 @@ __host__ int plan_f16(const KvAttnArgs& a, int64_t qtiles, int max_fused) {
 // (`mean`: mean length / T) blur the waves.  Within 8 % (geometric mean over 1 - 8 splits) of what 15 shapes took, 16 to 320 pairs
 // of 3000 to 33280 tokens, equal or spread down to a half; its choice is within 5 % of the best of them in all.  (Counting whole
 // waves for equal lengths chose up to 23 % worse.)
-__host__ double cost_clusters(int64_t pairs, int64_t T, double mean, int cluster, int ns) {
-  static const double place[8] = {1.0, 1.0, 0.943, 0.959, 0.946, 0.912, 0.875, 0.892};   // of two CTAs per SM, by cluster size
-  const double n = (double)pairs * ns, slots = 2.0 * sm_count() * place[cluster - 1], up = (double)((T + 512 * ns - 1) / (512 * ns) * 512);
+__host__ double cost_clusters(const KvPlaces& places, int64_t pairs, int64_t T, double mean, int cluster, int ns) {
+  const double n = (double)pairs * ns, slots = places.n[cluster], up = (double)((T + 512 * ns - 1) / (512 * ns) * 512);
   if (2.0 * n <= slots) return 0.0043 * up + 6.0 + 0.8 * ns;
   if (n <= slots) return 0.0076 * up + 6.0 + 0.8 * ns;
   double waves = n / slots;
@@ -105,17 +104,18 @@ __host__ double cost_clusters(int64_t pairs, int64_t T, double mean, int cluster
 // call, so it is left out where the model gives it less than 3 % or the call takes less than 60 us.
 __host__ KvSplits plan_clusters(int64_t pairs, int64_t T, double mean) {
   const double m_spread = mean > 0.0 ? mean : 0.75, m_even = mean > 0.0 ? mean : 1.0;
+  const KvPlaces places = kv_fast_places();
   const bool choose = mean <= 0.0 && pairs < (1 << 24);   // (the kernel counts pairs in 32 bits)
   double spread[9], even[9], least_spread = 1e30, least_even = 1e30;
   int ns_even[9], count = 0;
   for (int c = 1; c <= 8 && (c == 1 || T / c >= 256); count = c++) {
-    spread[c] = cost_clusters(pairs, T, m_spread, c, c);
-    even[c] = cost_clusters(pairs, T, m_even, c, c);
+    spread[c] = cost_clusters(places, pairs, T, m_spread, c, c);
+    even[c] = cost_clusters(places, pairs, T, m_even, c, c);
     ns_even[c] = c;
     if (choose && even[c] >= 60.0) {
       const double enough = 0.97 * even[c];
       for (int ns = 1; ns < c; ++ns) {
-        const double cost = c % ns == 0 ? cost_clusters(pairs, T, m_even, c, ns) : 1e30;
+        const double cost = c % ns == 0 ? cost_clusters(places, pairs, T, m_even, c, ns) : 1e30;
         if (cost < enough && cost < even[c]) { even[c] = cost; ns_even[c] = ns; }
       }
     }
@@ -127,7 +127,7 @@ __host__ KvSplits plan_clusters(int64_t pairs, int64_t T, double mean) {
     if (spread[c] / least_spread + even[c] / least_even < spread[best] / least_spread + even[best] / least_even - 1e-9) best = c;
   KvSplits s = {best, best, ns_even[best], 0.75f};
   while (s.ns_even != best && s.even_from < 1.f &&
-         cost_clusters(pairs, T, s.even_from, best, best) < cost_clusters(pairs, T, s.even_from, best, s.ns_even))
+         cost_clusters(places, pairs, T, s.even_from, best, best) < cost_clusters(places, pairs, T, s.even_from, best, s.ns_even))
     s.even_from += 0.03125f;
   return s;
 }

@@ -588,9 +588,10 @@ bool kv_fast_supported(const KvAttnArgs& a, const KvSeqTable* seqs) {
 }
 
 namespace {
+template <int BITS> size_t smem_of() { return (size_t)kWarps * (Geo<BITS>::STAGES * Geo<BITS>::STAGE_BYTES + Geo<BITS>::SB_BYTES) + 4 * 32 * 8 + 64; }
 template <int BITS, class TAB, bool CHOOSE = false>
 cudaError_t launch_fast_inst(const FastK& p, const TAB& tab, dim3 grid, cudaStream_t st) {
-  const size_t smem = (size_t)kWarps * (Geo<BITS>::STAGES * Geo<BITS>::STAGE_BYTES + Geo<BITS>::SB_BYTES) + 4 * 32 * 8 + 64;
+  const size_t smem = smem_of<BITS>();
   static bool done[64] = {};
   int dev = 0;
   cudaGetDevice(&dev);
@@ -619,6 +620,35 @@ cudaError_t launch_fast_inst(const FastK& p, const TAB& tab, dim3 grid, cudaStre
   return launch_kernel(kv_fast_kernel<BITS, TAB, CHOOSE>, grid, dim3(kWarps * 32), smem, st, p, tab);
 }
 }  // namespace
+
+// Looked up once per device.  (A cluster lies within one GPC, so not every size fills the chip: 296 CTAs of sizes 1 and 2 here, then
+// 279, 284, 280, 270, 259, 264.)
+KvPlaces kv_fast_places() {
+  static KvPlaces places[64] = {};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  std::lock_guard<std::mutex> lk(setup_mutex());
+  KvPlaces& p = places[dev >= 0 && dev < 64 ? dev : 0];
+  if (p.n[1] != 0 && dev >= 0 && dev < 64) return p;
+  auto kern = kv_fast_kernel<4, KvNoTable, false>;
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+  for (int c = 1; c <= 8; ++c) {
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)c; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+    cfg.gridDim = dim3((unsigned)c, 1024);
+    cfg.blockDim = dim3(kWarps * 32);
+    cfg.dynamicSmemBytes = smem_of<4>();
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int q = 0;
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(&q, kern, &cfg);
+    p.n[c] = e == cudaSuccess && q > 0 ? q * c : 2 * sm_count();
+  }
+  if (e != cudaSuccess) (void)cudaGetLastError();
+  return p;
+}
 
 cudaError_t launch_kv_fast(const KvAttnArgs& a, KvSplits splits, float* pm, float* pl, float* po,
                            cudaStream_t st, const KvSeqTable* seqs, bool fused) {

@@ -1,5 +1,5 @@
 // Tiled quantized matmul with the weight term in fp32, for widths the tcgen05 kernel does not take: y[M, N] = x[M, K] . What^T,
-// bf16 activations, 4- or 8-bit affine codes, group size 32 / 64 / 128, K any multiple of the group size, from about 33 tokens;
+// bf16 activations, 4- or 8-bit affine codes, group size 32 / 64 / 128, K any multiple of the group size, from 5 tokens on (which of them: the rule in api.cu);
 // and the same over rows sorted by expert (gather_qmm).
 //
 // Replaces mlx_quantized_matmul / mlx_gather_qmm (transpose = true; mlx-serve src/transformer.zig:20894-20983, :20763-20784) at
@@ -9,7 +9,7 @@
 // so the MMA multiplies the codes themselves, and every group's sums are scaled in fp32 (one FMA per output against four MMAs,
 // which take four times the issue slots' time).  tcgen05 would need an accumulator per group in tensor memory and the same
 // FMAs after reading it back; it serves the rounded-weight shapes instead.
-//  * CTA: 16 warps on a tile of TM tokens x 32 WN weight rows, K in stages of 64 through a ring of cp.async copies of x and W as
+//  * CTA: 8 warps on a tile of TM tokens x 32 WN weight rows, K in stages of 64 through a ring of cp.async copies of x and W as
 //    they are; one barrier per stage.
 //  * Codes become bf16 integers in registers: 4 bits 128 + c (a shift and a LOP3 per two codes), 8 bits exactly c.  The pairs cut
 //    out of a packed word are not neighbours in k; the activations' pairs are permuted alike (a byte permutation each).

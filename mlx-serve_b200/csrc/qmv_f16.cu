@@ -13,7 +13,7 @@
 //    three bf16 parts).
 //  * Activations become fp16 under one power-of-two scale per token and CTA (largest |x| to the top of the range): bf16
 //    values within 2^-24 of the token's largest keep all their bits, fp32 ones are split into two columns (22 bits).
-//  * Two producer warps stream W rows and the scales and biases (cp.async in 16-byte pieces, those of the scales from the
+//  * Four producer warps stream W rows and the scales and biases (cp.async in 16-byte pieces, those of the scales from the
 //    aligned address below: their rows may start anywhere) into a ring of stages; 16 consumer warps split a stage by (group of 64 k) x (16-row tile) and keep their sums in registers over the whole of K, so nothing
 //    is reduced until a block of 64 rows is finished, and a group's activation fragments are loaded once for all its tiles.
 //  * The CTAs of a cluster split K over the same rows when the activations are many (they would not fit, and every CTA
@@ -185,7 +185,7 @@ __global__ void __launch_bounds__(kThreads, 1) qmv_f16_kernel(const __grid_const
   if (cs > 1) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");   // waited for before the first remote write
 
   if (warp >= kCW) {
-    // =========================== producer warps: half of a stage's rows each ===========================
+    // =========================== producer warps: a quarter of a stage's rows each ===========================
     // the kernel before may have written the weights, unless the host knows better
     if (!p.early) asm volatile("griddepcontrol.wait;" ::: "memory");
     constexpr int LPR = GE::ROWB / 16, RPI = 32 / LPR, HR = kRB / kPW;   // lanes per row, rows per copy instruction, rows per warp
@@ -631,7 +631,7 @@ template <int BITS, int NT, int GS>
 cudaError_t launch_inst(const F16K& p, size_t smem, cudaStream_t st) {
   auto kern = qmv_f16_kernel<BITS, NT, GS>;
   static bool attr_done[64] = {};
-  static int clusters_of[64][4] = {};   // co-resident clusters of 1, 2, 4, 8 CTAs at the full footprint of the instantiation
+  static int clusters_of[64][4] = {};   // co-resident clusters of 2, 4, 8 CTAs at the full footprint of the instantiation; -1: none
   int dev = 0;
   cudaGetDevice(&dev);
   const int di = (dev >= 0 && dev < 64) ? dev : 0;
@@ -648,26 +648,22 @@ cudaError_t launch_inst(const F16K& p, size_t smem, cudaStream_t st) {
     if (!attr_done[di] || di != dev) {
       const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
       if (e != cudaSuccess) return e;
-      for (int i = 0; i < 4; ++i) {
-        const int c = 1 << i;
-        int n = sm_count() / c;
-        if (c > 1) {
-          cfg.gridDim = dim3(n * c);
-          cfg.dynamicSmemBytes = (size_t)227 * 1024;
-          attr[1].val.clusterDim.x = c;
-          cfg.attrs = &attr[1];
-          cfg.numAttrs = 1;
-          int q = 0;
-          if (cudaOccupancyMaxActiveClusters(&q, kern, &cfg) != cudaSuccess) { (void)cudaGetLastError(); q = 0; }
-          n = q < n ? q : n;
-        }
-        clusters_of[di][i] = n;
-      }
       note_reader((const void*)kern);
       attr_done[di] = true;
     }
+    if (p.cluster > 1 && (clusters_of[di][ci] == 0 || di != dev)) {
+      const int n = sm_count() / p.cluster;
+      cfg.gridDim = dim3(n * p.cluster);
+      cfg.dynamicSmemBytes = (size_t)227 * 1024;
+      attr[1].val.clusterDim.x = p.cluster;
+      cfg.attrs = &attr[1];
+      cfg.numAttrs = 1;
+      int q = 0;
+      if (cudaOccupancyMaxActiveClusters(&q, kern, &cfg) != cudaSuccess) { (void)cudaGetLastError(); q = 0; }
+      clusters_of[di][ci] = q < 1 ? -1 : (q < n ? q : n);
+    }
   }
-  int ncl = clusters_of[di][ci];
+  int ncl = p.cluster > 1 ? clusters_of[di][ci] : sm_count();
   if (ncl < 1) return cudaErrorInvalidConfiguration;
   const int most = (p.row0[p.nmat] + 7) / 8;           // a cluster has at least 8 rows
   ncl = ncl < most ? ncl : most;
