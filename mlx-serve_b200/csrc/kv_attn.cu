@@ -81,50 +81,60 @@ __host__ int plan_f16(const KvAttnArgs& a, int64_t qtiles, int max_fused) {
 }
 
 // Splits of the 4-bit integer kernel where they merge inside a cluster (no partials in memory).  A CTA reads a token of one kv head
-// in 4.3 ns alone on its SM and in 7.6 ns beside a second one, plus about 6 us of start and end and 0.8 us of merge per split.  While
+// in 4 ns alone on its SM and in 7.6 ns beside a second one, plus about 5 us of start and end and 0.8 us of merge per split.  While
 // all CTAs are resident the longest sequence decides, in rounds of 512 tokens a CTA; beyond, CTAs follow one another on the places
 // that clusters of that size can take.  A last wave that is nearly empty costs less than half a wave, as its CTAs have their SMs to
-// themselves (27 x 8 pairs of 20992 tokens: 1.46 waves of two splits take 134 us, 0.73 of one split 164); lengths that differ
-// (`mean`: mean length / T) blur the waves.  Within 8 % (geometric mean over 1 - 8 splits) of what 15 shapes took, 16 to 320 pairs
-// of 3000 to 33280 tokens, equal or spread down to a half; its choice is within 5 % of the best of them in all.  (Counting whole
-// waves for equal lengths chose up to 23 % worse.)
+// themselves (27 x 8 pairs of 20992 tokens: 1.46 waves of two splits take 134 us, 0.73 of one split 164), and about 3 us more the
+// emptier it is, which decides short calls (13 x 8 pairs of 4000: two splits 22.5 us, three in 1.12 waves 30.4); lengths that differ
+// (`mean`: mean length / T) blur the waves.  Within 8 % (geometric mean over 1 - 8 splits) of what 26 shapes took, 16 to 512 pairs
+// of 1024 to 33280 tokens, equal or spread down to a half; its choice is the best of them or within 5 % for all but four (12 %).
+// (Counting whole waves for equal lengths chose up to 34 % worse.)
 __host__ double cost_clusters(const KvPlaces& places, int64_t pairs, int64_t T, double mean, int cluster, int ns) {
   const double n = (double)pairs * ns, slots = places.n[cluster], up = (double)((T + 512 * ns - 1) / (512 * ns) * 512);
-  if (2.0 * n <= slots) return 0.0043 * up + 6.0 + 0.8 * ns;
-  if (n <= slots) return 0.0076 * up + 6.0 + 0.8 * ns;
+  if (2.0 * n <= 0.97 * slots) return 0.004 * up + 4.5 + 0.8 * ns;   // (with less to spare some CTAs share an SM)
+  if (n <= slots) return 0.0076 * up + 5.0 + 0.8 * ns;
   double waves = n / slots;
-  if (mean > 0.95) waves = waves + 0.15 > floor(waves) + 0.4 ? waves + 0.15 : floor(waves) + 0.4;
-  else waves += 0.4;
-  return (0.0076 * mean * (double)T / ns + 6.0) * waves + 0.8 * ns;
+  const double empty = ceil(waves) - waves;
+  if (mean > 0.95) waves = waves + 0.2 > floor(waves) + 0.4 ? waves + 0.2 : floor(waves) + 0.4;
+  else waves += 0.35;
+  return (0.0076 * mean * (double)T / ns + 5.0) * waves + 3.0 * empty + 0.8 * ns;
 }
 // `mean` 0: lengths that only the device knows.  The splits are those that lose least over lengths all alike and lengths spread evenly
-// down to half of the longest.  Equal lengths may still want fewer: the kernel then takes those when it finds the lengths alike,
-// several pairs to a cluster.  (16 x 8 pairs of 32768 tokens: 4 splits take 106 us spread and 137 equal, 2 splits 116 and 131; the
-// kernel that chooses 106 and 133.)  Finding out costs the start of every CTA a reduction over the lengths, up to 2 us of a small
-// call, so it is left out where the model gives it less than 3 % or the call takes less than 60 us.
+// down to half of the longest; below 60 us also, at a tenth of the weight, over one long sequence among short ones, which wants many
+// (13 x 8 pairs of 4000 tokens, one and two splits: 21.4 and 23.0 us equal, 20.4 and 15.2 one long).  In a longer call where equal
+// lengths want fewer splits, few enough for all CTAs to be resident, the kernel takes those when it finds the lengths alike, several
+// pairs to a cluster.  (16 x 8 pairs of 32768 tokens: 4 splits take 106 us spread and 137 equal, 2 splits 116 and 131; the kernel
+// that chooses 107 and 134.  Where the CTAs are not all resident, several pairs to a cluster lose: 27 x 8 pairs of 20992, two splits
+// alone 134 us, in clusters of four 176.)  Finding out costs the start of every CTA a reduction over the lengths, up to 2 us of a
+// small call, so it is left out where the model gives it less than 3 %.
 __host__ KvSplits plan_clusters(int64_t pairs, int64_t T, double mean) {
   const double m_spread = mean > 0.0 ? mean : 0.75, m_even = mean > 0.0 ? mean : 1.0;
   const KvPlaces places = kv_fast_places();
   const bool choose = mean <= 0.0 && pairs < (1 << 24);   // (the kernel counts pairs in 32 bits)
-  double spread[9], even[9], least_spread = 1e30, least_even = 1e30;
+  double spread[9], even[9], one[9], least_spread = 1e30, least_even = 1e30, least_one = 1e30;
   int ns_even[9], count = 0;
   for (int c = 1; c <= 8 && (c == 1 || T / c >= 256); count = c++) {
     spread[c] = cost_clusters(places, pairs, T, m_spread, c, c);
     even[c] = cost_clusters(places, pairs, T, m_even, c, c);
+    one[c] = cost_clusters(places, 1, T, 1.0, c, c);
     ns_even[c] = c;
     if (choose && even[c] >= 60.0) {
       const double enough = 0.97 * even[c];
       for (int ns = 1; ns < c; ++ns) {
-        const double cost = c % ns == 0 ? cost_clusters(places, pairs, T, m_even, c, ns) : 1e30;
+        const double cost = c % ns == 0 && pairs * ns <= places.n[c] ? cost_clusters(places, pairs, T, m_even, c, ns) : 1e30;
         if (cost < enough && cost < even[c]) { even[c] = cost; ns_even[c] = ns; }
       }
     }
     least_spread = spread[c] < least_spread ? spread[c] : least_spread;
     least_even = even[c] < least_even ? even[c] : least_even;
+    least_one = one[c] < least_one ? one[c] : least_one;
   }
   int best = 1;
-  for (int c = 2; c <= count; ++c)
-    if (spread[c] / least_spread + even[c] / least_even < spread[best] / least_spread + even[best] / least_even - 1e-9) best = c;
+  double best_loss = 1e30;
+  for (int c = 1; c <= count; ++c) {
+    const double loss = spread[c] / least_spread + even[c] / least_even + (mean > 0.0 || least_even >= 60.0 ? 0.0 : 0.1 * one[c] / least_one);
+    if (loss < best_loss - 1e-9) { best_loss = loss; best = c; }
+  }
   KvSplits s = {best, best, ns_even[best], 0.75f};
   while (s.ns_even != best && s.even_from < 1.f &&
          cost_clusters(places, pairs, T, s.even_from, best, best) < cost_clusters(places, pairs, T, s.even_from, best, s.ns_even))
