@@ -38,12 +38,12 @@ constexpr size_t kTiles = (size_t)12 * TILE + RAWB * RAW;
 constexpr int kBars = 2 * SMAX + 2 * RAWB + 4;
 constexpr size_t smem_of(bool grouped) { return kTiles + kBars * 8 + 48 + (grouped ? 2 * (kMaxE + 1) * 4 : 0); }
 static_assert(smem_of(true) <= 227 * 1024, "shared memory");
-// Limits of a bounded wait.  The time decides: how long the hardware holds a poll is its own choice below kNap, and in this kernel, where
-// other barriers of the CTA change all the time, it is 0.36 us whatever kNap says (20 us to 1 ms: 6300 polls in the 2.3 ms an epilogue
-// waits at K = 196608; a lone waiter is held for the whole of kNap).  A number of polls therefore was a limit of 1.5 ms (2^12), then of
-// 95 ms (2^18), which longer contractions outlive.
-constexpr uint32_t kPolls = 1u << 24, kNap = 20000;
-constexpr uint64_t kLimitNs = 4000000000ull;
+// Limit of a bounded wait: 2^22 polls, each held by the hardware for kNap ns at most -- a lone waiter's for all of it; in this kernel, where
+// other barriers of the CTA change all the time, 360 ns whatever kNap says (20 us to 1 ms: 6300 polls in the 2.3 ms an epilogue waits
+// at K = 196608) -- so 1.5 to 8 seconds.  (2^12 polls ended after 1.5 ms, 2^18 after 95 ms, which longer contractions outlive.  A
+// limit by the clock, in a function of its own behind 4096 polls, made the roles save registers around the call: 64 experts x 768 x
+// 2048 with 5168 rows 52.5 -> 54.0 us.)
+constexpr uint32_t kSpin = 1u << 22, kNap = 2000;
 
 __device__ int g_pair_error = 0;                 // 0, or the code of a wait that expired
 
@@ -59,28 +59,15 @@ struct Tile {
   int row0, row_end, units, nn0, nn1;            // tokens [row0, row_end), in units of nn0 and nn1 (multiples of 32, up to 256)
   int n0, nend, wrow0, wlast;                    // output columns; first weight row of the tile, last one of the matrix
 };
-__device__ __forceinline__ bool poll_cta(uint32_t addr, uint32_t parity) {
-  uint32_t done;
-  asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-               : "=r"(done) : "r"(addr), "r"(parity), "r"(kNap) : "memory");
-  return done != 0;
-}
-// (out of line: the waits of the running kernel end in the loop below)
-__device__ __noinline__ bool wait_long(uint32_t addr, uint32_t parity) {
-  uint64_t t0, now;
-  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t0));
-  for (uint32_t it = 0; it < kPolls; ++it) {
-    if (poll_cta(addr, parity)) return true;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
-    if (now - t0 > kLimitNs) break;
-  }
-  return false;
-}
 __device__ __forceinline__ bool wait_cta(uint64_t* bar, uint32_t parity) {
   const uint32_t addr = smem_u32(bar);
-  for (int it = 0; it < 4096; ++it)
-    if (poll_cta(addr, parity)) return true;
-  return wait_long(addr, parity);
+  for (uint32_t it = 0; it < kSpin; ++it) {
+    uint32_t done;
+    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                 : "=r"(done) : "r"(addr), "r"(parity), "r"(kNap) : "memory");
+    if (done) return true;
+  }
+  return false;
 }
 // (a shared::cluster address)
 __device__ __forceinline__ void arrive_addr(uint32_t bar) {
