@@ -48,19 +48,17 @@ def bf16_ulp(v):
     return 2.0 ** (np.floor(np.log2(a)) - 7)
 
 
-_TABLE = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "gpurun_out", "parity_table.jsonl")
+_TABLE = os.environ.get("QB200_PARITY_TABLE")
 
 
 def record(config: str, what: str, max_over_rms: float, frac_half_ulp=None, n=None):
     """Append one row of the measured-tolerance table (literal max|delta|/RMS and, for bf16 outputs, the fraction of
-    outputs within half a bf16 ulp of the oracle's unrounded value).  Written only where the scratch folder exists."""
-    try:
-        os.makedirs(os.path.dirname(_TABLE), exist_ok=True)
-        with open(_TABLE, "a") as f:
-            f.write(json.dumps({"config": config, "what": what, "max_abs_delta_over_rms": max_over_rms,
-                                "frac_within_half_ulp": frac_half_ulp, "outputs": n}) + "\n")
-    except OSError:
-        pass
+    outputs within half a bf16 ulp of the oracle's unrounded value) to the file that QB200_PARITY_TABLE names, if it is set."""
+    if not _TABLE:
+        return
+    with open(_TABLE, "a") as f:
+        f.write(json.dumps({"config": config, "what": what, "max_abs_delta_over_rms": max_over_rms,
+                            "frac_within_half_ulp": frac_half_ulp, "outputs": n}) + "\n")
 
 
 def half_ulp_fraction(got_f32: np.ndarray, ref_f32: np.ndarray) -> float:
