@@ -327,12 +327,12 @@ static int64_t wide_max_tokens() {
 static bool takes_wide(const QmmArgs& a) { return a.M > 8 && a.M <= wide_max_tokens() && qmv_wide_supported(a); }
 
 // What the tuned kernels decline -- K no multiple of 256, group size 32, group size 128 at 8 bits -- goes to one of four kernels,
-// by times of each over M 1 - 64, N 100 - 12000, K 128 - 4416 (us):
-//  * tiny products to the CUDA-core kernel, whose launch is the shortest (300 x 704, 8 tokens: 3.1 against 3.9);
-//  * 8 bits, K a multiple of 128, few weights and tokens to the integer MMA kernel (1137 x 640, 8 tokens: 3.1 against 4.3);
-//  * more than 8 tokens to the tiled kernel (4000 x 4416, 16 tokens: 10.9 against 18), up to 16 tokens only while the weights are
-//    few -- it reads them at half the streaming kernel's rate (12000 x 4416, 16 tokens: 31 against 24) --, and from 5 tokens where
-//    K is long and the rows of W are too few to occupy the streaming kernel (1137 x 4416, 8 tokens: 7.6 against 10.9);
+// by times of each over M 1 - 64, N 100 - 12000, K 128 - 4416 (us a call, replayed):
+//  * tiny products to the CUDA-core kernel, whose launch is the shortest (300 x 704, 8 tokens: 3.4 against 4.5);
+//  * 8 bits, K a multiple of 128, few weights and tokens to the integer MMA kernel (1137 x 640, 8 tokens: 3.6 against 5.2);
+//  * more than 8 tokens to the tiled kernel (4000 x 4416, 16 tokens: 13.4 against 23.7), up to 16 tokens only while the weights are
+//    few -- its time does not depend on the tokens, the streaming kernel's does (12000 x 4416: 35 against 25 at 9 tokens, 32 at 16) --, and from 5 tokens where
+//    K is long and the rows of W are too few to occupy the streaming kernel (1137 x 4416, 8 tokens: 9.4 against 13.7);
 //  * the rest to the fp16 streaming kernel.  (Where qmv_stream and qmv_wide serve a shape they are faster than either.)
 enum class Ragged { none, generic, mma, f16, tile };
 static Ragged ragged_kernel(const QmmArgs& a) {

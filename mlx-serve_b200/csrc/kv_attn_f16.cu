@@ -7,7 +7,7 @@
 // (src/transformer.zig:10216-10249); partials merged as src/transformer.zig:5194-5203.
 //
 // Organisation (HBM-bound by bytes: the packed codes are read once, straight from the strided cache views; what a kernel
-// of this kind runs out of first is issue slots, so the arithmetic is arranged around spending few of them per code):
+// of this kind runs out of in long batches is issue slots, so the arithmetic is arranged around spending few of them per code):
 //  * grid (split, kv head x query tile, sequence); 4 warps per CTA, three CTAs per SM.  A warp walks blocks of 64
 //    tokens with its own online softmax and its own cp.async ring, so no warp waits on another for data.
 //  * A code c (up to 8 bits) in the low bits of a 16-bit word IS the fp16 subnormal c * 2^-24, exactly: one AND turns a
@@ -25,7 +25,8 @@
 //    of one dim.  The V bias term is a plain fp32 dot of p with the biases.
 //  * The running reference r of the softmax (p = 2^(s - r)) is kept below the block maximum by the exponent of the
 //    block's largest V scale, so p * v_scale uses fp16's range from the top whatever the scales are.
-// Bound: issue slots.  408 warp instructions per 16 tokens at 4 bits and head dim 128 (ncu), IPC 2.1 with 12 warps per SM.
+// Bound: the latency of a warp's chain of dependent instructions, with few warps to hide it.  408 warp instructions per 16 tokens at
+// 4 bits and head dim 128; IPC 2.1 with 12 warps on an SM (long batches), 1.5 - 1.6 with the 7 - 9 that short ones leave there (ncu).
 // What it replaces and when it runs: the launch rule in kv_attn.cu.
 #include <mutex>
 

@@ -5,7 +5,8 @@
 // Replaces mlx_quantized_matmul / mlx_gather_qmm (transpose = true; mlx-serve src/transformer.zig:20894-20983, :20763-20784) at
 // such shapes, which ran on the CUDA cores (about 4 TFLOP/s; dense ones then in 32-token passes of the streaming kernel).
 //
-// Bound: the rate of the warp-level MMA (about 580 TFLOP/s of m16n8k16 on this part).  The weight term must not be rounded here,
+// Bound: at hundreds of tokens the rate of the warp-level MMA (about 580 TFLOP/s of m16n8k16 on this part); at tens of tokens the
+// dependent chain of a stage and its barrier (27 x 12000 x 4416: tensor pipe 27 % active, issue 0.40 per scheduler).  The weight term must not be rounded here,
 // so the MMA multiplies the codes themselves, and every group's sums are scaled in fp32 (one FMA per output against four MMAs,
 // which take four times the issue slots' time).  tcgen05 would need an accumulator per group in tensor memory and the same
 // FMAs after reading it back; it serves the rounded-weight shapes instead.
