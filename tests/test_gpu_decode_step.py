@@ -233,10 +233,13 @@ def test_swiglu_over_every_gate_pattern():
     gate = torch.arange(65536, dtype=torch.int32).to(torch.int16).view(torch.bfloat16)
     gate = gate[~torch.isnan(gate.float())]
     n = gate.numel() // 64 * 64
-    g32, up = gate[:n].float(), torch.full((n,), 1.5)
-    sy = 1.0 / (1.0 + torch.exp(g32.abs()))
-    sig = torch.where(g32 < 0, sy, 1.0 - sy).to(torch.bfloat16).float()
-    ref = ((g32 * sig).to(torch.bfloat16).float() * up).to(torch.bfloat16)
+    # In 64 bits, with fp32's overflow of the exponential: a gate of -0.0117 lies one fp32 step of the exponential from another bf16
+    # result, and results down to 1e-39 are subnormal, so fp32 on the host would tie the test to its vector library and its flushing mode.
+    g64, up = gate[:n].double(), torch.full((n,), 1.5)
+    e = torch.exp(g64.abs())
+    sy = 1.0 / (1.0 + torch.where(e > 3.4028235e38, torch.inf, e))
+    sig = torch.where(g64 < 0, sy, 1.0 - sy).to(torch.bfloat16).double()
+    ref = ((g64 * sig).to(torch.bfloat16).double() * up).to(torch.bfloat16)
     for shape in ((n // 64, 64), (n // 2, 2)):
         y = qb200.swiglu(gate[:n].view(shape).cuda(), up.to(torch.bfloat16).view(shape).cuda())
         assert torch.equal(y.cpu().view(-1).view(torch.int16)[~torch.isnan(ref.float())], ref.view(torch.int16)[~torch.isnan(ref.float())])
