@@ -86,19 +86,17 @@ __device__ __forceinline__ void tma_load_pair(uint32_t dst, const CUtensorMap* m
   asm volatile("cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
                ::"r"(dst), "l"(map), "r"(bar), "r"(x), "r"(y) : "memory");
 }
-// Executed by every lane (uniform operands); only the lane with `issue` set issues.
-__device__ __forceinline__ void umma2(uint32_t d, uint64_t ad, uint64_t bd, uint32_t idesc, uint32_t accum, uint32_t issue) {
-  asm volatile(
-      "{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %5, 0;\n\t"
-      "@q tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(d), "l"(ad), "l"(bd), "r"(idesc), "r"(accum), "r"(issue) : "memory");
+// Both by the elected lane.
+__device__ __forceinline__ void umma2(uint32_t d, uint64_t ad, uint64_t bd, uint32_t idesc, uint32_t accum) {
+  asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+               ::"r"(d), "l"(ad), "l"(bd), "r"(idesc), "r"(accum) : "memory");
 }
 // arrives at the barrier at this offset in both CTAs once the MMAs issued so far are complete
-__device__ __forceinline__ void commit2(uint32_t bar, uint32_t issue) {
+__device__ __forceinline__ void commit2(uint32_t bar) {
   asm volatile(
-      "{\n\t.reg .pred q;\n\t.reg .b16 lo, hi;\n\tmov.b32 {lo, hi}, %2;\n\tsetp.ne.b32 q, %1, 0;\n\t"
-      "@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], lo;\n\t}"
-      ::"r"(bar), "r"(issue), "r"(3u) : "memory");
+      "{\n\t.reg .b16 lo, hi;\n\tmov.b32 {lo, hi}, %1;\n\t"
+      "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], lo;\n\t}"
+      ::"r"(bar), "r"(3u) : "memory");
 }
 
 template <bool GROUPED>
@@ -135,7 +133,7 @@ __device__ __forceinline__ Tile tile_at(const PairK& p, const int* s_off, const 
 // uses is broadcast from lane 0, so that the compiler knows it to be the same in the whole warp and keeps it in uniform registers.
 struct Walk { uint32_t tmem, w_s, x_s, empty_s, acc_s; int tile0, ntiles, tstride, nkb; const int* s_off; const int* s_tcum; };
 template <bool GROUPED>
-__device__ __noinline__ void issue_walk(const PairK& p, const Walk a, uint32_t lead) {
+__device__ __noinline__ void issue_walk(const PairK& p, const Walk a) {
   auto U = [](uint32_t v) { return __shfl_sync(0xffffffffu, v, 0); };
   constexpr uint32_t idesc0 = (1u << 4) | (1u << 7) | (1u << 10) | ((256u >> 4) << 24);   // f32 += bf16 x bf16, M = 256
   const uint64_t hi = make_desc(0) & 0xFFFFFFFF00000000ull;
@@ -151,17 +149,22 @@ __device__ __noinline__ void issue_walk(const PairK& p, const Walk a, uint32_t l
       asm volatile("bar.sync %0, 64;" ::"r"(1 + st) : "memory");   // the scout has seen the stage (and the accumulators' slots) ready
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const uint32_t wd = wd0 + st * (TILE >> 4), xd = xd0 + st * xstep;
+      if (elect_one()) {
 #pragma unroll
-      for (int k = 0; k < BK / 16; ++k) umma2(d0, hi | (wd + 2 * k), hi | (xd + 2 * k), i0, kb > 0 || k > 0 ? 1u : 0u, lead);
-      if (units == 2) {
+        for (int k = 0; k < BK / 16; ++k) umma2(d0, hi | (wd + 2 * k), hi | (xd + 2 * k), i0, kb > 0 || k > 0 ? 1u : 0u);
+        if (units == 2) {
 #pragma unroll
-        for (int k = 0; k < BK / 16; ++k) umma2(d1, hi | (wd + 2 * k), hi | (xd + (TILE >> 4) + 2 * k), i1, kb > 0 || k > 0 ? 1u : 0u, lead);
+          for (int k = 0; k < BK / 16; ++k) umma2(d1, hi | (wd + 2 * k), hi | (xd + (TILE >> 4) + 2 * k), i1, kb > 0 || k > 0 ? 1u : 0u);
+        }
+        commit2(empty_s + st * 8u);
+        if (kb + 1 == nkb) {
+          commit2(acc_s + (u0 & 1) * 8u);
+          if (units == 2) commit2(acc_s + (~u0 & 1) * 8u);
+        }
       }
-      commit2(empty_s + st * 8u, lead);
+      __syncwarp();
       st = st + 1 == (uint32_t)S ? 0 : st + 1;
     }
-    commit2(acc_s + (u0 & 1) * 8u, lead);
-    if (units == 2) commit2(acc_s + (~u0 & 1) * 8u, lead);
     u0 += units;
   }
 }
@@ -268,7 +271,7 @@ __global__ void __launch_bounds__(kThreads, 1) qmm_pair_kernel(const __grid_cons
   auto failed = [&](int code) { s_fail = code; atomicCAS(&g_pair_error, 0, code); };
 
   if (warp == kXWarp) {
-    if (lane == 0) {
+    if (elect_one()) {
       int st = 0, round = 0;
       bool ok = true;
       for (int tile = tile0; tile < ntiles && ok; tile += tstride) {
@@ -294,7 +297,7 @@ __global__ void __launch_bounds__(kThreads, 1) qmm_pair_kernel(const __grid_cons
       }
     }
   } else if (warp == kWWarp) {
-    if (lane == 0) {
+    if (elect_one()) {
       int sb = 0;
       bool ok = true;
       for (int tile = tile0; tile < ntiles && ok; tile += tstride) {
@@ -314,7 +317,7 @@ __global__ void __launch_bounds__(kThreads, 1) qmm_pair_kernel(const __grid_cons
       Walk w;
       w.tmem = tmem; w.w_s = smem_u32(w_t); w.x_s = smem_u32(x_t); w.empty_s = smem_u32(empty); w.acc_s = smem_u32(acc_full);
       w.tile0 = tile0; w.ntiles = ntiles; w.tstride = tstride; w.nkb = nkb; w.s_off = s_off; w.s_tcum = s_tcum;
-      issue_walk<GROUPED>(p, w, lane == 0 ? 1u : 0u);
+      issue_walk<GROUPED>(p, w);
     }
   } else if (warp == kScoutWarp) {
     // The same walk as the issuer's, ahead of it: it arrives at a named barrier per stage, where the issuer meets it (a poll of an

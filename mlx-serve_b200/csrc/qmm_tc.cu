@@ -127,31 +127,17 @@ __device__ __forceinline__ uint32_t make_idesc(int bn) {
   d |= (uint32_t)(128 >> 4) << 24;
   return d;
 }
-// Both are executed by every lane of the issuing warp with the same operands (so that the compiler can keep
-// them in uniform registers and the loop around them stays convergent); only the lane with `issue` set
-// issues the instruction.
-__device__ __forceinline__ void umma(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accum, uint32_t issue) {
+// Both are executed by the elected lane of the issuing warp, which walks its loop convergent.
+__device__ __forceinline__ void umma(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accum) {
   asm volatile(
-      "{\n\t.reg .pred p, q;\n\t"
+      "{\n\t.reg .pred p;\n\t"
       "setp.ne.b32 p, %4, 0;\n\t"
-      "setp.ne.b32 q, %6, 0;\n\t"
-      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %5, %5, %5}, p;\n\t}"
-      ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accum), "r"(0u), "r"(issue)
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %5, %5, %5}, p;\n\t}"
+      ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accum), "r"(0u)
       : "memory");
 }
-__device__ __forceinline__ void umma_commit(uint64_t* bar, uint32_t issue) {
-  asm volatile(
-      "{\n\t.reg .pred q;\n\t"
-      "setp.ne.b32 q, %1, 0;\n\t"
-      "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}"
-      ::"r"(smem_u32(bar)), "r"(issue) : "memory");
-}
-__device__ __forceinline__ void umma_commit_addr(uint32_t bar_smem, uint32_t issue) {
-  asm volatile(
-      "{\n\t.reg .pred q;\n\t"
-      "setp.ne.b32 q, %1, 0;\n\t"
-      "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}"
-      ::"r"(bar_smem), "r"(issue) : "memory");
+__device__ __forceinline__ void umma_commit_addr(uint32_t bar_smem) {
+  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar_smem) : "memory");
 }
 // Tile t -> coordinates.  Dense: token block t % tiles_m (fastest, so that CTAs running side by side share
 // a weight tile through L2), weight block t / tiles_m.  Grouped: the expert whose tile range holds t, then
@@ -194,14 +180,14 @@ __device__ __forceinline__ TileCoord tile_coords(const TcK& p, int BN, const int
 
 // The MMA issuer's walk over this CTA's tiles and k-blocks, kept out of line: as part of the kernel's one big
 // function its loop was compiled into something three times slower than the same loop on its own (4 MMAs issued in
-// ~700 cycles against ~260).  Every lane of the warp runs it; `lead` marks the lane that issues.
+// ~700 cycles against ~260).  Every lane of the warp runs it; the elected one issues.
 struct IssuerArgs {
   uint32_t tmem_base, a_smem, b_smem, empty_smem, acc_full_smem;
   int tile0, ntiles, tstride, nkb, BN;
   const int* s_off; const int* s_tcum;
 };
 template <bool GROUPED, bool HALF>
-__device__ __noinline__ void issuer_walk(const TcK& p, const IssuerArgs a, uint32_t lead) {
+__device__ __noinline__ void issuer_walk(const TcK& p, const IssuerArgs a) {
   constexpr int STAGES = stages_of(GROUPED, HALF);
   constexpr int KPST = kb_per_stage_of(HALF);          // k-blocks per stage
   constexpr int A_STAGE = A_STAGE_BYTES;               // two x boxes: two token halves, or (few-token form) two k-blocks
@@ -227,24 +213,26 @@ __device__ __noinline__ void issuer_walk(const TcK& p, const IssuerArgs a, uint3
       const uint64_t ad0 = adesc0 + (uint64_t)(st * (A_STAGE >> 4)), bd0 = bdesc0 + (uint64_t)(st * (B_STAGE >> 4));
       // A tile without a second token half keeps two partial sums over K, in the columns the second
       // half would use (odd K steps go there; the epilogue adds them).
+      if (elect_one()) {
 #pragma unroll
-      for (int sub = 0; sub < KPST; ++sub) {
+        for (int sub = 0; sub < KPST; ++sub) {
 #pragma unroll
-        for (int k16 = 0; k16 < BK / 16; ++k16) {
-          if (!HALF && two_halves) {
-            const uint32_t accum = (kb > 0 || k16 > 0) ? 1u : 0u;
-            umma(d0, ad0 + 2 * k16, bd0 + 2 * k16, idesc, accum, lead);
-            umma(d0 + HALF_COLS, ad0 + ((128 * BK * 2) >> 4) + 2 * k16, bd0 + 2 * k16, idesc, accum, lead);
-          } else {
-            const uint32_t accum = (kb > 0 || sub > 0 || k16 > 1) ? 1u : 0u;
-            umma(d0 + (k16 & 1) * HALF_COLS, ad0 + sub * ((128 * BK * 2) >> 4) + 2 * k16, bd0 + sub * (B_SUB >> 4) + 2 * k16, idesc,
-                 accum, lead);
+          for (int k16 = 0; k16 < BK / 16; ++k16) {
+            if (!HALF && two_halves) {
+              const uint32_t accum = (kb > 0 || k16 > 0) ? 1u : 0u;
+              umma(d0, ad0 + 2 * k16, bd0 + 2 * k16, idesc, accum);
+              umma(d0 + HALF_COLS, ad0 + ((128 * BK * 2) >> 4) + 2 * k16, bd0 + 2 * k16, idesc, accum);
+            } else {
+              const uint32_t accum = (kb > 0 || sub > 0 || k16 > 1) ? 1u : 0u;
+              umma(d0 + (k16 & 1) * HALF_COLS, ad0 + sub * ((128 * BK * 2) >> 4) + 2 * k16, bd0 + sub * (B_SUB >> 4) + 2 * k16, idesc, accum);
+            }
           }
         }
+        umma_commit_addr(a.empty_smem + (uint32_t)st * 8u);   // frees this stage (A and B) once the MMAs above have read it
+        if (kb + KPST >= a.nkb) umma_commit_addr(a.acc_full_smem + (uint32_t)buf * 8u);
       }
-      umma_commit_addr(a.empty_smem + (uint32_t)st * 8u, lead);  // frees this stage (A and B) once the MMAs above have read it
+      __syncwarp();
     }
-    umma_commit_addr(a.acc_full_smem + (uint32_t)buf * 8u, lead);
   }
 }
 
@@ -340,7 +328,7 @@ __global__ void __launch_bounds__(kThreads, 1) qmm_tc_kernel(const __grid_consta
   // the same order inside the expert.
   auto coords = [&](int tile) { return tile_coords<GROUPED>(p, BN, s_off, s_tcum, tile); };
   if (warp == kTmaWarp) {
-    if (lane == 0) {
+    if (elect_one()) {
       // ---------------- TMA producer (one thread) ----------------
       int it = 0, fail = 0;
       for (int tile = tile0; tile < ntiles && !fail && !s_fail; tile += tstride) {
@@ -365,7 +353,7 @@ __global__ void __launch_bounds__(kThreads, 1) qmm_tc_kernel(const __grid_consta
       if (fail) { s_fail = fail; atomicCAS(&g_tc_error, 0, fail); }
     }
   } else if (warp == kWTmaWarp) {
-    if (lane == 0) {
+    if (elect_one()) {
       // ---------------- TMA producer of the packed codes (one thread) ----------------
       const int sb_per_tile = nkb / KPS;
       int sbk = 0, fail = 0;
@@ -384,7 +372,7 @@ __global__ void __launch_bounds__(kThreads, 1) qmm_tc_kernel(const __grid_consta
     }
   } else if (warp == kMmaWarp) {
     {
-      // ---------------- MMA issuer (the whole warp walks the loop, lane 0 issues) ----------------
+      // ---------------- MMA issuer (the whole warp walks the loop, the elected lane issues) ----------------
       // The issuer waits on nothing but its scout: the two walk the same (tile, k-block) sequence and meet at named
       // barrier 1 once per k-block, whatever happens.  When a wait of the scout runs out it records the failure and
       // stops waiting; the issuer then multiplies stale stages into an accumulator nobody trusts (the status word
@@ -394,7 +382,7 @@ __global__ void __launch_bounds__(kThreads, 1) qmm_tc_kernel(const __grid_consta
       ia.empty_smem = smem_u32(empty); ia.acc_full_smem = smem_u32(acc_full);
       ia.tile0 = tile0; ia.ntiles = ntiles; ia.tstride = tstride; ia.nkb = nkb; ia.BN = BN;
       ia.s_off = s_off; ia.s_tcum = s_tcum;
-      issuer_walk<GROUPED, HALF>(p, ia, lane == 0 ? 1u : 0u);
+      issuer_walk<GROUPED, HALF>(p, ia);
     }
   } else if (warp == kScoutWarp) {
     // ---------------- the issuer's scout: the same walk, one meeting per k-block ----------------
