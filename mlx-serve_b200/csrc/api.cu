@@ -223,7 +223,7 @@ QB200_API void qb200_set_error_handler(qb200_error_handler_func handler, void* d
 QB200_API const char* qb200_last_error(void) { return g_last_error.c_str(); }
 QB200_API const char* qb200_version(void) { return "qb200 0.1 (sm_100a)"; }
 QB200_API int qb200_debug_tc_status(void) {
-  for (int code : {qmm_tc_error_code(), qmm_pair_error_code(), qmv_f16_error_code()})
+  for (int code : {qmm_tc_error_code(), qmm_pair_error_code(), qmv_f16_error_code(), qmv_tmem_error_code()})
     if (code) return code;
   return qmv_wide_error_code();
 }
@@ -232,6 +232,7 @@ QB200_API void qb200_debug_tc_reset(void) {
   qmv_wide_error_reset();
   qmv_f16_error_reset();
   qmm_pair_error_reset();
+  qmv_tmem_error_reset();
 }
 
 QB200_API void qb200_debug_wait_polls(int polls) { wait_polls() = polls; }
@@ -311,12 +312,12 @@ static int prepare_qmm(qb200_tensor* res, const qb200_tensor* x, const qb200_ten
   return QB200_OK;
 }
 
-// Routing by token count.  Up to 8 tokens: the narrow streaming kernel (one launch).  9 .. 32 (bf16 activations): the
-// wide streaming kernel, which reads every packed word once for up to 64 tokens per pass.  Above that the
-// tensor-core kernel, whose time does not depend on the token count up to 128 (measured on the C2 layer through the
-// batch entry: 110 us at 32 tokens and 170 us at 64 on the wide kernel, 140 / 143 / 149 us at 32 / 64 / 128 on the
-// tensor-core kernel).  QB200_WIDE_MAX_TOKENS in the environment moves the upper limit (0 turns the wide kernel off,
-// 64 is the most it serves; a diagnostic for measuring the crossover, read once).
+// Routing by token count.  Up to 8 tokens: the narrow streaming kernel (one launch).  9 .. 64 (bf16 activations on 16-byte rows): the
+// kernel that streams weights through tensor memory (us, before -> there, 4-bit 4096 x 4096: 13.5 -> 9.4 at 9 tokens, 16.8 -> 10.3 at
+// 32, 26.6 -> 11.7 at 64; 512 x 512: 6.4 -> 4.1, 7.8 -> 4.5, 7.0 -> 5.6); 9 .. 32 of activations that TMA does not take: the wide
+// streaming kernel.  Above that the tensor-core kernel, whose time does not depend on the token count up to 128.
+// QB200_WIDE_MAX_TOKENS in the environment moves the upper limit of the wide kernel (0 turns it off, 64 is the most it serves; a
+// diagnostic for measuring the crossover, read once).
 static int64_t wide_max_tokens() {
   static const int64_t v = [] {
     const char* e = getenv("QB200_WIDE_MAX_TOKENS");
@@ -336,7 +337,7 @@ static bool takes_wide(const QmmArgs& a) { return a.M > 8 && a.M <= wide_max_tok
 //  * the rest to the fp16 streaming kernel.  (Where qmv_stream and qmv_wide serve a shape they are faster than either.)
 enum class Ragged { none, generic, mma, f16, tile };
 static Ragged ragged_kernel(const QmmArgs& a) {
-  if (takes_wide(a) || (a.M > 8 && qmm_tc_supported(a)) || qmv_stream_supported(a)) return Ragged::none;
+  if (takes_wide(a) || qmv_tmem_supported(a) || (a.M > 8 && qmm_tc_supported(a)) || qmv_stream_supported(a)) return Ragged::none;
   const bool mma = qmv_mma_supported(a), f16 = qmv_f16_supported(a), tile = qmm_tile_supported(a);
   if ((double)a.M * a.N * a.K * a.nbatch <= 3.6e6 && !mma) return Ragged::generic;
   if (mma) {
@@ -358,6 +359,7 @@ static bool launched(cudaError_t e) {
 static cudaError_t dispatch_qmm(const QmmArgs& a, cudaStream_t s) {
   if (!a.transpose) return qmv_rows_supported(a) ? launch_qmv_rows(a, s) : launch_qmm_generic(a, s);
   if (a.nbatch > 1 && qmv_shortk_supported(a)) return launch_qmv_shortk(a, s);   // one W per batch element, short K: q @ K^T
+  if (qmv_tmem_supported(a)) return launch_qmv_tmem(a, s);
   if (takes_wide(a)) return launch_qmv_wide(a, s);
   if (qmm_pair_supported(a) && launched(launch_qmm_pair(a, s))) return cudaSuccess;
   if (a.M > wide_max_tokens() && a.M > 8 && qmm_tc_supported(a)) return launch_qmm_tc(a, s);
@@ -401,23 +403,26 @@ QB200_API int qb200_quantized_matmul_batch(qb200_tensor* const* res, const qb200
     const int n = count - i0 < kChunk ? count - i0 : kChunk;
     QmmArgs a[kChunk];
     bool empty[kChunk];
-    bool fuse = n > 1, wide = n > 1, f16 = n > 1;
+    bool fuse = n > 1, tmem = n > 1, wide = n > 1, f16 = n > 1;
     for (int i = 0; i < n; ++i) {
       int st = prepare_qmm(res[i0 + i], x, w[i0 + i], scales[i0 + i], biases[i0 + i], transpose_w, group_size, bits,
                            mode, &a[i], &empty[i]);
       if (st) return st;
       // the matrices share a launch where the single call would take a streaming kernel (same rule as dispatch_qmm)
       f16 = f16 && !empty[i] && a[i].K == a[0].K && ragged_kernel(a[i]) == Ragged::f16;
+      tmem = tmem && !empty[i] && qmv_tmem_supported(a[i]) && a[i].K == a[0].K;
       wide = wide && !empty[i] && takes_wide(a[i]) && a[i].K == a[0].K;
       fuse = fuse && !empty[i] && a[i].M <= 8 && qmv_stream_supported(a[i]) && a[i].K == a[0].K;
     }
     // beyond the streaming kernels' widths, up to 256 tokens: one launch of the tensor-core kernel over all matrices
-    bool tc = n > 1 && !wide && !fuse && !f16;
+    bool tc = n > 1 && !tmem && !wide && !fuse && !f16;
     for (int i = 0; i < n && tc; ++i) tc = !empty[i] && a[i].M > wide_max_tokens() && a[i].M > 8 && !qmm_pair_supported(a[i]);
     tc = tc && qmm_tc_multi_supported(a, n);
     cudaError_t e = cudaSuccess;
     if (f16 && launched(launch_qmv_f16_multi(a, n, (cudaStream_t)s))) {
       // one launch has taken all of them
+    } else if (tmem) {
+      e = launch_qmv_tmem_multi(a, n, (cudaStream_t)s);
     } else if (wide) {
       e = launch_qmv_wide_multi(a, n, (cudaStream_t)s);
     } else if (tc) {

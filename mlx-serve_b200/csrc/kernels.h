@@ -155,6 +155,13 @@ cudaError_t launch_qmv_wide_multi(const QmmArgs* a, int count, cudaStream_t st);
 int qmv_wide_error_code();    // 0, or the code of a bounded wait that expired
 void qmv_wide_error_reset();
 
+// ---- qmv_tmem.cu : 9..128 tokens, weights streamed through tensor memory, every packed word read once ----
+bool qmv_tmem_supported(const QmmArgs& a);
+cudaError_t launch_qmv_tmem(const QmmArgs& a, cudaStream_t st);
+cudaError_t launch_qmv_tmem_multi(const QmmArgs* a, int count, cudaStream_t st);   // same x, <= 4 matrices
+int qmv_tmem_error_code();    // 0, or the code of a bounded wait that expired
+void qmv_tmem_error_reset();
+
 // ---- qmm_tc.cu : prefill widths on tcgen05 (dequantise into the swizzled smem operand, TMEM accumulate) ----
 bool qmm_tc_supported(const QmmArgs& a);
 cudaError_t launch_qmm_tc(const QmmArgs& a, cudaStream_t st);

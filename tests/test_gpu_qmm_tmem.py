@@ -1,0 +1,63 @@
+"""The kernel that streams weights through tensor memory (9 - 64 tokens): edges of its token blocks, row tiles and shares of K, scales on
+either side of what its conversion takes at once, several matrices in a call, a device that places no clusters -- against the CPU
+oracle (weight term rounded to bf16 once)."""
+import numpy as np
+import pytest
+import torch
+
+from oracle import qoracle as qo
+from test_gpu_qmm import _run
+from util import dev_triple, gate_bf16, make_weight, rand_bf16, to_dev_bf16
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("bits,gs,M,N,K", [
+    (4, 64, 9, 1, 256), (4, 64, 16, 127, 512), (4, 128, 17, 128, 768), (4, 64, 32, 129, 1280),      # one row; edges of tiles; scales' rows of 24, 40 bytes
+    (4, 64, 33, 300, 2048), (4, 64, 48, 640, 256), (4, 128, 64, 513, 1024), (4, 64, 64, 100, 4352),
+    (8, 64, 9, 130, 256), (8, 128, 16, 257, 1792), (8, 64, 27, 64, 3072), (8, 64, 49, 200, 512), (8, 128, 64, 129, 768),
+    (4, 64, 13, 20000, 256), (8, 64, 32, 9000, 512),                                                # several tiles a cluster
+    (4, 64, 20, 256, 16384), (8, 64, 64, 140, 8192)])                                               # x in a ring
+def test_edges(bits, gs, M, N, K):
+    import qb200
+    rng = np.random.default_rng(bits * 100 + gs + M + N + K)
+    q, s, b = make_weight(rng, (N, K), gs, bits)
+    _run(rand_bf16(rng, (M, K)), q, s, b, gs, bits)
+    assert qb200.lib().qb200_debug_tc_status() == 0
+
+
+@pytest.mark.parametrize("bits", [4, 8])
+def test_scales_of_all_sizes(bits):
+    """Groups from 2^-30 to 2^30: those that the conversion of codes as subnormals takes, those beyond, and both in a unit."""
+    import qb200
+    rng = np.random.default_rng(bits)
+    M, N, K = 24, 256, 1024
+    w = rand_bf16(rng, (N, K)) * np.exp2(rng.integers(-30, 31, (N, K // 64))).astype(np.float32).repeat(64, 1)
+    w[:128] = rand_bf16(rng, (128, K), 0.02)
+    w[5, 64:128] = 1000.0 * rand_bf16(rng, (64,))
+    q, s, b = qo.quantize(w, 64, bits)
+    x = rand_bf16(rng, (M, K))
+    y = qb200.quantized_matmul(to_dev_bf16(qo.f32_to_bf16(x)), *dev_triple(q, s, b), True, 64, bits).float().cpu().numpy()
+    ref = qo.qmm(x, q, s, b, 64, bits, bf16_weights=True)
+    for n in range(N):   # (a row's own size)
+        gate_bf16(y[:, n], ref[:, n], f"row {n}")
+
+
+def test_several_matrices():
+    import qb200
+    rng = np.random.default_rng(5)
+    K, M, rows = 1024, 19, (700, 33, 128, 250)
+    ws = [make_weight(rng, (n, K), 64, 4) for n in rows]
+    x = rand_bf16(rng, (M, K))
+    dev, dx = [dev_triple(*w) for w in ws], to_dev_bf16(qo.f32_to_bf16(x))
+    outs = [torch.empty((M, n), dtype=torch.bfloat16, device="cuda") for n in rows]
+    qb200.quantized_matmul_batch(dx, dev, outs, True, 64, 4)
+    for y, w, d in zip(outs, ws, dev):
+        gate_bf16(y.float().cpu().numpy(), qo.qmm(x, *w, 64, 4, bf16_weights=True), "several matrices")
+    qb200.lib().qb200_debug_refuse_clusters(True)
+    try:
+        alone = qb200.quantized_matmul(dx, *dev[0], True, 64, 4)
+    finally:
+        qb200.lib().qb200_debug_refuse_clusters(False)
+    gate_bf16(alone.float().cpu().numpy(), qo.qmm(x, *ws[0], 64, 4, bf16_weights=True), "no clusters")
+    assert qb200.lib().qb200_debug_tc_status() == 0
