@@ -31,14 +31,13 @@ namespace {
 constexpr int kMaxMat = 4, kMaxNt = 64, kMaxCluster = 8;
 constexpr int CK = 256;                                   // K values of a unit
 constexpr int kMaxCodes = 8, kSlots = 6, kMaxX = 16;      // ring depths: packed codes; A operand (half units, of all groups); units of x in shared memory
-// GRP converting groups: three up to 32 tokens, two beyond, where tensor memory has no room for three accumulators.
-template <int GRP> struct Form {
-  static constexpr int kOwn = kSlots / GRP;                // slots of a group
-  static constexpr int kEpi0 = 4 * GRP, kCodesWarp = kEpi0 + 4, kXWarp = kCodesWarp + 1, kThreads = (kXWarp + 1) * 32;   // first warps of the roles
-};
+// Warps: GRP groups of four that convert, four of the epilogue, one each for codes and x, one issuer a group.  (Three groups: 28672 x 4096
+// 31.4 us against 26.6 at 27 tokens, for whose three accumulators tensor memory has room once, not twice; the same at 9.)
+constexpr int GRP = 2, kOwn = kSlots / GRP;                // slots of a group
+constexpr int kEpi0 = 4 * GRP, kCodesWarp = kEpi0 + 4, kXWarp = kCodesWarp + 1, kMmaWarp = kXWarp + 1, kThreads = (kMmaWarp + GRP) * 32;
 constexpr uint32_t kSpin = 1u << 22, kNap = 2000;         // polls of a bounded wait; ns the hardware may hold one
 constexpr int kBars = 2 * kMaxCodes + kSlots + 2 * kMaxX + 4 + 4;
-constexpr size_t kBarBytes = kBars * 8 + 32, kSmem = 225 * 1024;
+constexpr size_t kBarBytes = kBars * 8 + 32, kSmem = 225 * 1024, kSmemTwo = 113 * 1024;
 __device__ int g_tmem_error = 0;                          // 0, or the code of a wait that expired
 
 struct TmMaps { CUtensorMap w[kMaxMat], s[kMaxMat], b[kMaxMat]; };
@@ -73,6 +72,12 @@ __device__ __forceinline__ bool wait_cta(uint64_t* bar, uint32_t parity) {
     if (done) return true;
   }
   return false;
+}
+__device__ __forceinline__ bool test_cta(uint64_t* bar, uint32_t parity) {
+  uint32_t done;
+  asm volatile("{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+               : "=r"(done) : "r"(smem_u32(bar)), "r"(parity) : "memory");
+  return done != 0;
 }
 // A whole warp waits.  All lanes poll (107 cycles when the phase is complete; one lane for the others, 134 and a divergent branch).
 __device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity) { return __all_sync(0xffffffffu, wait_cta(bar, parity)); }
@@ -194,14 +199,12 @@ __device__ __forceinline__ void tmem_ld4(uint32_t taddr, uint32_t (&r)[4]) {
   asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(taddr));
 }
 
-template <int BITS, int GRP>
-__global__ void __launch_bounds__(Form<GRP>::kThreads, 1) qmv_tmem_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ TmMaps wm,
+template <int BITS, int PER_SM>
+__global__ void __launch_bounds__(kThreads, PER_SM) qmv_tmem_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ TmMaps wm,
                                                                const __grid_constant__ TmK p) {
   extern __shared__ __align__(1024) unsigned char smem[];
   constexpr int kCodes = 128 * CK * BITS / 8;              // packed codes of a unit: 128-byte rows, one box at 4 bits, two at 8
   constexpr int kStage = kCodes + 2 * 2048;                // and blocks of 8 scales and 8 biases of its rows, 16 bytes each
-  using F = Form<GRP>;
-  constexpr int kEpi0 = F::kEpi0, kCodesWarp = F::kCodesWarp, kXWarp = F::kXWarp, kThreads = F::kThreads;
   // (the warp's number from lane 0: what follows from it is then the same in the whole warp to the compiler, too)
   const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = tid & 31;
   const int CS = p.cs, XS = p.xs, nt = p.nt, C = p.cluster;
@@ -324,76 +327,63 @@ __global__ void __launch_bounds__(Form<GRP>::kThreads, 1) qmv_tmem_kernel(const 
   auto peers_ready = [&] { if (C > 1) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); };   // once by every thread
 
   if (warp < kEpi0) {
-    // ---- convert this thread's weight row, unit by unit, and multiply: the group's first warp issues the MMAs ----
-    // A wait that runs out ends the others', too, and no MMA is issued any more; but every warp keeps every meeting of its group.
-    const int grp = warp >> 2, q = warp & 3, r = q * 32 + lane;
-    const uint32_t lane_off = (uint32_t)(q * 32) << 16, a_g = a0 + grp * (F::kOwn * 64);
-    const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (((uint32_t)nt >> 3) << 17) | ((128u >> 4) << 24);   // f32 += bf16 x bf16, M = 128
-    const uint64_t dhi = make_desc(0) & 0xFFFFFFFF00000000ull;
-    const uint32_t xd0 = (uint32_t)make_desc(smem_u32(xs));
+    // ---- convert this thread's weight row, unit by unit ----
+    // A wait that runs out ends the others', too; but every warp keeps every meeting with its group's issuer, by then one at a time.
+    const int grp = warp >> 2, q = warp & 3, r = q * 32 + lane, mine = total > grp ? (total - grp + GRP - 1) / GRP : 0;
+    const uint32_t a_g = a0 + grp * (kOwn * 64) + ((uint32_t)(q * 32) << 16);
     bool ok = true;
-    auto wait = [&](uint64_t* bar, int phase) { if (ok) ok = warp_wait(bar, (uint32_t)phase & 1); };
-    int st = grp, cround = 0, slot = 0, round = 0, xi = grp % XS, xround = 0;   // (CS and a ring's XS are multiples of GRP: a stage is always for the same group)
-    int k = grp;
-    for (int t = 0; t < tiles; ++t, k -= ku) {
-      const int d = p.dbufs == 2 ? t & 1 : 0, dround = p.dbufs == 2 ? t >> 1 : t;
-      const uint32_t dt = tmem + (uint32_t)((d * GRP + grp) * nt);
-      const bool mine = k < ku;
-      uint32_t acc = 0;
-      if (!p.ring) xi = k;
-      for (; k < ku; k += GRP) {
-        const unsigned char* row = codes + st * kStage + r * 128;
-        wait(&codes_full[st], cround);
-        const int e = ((k0 + k) << (2 - p.gshift)) & 7;
-        const unsigned char* sbp = codes + st * kStage + kCodes + r * 16 + e * 2;
-        uint2 sv, bv;
-        if (p.gshift == 0) {
-          sv = *(const uint2*)sbp;
-          bv = *(const uint2*)(sbp + 2048);
-        } else {
-          const uint32_t s2 = *(const uint32_t*)sbp, b2 = *(const uint32_t*)(sbp + 2048);
-          sv = make_uint2(__byte_perm(s2, 0, 0x1010), __byte_perm(s2, 0, 0x3232));
-          bv = make_uint2(__byte_perm(b2, 0, 0x1010), __byte_perm(b2, 0, 0x3232));
-        }
-        const bool fits = __all_sync(0xffffffffu, fits_subnormal<BITS>(sv.x) && fits_subnormal<BITS>(sv.x >> 16) && fits_subnormal<BITS>(sv.y) && fits_subnormal<BITS>(sv.y >> 16));
-#pragma unroll 1
-        for (int h = 0; h < 2; ++h) {
-          const uint32_t a_s = a_g + (uint32_t)slot * 64;
-          if (round > 0) wait(&empty[grp * F::kOwn + slot], round - 1);
-          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          if (fits) convert_half<BITS, true>(row, r & 7, h, sv.x, bv.x, a_s + lane_off);
-          else convert_half<BITS, false>(row, r & 7, h, sv.x, bv.x, a_s + lane_off);
-          sv.x = sv.y;
-          bv.x = bv.y;
-          asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-          asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-          if (h == 0 && (p.ring || t == 0)) wait(&x_full[xi], xround);
-          if (h > 0 && lane == 0) mbar_arrive(&codes_empty[st]);   // (only now that the words have been consumed)
-          asm volatile("bar.sync %0, 128;" ::"r"(2 + grp) : "memory");
-          if (q == 0) {
-            if (acc == 0 && dround > 0) wait(&d_empty[d], dround - 1);
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            if (ok && elect_one()) {
-              const uint32_t xd = xd0 + (uint32_t)((xi * 4 + h * 2) * nt * 8), xk = (uint32_t)nt * 8;
-#pragma unroll
-              for (int m = 0; m < 8; ++m) umma_ta(dt, a_s + m * 8, dhi | (xd + (m >> 2) * xk + 2 * (m & 3)), idesc, m > 0 ? 1u : acc);
-              commit1(smem_u32(&empty[grp * F::kOwn + slot]));
-              if (h > 0 && p.ring) commit1(smem_u32(&x_empty[xi]));
-              if (h > 0 && k + GRP >= ku) commit1(smem_u32(&d_full[d]));
-            }
-            __syncwarp();
-          }
-          acc = 1;
-          if (++slot == F::kOwn) { slot = 0; ++round; }
-        }
-        st += GRP;
-        if (st >= CS) { st -= CS; ++cround; }
-        xi += GRP;
-        if (p.ring && xi >= XS) { xi -= XS; ++xround; }
+    auto wait = [&](bool ready, uint64_t* bar, int phase) { if (!ready && ok) ok = warp_wait(bar, (uint32_t)phase & 1); };
+    int st = grp, cround = 0, slot = 0, round = 0;           // (CS is a multiple of GRP: a stage is always for the same group)
+    int e = (k0 + grp % ku) << (2 - p.gshift), k = grp % ku; // the unit's first group of scales
+    uint2 sv, bv;
+    auto read_scales = [&]() {
+      const unsigned char* sbp = codes + st * kStage + kCodes + r * 16 + (e & 7) * 2;
+      if (p.gshift == 0) {
+        sv = *(const uint2*)sbp;
+        bv = *(const uint2*)(sbp + 2048);
+      } else {
+        const uint32_t s2 = *(const uint32_t*)sbp, b2 = *(const uint32_t*)(sbp + 2048);
+        sv = make_uint2(__byte_perm(s2, 0, 0x1010), __byte_perm(s2, 0, 0x3232));
+        bv = make_uint2(__byte_perm(b2, 0, 0x1010), __byte_perm(b2, 0, 0x3232));
       }
-      if (!mine && q == 0) {                               // (a tile of fewer units than groups)
-        if (dround > 0) wait(&d_empty[d], dround - 1);
-        if (ok && lane == 0) mbar_arrive(&d_full[d]);
+    };
+    bool codes_ready = false, slot_ready = true;
+    for (int i = 0; i < mine; ++i) {
+      if (!codes_ready) {
+        wait(false, &codes_full[st], cround);
+        read_scales();
+      }
+      const unsigned char* row = codes + st * kStage + r * 128;
+      uint64_t* done = &codes_empty[st];
+      const bool fits = __all_sync(0xffffffffu, fits_subnormal<BITS>(sv.x) && fits_subnormal<BITS>(sv.x >> 16) && fits_subnormal<BITS>(sv.y) && fits_subnormal<BITS>(sv.y >> 16));
+#pragma unroll 1
+      for (int h = 0; h < 2; ++h) {
+        wait(slot_ready, &empty[grp * kOwn + slot], round - 1);
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const uint32_t a_s = a_g + (uint32_t)slot * 64;
+        if (fits) convert_half<BITS, true>(row, r & 7, h, sv.x, bv.x, a_s);
+        else convert_half<BITS, false>(row, r & 7, h, sv.x, bv.x, a_s);
+        sv.x = sv.y;
+        bv.x = bv.y;
+        // what the next half needs is looked for while this one's stores end
+        const int id = 2 + grp * kOwn + slot;
+        if (++slot == kOwn) { slot = 0; ++round; }
+        slot_ready = round == 0 || test_cta(&empty[grp * kOwn + slot], (uint32_t)(round - 1) & 1);
+        if (h) {
+          st += GRP;
+          if (st >= CS) { st -= CS; ++cround; }
+          k += GRP;
+          while (k >= ku) k -= ku;
+          e = (k0 + k) << (2 - p.gshift);
+          codes_ready = i + 1 < mine && __all_sync(0xffffffffu, test_cta(&codes_full[st], (uint32_t)cround & 1));
+          if (codes_ready) read_scales();
+        }
+        slot_ready = __all_sync(0xffffffffu, slot_ready);
+        asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        if (ok) asm volatile("bar.arrive %0, 160;" ::"r"(id) : "memory");
+        else asm volatile("bar.sync %0, 160;" ::"r"(id) : "memory");
+        if (h && lane == 0) mbar_arrive(done);               // (only now that the words have been consumed)
       }
     }
     if (!ok && !s_fail) failed(404);
@@ -493,7 +483,7 @@ __global__ void __launch_bounds__(Form<GRP>::kThreads, 1) qmv_tmem_kernel(const 
     if (window_ok && CS < total) copy_units(CS, total);
     __syncwarp();
     peers_ready();
-  } else {
+  } else if (warp == kXWarp) {
     if (elect_one()) {
       grid_wait();                                         // x, and whatever used y last
       asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -519,6 +509,49 @@ __global__ void __launch_bounds__(Form<GRP>::kThreads, 1) qmv_tmem_kernel(const 
     }
     __syncwarp();
     peers_ready();
+  } else {
+    // ---- a group's issuer: the MMAs of every half unit that the group has converted, into the group's accumulator ----
+    const int grp = warp - kMmaWarp;
+    const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (((uint32_t)nt >> 3) << 17) | ((128u >> 4) << 24);   // f32 += bf16 x bf16, M = 128
+    const uint64_t dhi = make_desc(0) & 0xFFFFFFFF00000000ull;
+    const uint32_t xd0 = (uint32_t)make_desc(smem_u32(xs)), a_g = a0 + grp * (kOwn * 64), xk = (uint32_t)nt * 8;
+    bool ok = true;
+    auto wait = [&](uint64_t* bar, int phase) { if (ok) ok = warp_wait(bar, (uint32_t)phase & 1); };
+    int slot = 0, xi = grp % XS, xround = 0, k = grp;        // (a ring's XS is a multiple of GRP, too)
+    for (int t = 0; t < tiles; ++t, k -= ku) {
+      const int d = p.dbufs == 2 ? t & 1 : 0, dround = p.dbufs == 2 ? t >> 1 : t;
+      const uint32_t dt = tmem + (uint32_t)((d * GRP + grp) * nt);
+      const bool mine = k < ku;
+      if (dround > 0) wait(&d_empty[d], dround - 1);
+      uint32_t acc = 0;
+      if (!p.ring) xi = k;
+      for (; k < ku; k += GRP) {
+        if (p.ring || t == 0) wait(&x_full[xi], xround);
+#pragma unroll 1
+        for (int h = 0; h < 2; ++h) {
+          asm volatile("bar.sync %0, 160;" ::"r"(2 + grp * kOwn + slot) : "memory");
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          if (ok && elect_one()) {
+            const uint32_t xd = xd0 + (uint32_t)((xi * 4 + h * 2) * nt * 8), a_s = a_g + (uint32_t)slot * 64;
+#pragma unroll
+            for (int m = 0; m < 8; ++m) umma_ta(dt, a_s + m * 8, dhi | (xd + (m >> 2) * xk + 2 * (m & 3)), idesc, m > 0 ? 1u : acc);
+            commit1(smem_u32(&empty[grp * kOwn + slot]));
+            if (h > 0 && p.ring) commit1(smem_u32(&x_empty[xi]));
+            if (h > 0 && k + GRP >= ku) commit1(smem_u32(&d_full[d]));
+          }
+          __syncwarp();
+          acc = 1;
+          if (++slot == kOwn) slot = 0;
+        }
+        xi += GRP;
+        if (p.ring && xi >= XS) { xi -= XS; ++xround; }
+      }
+      if (!mine && ok && lane == 0) mbar_arrive(&d_full[d]);   // (a tile of fewer units than groups)
+      __syncwarp();
+    }
+    if (!ok && !s_fail) failed(401);
+    __syncwarp();
+    peers_ready();
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
@@ -541,10 +574,10 @@ bool make_map(CUtensorMap* m, CUtensorMapDataType t, const void* base, int64_t c
                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-cudaLaunchConfig_t config(int threads, cudaLaunchAttribute (&attr)[2], int grid, int cluster, size_t smem, cudaStream_t st) {
+cudaLaunchConfig_t config(cudaLaunchAttribute (&attr)[2], int grid, int cluster, size_t smem, cudaStream_t st) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)grid);
-  cfg.blockDim = dim3((unsigned)threads);
+  cfg.blockDim = dim3(kThreads);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -556,7 +589,7 @@ cudaLaunchConfig_t config(int threads, cudaLaunchAttribute (&attr)[2], int grid,
   return cfg;
 }
 // Clusters of this size that the device holds at once (0: none), looked up once per device; index 1: its SMs.
-template <int BITS, int GRP>
+template <int BITS, int PER_SM>
 cudaError_t clusters_of(int cluster, int* n) {
   static int cached[64][kMaxCluster + 1] = {};
   int dev = 0;
@@ -566,14 +599,14 @@ cudaError_t clusters_of(int cluster, int* n) {
   const int sms = sm_count();
   std::lock_guard<std::mutex> lk(setup_mutex());
   if (cached[dev][0] == 0) {
-    auto kern = qmv_tmem_kernel<BITS, GRP>;
+    auto kern = qmv_tmem_kernel<BITS, PER_SM>;
     e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem);
     if (e != cudaSuccess) return e;
     note_reader((const void*)kern);
     cached[dev][1] = sms;
     for (int c = 2; c <= kMaxCluster; ++c) {
       cudaLaunchAttribute attr[2];
-      cudaLaunchConfig_t cfg = config(Form<GRP>::kThreads, attr, sms / c * c, c, kSmem, nullptr);
+      cudaLaunchConfig_t cfg = config(attr, sms / c * c, c, kSmem, nullptr);
       cfg.attrs = &attr[1];
       cfg.numAttrs = 1;
       int q = 0;
@@ -588,12 +621,12 @@ cudaError_t clusters_of(int cluster, int* n) {
 
 // The cluster size: waves of tiles x (units of a tile's share + hand-over of its sums), in units of about 0.65 us
 struct Plan { int cluster, ncl, per, ku; };                // CTAs that split K, clusters, tiles and units of K of one at most
-template <int BITS, int GRP>
+template <int BITS, int PER_SM>
 cudaError_t plan(const TmK& p, int most, Plan* out) {
   const int ntiles = p.tile0[kMaxMat];
   double best = -1.0;
   for (int c = 1, n = 0; c <= most && c <= p.spb; ++c) {
-    const cudaError_t e = clusters_of<BITS, GRP>(c, &n);
+    const cudaError_t e = clusters_of<BITS, PER_SM>(c, &n);
     if (e != cudaSuccess) return e;
     if (n < 1) continue;
     const int t = (ntiles + n - 1) / n, ku = (p.spb + c - 1) / c;
@@ -603,19 +636,20 @@ cudaError_t plan(const TmK& p, int most, Plan* out) {
   return best < 0 ? cudaErrorInvalidConfiguration : cudaSuccess;
 }
 
-template <int BITS, int GRP>
-cudaError_t launch_form(const CUtensorMap& xmap, const TmMaps& wm, TmK p, cudaStream_t st) {
+template <int BITS, int PER_SM>
+cudaError_t launch_inst(const CUtensorMap& xmap, const TmMaps& wm, TmK p, cudaStream_t st) {
   constexpr int stage = 128 * CK * BITS / 8 + 2 * 2048;
   p.dbufs = 2 * GRP * p.nt <= 128 ? 2 : 1;                 // 512 columns of tensor memory: 6 x 64 for the A operand, groups x accumulators x tokens
   for (int most : {kMaxCluster, 1}) {                      // (where the device places no such cluster: CTAs by themselves)
     Plan pl;
-    cudaError_t e = plan<BITS, GRP>(p, most, &pl);
+    cudaError_t e = plan<BITS, PER_SM>(p, most, &pl);
     if (e != cudaSuccess) return e;
-    const int c = pl.cluster, xu = p.nt * 512, rx1 = c > 1 ? c * ((p.nt / 4 + c - 1) / c) * 2048 : 0, room = (int)(kSmem - kBarBytes);
+    const int c = pl.cluster, xu = p.nt * 512, rx1 = c > 1 ? c * ((p.nt / 4 + c - 1) / c) * 2048 : 0, room = (int)((PER_SM == 2 ? kSmemTwo : kSmem) - kBarBytes);
     p.cluster = c;
     p.rx = pl.per > 1 && c > 1 && room - 2 * rx1 >= 3 * xu + 3 * stage ? 2 : 1;
     const int left = room - p.rx * rx1;
-    p.ring = (left - 4 * stage) / xu < pl.ku || pl.ku > kMaxX;   // x whole where that leaves four stages of codes
+    const int keep = pl.per > 1 ? 4 : 6;                   // x whole where that leaves four stages of codes; six where it is read once
+    p.ring = (left - keep * stage) / xu < pl.ku || pl.ku > kMaxX;
     p.xs = pl.ku;
     if (p.ring) {
       p.xs = (left - 6 * stage) / xu;
@@ -628,18 +662,13 @@ cudaError_t launch_form(const CUtensorMap& xmap, const TmMaps& wm, TmK p, cudaSt
     p.cs = p.cs / GRP * GRP;
     if (p.cs < GRP) return cudaErrorInvalidConfiguration;
     cudaLaunchAttribute attr[2];
-    const cudaLaunchConfig_t cfg = config(Form<GRP>::kThreads, attr, pl.ncl * c, c, (size_t)(p.cs * stage + p.xs * xu + p.rx * rx1) + kBarBytes, st);
-    e = c > 1 ? launch_clusters(cfg, qmv_tmem_kernel<BITS, GRP>, xmap, wm, p) : cudaLaunchKernelEx(&cfg, qmv_tmem_kernel<BITS, GRP>, xmap, wm, p);
+    const cudaLaunchConfig_t cfg = config(attr, pl.ncl * c, c, (size_t)(p.cs * stage + p.xs * xu + p.rx * rx1) + kBarBytes, st);
+    e = c > 1 ? launch_clusters(cfg, qmv_tmem_kernel<BITS, PER_SM>, xmap, wm, p) : cudaLaunchKernelEx(&cfg, qmv_tmem_kernel<BITS, PER_SM>, xmap, wm, p);
     if (e == cudaSuccess || c == 1) return e;
     (void)cudaGetLastError();
   }
   return cudaErrorInvalidConfiguration;
 }
-template <int BITS>
-cudaError_t launch_inst(const CUtensorMap& xmap, const TmMaps& wm, const TmK& p, cudaStream_t st) {
-  return p.nt <= 32 ? launch_form<BITS, 3>(xmap, wm, p, st) : launch_form<BITS, 2>(xmap, wm, p, st);
-}
-
 }  // namespace
 
 bool qmv_tmem_supported(const QmmArgs& a) {
@@ -687,7 +716,11 @@ cudaError_t launch_qmv_tmem_multi(const QmmArgs* a, int count, cudaStream_t st) 
   p.tile0[kMaxMat] = tiles;
   if (!make_map(&xmap, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, (const uint16_t*)a[0].x + a[0].xb.offset(0), a[0].K, a[0].M, a[0].ldx * 2, 64, p.nt)) return cudaErrorInvalidValue;
   p.early = weights_settled(st);
-  return bits == 4 ? launch_inst<4>(xmap, wm, p, st) : launch_inst<8>(xmap, wm, p, st);
+  // Up to 16 tokens at 4 bits two CTAs fit an SM (64 registers, 113 KB), so that the next launch's is set up and has filled its ring when
+  // this one ends: a layer of Llama-3-8B's projections 51.7 us against 57.5.  With more to hold, the shallower rings cost more than that
+  // (27 tokens 73 against 61, 9 at 8 bits 76 / 59), as a launch of a few units has nothing to gain.
+  if (bits == 8) return launch_inst<8, 1>(xmap, wm, p, st);
+  return p.nt <= 16 && tiles * p.spb > 4 ? launch_inst<4, 2>(xmap, wm, p, st) : launch_inst<4, 1>(xmap, wm, p, st);
 }
 cudaError_t launch_qmv_tmem(const QmmArgs& a, cudaStream_t st) { return launch_qmv_tmem_multi(&a, 1, st); }
 
