@@ -394,6 +394,10 @@ __global__ void __launch_bounds__(kThreads, PER_SM) qmv_tmem_kernel(const __grid
     const int q = warp & 3, r = q * 32 + lane, ng = nt / 4;
     const int g0 = ng * rank / C, g1 = ng * (rank + 1) / C;                   // groups of four tokens that this CTA stores
     const uint32_t lane_off = (uint32_t)(q * 32) << 16, rx_s = smem_u32(rx);
+    if (q == 0) {   // (when tensor memory is this CTA's: a dependent that took it first, and waits for this grid, would never give it back)
+      grid_wait();
+      asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    }
     bool ok = true, seen = false;
     for (int j = 0; j < tiles && ok; ++j) {
       const int tile = cl + j * ncl, d = p.dbufs == 2 ? j & 1 : 0, b = p.rx == 2 ? j & 1 : 0;
@@ -486,7 +490,6 @@ __global__ void __launch_bounds__(kThreads, PER_SM) qmv_tmem_kernel(const __grid
   } else if (warp == kXWarp) {
     if (elect_one()) {
       grid_wait();                                         // x, and whatever used y last
-      asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
       const uint32_t kb = (uint32_t)nt * 128u;
       auto load_x = [&](int k, int st) {
         mbar_expect_tx(&x_full[st], 4 * kb);
