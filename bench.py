@@ -280,9 +280,7 @@ def main():
 
     def launches_per_layer(m):
         calls = 7 if args.no_batch else 4
-        if 8 < m <= 32:
-            return 2 * calls                  # the wide streaming kernel and its activation pre-arrangement
-        return calls if m <= 256 else 7       # the narrow streaming kernel, the tensor-core kernel: one launch per call; CTA pairs: per projection
+        return calls if m <= 256 else 7       # the streaming, tensor-memory and tensor-core kernels: one launch per call; CTA pairs: per projection
 
     # ------------------------------------------------------------------ the other configurations
     def cfg_c1():
@@ -479,8 +477,8 @@ def main():
         """A whole decode tick of one Llama-3-8B-shaped layer through the library (forwardBatchedDecode's layer body,
         src/transformer.zig:9656-9861): q/k/v, rope + cache append, attention over per-sequence 4-bit caches (one launch: the splits of a
         sequence merge inside a thread-block cluster), o, add + norm, gate/up, SwiGLU, down, add + the next layer's input
-        norm -- 10 calls (plus one norm before the
-        first layer), from 9 sequences on 14 launches: the wide streaming kernel is two.  8 layers' weights rotate so the weights stream from HBM."""
+        norm -- 10 launches (plus one norm before the
+        first layer).  8 layers' weights rotate so the weights stream from HBM."""
         Hd, Hq, Hkv, D, F, NL = 4096, 32, 8, 128, 14336, 8
         lw = layers[:NL] if len(layers) >= NL else None
         if lw is None:
@@ -532,7 +530,7 @@ def main():
             ms = time_graph(gr, 20, sync_ranks=False) / 20 / NL
             kv_bytes = sum(2 * Hkv * (lens[n] + 1) * (D * 4 // 8 + 8) for n in range(N))
             by = layer_bytes(N) + kv_bytes
-            res[f"N{N}_T{T}"] = {"us_per_layer_tick": ms * 1e3, "launches_per_layer": 10 if N <= 8 else 14, "tokens_per_s_through_32_layers": N / (32 * ms * 1e-3),
+            res[f"N{N}_T{T}"] = {"us_per_layer_tick": ms * 1e3, "launches_per_layer": 10, "tokens_per_s_through_32_layers": N / (32 * ms * 1e-3),
                                   "bytes_per_layer_tick": by, "GBps": by / (ms * 1e-3) / 1e9, "frac_of_hbm_peak": by / (ms * 1e-3) / 1e9 / hbm_peak}
             del gr, kt, vt, kviews, vviews
         return res

@@ -148,14 +148,14 @@ bool qmv_stream_supported(const QmmArgs& a);
 cudaError_t launch_qmv_stream(const QmmArgs& a, cudaStream_t st);
 cudaError_t launch_qmv_stream_multi(const QmmArgs* a, int count, cudaStream_t st);  // same x, <= 4 matrices
 
-// ---- qmv_wide.cu : 9..32 tokens per pass, every packed word read once (stream-K over a persistent grid) ----
+// ---- qmv_wide.cu : 9..32 tokens per pass of activations that TMA does not take, every packed word read once (stream-K over a persistent grid) ----
 bool qmv_wide_supported(const QmmArgs& a);
 cudaError_t launch_qmv_wide(const QmmArgs& a, cudaStream_t st);
 cudaError_t launch_qmv_wide_multi(const QmmArgs* a, int count, cudaStream_t st);   // same x, <= 4 matrices
 int qmv_wide_error_code();    // 0, or the code of a bounded wait that expired
 void qmv_wide_error_reset();
 
-// ---- qmv_tmem.cu : 9..128 tokens, weights streamed through tensor memory, every packed word read once ----
+// ---- qmv_tmem.cu : 9..64 tokens, weights streamed through tensor memory, every packed word read once ----
 bool qmv_tmem_supported(const QmmArgs& a);
 cudaError_t launch_qmv_tmem(const QmmArgs& a, cudaStream_t st);
 cudaError_t launch_qmv_tmem_multi(const QmmArgs* a, int count, cudaStream_t st);   // same x, <= 4 matrices

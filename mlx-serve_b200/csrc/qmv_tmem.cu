@@ -3,23 +3,25 @@
 // widths its scheduler batches, src/scheduler.zig:5147, and prompts of a few dozen tokens).
 //
 // Bound: the conversion and what a unit of 128 rows x 256 K costs beside it.  Converting takes 645 of a scheduler's issue slots a unit
-// (its bytes take 870 cycles at the copy bandwidth), the waits, votes and fences around it about 1800 cycles of latency in each group,
-// of which the three groups hide two thirds; the MMAs are 16 of 16 cycles.  us a layer of Llama-3-8B's projections (218 M weights, four
-// launches, replayed), before -> after: 27 tokens 110 -> 76 (a streaming kernel on mma.sync before), 64 tokens 143 -> 98 (tcgen05 with
-// the weights through shared memory); 4096 x 4096 alone: 13.5 -> 9.4 at 9, 16.8 -> 10.3 at 32, 26.6 -> 11.7 at 64.
+// (its bytes take 870 cycles at the copy bandwidth), of a group's 3300 cycles a unit 2400 are conversion beside the other group's; the MMAs
+// are 16 of 16 cycles.  us a layer of Llama-3-8B's projections (218 M weights, four launches, each replayed), before -> after: 16 tokens
+// 85 -> 52, 27 tokens 110 -> 61 (a streaming kernel on mma.sync before), 64 tokens 143 -> 75 (tcgen05 with the weights through shared
+// memory); 4096 x 4096 alone 13.5 -> 5.9 at 16, 16.8 -> 8.8 at 32, 26.6 -> 10.3 at 64; 512 x 512 6.4 -> 3.9, 7.8 -> 3.4, 6.9 -> 4.9.
 //  * A thread converts a weight row.  Its codes lie in a lane of registers and go to the same lane of tensor memory, the A operand of
 //    the MMA: no shuffles, no shared-memory tile, scale and bias one register each.
-//  * A group of four warps takes units in turn, half a unit (64 columns of tensor memory) at a time, and its first warp issues that
-//    half's MMAs into the group's own accumulator -- an issuer of its own would have to be woken for every half unit, and two threads'
-//    MMAs into one accumulator have no order.  The epilogue's warps add the accumulators, group by group from the tile's first unit on.
+//  * A group of four warps takes units in turn, half a unit (64 columns of tensor memory) at a time, and meets its issuer at a named barrier
+//    per slot without waiting; whether the next slot and the next codes are there is looked at while the stores of this half end.  An
+//    accumulator per group, as two threads' MMAs into one have no order; the epilogue's warps add them, from the tile's first unit's on.
 //  * One thread copies packed codes (128-byte rows), scales and biases by TMA, one x, the B operand as it is.
 //  * The CTAs of a cluster split K, each the same part for every tile of 128 rows that the cluster walks, so that its part of x mostly
 //    stays in shared memory.  At the end of a tile each hands its fp32 sums to the CTA that owns the tokens (asynchronous remote
 //    stores that count at the owner's barrier), which adds them in rank order and stores: no scratch memory, no waiting for whoever
 //    is last, and the order of the sum does not depend on timing.
-// Not kept: two CTAs an SM (512 threads at 64 registers, 113 KB: 4096 x 4096 in 6.5 us where launches of it follow each other, but a
-// layer of different matrices 359 us against 303, four deep); stream-K over all SMs with partial sums in memory (9 us for the last CTA
-// of a tile); an issuer and a scout of their own; scales read by the converting threads, or by cp.async of 8 bytes a row.
+// Not kept: stream-K over all SMs with partial sums in memory (9 us for the last CTA of a tile); one issuer, with or without a scout, for
+// all groups (a poll of a barrier costs 107 cycles, half a unit's MMAs 130); MMAs issued by a converting warp (800 cycles a unit that the
+// group waits for); scales read by the converting threads, or by cp.async of 8 bytes a row (their latency, 1000 cycles a unit of one warp);
+// the conversion unrolled over a unit (14 KB: an eighth of the rate, waiting for instructions); two forms of the kernel for short and long
+// launches (a layer, four deep: 359 us against 303 with one -- launches of different kernels refetch their instructions).
 // Every mbarrier wait is bounded: on expiry the kernel records a code, no more MMAs are issued, every warp still keeps the meetings of
 // its group, and tensor memory is freed.
 #include "stream_ptx.cuh"
