@@ -9,8 +9,12 @@
 // the M side because their number is a multiple of 256 in most models while token counts are ragged: N goes in steps of 32, so an
 // expert of 270 rows costs 288 and the tokens of a prompt divide evenly over the waves of tiles.
 //
-//  * Cluster of two CTAs, persistent, one pair per two SMs.  A tile is one or two units of up to 256 tokens.  Accumulators: two
-//    slots of 256 columns of tensor memory that units take in turn: the epilogue of one-unit tiles runs beside the next tile.
+//  * Cluster of two CTAs, persistent, one pair per two SMs.  A tile is one or two units of up to 256 tokens.  Accumulators: a
+//    ring of 16 blocks of 32 columns of tensor memory.  A unit takes the next blocks, the epilogue gives every block back as soon as it
+//    has read it, and so works beside the next tile except for the blocks that two tiles have in common (two tiles of 288 tokens: 64
+//    of 512 columns).  With two slots of 256 columns a tile of two units began after the whole epilogue of the one before, 6800 of
+//    16800 cycles at K = 768 (128 experts, us, before -> after: 256 rows an expert 768 x 2048 123 -> 117, 2048 x 768 134 -> 115; 290
+//    rows 132 -> 124, 148 -> 126).
 //  * Roles per CTA: twelve warps convert weights (three groups of four that take k-blocks in turn, a thread per weight row), four
 //    are the epilogue, and one each loads x, loads packed codes, issues the MMAs (CTA 0 only: its instructions read both CTAs'
 //    operands) and scouts for the issuer (CTA 0).  These four share a scheduler without any converting warp: beside one, the
@@ -35,7 +39,8 @@ constexpr int TILE = 128 * BK * 2, RAW = 128 * 128;   // 128 rows of one k-block
 constexpr int kMaxE = 256;                            // experts whose tables fit beside the rings; more take the room of a sixth stage
 // two units a tile: 4 stages of weights and two boxes of x; one unit: 6 stages of weights and one
 constexpr size_t kTiles = (size_t)12 * TILE + RAWB * RAW;
-constexpr int kBars = 2 * SMAX + 2 * RAWB + 4;
+constexpr int kCols = 16;                            // accumulators: a ring of blocks of 32 columns of tensor memory
+constexpr int kBars = 2 * SMAX + 2 * RAWB + 2 * kCols;
 constexpr size_t smem_of(bool grouped) { return kTiles + kBars * 8 + 48 + (grouped ? 2 * (kMaxE + 1) * 4 : 0); }
 static_assert(smem_of(true) <= 227 * 1024, "shared memory");
 // Limit of a bounded wait: 2^22 polls, each held by the hardware for kNap ns at most -- a lone waiter's for all of it; in this kernel, where
@@ -56,7 +61,8 @@ struct PairK {
   const void* rhs; int rhs_i64; int E;           // grouped: expert of every row, ascending
 };
 struct Tile {
-  int row0, row_end, units, nn0, nn1;            // tokens [row0, row_end), in units of nn0 and nn1 (multiples of 32, up to 256)
+  int row0, row_end, q;                          // tokens [row0, row_end), in steps of 32
+  int units, nn0, nn1, col0, col1;               // units of nn0 and nn1 tokens (multiples of 32, up to 256), from these blocks of columns on
   int n0, nend, wrow0, wlast;                    // output columns; first weight row of the tile, last one of the matrix
 };
 __device__ __forceinline__ bool wait_cta(uint64_t* bar, uint32_t parity) {
@@ -122,11 +128,34 @@ __device__ __forceinline__ Tile tile_at(const PairK& p, const int* s_off, const 
   }
   c.n0 = nb * 256;
   c.nend = c.n0 + 256 < p.N ? c.n0 + 256 : p.N;
-  const int q = c.row_end > c.row0 ? (c.row_end - c.row0 + 31) >> 5 : 1;
-  c.units = q > 8 ? 2 : 1;
-  c.nn0 = c.units == 2 ? ((q + 1) >> 1) << 5 : q << 5;
-  c.nn1 = (q << 5) - c.nn0;
+  c.q = c.row_end > c.row0 ? (c.row_end - c.row0 + 31) >> 5 : 1;
   return c;
+}
+// Where the accumulators of the next tile lie in the ring.  A unit is contiguous.  A tile that the ring's end would cut is cut there into
+// its two units, if x has room for two; a tile that is one unit only if starting at block 0 it met the tile before (two such tiles of 224
+// or 256 tokens take turns uncut: cutting them cost 3 %).
+struct Ring { int pos = 0, prev = 0; };          // the next free block; the first one of the tile before
+__device__ __forceinline__ void place(Tile& c, Ring& r, bool two) {
+  const int q = c.q;
+  int a = q, pos = r.pos;
+  if (q > 8 || (two && pos + q > kCols && q > r.prev)) {
+    a = kCols - pos;
+    if (pos + q <= kCols || a > 8 || q - a > 8) {
+      a = (q + 1) >> 1;
+      if (pos + q > kCols && (pos + a > kCols || q - a > pos)) pos = 0;
+    }
+  } else if (pos + q > kCols) {
+    pos = 0;
+  }
+  const int b = q - a;
+  c.units = b ? 2 : 1;
+  c.nn0 = a << 5;
+  c.nn1 = b << 5;
+  c.col0 = r.prev = pos;
+  pos += a;
+  if (pos + b > kCols) pos = 0;
+  c.col1 = pos;
+  r.pos = (pos + b) & (kCols - 1);
 }
 
 // The issuer's walk, out of line (as part of the big function its loop compiles into something much slower).  Everything the loop
@@ -140,11 +169,14 @@ __device__ __noinline__ void issue_walk(const PairK& p, const Walk a) {
   const uint32_t wd0 = U((uint32_t)make_desc(a.w_s)), xd0 = U((uint32_t)make_desc(a.x_s)), tmem = U(a.tmem), empty_s = U(a.empty_s), acc_s = U(a.acc_s);
   const int nkb = (int)U((uint32_t)a.nkb), S = (int)U((uint32_t)p.stages), ntiles = (int)U((uint32_t)a.ntiles), tstride = (int)U((uint32_t)a.tstride);
   const uint32_t xstep = U((uint32_t)((p.hmax >> 8) * (TILE >> 4)));   // a stage of x, in the descriptor's 16-byte units
-  uint32_t st = 0, u0 = 0;
+  const bool two = U((uint32_t)p.hmax) > 256u;
+  uint32_t st = 0;
+  Ring ring;
   for (int tile = (int)U((uint32_t)a.tile0); tile < ntiles; tile += tstride) {
-    const Tile tc = tile_at<GROUPED>(p, a.s_off, a.s_tcum, tile);
+    Tile tc = tile_at<GROUPED>(p, a.s_off, a.s_tcum, tile);
+    place(tc, ring, two);
     const uint32_t units = U((uint32_t)tc.units), i0 = U(idesc0 | ((uint32_t)(tc.nn0 >> 3) << 17)), i1 = U(idesc0 | ((uint32_t)(tc.nn1 >> 3) << 17));
-    const uint32_t d0 = tmem + (u0 & 1) * 256, d1 = tmem + (~u0 & 1) * 256;
+    const uint32_t c0 = U((uint32_t)tc.col0), c1 = U((uint32_t)tc.col1), d0 = tmem + c0 * 32, d1 = tmem + c1 * 32;
     for (int kb = 0; kb < nkb; ++kb) {
       asm volatile("bar.sync %0, 64;" ::"r"(1 + st) : "memory");   // the scout has seen the stage (and the accumulators' slots) ready
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -152,20 +184,18 @@ __device__ __noinline__ void issue_walk(const PairK& p, const Walk a) {
       if (elect_one()) {
 #pragma unroll
         for (int k = 0; k < BK / 16; ++k) umma2(d0, hi | (wd + 2 * k), hi | (xd + 2 * k), i0, kb > 0 || k > 0 ? 1u : 0u);
+        const bool last = kb + 1 == nkb;
+        if (last) commit2(acc_s + c0 * 8u);
         if (units == 2) {
 #pragma unroll
           for (int k = 0; k < BK / 16; ++k) umma2(d1, hi | (wd + 2 * k), hi | (xd + (TILE >> 4) + 2 * k), i1, kb > 0 || k > 0 ? 1u : 0u);
+          if (last) commit2(acc_s + c1 * 8u);
         }
         commit2(empty_s + st * 8u);
-        if (kb + 1 == nkb) {
-          commit2(acc_s + (u0 & 1) * 8u);
-          if (units == 2) commit2(acc_s + (~u0 & 1) * 8u);
-        }
       }
       __syncwarp();
       st = st + 1 == (uint32_t)S ? 0 : st + 1;
     }
-    u0 += units;
   }
 }
 
@@ -210,8 +240,8 @@ __global__ void __launch_bounds__(kThreads, 1) qmm_pair_kernel(const __grid_cons
   unsigned char* x_t = smem + S * TILE;                    // [S][units][128 x 64 bf16]: its tokens
   unsigned char* raw = smem + 12 * TILE;                   // [RAWB][128 x 128 bytes of codes]
   uint64_t* full = (uint64_t*)(raw + RAWB * RAW);
-  uint64_t *empty = full + SMAX, *raw_full = empty + SMAX, *raw_empty = raw_full + RAWB, *acc_full = raw_empty + RAWB, *acc_empty = acc_full + 2;
-  uint32_t* tmem_slot = (uint32_t*)(acc_empty + 2);
+  uint64_t *empty = full + SMAX, *raw_full = empty + SMAX, *raw_empty = raw_full + RAWB, *acc_full = raw_empty + RAWB, *acc_empty = acc_full + kCols;
+  uint32_t* tmem_slot = (uint32_t*)(acc_empty + kCols);
   volatile int& s_fail = *(volatile int*)(tmem_slot + 1);
   volatile int* s_go = (volatile int*)(tmem_slot + 2);     // [DQG][2]
   int* s_off = (int*)(tmem_slot + 2 + 2 * DQG + 2);                      // [E + 1] first row of every expert
@@ -224,7 +254,7 @@ __global__ void __launch_bounds__(kThreads, 1) qmm_pair_kernel(const __grid_cons
   if (tid == 0) {
     for (int i = 0; i < SMAX; ++i) { mbar_init(&full[i], 1 + 2 * WPG); mbar_init(&empty[i], 1); }
     for (int i = 0; i < RAWB; ++i) { mbar_init(&raw_full[i], 1); mbar_init(&raw_empty[i], WPG * KPS + (KPS < DQG ? DQG - KPS : 0)); }
-    for (int i = 0; i < 2; ++i) { mbar_init(&acc_full[i], 1); mbar_init(&acc_empty[i], 8); }
+    for (int i = 0; i < kCols; ++i) { mbar_init(&acc_full[i], 1); mbar_init(&acc_empty[i], 8); }
     s_fail = (smem_u32(smem) & 1023u) ? 308 : 0;           // misaligned window: every role leaves at once
     if (s_fail) atomicCAS(&g_pair_error, 0, 308);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -274,8 +304,10 @@ __global__ void __launch_bounds__(kThreads, 1) qmm_pair_kernel(const __grid_cons
     if (elect_one()) {
       int st = 0, round = 0;
       bool ok = true;
+      Ring ring;
       for (int tile = tile0; tile < ntiles && ok; tile += tstride) {
-        const Tile tc = at(tile);
+        Tile tc = at(tile);
+        place(tc, ring, p.hmax > 256);
         // boxes of 64 tokens of unit u that CTA r loads
         auto boxes = [&](int r, int u) {
           const int half = (u ? tc.nn1 : tc.nn0) >> 1, t0 = tc.row0 + (u ? tc.nn0 : 0) + r * half;
@@ -324,14 +356,18 @@ __global__ void __launch_bounds__(kThreads, 1) qmm_pair_kernel(const __grid_cons
     // mbarrier by the issuing thread costs more than the meeting).  When a wait runs out the scout only paces the issuer, which
     // then multiplies stale stages into accumulators nobody trusts (the status word says so).
     if (rank == 0) {
-      int st = 0, round = 0, u0 = 0, fail = 0;
+      int st = 0, round = 0, fail = 0;
+      Ring ring;
+      uint32_t used = 0, par = 0;                        // blocks that had a tile before; how often, modulo 2
       for (int tile = tile0; tile < ntiles; tile += tstride) {
-        const int units = at(tile).units;
-        for (int j = 0; j < units; ++j) {
-          const int use = (u0 + j) >> 1;
-          if (!fail && use >= 1 && !warp_wait(lane, [&] { return wait_cta(&acc_empty[(u0 + j) & 1], (use - 1) & 1); })) fail = 306;
-        }
-        u0 += units;
+        Tile tc = at(tile);
+        place(tc, ring, p.hmax > 256);
+        // a lane per block
+        const uint32_t mine = (((1u << (tc.nn0 >> 5)) - 1) << tc.col0) | (((1u << (tc.nn1 >> 5)) - 1) << tc.col1);
+        const bool held = lane < kCols && (mine & used) >> lane & 1;
+        if (!fail && !__all_sync(0xffffffffu, !held || wait_cta(&acc_empty[lane], ~(par >> lane) & 1))) fail = 306;
+        used |= mine;
+        par ^= mine;
         for (int kb = 0; kb < nkb; ++kb) {
           if (!fail && !warp_wait(lane, [&] { return wait_cta(&full[st], round & 1); })) fail = 301;
           if (!fail) asm volatile("bar.arrive %0, 64;" ::"r"(1 + st) : "memory");
@@ -431,31 +467,32 @@ __global__ void __launch_bounds__(kThreads, 1) qmm_pair_kernel(const __grid_cons
   } else {
     // epilogue: this CTA's 128 weight rows (lanes) x the tokens (columns) of every unit
     const int q = warp & 3;
-    int u0 = 0;
+    Ring ring;
+    uint32_t par = 0;                                      // how often a unit began at a block, modulo 2
     bool ok = true;
     for (int tile = tile0; tile < ntiles && ok; tile += tstride) {
-      const Tile tc = at(tile);
+      Tile tc = at(tile);
+      place(tc, ring, p.hmax > 256);
       const int n = tc.n0 + rank * 128 + q * 32 + lane;
       for (int j = 0; j < tc.units; ++j) {
-        const int slot = (u0 + j) & 1;
-        ok = warp_wait(lane, [&] { return wait_cta(&acc_full[slot], ((u0 + j) >> 1) & 1); });
+        const int col = j ? tc.col1 : tc.col0;
+        ok = warp_wait(lane, [&] { return wait_cta(&acc_full[col], (par >> col) & 1); });
         if (!ok || s_fail) { ok = false; break; }
+        par ^= 1u << col;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const int t0 = tc.row0 + (j ? tc.nn0 : 0), nt = j ? tc.nn1 : tc.nn0;
-        if (n - lane < tc.nend) {
+        const uint32_t freed = full0 + (uint32_t)((unsigned char*)&acc_empty[col] - (unsigned char*)full);
 #pragma unroll 1
-          for (int c0 = 0; c0 < nt; c0 += 32) {
-            uint32_t v[32];
-            tmem_ld32(tmem + ((uint32_t)(q * 32) << 16) + slot * 256 + c0, v);
-            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-            store_cols32(p.y + (int64_t)(t0 + c0) * p.ldy, p.ldy, v, tc.row_end - (t0 + c0), n, tc.nend, p.y_vec != 0, lane);
-          }
+        for (int c0 = 0; c0 < nt; c0 += 32) {
+          uint32_t v[32];
+          tmem_ld32(tmem + ((uint32_t)(q * 32) << 16) + col * 32 + c0, v);
+          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+          asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+          __syncwarp();
+          if (lane == 0) arrive_addr(freed + (uint32_t)c0 / 4);   // the block may be overwritten
+          if (n - lane < tc.nend) store_cols32(p.y + (int64_t)(t0 + c0) * p.ldy, p.ldy, v, tc.row_end - (t0 + c0), n, tc.nend, p.y_vec != 0, lane);
         }
-        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-        __syncwarp();
-        if (lane == 0) arrive_addr(full0 + (uint32_t)((unsigned char*)&acc_empty[slot] - (unsigned char*)full));   // the slot may be overwritten
       }
-      u0 += tc.units;
     }
     if (!ok && !s_fail) failed(305);
   }
@@ -548,7 +585,8 @@ cudaError_t launch_gather_pair(const GatherArgs& a, cudaStream_t st) {
   p.s = (const uint16_t*)a.s; p.b = (const uint16_t*)a.b; p.y = (uint16_t*)a.y;
   p.lds = a.K / a.gs; p.ldy = a.N; p.M = (int)a.I; p.N = (int)a.N; p.K = (int)a.K; p.gshift = a.gs == 128 ? 1 : 0;
   p.rhs = a.rhs; p.rhs_i64 = a.rhs_dtype == QB200_INT64; p.E = (int)a.E;
-  // two units where many experts have more than 256 rows (256 on average: 129 us against 147 with one)
+  // two units where many experts have more than 256 rows (128 experts +- 12 %, 768 x 2048 / 2048 x 768, us, two units and one: 256 rows
+  // on average 116 / 135 and 115 / 149, 230 113 / 109 and 112 / 115, 180 108 / 106 and 107 / 111)
   p.hmax = a.I > 200 * a.E && a.E <= kMaxE ? 512 : 256;
   return launch_pair(p, a.x, a.K, a.w, a.E * a.N, a.K * a.bits / 32, a.bits, true, sm_count() / 2, st);
 }
