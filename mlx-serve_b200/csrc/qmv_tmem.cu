@@ -39,7 +39,12 @@ constexpr int GRP = 2, kOwn = kSlots / GRP;                // slots of a group
 constexpr int kEpi0 = 4 * GRP, kCodesWarp = kEpi0 + 4, kXWarp = kCodesWarp + 1, kMmaWarp = kXWarp + 1, kThreads = (kMmaWarp + GRP) * 32;
 constexpr uint32_t kSpin = 1u << 22, kNap = 2000;         // polls of a bounded wait; ns the hardware may hold one
 constexpr int kBars = 2 * kMaxCodes + kSlots + 2 * kMaxX + 4 + 4;
-constexpr size_t kBarBytes = kBars * 8 + 32, kSmem = 225 * 1024, kSmemTwo = 113 * 1024;
+constexpr size_t kBarBytes = kBars * 8 + 32, kSmem = 225 * 1024;
+// One CTA an SM: each allocates all of tensor memory.  Were there room for a second one of the grid (or of another stream's), it would wait
+// for the first one's, its peers for its sums, and another cluster's CTAs the other way round.  (At 16 tokens two an SM, the next launch's
+// beside this one's, took 51.7 us a layer of Llama-3-8B's projections against 57.5, and had just that fault.)
+constexpr size_t kSmemLeast = 116 * 1024;
+static_assert(2 * kSmemLeast > 228 * 1024, "two CTAs would fit an SM");
 __device__ int g_tmem_error = 0;                          // 0, or the code of a wait that expired
 
 struct TmMaps { CUtensorMap w[kMaxMat], s[kMaxMat], b[kMaxMat]; };
@@ -201,8 +206,8 @@ __device__ __forceinline__ void tmem_ld4(uint32_t taddr, uint32_t (&r)[4]) {
   asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(taddr));
 }
 
-template <int BITS, int PER_SM>
-__global__ void __launch_bounds__(kThreads, PER_SM) qmv_tmem_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ TmMaps wm,
+template <int BITS>
+__global__ void __launch_bounds__(kThreads, 1) qmv_tmem_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ TmMaps wm,
                                                                const __grid_constant__ TmK p) {
   extern __shared__ __align__(1024) unsigned char smem[];
   constexpr int kCodes = 128 * CK * BITS / 8;              // packed codes of a unit: 128-byte rows, one box at 4 bits, two at 8
@@ -594,7 +599,7 @@ cudaLaunchConfig_t config(cudaLaunchAttribute (&attr)[2], int grid, int cluster,
   return cfg;
 }
 // Clusters of this size that the device holds at once (0: none), looked up once per device; index 1: its SMs.
-template <int BITS, int PER_SM>
+template <int BITS>
 cudaError_t clusters_of(int cluster, int* n) {
   static int cached[64][kMaxCluster + 1] = {};
   int dev = 0;
@@ -604,7 +609,7 @@ cudaError_t clusters_of(int cluster, int* n) {
   const int sms = sm_count();
   std::lock_guard<std::mutex> lk(setup_mutex());
   if (cached[dev][0] == 0) {
-    auto kern = qmv_tmem_kernel<BITS, PER_SM>;
+    auto kern = qmv_tmem_kernel<BITS>;
     e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem);
     if (e != cudaSuccess) return e;
     note_reader((const void*)kern);
@@ -626,12 +631,12 @@ cudaError_t clusters_of(int cluster, int* n) {
 
 // The cluster size: waves of tiles x (units of a tile's share + hand-over of its sums), in units of about 0.65 us
 struct Plan { int cluster, ncl, per, ku; };                // CTAs that split K, clusters, tiles and units of K of one at most
-template <int BITS, int PER_SM>
+template <int BITS>
 cudaError_t plan(const TmK& p, int most, Plan* out) {
   const int ntiles = p.tile0[kMaxMat];
   double best = -1.0;
   for (int c = 1, n = 0; c <= most && c <= p.spb; ++c) {
-    const cudaError_t e = clusters_of<BITS, PER_SM>(c, &n);
+    const cudaError_t e = clusters_of<BITS>(c, &n);
     if (e != cudaSuccess) return e;
     if (n < 1) continue;
     const int t = (ntiles + n - 1) / n, ku = (p.spb + c - 1) / c;
@@ -641,15 +646,15 @@ cudaError_t plan(const TmK& p, int most, Plan* out) {
   return best < 0 ? cudaErrorInvalidConfiguration : cudaSuccess;
 }
 
-template <int BITS, int PER_SM>
+template <int BITS>
 cudaError_t launch_inst(const CUtensorMap& xmap, const TmMaps& wm, TmK p, cudaStream_t st) {
   constexpr int stage = 128 * CK * BITS / 8 + 2 * 2048;
   p.dbufs = 2 * GRP * p.nt <= 128 ? 2 : 1;                 // 512 columns of tensor memory: 6 x 64 for the A operand, groups x accumulators x tokens
   for (int most : {kMaxCluster, 1}) {                      // (where the device places no such cluster: CTAs by themselves)
     Plan pl;
-    cudaError_t e = plan<BITS, PER_SM>(p, most, &pl);
+    cudaError_t e = plan<BITS>(p, most, &pl);
     if (e != cudaSuccess) return e;
-    const int c = pl.cluster, xu = p.nt * 512, rx1 = c > 1 ? c * ((p.nt / 4 + c - 1) / c) * 2048 : 0, room = (int)((PER_SM == 2 ? kSmemTwo : kSmem) - kBarBytes);
+    const int c = pl.cluster, xu = p.nt * 512, rx1 = c > 1 ? c * ((p.nt / 4 + c - 1) / c) * 2048 : 0, room = (int)(kSmem - kBarBytes);
     p.cluster = c;
     p.rx = pl.per > 1 && c > 1 && room - 2 * rx1 >= 3 * xu + 3 * stage ? 2 : 1;
     const int left = room - p.rx * rx1;
@@ -666,9 +671,10 @@ cudaError_t launch_inst(const CUtensorMap& xmap, const TmMaps& wm, TmK p, cudaSt
     if (p.cs > kMaxCodes) p.cs = kMaxCodes;
     p.cs = p.cs / GRP * GRP;
     if (p.cs < GRP) return cudaErrorInvalidConfiguration;
+    const size_t smem = (size_t)(p.cs * stage + p.xs * xu + p.rx * rx1) + kBarBytes;
     cudaLaunchAttribute attr[2];
-    const cudaLaunchConfig_t cfg = config(attr, pl.ncl * c, c, (size_t)(p.cs * stage + p.xs * xu + p.rx * rx1) + kBarBytes, st);
-    e = c > 1 ? launch_clusters(cfg, qmv_tmem_kernel<BITS, PER_SM>, xmap, wm, p) : cudaLaunchKernelEx(&cfg, qmv_tmem_kernel<BITS, PER_SM>, xmap, wm, p);
+    const cudaLaunchConfig_t cfg = config(attr, pl.ncl * c, c, smem < kSmemLeast ? kSmemLeast : smem, st);
+    e = c > 1 ? launch_clusters(cfg, qmv_tmem_kernel<BITS>, xmap, wm, p) : cudaLaunchKernelEx(&cfg, qmv_tmem_kernel<BITS>, xmap, wm, p);
     if (e == cudaSuccess || c == 1) return e;
     (void)cudaGetLastError();
   }
@@ -721,11 +727,7 @@ cudaError_t launch_qmv_tmem_multi(const QmmArgs* a, int count, cudaStream_t st) 
   p.tile0[kMaxMat] = tiles;
   if (!make_map(&xmap, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, (const uint16_t*)a[0].x + a[0].xb.offset(0), a[0].K, a[0].M, a[0].ldx * 2, 64, p.nt)) return cudaErrorInvalidValue;
   p.early = weights_settled(st);
-  // Up to 16 tokens at 4 bits two CTAs fit an SM (64 registers, 113 KB), so that the next launch's is set up and has filled its ring when
-  // this one ends: a layer of Llama-3-8B's projections 51.7 us against 57.5.  With more to hold, the shallower rings cost more than that
-  // (27 tokens 73 against 61, 9 at 8 bits 76 / 59), as a launch of a few units has nothing to gain.
-  if (bits == 8) return launch_inst<8, 1>(xmap, wm, p, st);
-  return p.nt <= 16 && tiles * p.spb > 4 ? launch_inst<4, 2>(xmap, wm, p, st) : launch_inst<4, 1>(xmap, wm, p, st);
+  return bits == 8 ? launch_inst<8>(xmap, wm, p, st) : launch_inst<4>(xmap, wm, p, st);
 }
 cudaError_t launch_qmv_tmem(const QmmArgs& a, cudaStream_t st) { return launch_qmv_tmem_multi(&a, 1, st); }
 
