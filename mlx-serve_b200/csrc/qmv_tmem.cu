@@ -5,8 +5,8 @@
 // Bound: the conversion and what a unit of 128 rows x 256 K costs beside it.  Converting takes 645 of a scheduler's issue slots a unit
 // (its bytes take 870 cycles at the copy bandwidth), of a group's 3300 cycles a unit 2400 are conversion beside the other group's; the MMAs
 // are 16 of 16 cycles.  us a layer of Llama-3-8B's projections (218 M weights, four launches, each replayed), before -> after: 16 tokens
-// 85 -> 52, 27 tokens 110 -> 61 (a streaming kernel on mma.sync before), 64 tokens 143 -> 75 (tcgen05 with the weights through shared
-// memory); 4096 x 4096 alone 13.5 -> 5.9 at 16, 16.8 -> 8.8 at 32, 26.6 -> 10.3 at 64; 512 x 512 6.4 -> 3.9, 7.8 -> 3.4, 6.9 -> 4.9.
+// 85 -> 58, 27 tokens 110 -> 61 (a streaming kernel on mma.sync before), 64 tokens 143 -> 75 (tcgen05 with the weights through shared
+// memory); 4096 x 4096 alone 16.8 -> 8.8 at 32, 26.6 -> 10.3 at 64; 512 x 512 7.8 -> 3.4, 6.9 -> 4.9.
 //  * A thread converts a weight row.  Its codes lie in a lane of registers and go to the same lane of tensor memory, the A operand of
 //    the MMA: no shuffles, no shared-memory tile, scale and bias one register each.
 //  * A group of four warps takes units in turn, half a unit (64 columns of tensor memory) at a time, and meets its issuer at a named barrier
