@@ -536,7 +536,8 @@ __global__ void __launch_bounds__(kThreads, 1) qmv_tmem_kernel(const __grid_cons
       uint32_t acc = 0;
       if (!p.ring) xi = k;
       for (; k < ku; k += GRP) {
-        if (p.ring || t == 0) wait(&x_full[xi], xround);
+        // (x that stays: units of K change groups from tile to tile where ku is odd, so a group has met all of its units after GRP tiles)
+        if (p.ring || t < GRP) wait(&x_full[xi], xround);
 #pragma unroll 1
         for (int h = 0; h < 2; ++h) {
           asm volatile("bar.sync %0, 160;" ::"r"(2 + grp * kOwn + slot) : "memory");

@@ -16,7 +16,7 @@ pytestmark = pytest.mark.gpu
     (4, 64, 9, 1, 256), (4, 64, 16, 127, 512), (4, 128, 17, 128, 768), (4, 64, 32, 129, 1280),      # one row; edges of tiles; scales' rows of 24, 40 bytes
     (4, 64, 33, 300, 2048), (4, 64, 48, 640, 256), (4, 128, 64, 513, 1024), (4, 64, 64, 100, 4352),
     (8, 64, 9, 130, 256), (8, 128, 16, 257, 1792), (8, 64, 27, 64, 3072), (8, 64, 49, 200, 512), (8, 128, 64, 129, 768),
-    (4, 64, 13, 20000, 256), (8, 64, 32, 9000, 512),                                                # several tiles a cluster
+    (4, 64, 13, 20000, 256), (8, 64, 32, 9000, 512), (8, 64, 32, 30000, 512),                       # (on 148 SMs) two tiles a CTA, one, two
     (4, 64, 20, 256, 16384), (8, 64, 64, 140, 8192)])                                               # x in a ring
 def test_edges(bits, gs, M, N, K):
     import qb200
@@ -60,4 +60,66 @@ def test_several_matrices():
     finally:
         qb200.lib().qb200_debug_refuse_clusters(False)
     gate_bf16(alone.float().cpu().numpy(), qo.qmm(x, *ws[0], 64, 4, bf16_weights=True), "no clusters")
+    assert qb200.lib().qb200_debug_tc_status() == 0
+
+
+def _weight(n, k, gs, bits, g):
+    import qb200
+    return qb200.quantize((torch.randn((n, k), device="cuda", generator=g) * 0.02).to(torch.bfloat16), gs, bits)
+
+
+def _gate_exact(y, x, w, gs, bits, what):
+    """Every output against the 64-bit sum: the rounding of the result to bf16 (2^-8 of it at most), and fp32 sums of K products in any
+    order (2^-23 a step)."""
+    import qb200
+    wd, xd = qb200.dequantize(*w, gs, bits, dtype=torch.bfloat16).double(), x.double()
+    ref = xd @ wd.t()
+    tol = 2.0 ** -8 * ref.abs() + x.shape[1] * 2.0 ** -23 * (xd.abs() @ wd.abs().t())
+    bad = ~((y.double() - ref).abs() <= tol)
+    assert not bool(bad.any()), f"{what}: {int(bad.sum())} of {bad.numel()}"
+
+
+# (on 148 SMs: tiles of 128 rows, the CTAs that share a row tile, units of K of one)
+@pytest.mark.parametrize("bits,gs,M,N,K", [
+    (4, 64, 9, 19500, 256), (4, 64, 32, 40000, 256), (8, 64, 17, 40000, 256), (4, 128, 64, 40000, 256),    # 1 CTA, 1 unit: the second group's first one is in the second tile
+    (4, 64, 16, 40000, 768), (8, 128, 32, 19500, 1280), (4, 64, 25, 11264, 2560)])                         # odd shares: units change groups from tile to tile
+def test_activations_of_the_kernel_before(bits, gs, M, N, K):
+    """Two linears in a graph, the first one's output the second one's activations: the second is let in early and converts its weights
+    meanwhile, and has to wait for every unit of x."""
+    import qb200
+    g = torch.Generator(device="cuda").manual_seed(N + K + M)
+    w1, w2 = _weight(K, 14336, 64, 4, g), _weight(N, K, gs, bits, g)
+    x = torch.randn((M, 14336), device="cuda", generator=g).to(torch.bfloat16)
+    h, y = (torch.zeros((M, n), dtype=torch.bfloat16, device="cuda") for n in (K, N))
+
+    def chain():
+        qb200.quantized_matmul(x, *w1, True, 64, 4, out=h)
+        qb200.quantized_matmul(h, *w2, True, gs, bits, out=y)
+
+    chain()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        chain()
+    for i in range(5):
+        x.copy_(torch.randn(x.shape, device="cuda", generator=g))
+        torch.cuda.synchronize()
+        graph.replay()
+        _gate_exact(h, x, w1, 64, 4, f"first, replay {i}")
+        _gate_exact(y, h, w2, gs, bits, f"second, replay {i}")
+    assert qb200.lib().qb200_debug_tc_status() == 0
+
+
+@pytest.mark.parametrize("M", [16, 32, 64])
+@pytest.mark.parametrize("bits,gs,N,K", [
+    (4, 64, 28672, 4096), (8, 64, 13000, 4096),     # clusters of four, seven and three tiles each
+    (4, 128, 11648, 2560), (4, 64, 12000, 2304)])   # clusters of three, two tiles each: shares of 3, 3, 4 units and of 3
+def test_several_tiles_a_cluster(bits, gs, N, K, M):
+    import qb200
+    g = torch.Generator(device="cuda").manual_seed(N + K + M)
+    w = _weight(N, K, gs, bits, g)
+    x = torch.randn((M, K), device="cuda", generator=g).to(torch.bfloat16)
+    y = qb200.quantized_matmul(x, *w, True, gs, bits)
+    _gate_exact(y, x, w, gs, bits, f"{M} x {N} x {K}")
+    assert torch.equal(qb200.quantized_matmul(x, *w, True, gs, bits), y)   # the order of the sum does not depend on timing
     assert qb200.lib().qb200_debug_tc_status() == 0
