@@ -685,6 +685,11 @@ template <int BITS>
 cudaError_t launch_bits(const StreamK& p, cudaStream_t st) {
   int nt; bool m1;
   pick_inst(p, &nt, &m1);
+  if (m1) {   // (a last block of one token, whose K the other blocks stage in passes, may be too long for the one-token form)
+    StreamK q = p;
+    int grid; size_t smem;
+    m1 = plan_stream(q, 1, true, &grid, &smem);
+  }
   if (m1) return launch_inst<BITS, 1, true>(p, st);
   if (nt == 1) return launch_inst<BITS, 1, false>(p, st);
   return launch_inst<BITS, 2, false>(p, st);

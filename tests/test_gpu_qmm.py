@@ -282,6 +282,19 @@ def test_fp32_activations_just_below_a_power_of_two(M):
     gate_f32(y.cpu().numpy(), ref, "fp32 activations at the clamp")
 
 
+@pytest.mark.parametrize("bits", [4, 8])
+@pytest.mark.parametrize("M", [9, 17, 33])
+def test_last_block_of_one_token_at_a_long_contraction(M, bits):
+    """fp32 activations go in blocks of eight tokens; the last one's single token has a K that the one-token form does not stage."""
+    import qb200
+    rng = np.random.default_rng(M + bits)
+    K = 33024
+    q, s, b = make_weight(rng, (100, K), 64, bits)
+    x = rand_bf16(rng, (M, K))
+    y = qb200.quantized_matmul(torch.from_numpy(x).cuda(), *dev_triple(q, s, b), True, 64, bits)
+    gate_f32(y.cpu().numpy(), qo.qmm(x, q, s, b, 64, bits), "fp32 activations")
+
+
 def test_strided_operands_and_1d_x():
     import qb200
     rng = np.random.default_rng(13)
