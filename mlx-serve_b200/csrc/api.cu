@@ -327,6 +327,8 @@ static int64_t wide_max_tokens() {
   return v;
 }
 static bool takes_wide(const QmmArgs& a) { return a.M > 8 && a.M <= wide_max_tokens() && qmv_wide_supported(a); }
+// (up to 32 tokens, what the wide kernel does not serve -- a contraction above 16384 -- keeps the narrow one's weights in fp32)
+static bool takes_tmem(const QmmArgs& a) { return qmv_tmem_supported(a) && (a.M > 32 || qmv_wide_supported(a) || !qmv_stream_supported(a)); }
 
 // What the tuned kernels decline -- K no multiple of 256, group size 32, group size 128 at 8 bits -- goes to one of four kernels,
 // by times of each over M 1 - 64, N 100 - 12000, K 128 - 4416 (us a call, replayed):
@@ -338,7 +340,7 @@ static bool takes_wide(const QmmArgs& a) { return a.M > 8 && a.M <= wide_max_tok
 //  * the rest to the fp16 streaming kernel.  (Where qmv_stream and qmv_wide serve a shape they are faster than either.)
 enum class Ragged { none, generic, mma, f16, tile };
 static Ragged ragged_kernel(const QmmArgs& a) {
-  if (takes_wide(a) || qmv_tmem_supported(a) || (a.M > 8 && qmm_tc_supported(a)) || qmv_stream_supported(a)) return Ragged::none;
+  if (takes_wide(a) || (a.M > 8 && qmm_tc_supported(a)) || qmv_stream_supported(a)) return Ragged::none;
   const bool mma = qmv_mma_supported(a), f16 = qmv_f16_supported(a), tile = qmm_tile_supported(a);
   if ((double)a.M * a.N * a.K * a.nbatch <= 3.6e6 && !mma) return Ragged::generic;
   if (mma) {
@@ -360,7 +362,7 @@ static bool launched(cudaError_t e) {
 static cudaError_t dispatch_qmm(const QmmArgs& a, cudaStream_t s) {
   if (!a.transpose) return qmv_rows_supported(a) ? launch_qmv_rows(a, s) : launch_qmm_generic(a, s);
   if (a.nbatch > 1 && qmv_shortk_supported(a)) return launch_qmv_shortk(a, s);   // one W per batch element, short K: q @ K^T
-  if (qmv_tmem_supported(a)) return launch_qmv_tmem(a, s);
+  if (takes_tmem(a)) return launch_qmv_tmem(a, s);
   if (takes_wide(a)) return launch_qmv_wide(a, s);
   if (qmm_pair_supported(a) && launched(launch_qmm_pair(a, s))) return cudaSuccess;
   if (a.M > wide_max_tokens() && a.M > 8 && qmm_tc_supported(a)) return launch_qmm_tc(a, s);
@@ -411,7 +413,7 @@ QB200_API int qb200_quantized_matmul_batch(qb200_tensor* const* res, const qb200
       if (st) return st;
       // the matrices share a launch where the single call would take a streaming kernel (same rule as dispatch_qmm)
       f16 = f16 && !empty[i] && a[i].K == a[0].K && ragged_kernel(a[i]) == Ragged::f16;
-      tmem = tmem && !empty[i] && qmv_tmem_supported(a[i]) && a[i].K == a[0].K;
+      tmem = tmem && !empty[i] && takes_tmem(a[i]) && a[i].K == a[0].K;
       wide = wide && !empty[i] && takes_wide(a[i]) && a[i].K == a[0].K;
       fuse = fuse && !empty[i] && a[i].M <= 8 && qmv_stream_supported(a[i]) && a[i].K == a[0].K;
     }

@@ -26,6 +26,21 @@ def test_edges(bits, gs, M, N, K):
     assert qb200.lib().qb200_debug_tc_status() == 0
 
 
+@pytest.mark.parametrize("bits,gs,M,N,K", [(4, 64, 12, 500, 16640), (8, 64, 32, 300, 20480), (4, 128, 20, 400, 28672), (8, 128, 9, 100, 16640), (4, 64, 33, 200, 16640)])
+def test_long_contractions(bits, gs, M, N, K):
+    """Above 16384 the weight term is fp32 up to 32 tokens, but at 8 bits of groups of 128; alone and two matrices in a call."""
+    import qb200
+    rng = np.random.default_rng(M + N + K)
+    q, s, b = make_weight(rng, (N, K), gs, bits)
+    x = rand_bf16(rng, (M, K))
+    _run(x, q, s, b, gs, bits)
+    dw, dx = dev_triple(q, s, b), to_dev_bf16(qo.f32_to_bf16(x))
+    outs = [torch.empty((M, N), dtype=torch.bfloat16, device="cuda") for _ in range(2)]
+    qb200.quantized_matmul_batch(dx, [dw, dw], outs, True, gs, bits)
+    for y in outs:
+        gate_bf16(y.float().cpu().numpy(), qo.qmm(x, q, s, b, gs, bits, bf16_weights=M > 32 or gs * bits == 1024), "two matrices")
+
+
 @pytest.mark.parametrize("bits", [4, 8])
 def test_scales_of_all_sizes(bits):
     """Groups from 2^-30 to 2^30: those that the conversion of codes as subnormals takes, those beyond, and both in a unit."""
