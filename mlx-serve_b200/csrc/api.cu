@@ -353,7 +353,8 @@ static Ragged ragged_kernel(const QmmArgs& a) {
   return mma ? Ragged::mma : Ragged::generic;
 }
 
-// Kernels whose launch is a cluster give way to the ones that served their shapes before where the device places none.
+// Kernels whose launch is a cluster, or whose rows the driver has to describe (a pitch that its tensor maps do not take), give way to the
+// ones that served their shapes before.
 static bool launched(cudaError_t e) {
   if (e == cudaSuccess) return true;
   (void)cudaGetLastError();
@@ -362,7 +363,7 @@ static bool launched(cudaError_t e) {
 static cudaError_t dispatch_qmm(const QmmArgs& a, cudaStream_t s) {
   if (!a.transpose) return qmv_rows_supported(a) ? launch_qmv_rows(a, s) : launch_qmm_generic(a, s);
   if (a.nbatch > 1 && qmv_shortk_supported(a)) return launch_qmv_shortk(a, s);   // one W per batch element, short K: q @ K^T
-  if (takes_tmem(a)) return launch_qmv_tmem(a, s);
+  if (takes_tmem(a) && launched(launch_qmv_tmem(a, s))) return cudaSuccess;
   if (takes_wide(a)) return launch_qmv_wide(a, s);
   if (qmm_pair_supported(a) && launched(launch_qmm_pair(a, s))) return cudaSuccess;
   if (a.M > wide_max_tokens() && a.M > 8 && qmm_tc_supported(a)) return launch_qmm_tc(a, s);
@@ -418,20 +419,22 @@ QB200_API int qb200_quantized_matmul_batch(qb200_tensor* const* res, const qb200
       fuse = fuse && !empty[i] && a[i].M <= 8 && qmv_stream_supported(a[i]) && a[i].K == a[0].K;
     }
     // beyond the streaming kernels' widths, up to 256 tokens: one launch of the tensor-core kernel over all matrices
-    bool tc = n > 1 && !tmem && !wide && !fuse && !f16;
-    for (int i = 0; i < n && tc; ++i) tc = !empty[i] && a[i].M > wide_max_tokens() && a[i].M > 8 && !qmm_pair_supported(a[i]);
-    tc = tc && qmm_tc_multi_supported(a, n);
+    auto takes_tc = [&] {
+      for (int i = 0; i < n; ++i)
+        if (empty[i] || a[i].M <= wide_max_tokens() || a[i].M <= 8 || qmm_pair_supported(a[i])) return false;
+      return qmm_tc_multi_supported(a, n);
+    };
     cudaError_t e = cudaSuccess;
     if (f16 && launched(launch_qmv_f16_multi(a, n, (cudaStream_t)s))) {
       // one launch has taken all of them
-    } else if (tmem) {
-      e = launch_qmv_tmem_multi(a, n, (cudaStream_t)s);
+    } else if (tmem && launched(launch_qmv_tmem_multi(a, n, (cudaStream_t)s))) {
+      // and here
     } else if (wide) {
       e = launch_qmv_wide_multi(a, n, (cudaStream_t)s);
-    } else if (tc) {
-      e = launch_qmm_tc_multi(a, n, (cudaStream_t)s);
     } else if (fuse) {
       e = launch_qmv_stream_multi(a, n, (cudaStream_t)s);
+    } else if (n > 1 && !f16 && takes_tc()) {
+      e = launch_qmm_tc_multi(a, n, (cudaStream_t)s);
     } else {
       for (int i = 0; i < n && e == cudaSuccess; ++i)
         if (!empty[i]) e = dispatch_qmm(a[i], (cudaStream_t)s);

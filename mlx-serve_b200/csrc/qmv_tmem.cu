@@ -688,6 +688,7 @@ bool qmv_tmem_supported(const QmmArgs& a) {
   if (!((a.bits == 4 || a.bits == 8) && (a.gs == 64 || a.gs == 128))) return false;
   if (a.M <= 8 || a.M > kMaxNt || a.N < 1 || a.N > (1 << 24) || a.K < CK || a.K % CK != 0 || a.K > (1 << 20)) return false;
   if ((((uintptr_t)a.x) & 15) != 0 || (a.ldx * 2) % 16 != 0 || (((uintptr_t)a.w) & 15) != 0 || (a.ldw * 4) % 16 != 0) return false;
+  if (a.ldx < a.K || a.ldw * 32 < a.K * a.bits) return false;   // broadcast or overlapping rows: no form of a tensor map
   const uintptr_t al = a.gs == 64 ? 7 : 3;   // a unit's scales in one access
   if ((((uintptr_t)a.s) & al) != 0 || (((uintptr_t)a.b) & al) != 0 || (a.lds * 2) & (int64_t)al) return false;
   return get_encode() != nullptr;
@@ -715,7 +716,7 @@ cudaError_t launch_qmv_tmem_multi(const QmmArgs* a, int count, cudaStream_t st) 
     p.lds[i] = q.lds; p.ldy[i] = q.ldy;
     p.tile0[i] = tiles;
     if (i < count) tiles += ((int)q.N + 127) / 128;
-    p.sb_tma = p.sb_tma && q.lds % 8 == 0 && (((uintptr_t)p.s[i] | (uintptr_t)p.b[i]) & 15) == 0;
+    p.sb_tma = p.sb_tma && q.lds % 8 == 0 && q.lds >= q.K / q.gs && (((uintptr_t)p.s[i] | (uintptr_t)p.b[i]) & 15) == 0;
   }
   for (int i = 0; i < count; ++i) {
     const QmmArgs& q = a[i];

@@ -138,3 +138,48 @@ def test_several_tiles_a_cluster(bits, gs, N, K, M):
     _gate_exact(y, x, w, gs, bits, f"{M} x {N} x {K}")
     assert torch.equal(qb200.quantized_matmul(x, *w, True, gs, bits), y)   # the order of the sum does not depend on timing
     assert qb200.lib().qb200_debug_tc_status() == 0
+
+
+@pytest.mark.parametrize("bits,gs", [(4, 64), (8, 64), (4, 128)])
+@pytest.mark.parametrize("M,N,K", [(9, 130, 256), (16, 640, 1280), (20, 1000, 2048), (32, 300, 4352)])
+def test_activations_off_16_bytes(bits, gs, M, N, K):
+    """Rows of x that no tensor map takes: the wide streaming kernel, alone and two matrices in a call."""
+    import qb200
+    rng = np.random.default_rng(M + N + K)
+    ws = [make_weight(rng, (n, K), gs, bits) for n in (N, 77)]
+    x = rand_bf16(rng, (M, K + 5))
+    dx, dev = to_dev_bf16(qo.f32_to_bf16(x))[:, 3:K + 3], [dev_triple(*w) for w in ws]
+    refs = [qo.qmm(np.ascontiguousarray(x[:, 3:K + 3]), *w, gs, bits, bf16_weights=True) for w in ws]
+    gate_bf16(qb200.quantized_matmul(dx, *dev[0], True, gs, bits).float().cpu().numpy(), refs[0], "alone")
+    outs = [torch.empty((M, n), dtype=torch.bfloat16, device="cuda") for n in (N, 77)]
+    qb200.quantized_matmul_batch(dx, dev, outs, True, gs, bits)
+    for y, ref in zip(outs, refs):
+        gate_bf16(y.float().cpu().numpy(), ref, "two matrices")
+    assert qb200.lib().qb200_debug_tc_status() == 0
+
+
+@pytest.mark.parametrize("M", [9, 32])
+def test_rows_that_no_tensor_map_takes(M):
+    """Broadcast and overlapping rows of x, of the weights and of their scales, and a single row of a pitch beyond a map's."""
+    import qb200
+    rng = np.random.default_rng(M)
+    N, K = 200, 512
+    w, x = make_weight(rng, (N, K), 64, 4), rand_bf16(rng, (M, K))
+    dev, dx, flat = dev_triple(*w), to_dev_bf16(qo.f32_to_bf16(x)), rand_bf16(rng, (K + 8 * M,))
+    slid = np.stack([flat[8 * i:8 * i + K] for i in range(M)])
+    cases = {
+        "x of one row": (dx[:1].expand(M, K), dev, x[:1].repeat(M, 0), w),
+        "x as windows": (to_dev_bf16(qo.f32_to_bf16(flat)).as_strided((M, K), (8, 1)), dev, slid, w),
+        "weights of one row": (dx, [t[:1].expand(N, t.shape[1]) for t in dev], x, [t[:1].repeat(N, 0) for t in w]),
+        "scales of one row": (dx, [dev[0]] + [t[:1].expand(N, t.shape[1]) for t in dev[1:]], x, [w[0]] + [t[:1].repeat(N, 0) for t in w[1:]]),
+        "one row, no pitch": (dx, [t.as_strided((1, t.shape[1]), (0, 1)) for t in dev], x, [t[:1] for t in w]),
+        "one row, any pitch": (dx, [t.as_strided((1, t.shape[1]), (1 << 40, 1)) for t in dev], x, [t[:1] for t in w]),
+    }
+    for what, (xd, wd, xh, wh) in cases.items():
+        ref = qo.qmm(np.ascontiguousarray(xh), *[np.ascontiguousarray(t) for t in wh], 64, 4, bf16_weights=True)
+        gate_bf16(qb200.quantized_matmul(xd, *wd, True, 64, 4).float().cpu().numpy(), ref, what)
+        outs = [torch.empty((M, ref.shape[1]), dtype=torch.bfloat16, device="cuda") for _ in range(2)]
+        qb200.quantized_matmul_batch(xd, [wd, wd], outs, True, 64, 4)
+        for y in outs:
+            gate_bf16(y.float().cpu().numpy(), ref, what + ", twice")
+    assert qb200.lib().qb200_debug_tc_status() == 0
