@@ -108,8 +108,8 @@ QB200_API int qb200_debug_tc_status(void);
 /* Clears that code (it is sticky: once set it stays until cleared).  A host should read the status once per step
  * after its stream synchronisation -- a non-zero code means a result of that step is incomplete -- and clear it. */
 QB200_API void qb200_debug_tc_reset(void);
-/* For tests of that: how many polls a wait of the fp16 streaming kernel takes before it gives up, in the launches of the calling
- * thread from now on (below 0: none, so that the kernel gives up at its first wait; 0: the kernel's own limit). */
+/* For tests of that: how many polls a wait of the fp16 streaming kernel and of the tensor-memory kernel takes before it gives up, in the
+ * launches of the calling thread from now on (below 0: none, so that the kernel gives up at its first wait; 0: the kernel's own limit). */
 QB200_API void qb200_debug_wait_polls(int polls);
 /* For tests: whether a linear launched on this stream now would read its weights before the kernels ahead of it are complete.  It does
  * only under stream capture, behind kernels of this library that write no weights; weights may come from earlier work in the stream

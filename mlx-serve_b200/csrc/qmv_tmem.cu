@@ -22,8 +22,9 @@
 // group waits for); scales read by the converting threads, or by cp.async of 8 bytes a row (their latency, 1000 cycles a unit of one warp);
 // the conversion unrolled over a unit (14 KB: an eighth of the rate, waiting for instructions); two forms of the kernel for short and long
 // launches (a layer, four deep: 359 us against 303 with one -- launches of different kernels refetch their instructions).
-// Every mbarrier wait is bounded: on expiry the kernel records a code, no more MMAs are issued, every warp still keeps the meetings of
-// its group, and tensor memory is freed.
+// Every mbarrier wait is bounded.  A role whose wait runs out records a code and issues no more copies or MMAs, so that the waits of the
+// others run out in turn and nothing is stored; converting warps and issuers still keep every meeting, and tensor memory is freed.  (The
+// loops are delicate: a failure word looked at between two polls, or a limit that is no constant, cost 2 - 5 % of a launch.)
 #include "stream_ptx.cuh"
 #include "tc_ptx.cuh"
 
@@ -60,6 +61,7 @@ struct TmK {
   int rx;                    // buffers for the peers' sums: 2, or 1 where a cluster has one tile
   int sb_tma;                // scales and biases by TMA: their rows are 16-byte aligned
   int early;                 // the weights may be read before the previous grid is complete
+  uint32_t polls;            // SHORT: of a wait, before it gives up
 };
 
 #define QB_SEL4(arr, i) ((i) == 0 ? (arr)[0] : ((i) == 1 ? (arr)[1] : ((i) == 2 ? (arr)[2] : (arr)[3])))
@@ -70,9 +72,9 @@ __device__ __forceinline__ int mat_of(const TmK& p, int tile) {
   if (p.nmat > 3 && tile >= p.tile0[3]) mi = 3;
   return mi;
 }
-__device__ __forceinline__ bool wait_cta(uint64_t* bar, uint32_t parity) {
+__device__ __forceinline__ bool wait_cta(uint64_t* bar, uint32_t parity, uint32_t polls) {
   const uint32_t addr = smem_u32(bar);
-  for (uint32_t it = 0; it < kSpin; ++it) {
+  for (uint32_t it = 0; it < polls; ++it) {
     uint32_t done;
     asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\tselp.u32 %0, 1, 0, p;\n\t}"
                  : "=r"(done) : "r"(addr), "r"(parity), "r"(kNap) : "memory");
@@ -87,7 +89,7 @@ __device__ __forceinline__ bool test_cta(uint64_t* bar, uint32_t parity) {
   return done != 0;
 }
 // A whole warp waits.  All lanes poll (107 cycles when the phase is complete; one lane for the others, 134 and a divergent branch).
-__device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity) { return __all_sync(0xffffffffu, wait_cta(bar, parity)); }
+__device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity, uint32_t polls) { return __all_sync(0xffffffffu, wait_cta(bar, parity, polls)); }
 __device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void umma_ta(uint32_t d, uint32_t a, uint64_t bd, uint32_t idesc, uint32_t accum) {
   asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
@@ -206,7 +208,8 @@ __device__ __forceinline__ void tmem_ld4(uint32_t taddr, uint32_t (&r)[4]) {
   asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(taddr));
 }
 
-template <int BITS>
+// SHORT: the launch says how long a wait may be, for tests of waits that run out
+template <int BITS, bool SHORT>
 __global__ void __launch_bounds__(kThreads, 1) qmv_tmem_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ TmMaps wm,
                                                                const __grid_constant__ TmK p) {
   extern __shared__ __align__(1024) unsigned char smem[];
@@ -215,6 +218,12 @@ __global__ void __launch_bounds__(kThreads, 1) qmv_tmem_kernel(const __grid_cons
   // (the warp's number from lane 0: what follows from it is then the same in the whole warp to the compiler, too)
   const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = tid & 31;
   const int CS = p.cs, XS = p.xs, nt = p.nt, C = p.cluster;
+  const uint32_t polls = SHORT ? p.polls : kSpin;
+  if (smem_u32(smem) & 1023u) {                            // a misaligned window: all CTAs alike leave, behind whatever comes before
+    grid_wait();
+    if (tid == 0) atomicCAS(&g_tmem_error, 0, 408);
+    return;
+  }
   unsigned char* codes = smem;                             // [CS][kStage]
   unsigned char* xs = smem + CS * kStage;                  // [XS][4 k-blocks][nt x 128 bytes]
   unsigned char* rx = xs + XS * nt * 512;                  // [p.rx][C ranks][4-token groups that this CTA owns][128 rows][16 bytes]
@@ -272,7 +281,7 @@ __global__ void __launch_bounds__(kThreads, 1) qmv_tmem_kernel(const __grid_cons
     if (p.sb_tma) {
       if (elect_one()) {
         for (int i = from; i < to; ++i) {
-          if (l_round > 0 && !wait_cta(&codes_empty[l_st], (uint32_t)(l_round - 1) & 1)) { failed(407); break; }
+          if (l_round > 0 && !wait_cta(&codes_empty[l_st], (uint32_t)(l_round - 1) & 1, polls)) { failed(407); break; }
           if (s_fail) break;
           next_unit();
           copy_codes();
@@ -282,9 +291,9 @@ __global__ void __launch_bounds__(kThreads, 1) qmv_tmem_kernel(const __grid_cons
       __syncwarp();
     } else {
       for (int i = from; i < to; ++i) {
-        const bool go = l_round == 0 || warp_wait(&codes_empty[l_st], (uint32_t)(l_round - 1) & 1);
+        const bool go = l_round == 0 || warp_wait(&codes_empty[l_st], (uint32_t)(l_round - 1) & 1, polls);
         if (!go && lane == 0) failed(407);
-        if (!go || s_fail) break;
+        if (!__all_sync(0xffffffffu, go && !s_fail)) break;
         next_unit();
         if (elect_one()) copy_codes();
         __syncwarp();
@@ -295,18 +304,13 @@ __global__ void __launch_bounds__(kThreads, 1) qmv_tmem_kernel(const __grid_cons
   };
 
   // Set-up, each role its part: the first copies of codes and scales are under way before the barriers of the other roles exist.
-  const bool window_ok = (smem_u32(smem) & 1023u) == 0;
   if (warp == kCodesWarp) {
     if (lane < CS) { mbar_init(&codes_full[lane], p.sb_tma ? 1 : 1 + 32); mbar_init(&codes_empty[lane], 4); }
-    if (lane == 0) s_fail = window_ok ? 0 : 408;           // misaligned window: every role leaves at once
+    if (lane == 0) s_fail = 0;
     asm volatile("fence.mbarrier_init.release.cluster;\n\tfence.proxy.async.shared::cta;" ::: "memory");
     __syncwarp();
-    if (window_ok) {
-      if (!p.early) grid_wait();
-      copy_units(0, CS < total ? CS : total);
-    }
-    if (lane == 0 && !window_ok) atomicCAS(&g_tmem_error, 0, 408);
-    __syncwarp();
+    if (!p.early) grid_wait();
+    copy_units(0, CS < total ? CS : total);
   } else if (warp == kXWarp) {
     auto init = [&](uint64_t* bar, int n, int count) { if (lane < n) mbar_init(&bar[lane], (uint32_t)count); };
     init(empty, kSlots, 1);
@@ -335,11 +339,9 @@ __global__ void __launch_bounds__(kThreads, 1) qmv_tmem_kernel(const __grid_cons
 
   if (warp < kEpi0) {
     // ---- convert this thread's weight row, unit by unit ----
-    // A wait that runs out ends the others', too; but every warp keeps every meeting with its group's issuer, by then one at a time.
     const int grp = warp >> 2, q = warp & 3, r = q * 32 + lane, mine = total > grp ? (total - grp + GRP - 1) / GRP : 0;
     const uint32_t a_g = a0 + grp * (kOwn * 64) + ((uint32_t)(q * 32) << 16);
     bool ok = true;
-    auto wait = [&](bool ready, uint64_t* bar, int phase) { if (!ready && ok) ok = warp_wait(bar, (uint32_t)phase & 1); };
     int st = grp, cround = 0, slot = 0, round = 0;           // (CS is a multiple of GRP: a stage is always for the same group)
     int e = (k0 + grp % ku) << (2 - p.gshift), k = grp % ku; // the unit's first group of scales
     uint2 sv, bv;
@@ -355,17 +357,20 @@ __global__ void __launch_bounds__(kThreads, 1) qmv_tmem_kernel(const __grid_cons
       }
     };
     bool codes_ready = false, slot_ready = true;
-    for (int i = 0; i < mine; ++i) {
+    int i = 0, h = 0;
+    for (; i < mine; ++i) {
       if (!codes_ready) {
-        wait(false, &codes_full[st], cround);
+        ok = warp_wait(&codes_full[st], (uint32_t)cround & 1, polls);
         read_scales();
       }
+      if (!ok) break;
       const unsigned char* row = codes + st * kStage + r * 128;
       uint64_t* done = &codes_empty[st];
       const bool fits = __all_sync(0xffffffffu, fits_subnormal<BITS>(sv.x) && fits_subnormal<BITS>(sv.x >> 16) && fits_subnormal<BITS>(sv.y) && fits_subnormal<BITS>(sv.y >> 16));
 #pragma unroll 1
-      for (int h = 0; h < 2; ++h) {
-        wait(slot_ready, &empty[grp * kOwn + slot], round - 1);
+      for (h = 0; h < 2; ++h) {
+        if (!slot_ready) ok = warp_wait(&empty[grp * kOwn + slot], (uint32_t)(round - 1) & 1, polls);
+        if (!ok) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t a_s = a_g + (uint32_t)slot * 64;
         if (fits) convert_half<BITS, true>(row, r & 7, h, sv.x, bv.x, a_s);
@@ -388,12 +393,23 @@ __global__ void __launch_bounds__(kThreads, 1) qmv_tmem_kernel(const __grid_cons
         slot_ready = __all_sync(0xffffffffu, slot_ready);
         asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-        if (ok) asm volatile("bar.arrive %0, 160;" ::"r"(id) : "memory");
-        else asm volatile("bar.sync %0, 160;" ::"r"(id) : "memory");
+        asm volatile("bar.arrive %0, 160;" ::"r"(id) : "memory");
         if (h && lane == 0) mbar_arrive(done);               // (only now that the words have been consumed)
       }
+      if (!ok) break;
     }
-    if (!ok && !s_fail) failed(404);
+    if (!ok) {
+      // A wait ran out: this warp converts no more, but keeps its meetings with the issuer, each behind the one before in that slot, which
+      // the issuer frees whatever happens.  (Met ahead of it, the named barrier would count this warp for the issuer; both would then wait
+      // for good.)
+      if (lane == 0 && !s_fail) failed(404);
+      __syncwarp();
+      for (int n = 2 * (mine - i) - (h == 1); n > 0; --n) {
+        if (round > 0) warp_wait(&empty[grp * kOwn + slot], (uint32_t)(round - 1) & 1, 8 * kSpin);
+        asm volatile("bar.arrive %0, 160;" ::"r"(2 + grp * kOwn + slot) : "memory");
+        if (++slot == kOwn) { slot = 0; ++round; }
+      }
+    }
     __syncwarp();
     peers_ready();
   } else if (warp < kCodesWarp) {
@@ -409,8 +425,8 @@ __global__ void __launch_bounds__(kThreads, 1) qmv_tmem_kernel(const __grid_cons
     for (int j = 0; j < tiles && ok; ++j) {
       const int tile = cl + j * ncl, d = p.dbufs == 2 ? j & 1 : 0, b = p.rx == 2 ? j & 1 : 0;
       if (C > 1 && g1 > g0 && tid == kEpi0 * 32) mbar_expect_tx(&rx_full[b], (uint32_t)((C - 1) * (g1 - g0) * 2048));
-      ok = warp_wait(&d_full[d], (uint32_t)(p.dbufs == 2 ? j >> 1 : j) & 1) && (C == 1 || j < p.rx || warp_wait(&rx_free[b], (uint32_t)(j / p.rx - 1) & 1)) &&
-           !s_fail;
+      ok = warp_wait(&d_full[d], (uint32_t)(p.dbufs == 2 ? j >> 1 : j) & 1, polls) && (C == 1 || j < p.rx || warp_wait(&rx_free[b], (uint32_t)(j / p.rx - 1) & 1, polls)) &&
+           __all_sync(0xffffffffu, !s_fail);
       if (!ok) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const int mi = mat_of(p, tile), n = (tile - QB_SEL4(p.tile0, mi)) * 128 + r;
@@ -467,7 +483,7 @@ __global__ void __launch_bounds__(kThreads, 1) qmv_tmem_kernel(const __grid_cons
         }
       }
       if (C > 1 && g1 > g0) {
-        ok = warp_wait(&rx_full[b], (uint32_t)(j / p.rx) & 1) && !s_fail;
+        ok = warp_wait(&rx_full[b], (uint32_t)(j / p.rx) & 1, polls) && __all_sync(0xffffffffu, !s_fail);
         if (!ok) break;
 #pragma unroll 1
         for (int g = g0; g < g1; ++g) {
@@ -491,7 +507,7 @@ __global__ void __launch_bounds__(kThreads, 1) qmv_tmem_kernel(const __grid_cons
     __syncwarp();
     if (!ok && C > 1 && !seen) peers_ready();
   } else if (warp == kCodesWarp) {
-    if (window_ok && CS < total) copy_units(CS, total);
+    if (CS < total) copy_units(CS, total);
     __syncwarp();
     peers_ready();
   } else if (warp == kXWarp) {
@@ -509,7 +525,7 @@ __global__ void __launch_bounds__(kThreads, 1) qmv_tmem_kernel(const __grid_cons
       } else {
         int k = 0, st = 0, round = 0;
         for (int i = 0; i < total; ++i) {
-          if (round > 0 && !wait_cta(&x_empty[st], (uint32_t)(round - 1) & 1)) { failed(403); break; }
+          if (round > 0 && !wait_cta(&x_empty[st], (uint32_t)(round - 1) & 1, polls)) { failed(403); break; }
           if (s_fail) break;
           load_x(k, st);
           if (++k == ku) k = 0;
@@ -526,7 +542,7 @@ __global__ void __launch_bounds__(kThreads, 1) qmv_tmem_kernel(const __grid_cons
     const uint64_t dhi = make_desc(0) & 0xFFFFFFFF00000000ull;
     const uint32_t xd0 = (uint32_t)make_desc(smem_u32(xs)), a_g = a0 + grp * (kOwn * 64), xk = (uint32_t)nt * 8;
     bool ok = true;
-    auto wait = [&](uint64_t* bar, int phase) { if (ok) ok = warp_wait(bar, (uint32_t)phase & 1); };
+    auto wait = [&](uint64_t* bar, int phase) { if (ok) ok = warp_wait(bar, (uint32_t)phase & 1, polls); };
     int slot = 0, xi = grp % XS, xround = 0, k = grp;        // (a ring's XS is a multiple of GRP, too)
     for (int t = 0; t < tiles; ++t, k -= ku) {
       const int d = p.dbufs == 2 ? t & 1 : 0, dround = p.dbufs == 2 ? t >> 1 : t;
@@ -542,7 +558,9 @@ __global__ void __launch_bounds__(kThreads, 1) qmv_tmem_kernel(const __grid_cons
         for (int h = 0; h < 2; ++h) {
           asm volatile("bar.sync %0, 160;" ::"r"(2 + grp * kOwn + slot) : "memory");
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          if (ok && elect_one()) {
+          if (!ok) {                                         // a wait ran out: no more MMAs, but the converting warps go by these meetings
+            if (lane == 0) mbar_arrive(&empty[grp * kOwn + slot]);
+          } else if (elect_one()) {
             const uint32_t xd = xd0 + (uint32_t)((xi * 4 + h * 2) * nt * 8), a_s = a_g + (uint32_t)slot * 64;
 #pragma unroll
             for (int m = 0; m < 8; ++m) umma_ta(dt, a_s + m * 8, dhi | (xd + (m >> 2) * xk + 2 * (m & 3)), idesc, m > 0 ? 1u : acc);
@@ -561,6 +579,8 @@ __global__ void __launch_bounds__(kThreads, 1) qmv_tmem_kernel(const __grid_cons
       __syncwarp();
     }
     if (!ok && !s_fail) failed(401);
+    if (s_fail)
+      for (int i = 0; i < 1000; ++i) __nanosleep(1000);    // (MMAs may still be on their way)
     __syncwarp();
     peers_ready();
   }
@@ -610,10 +630,12 @@ cudaError_t clusters_of(int cluster, int* n) {
   const int sms = sm_count();
   std::lock_guard<std::mutex> lk(setup_mutex());
   if (cached[dev][0] == 0) {
-    auto kern = qmv_tmem_kernel<BITS>;
-    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem);
-    if (e != cudaSuccess) return e;
-    note_reader((const void*)kern);
+    auto kern = qmv_tmem_kernel<BITS, false>;
+    for (auto k : {kern, qmv_tmem_kernel<BITS, true>}) {
+      e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem);
+      if (e != cudaSuccess) return e;
+      note_reader((const void*)k);
+    }
     cached[dev][1] = sms;
     for (int c = 2; c <= kMaxCluster; ++c) {
       cudaLaunchAttribute attr[2];
@@ -675,7 +697,8 @@ cudaError_t launch_inst(const CUtensorMap& xmap, const TmMaps& wm, TmK p, cudaSt
     const size_t smem = (size_t)(p.cs * stage + p.xs * xu + p.rx * rx1) + kBarBytes;
     cudaLaunchAttribute attr[2];
     const cudaLaunchConfig_t cfg = config(attr, pl.ncl * c, c, smem < kSmemLeast ? kSmemLeast : smem, st);
-    e = c > 1 ? launch_clusters(cfg, qmv_tmem_kernel<BITS>, xmap, wm, p) : cudaLaunchKernelEx(&cfg, qmv_tmem_kernel<BITS>, xmap, wm, p);
+    auto kern = wait_polls() == 0 ? qmv_tmem_kernel<BITS, false> : qmv_tmem_kernel<BITS, true>;
+    e = c > 1 ? launch_clusters(cfg, kern, xmap, wm, p) : cudaLaunchKernelEx(&cfg, kern, xmap, wm, p);
     if (e == cudaSuccess || c == 1) return e;
     (void)cudaGetLastError();
   }
@@ -729,6 +752,7 @@ cudaError_t launch_qmv_tmem_multi(const QmmArgs* a, int count, cudaStream_t st) 
   p.tile0[kMaxMat] = tiles;
   if (!make_map(&xmap, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, (const uint16_t*)a[0].x + a[0].xb.offset(0), a[0].K, a[0].M, a[0].ldx * 2, 64, p.nt)) return cudaErrorInvalidValue;
   p.early = weights_settled(st);
+  p.polls = wait_polls() > 0 ? (uint32_t)wait_polls() : 0;
   return bits == 8 ? launch_inst<8>(xmap, wm, p, st) : launch_inst<4>(xmap, wm, p, st);
 }
 cudaError_t launch_qmv_tmem(const QmmArgs& a, cudaStream_t st) { return launch_qmv_tmem_multi(&a, 1, st); }

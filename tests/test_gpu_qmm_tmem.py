@@ -183,3 +183,33 @@ def test_rows_that_no_tensor_map_takes(M):
         for y in outs:
             gate_bf16(y.float().cpu().numpy(), ref, what + ", twice")
     assert qb200.lib().qb200_debug_tc_status() == 0
+
+
+@pytest.mark.parametrize("bits,M,N,K", [
+    (4, 16, 28672, 4096), (4, 64, 11648, 2560),      # clusters with several tiles
+    (4, 13, 40000, 768), (8, 64, 300, 8192)])        # CTAs by themselves; x in a ring
+def test_waits_that_run_out(bits, M, N, K):
+    """A wait that gives up ends the launch: its status is set, nothing is stored behind it, and the next launch is as ever."""
+    import qb200
+    L = qb200.lib()
+    g = torch.Generator(device="cuda").manual_seed(N + K + M)
+    w = _weight(N, K, 64, bits, g)
+    x = torch.randn((M, K), device="cuda", generator=g).to(torch.bfloat16)
+    good = qb200.quantized_matmul(x, *w, True, 64, bits)
+    assert L.qb200_debug_tc_status() == 0
+    try:
+        for polls in (-1, 1, 2, 5):
+            y = torch.full_like(good, float("nan"))
+            L.qb200_debug_wait_polls(polls)
+            qb200.quantized_matmul(x, *w, True, 64, bits, out=y)
+            status, done = L.qb200_debug_tc_status(), ~torch.isnan(y)
+            assert status in (401, 403, 404, 405, 407) or (polls > 0 and status == 0)
+            assert bool((y[done] == good[done]).all())
+            assert (status == 0) == bool(done.all())
+            assert polls > 0 or not bool(done.any())
+            L.qb200_debug_tc_reset()
+    finally:
+        L.qb200_debug_wait_polls(0)
+        L.qb200_debug_tc_reset()
+    assert torch.equal(qb200.quantized_matmul(x, *w, True, 64, bits), good)
+    assert L.qb200_debug_tc_status() == 0
