@@ -48,7 +48,7 @@ static_assert(smem_of(true) <= 227 * 1024, "shared memory");
 // at K = 196608) -- so 1.5 to 8 seconds.  (2^12 polls ended after 1.5 ms, 2^18 after 95 ms, which longer contractions outlive.  A
 // limit by the clock, in a function of its own behind 4096 polls, made the roles save registers around the call: 64 experts x 768 x
 // 2048 with 5168 rows 52.5 -> 54.0 us.)
-constexpr uint32_t kSpin = 1u << 22, kNap = 2000;
+constexpr uint32_t kSpin = 1u << 22;
 
 __device__ int g_pair_error = 0;                 // 0, or the code of a wait that expired
 
@@ -65,16 +65,6 @@ struct Tile {
   int units, nn0, nn1, col0, col1;               // units of nn0 and nn1 tokens (multiples of 32, up to 256), from these blocks of columns on
   int n0, nend, wrow0, wlast;                    // output columns; first weight row of the tile, last one of the matrix
 };
-__device__ __forceinline__ bool wait_cta(uint64_t* bar, uint32_t parity) {
-  const uint32_t addr = smem_u32(bar);
-  for (uint32_t it = 0; it < kSpin; ++it) {
-    uint32_t done;
-    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-                 : "=r"(done) : "r"(addr), "r"(parity), "r"(kNap) : "memory");
-    if (done) return true;
-  }
-  return false;
-}
 // (a shared::cluster address)
 __device__ __forceinline__ void arrive_addr(uint32_t bar) {
   asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
@@ -316,7 +306,7 @@ __global__ void __launch_bounds__(kThreads, 1) qmm_pair_kernel(const __grid_cons
         const int b0 = boxes(rank, 0), b1 = boxes(rank, 1), all = boxes(0, 0) + boxes(0, 1) + boxes(1, 0) + boxes(1, 1);
         const int t0 = tc.row0 + rank * (tc.nn0 >> 1), t1 = tc.row0 + tc.nn0 + rank * (tc.nn1 >> 1);
         for (int kb = 0; kb < nkb; ++kb) {
-          if (round > 0 && !wait_cta(&empty[st], (round - 1) & 1)) { failed(303); ok = false; break; }
+          if (round > 0 && !wait_cta(&empty[st], (round - 1) & 1, kSpin)) { failed(303); ok = false; break; }
           if (s_fail) { ok = false; break; }
           if (rank == 0) mbar_expect_tx(&full[st], (uint32_t)(all * (TILE / 2)));   // the copies of both CTAs complete at CTA 0's barrier
           const uint32_t dst = smem_u32(x_t + st * xbox * TILE), bar = full0 + (uint32_t)st * 8u;
@@ -337,7 +327,7 @@ __global__ void __launch_bounds__(kThreads, 1) qmm_pair_kernel(const __grid_cons
         const int n = tc.wrow0 + rank * 128;
         for (int k = 0; k < nkb / KPS; ++k, ++sb) {
           const int buf = sb % RAWB;
-          if (sb >= RAWB && !wait_cta(&raw_empty[buf], ((sb / RAWB) - 1) & 1)) { failed(307); ok = false; break; }
+          if (sb >= RAWB && !wait_cta(&raw_empty[buf], ((sb / RAWB) - 1) & 1, kSpin)) { failed(307); ok = false; break; }
           if (s_fail) { ok = false; break; }
           mbar_expect_tx(&raw_full[buf], (uint32_t)RAW);
           tma_load_2d(smem_u32(raw + buf * RAW), &wmap, &raw_full[buf], k * 32, n);
@@ -365,11 +355,11 @@ __global__ void __launch_bounds__(kThreads, 1) qmm_pair_kernel(const __grid_cons
         // a lane per block
         const uint32_t mine = (((1u << (tc.nn0 >> 5)) - 1) << tc.col0) | (((1u << (tc.nn1 >> 5)) - 1) << tc.col1);
         const bool held = lane < kCols && (mine & used) >> lane & 1;
-        if (!fail && !__all_sync(0xffffffffu, !held || wait_cta(&acc_empty[lane], ~(par >> lane) & 1))) fail = 306;
+        if (!fail && !__all_sync(0xffffffffu, !held || wait_cta(&acc_empty[lane], ~(par >> lane) & 1, kSpin))) fail = 306;
         used |= mine;
         par ^= mine;
         for (int kb = 0; kb < nkb; ++kb) {
-          if (!fail && !warp_wait(lane, [&] { return wait_cta(&full[st], round & 1); })) fail = 301;
+          if (!fail && !warp_wait(lane, [&] { return wait_cta(&full[st], round & 1, kSpin); })) fail = 301;
           if (!fail) asm volatile("bar.arrive %0, 64;" ::"r"(1 + st) : "memory");
           else {
             if (!s_fail && lane == 0) failed(fail);
@@ -429,12 +419,12 @@ __global__ void __launch_bounds__(kThreads, 1) qmm_pair_kernel(const __grid_cons
         // Pieces without a k-block of this group are seen and released too: a parity names a phase only to who follows every one.
         bool go = true;
         for (; KPS < DQG && seen < sb; ++seen) {
-          go = go && wait_cta(&raw_full[seen % RAWB], (seen / RAWB) & 1);
+          go = go && wait_cta(&raw_full[seen % RAWB], (seen / RAWB) & 1, kSpin);
           mbar_arrive(&raw_empty[seen % RAWB]);
         }
         seen = sb + 1;
-        go = go && wait_cta(&raw_full[buf], (sb / RAWB) & 1);
-        if (go && round > 0) go = wait_cta(&empty[st], (round - 1) & 1);
+        go = go && wait_cta(&raw_full[buf], (sb / RAWB) & 1, kSpin);
+        if (go && round > 0) go = wait_cta(&empty[st], (round - 1) & 1, kSpin);
         s_go[grp * 2 + turn] = go && !s_fail;
       }
       asm volatile("bar.sync %0, 128;" ::"r"(1 + SMAX + grp) : "memory");
@@ -476,7 +466,7 @@ __global__ void __launch_bounds__(kThreads, 1) qmm_pair_kernel(const __grid_cons
       const int n = tc.n0 + rank * 128 + q * 32 + lane;
       for (int j = 0; j < tc.units; ++j) {
         const int col = j ? tc.col1 : tc.col0;
-        ok = warp_wait(lane, [&] { return wait_cta(&acc_full[col], (par >> col) & 1); });
+        ok = warp_wait(lane, [&] { return wait_cta(&acc_full[col], (par >> col) & 1, kSpin); });
         if (!ok || s_fail) { ok = false; break; }
         par ^= 1u << col;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -527,13 +517,6 @@ cudaError_t launch_inst(const CUtensorMap& xmap, const CUtensorMap& wmap, const 
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   return launch_clusters(cfg, kern, xmap, wmap, p);
-}
-bool make_map(CUtensorMap* m, CUtensorMapDataType t, const void* base, int64_t cols, int64_t rows, int64_t pitch, int bc, int br) {
-  const EncodeFn enc = get_encode();
-  const cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows}, strides[1] = {(cuuint64_t)pitch};
-  const cuuint32_t box[2] = {(cuuint32_t)bc, (cuuint32_t)br}, es[2] = {1, 1};
-  return enc && enc(m, t, 2, (void*)base, dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-                    CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 // wrows: weight rows in all (E * N in the grouped form)
 cudaError_t launch_pair(PairK& p, const void* x, int64_t ldx, const uint32_t* w, int64_t wrows, int64_t ldw, int bits, bool grouped, int pairs, cudaStream_t st) {

@@ -38,7 +38,7 @@ constexpr int kMaxCodes = 8, kSlots = 6, kMaxX = 16;      // ring depths: packed
 // 31.4 us against 26.6 at 27 tokens, for whose three accumulators tensor memory has room once, not twice; the same at 9.)
 constexpr int GRP = 2, kOwn = kSlots / GRP;                // slots of a group
 constexpr int kEpi0 = 4 * GRP, kCodesWarp = kEpi0 + 4, kXWarp = kCodesWarp + 1, kMmaWarp = kXWarp + 1, kThreads = (kMmaWarp + GRP) * 32;
-constexpr uint32_t kSpin = 1u << 22, kNap = 2000;         // polls of a bounded wait; ns the hardware may hold one
+constexpr uint32_t kSpin = 1u << 22;                      // polls of a bounded wait
 constexpr int kBars = 2 * kMaxCodes + kSlots + 2 * kMaxX + 4 + 4;
 constexpr size_t kBarBytes = kBars * 8 + 32, kSmem = 225 * 1024;
 // One CTA an SM: each allocates all of tensor memory.  Were there room for a second one of the grid (or of another stream's), it would wait
@@ -71,16 +71,6 @@ __device__ __forceinline__ int mat_of(const TmK& p, int tile) {
   if (p.nmat > 2 && tile >= p.tile0[2]) mi = 2;
   if (p.nmat > 3 && tile >= p.tile0[3]) mi = 3;
   return mi;
-}
-__device__ __forceinline__ bool wait_cta(uint64_t* bar, uint32_t parity, uint32_t polls) {
-  const uint32_t addr = smem_u32(bar);
-  for (uint32_t it = 0; it < polls; ++it) {
-    uint32_t done;
-    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-                 : "=r"(done) : "r"(addr), "r"(parity), "r"(kNap) : "memory");
-    if (done) return true;
-  }
-  return false;
 }
 __device__ __forceinline__ bool test_cta(uint64_t* bar, uint32_t parity) {
   uint32_t done;
@@ -594,15 +584,6 @@ __global__ void __launch_bounds__(kThreads, 1) qmv_tmem_kernel(const __grid_cons
     __syncthreads();
     if (C > 1) cluster_sync_tc();
   }
-}
-
-bool make_map(CUtensorMap* m, CUtensorMapDataType t, const void* base, int64_t cols, int64_t rows, int64_t pitch, int bc, int br,
-              CUtensorMapSwizzle swizzle = CU_TENSOR_MAP_SWIZZLE_128B) {
-  const EncodeFn enc = get_encode();
-  const cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows}, strides[1] = {(cuuint64_t)pitch};
-  const cuuint32_t box[2] = {(cuuint32_t)bc, (cuuint32_t)br}, es[2] = {1, 1};
-  return enc && enc(m, t, 2, (void*)base, dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
 cudaLaunchConfig_t config(cudaLaunchAttribute (&attr)[2], int grid, int cluster, size_t smem, cudaStream_t st) {

@@ -64,6 +64,18 @@ __device__ __forceinline__ bool mbar_wait_backoff(uint64_t* bar, uint32_t parity
   }
   return false;
 }
+// The same with a number of polls of the caller's, each held by the hardware for kNap ns at most.
+constexpr uint32_t kNap = 2000;
+__device__ __forceinline__ bool wait_cta(uint64_t* bar, uint32_t parity, uint32_t polls) {
+  const uint32_t addr = smem_u32(bar);
+  for (uint32_t it = 0; it < polls; ++it) {
+    uint32_t done;
+    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                 : "=r"(done) : "r"(addr), "r"(parity), "r"(kNap) : "memory");
+    if (done) return true;
+  }
+  return false;
+}
 // One lane of a converged warp.  By elect.sync the compiler knows that it is one: behind it an MMA issues in 9 - 16 cycles, behind
 // `lane == 0` in 73, commits and copies alike.
 __device__ __forceinline__ bool elect_one() {
@@ -166,6 +178,16 @@ inline EncodeFn get_encode() {
       fn = (EncodeFn)sym;
   }
   return fn;
+}
+
+// A matrix of `rows` rows of `cols` elements, `pitch` bytes apart, in boxes of br x bc; false where the driver declines it.
+inline bool make_map(CUtensorMap* m, CUtensorMapDataType t, const void* base, int64_t cols, int64_t rows, int64_t pitch, int bc, int br,
+                     CUtensorMapSwizzle swizzle = CU_TENSOR_MAP_SWIZZLE_128B) {
+  const EncodeFn enc = get_encode();
+  const cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows}, strides[1] = {(cuuint64_t)pitch};
+  const cuuint32_t box[2] = {(cuuint32_t)bc, (cuuint32_t)br}, es[2] = {1, 1};
+  return enc && enc(m, t, 2, (void*)base, dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
 }  // namespace qb
