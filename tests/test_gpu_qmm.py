@@ -38,11 +38,11 @@ def _run(x32, q, s, b, gs, bits, transpose=True, tag=None):
 
 
 def _tensor_core_route(M, K, bits, gs):
-    """The dispatch rule of qb200_quantized_matmul for bf16 activations: from 9 tokens a kernel that rounds the weight
-    term to bf16 once, as the reference's dense route does -- the wide streaming kernel (4/8 bits at group 64, 4 bits
-    at group 128, K a multiple of 256 up to 16384; 9..32 tokens) or the tcgen05 kernel (K a multiple of 256, 4/8 bits,
-    group 64/128; from 33 tokens, and where the wide kernel does not serve); up to 8 tokens, and for other formats,
-    the fp32 weight term."""
+    """The dispatch rule of qb200_quantized_matmul for bf16 activations: from 9 tokens, with K a multiple of 256, 4 or 8
+    bits and group 64 or 128, a kernel that rounds the weight term to bf16 once, as the reference's dense route does --
+    the tensor-memory kernel up to 64 tokens (the wide streaming one up to 32 for rows that no tensor map takes), the
+    tcgen05 kernels above; up to 8 tokens, for other formats, and at 9..32 tokens above K = 16384 (but for 8 bits at
+    group 128), the fp32 weight term."""
     tc_ok = K % 256 == 0 and bits in (4, 8) and gs in (64, 128)
     return tc_ok and M > 8 and (M > 32 or K <= 16384 or (bits, gs) == (8, 128))
 
@@ -73,9 +73,7 @@ def test_config2_llama_projections(proj, M):
                                    (31, 640, 4096), (16, 14336, 4096), (12, 256, 256), (40, 1000, 2048), (64, 640, 4096),
                                    (57, 4096, 1024), (33, 16, 512)])
 def test_nine_to_sixty_four_tokens(bits, gs, M, N, K):
-    """9..32 tokens: the wide streaming kernel reads the weights once per pass (16- and 32-token forms, ragged token
-    counts and row counts, K from one ring stage to the longest projection, work cut over the CTAs inside tile blocks);
-    33..64 tokens take the tensor-core kernel."""
+    """Ragged token counts and row counts, K from one unit to the longest projection: the tensor-memory kernel."""
     rng = np.random.default_rng(M * 7 + N + K + bits)
     q, s, b = make_weight(rng, (N, K), gs, bits)
     _run(rand_bf16(rng, (M, K)), q, s, b, gs, bits)
@@ -389,10 +387,31 @@ def test_config4_full_size_vs_dequantize_plus_fp32_matmul(bits):
 @pytest.mark.parametrize("M,N,K", [(128, 4096, 4096), (64, 1024, 4096), (100, 1000, 2048), (128, 512, 14336),
                                    (256, 4096, 4096), (200, 1024, 2048)])
 def test_few_token_split_k_shapes(bits, gs, M, N, K):
-    """32..256 tokens against few weight rows: the tensor-core kernel cuts K over the CTAs of a cluster and adds
-    the partial accumulators in rank 0 (C2's M = 128 projections: q/o 4096x4096, k/v 1024x4096, down K = 14336)."""
+    """Up to 256 tokens against few weight rows: above 64 the tensor-core kernel cuts K over the CTAs of a cluster and
+    adds the partial accumulators in rank 0 (C2's M = 128 projections: q/o 4096x4096, k/v 1024x4096, down K = 14336)."""
     import qb200
     rng = np.random.default_rng(M + N + K + bits + gs)
     q, s, b = make_weight(rng, (N, K), gs, bits)
     _run(rand_bf16(rng, (M, K)), q, s, b, gs, bits)
+    assert qb200.lib().qb200_debug_tc_status() == 0
+
+
+@pytest.mark.parametrize("bits,gs", [(4, 64), (8, 64), (4, 128), (8, 128)])
+@pytest.mark.parametrize("M,N,K", [(9, 200, 512), (32, 1024, 4096), (33, 640, 1024), (64, 1000, 4096), (64, 257, 14336)])
+def test_few_tokens_with_unaligned_scales(bits, gs, M, N, K):
+    """Scales and biases as views whose rows are off 4 bytes, which the kernels for few tokens decline: the tensor-core
+    kernel's few-token form, with and without K split over a cluster; alone and two matrices in a call."""
+    import qb200
+    rng = np.random.default_rng(M + N + K + bits + gs)
+    q, s, b = make_weight(rng, (N, K), gs, bits)
+    x = rand_bf16(rng, (M, K))
+    dx, (dq, ds, db) = to_dev_bf16(qo.f32_to_bf16(x)), dev_triple(q, s, b)
+    off = [torch.cat([t[:, :1], t, t[:, :2]], 1)[:, 1:1 + t.shape[1]] for t in (ds, db)]
+    ref = qo.qmm(x, q, s, b, gs, bits, True, bf16_weights=True)
+    y = qb200.quantized_matmul(dx, dq, *off, True, gs, bits)
+    gate_bf16(y.float().cpu().numpy(), ref, "alone")
+    outs = [torch.empty_like(y) for _ in range(2)]
+    qb200.quantized_matmul_batch(dx, [(dq, *off)] * 2, outs, True, gs, bits)
+    for o in outs:
+        gate_bf16(o.float().cpu().numpy(), ref, "two matrices")
     assert qb200.lib().qb200_debug_tc_status() == 0
