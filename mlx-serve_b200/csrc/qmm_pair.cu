@@ -14,7 +14,9 @@
 //    has read it, and so works beside the next tile except for the blocks that two tiles have in common (two tiles of 288 tokens: 64
 //    of 512 columns).  With two slots of 256 columns a tile of two units began after the whole epilogue of the one before, 6800 of
 //    16800 cycles at K = 768 (128 experts, us, before -> after: 256 rows an expert 768 x 2048 123 -> 117, 2048 x 768 134 -> 115; 290
-//    rows 132 -> 124, 148 -> 126).
+//    rows 132 -> 124, 148 -> 126).  Launches of one-unit tiles are a form of their own, without the arithmetic of cut tiles, whose epilogue
+//    gives its blocks back at the end of a tile: with one form for both they took 150 cycles a block and 0.2 us a tile more (us, two slots,
+//    one form, two forms: 2048 tokens, 14336 x 256 25.6, 29.0, 25.2; 1138 tokens, 14147 x 768 53.3, 59.1, 53.7).
 //  * Roles per CTA: twelve warps convert weights (three groups of four that take k-blocks in turn, a thread per weight row), four
 //    are the epilogue, and one each loads x, loads packed codes, issues the MMAs (CTA 0 only: its instructions read both CTAs'
 //    operands) and scouts for the issuer (CTA 0).  These four share a scheduler without any converting warp: beside one, the
@@ -69,6 +71,9 @@ struct Tile {
 __device__ __forceinline__ void arrive_addr(uint32_t bar) {
   asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
 }
+__device__ __forceinline__ void arrive_if(uint32_t bar, bool yes) {
+  asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %1, 0;\n\t@p mbarrier.arrive.shared::cluster.b64 _, [%0];\n\t}" ::"r"(bar), "r"((uint32_t)yes) : "memory");
+}
 // A whole warp waits: one lane polls (thirty-two lanes polling one barrier are served one after another, and sixteen warps of them
 // kept the copies' own arrivals waiting for thousands of cycles), the others follow.
 template <class F>
@@ -121,14 +126,24 @@ __device__ __forceinline__ Tile tile_at(const PairK& p, const int* s_off, const 
   c.q = c.row_end > c.row0 ? (c.row_end - c.row0 + 31) >> 5 : 1;
   return c;
 }
-// Where the accumulators of the next tile lie in the ring.  A unit is contiguous.  A tile that the ring's end would cut is cut there into
-// its two units, if x has room for two; a tile that is one unit only if starting at block 0 it met the tile before (two such tiles of 224
-// or 256 tokens take turns uncut: cutting them cost 3 %).
+// Where the accumulators of the next tile lie in the ring.  A unit is contiguous.  Tiles of one unit (TWO = false) start over where the
+// ring's end would cut them.  Else a tile that the end would cut is cut there into its two units, or, as one unit, moved to block 0 where
+// that does not meet the tile before (two tiles of 224 or 256 tokens take turns uncut: cutting them cost 3 %).
 struct Ring { int pos = 0, prev = 0; };          // the next free block; the first one of the tile before
-__device__ __forceinline__ void place(Tile& c, Ring& r, bool two) {
+template <bool TWO>
+__device__ __forceinline__ void place(Tile& c, Ring& r) {
   const int q = c.q;
   int a = q, pos = r.pos;
-  if (q > 8 || (two && pos + q > kCols && q > r.prev)) {
+  if constexpr (!TWO) {
+    if (pos + q > kCols) pos = 0;
+    c.units = 1;
+    c.nn0 = q << 5;
+    c.nn1 = 0;
+    c.col0 = c.col1 = pos;
+    r.pos = pos + q;
+    return;
+  }
+  if (q > 8 || (pos + q > kCols && q > r.prev)) {
     a = kCols - pos;
     if (pos + q <= kCols || a > 8 || q - a > 8) {
       a = (q + 1) >> 1;
@@ -151,20 +166,19 @@ __device__ __forceinline__ void place(Tile& c, Ring& r, bool two) {
 // The issuer's walk, out of line (as part of the big function its loop compiles into something much slower).  Everything the loop
 // uses is broadcast from lane 0, so that the compiler knows it to be the same in the whole warp and keeps it in uniform registers.
 struct Walk { uint32_t tmem, w_s, x_s, empty_s, acc_s; int tile0, ntiles, tstride, nkb; const int* s_off; const int* s_tcum; };
-template <bool GROUPED>
+template <bool GROUPED, bool TWO>
 __device__ __noinline__ void issue_walk(const PairK& p, const Walk a) {
   auto U = [](uint32_t v) { return __shfl_sync(0xffffffffu, v, 0); };
   constexpr uint32_t idesc0 = (1u << 4) | (1u << 7) | (1u << 10) | ((256u >> 4) << 24);   // f32 += bf16 x bf16, M = 256
   const uint64_t hi = make_desc(0) & 0xFFFFFFFF00000000ull;
   const uint32_t wd0 = U((uint32_t)make_desc(a.w_s)), xd0 = U((uint32_t)make_desc(a.x_s)), tmem = U(a.tmem), empty_s = U(a.empty_s), acc_s = U(a.acc_s);
   const int nkb = (int)U((uint32_t)a.nkb), S = (int)U((uint32_t)p.stages), ntiles = (int)U((uint32_t)a.ntiles), tstride = (int)U((uint32_t)a.tstride);
-  const uint32_t xstep = U((uint32_t)((p.hmax >> 8) * (TILE >> 4)));   // a stage of x, in the descriptor's 16-byte units
-  const bool two = U((uint32_t)p.hmax) > 256u;
+  constexpr uint32_t xstep = (TWO ? 2 : 1) * (TILE >> 4);              // a stage of x, in the descriptor's 16-byte units
   uint32_t st = 0;
   Ring ring;
   for (int tile = (int)U((uint32_t)a.tile0); tile < ntiles; tile += tstride) {
     Tile tc = tile_at<GROUPED>(p, a.s_off, a.s_tcum, tile);
-    place(tc, ring, two);
+    place<TWO>(tc, ring);
     const uint32_t units = U((uint32_t)tc.units), i0 = U(idesc0 | ((uint32_t)(tc.nn0 >> 3) << 17)), i1 = U(idesc0 | ((uint32_t)(tc.nn1 >> 3) << 17));
     const uint32_t c0 = U((uint32_t)tc.col0), c1 = U((uint32_t)tc.col1), d0 = tmem + c0 * 32, d1 = tmem + c1 * 32;
     for (int kb = 0; kb < nkb; ++kb) {
@@ -176,7 +190,7 @@ __device__ __noinline__ void issue_walk(const PairK& p, const Walk a) {
         for (int k = 0; k < BK / 16; ++k) umma2(d0, hi | (wd + 2 * k), hi | (xd + 2 * k), i0, kb > 0 || k > 0 ? 1u : 0u);
         const bool last = kb + 1 == nkb;
         if (last) commit2(acc_s + c0 * 8u);
-        if (units == 2) {
+        if (TWO && units == 2) {
 #pragma unroll
           for (int k = 0; k < BK / 16; ++k) umma2(d1, hi | (wd + 2 * k), hi | (xd + (TILE >> 4) + 2 * k), i1, kb > 0 || k > 0 ? 1u : 0u);
           if (last) commit2(acc_s + c1 * 8u);
@@ -220,12 +234,14 @@ __device__ __forceinline__ void store_cols32(uint16_t* y, int64_t ldy, const uin
   }
 }
 
-template <int BITS, bool GROUPED>
+// TWO: tiles of up to two units, 512 tokens
+template <int BITS, bool GROUPED, bool TWO>
 __global__ void __launch_bounds__(kThreads, 1) qmm_pair_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap wmap,
                                                                const __grid_constant__ PairK p) {
   extern __shared__ __align__(1024) unsigned char smem[];
   constexpr int KPS = 128 * 8 / (BK * BITS);   // k-blocks per 128-byte piece of packed codes (4 or 2)
-  const int S = p.stages, xbox = p.hmax >> 8;
+  constexpr int xbox = TWO ? 2 : 1;
+  const int S = p.stages;
   unsigned char* w_t = smem;                               // [S][128 x 64 bf16]: this CTA's weight rows
   unsigned char* x_t = smem + S * TILE;                    // [S][units][128 x 64 bf16]: its tokens
   unsigned char* raw = smem + 12 * TILE;                   // [RAWB][128 x 128 bytes of codes]
@@ -241,12 +257,15 @@ __global__ void __launch_bounds__(kThreads, 1) qmm_pair_kernel(const __grid_cons
   const int rank = (int)cluster_rank_tc();
   const int nkb = p.K / BK, tile0 = (int)blockIdx.x >> 1, tstride = (int)gridDim.x >> 1;
 
-  if (tid == 0) {
-    for (int i = 0; i < SMAX; ++i) { mbar_init(&full[i], 1 + 2 * WPG); mbar_init(&empty[i], 1); }
-    for (int i = 0; i < RAWB; ++i) { mbar_init(&raw_full[i], 1); mbar_init(&raw_empty[i], WPG * KPS + (KPS < DQG ? DQG - KPS : 0)); }
-    for (int i = 0; i < kCols; ++i) { mbar_init(&acc_full[i], 1); mbar_init(&acc_empty[i], 8); }
-    s_fail = (smem_u32(smem) & 1023u) ? 308 : 0;           // misaligned window: every role leaves at once
-    if (s_fail) atomicCAS(&g_pair_error, 0, 308);
+  if (warp == 0) {
+    auto init = [&](uint64_t* bar, int n, int count) { if (lane < n) mbar_init(&bar[lane], (uint32_t)count); };
+    init(full, SMAX, 1 + 2 * WPG); init(empty, SMAX, 1);
+    init(raw_full, RAWB, 1); init(raw_empty, RAWB, WPG * KPS + (KPS < DQG ? DQG - KPS : 0));
+    init(acc_full, kCols, 1); init(acc_empty, kCols, 8);
+    if (lane == 0) {
+      s_fail = (smem_u32(smem) & 1023u) ? 308 : 0;         // misaligned window: every role leaves at once
+      if (s_fail) atomicCAS(&g_pair_error, 0, 308);
+    }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   int ntiles = p.ntiles;
@@ -297,7 +316,7 @@ __global__ void __launch_bounds__(kThreads, 1) qmm_pair_kernel(const __grid_cons
       Ring ring;
       for (int tile = tile0; tile < ntiles && ok; tile += tstride) {
         Tile tc = at(tile);
-        place(tc, ring, p.hmax > 256);
+        place<TWO>(tc, ring);
         // boxes of 64 tokens of unit u that CTA r loads
         auto boxes = [&](int r, int u) {
           const int half = (u ? tc.nn1 : tc.nn0) >> 1, t0 = tc.row0 + (u ? tc.nn0 : 0) + r * half;
@@ -339,7 +358,7 @@ __global__ void __launch_bounds__(kThreads, 1) qmm_pair_kernel(const __grid_cons
       Walk w;
       w.tmem = tmem; w.w_s = smem_u32(w_t); w.x_s = smem_u32(x_t); w.empty_s = smem_u32(empty); w.acc_s = smem_u32(acc_full);
       w.tile0 = tile0; w.ntiles = ntiles; w.tstride = tstride; w.nkb = nkb; w.s_off = s_off; w.s_tcum = s_tcum;
-      issue_walk<GROUPED>(p, w);
+      issue_walk<GROUPED, TWO>(p, w);
     }
   } else if (warp == kScoutWarp) {
     // The same walk as the issuer's, ahead of it: it arrives at a named barrier per stage, where the issuer meets it (a poll of an
@@ -351,7 +370,7 @@ __global__ void __launch_bounds__(kThreads, 1) qmm_pair_kernel(const __grid_cons
       uint32_t used = 0, par = 0;                        // blocks that had a tile before; how often, modulo 2
       for (int tile = tile0; tile < ntiles; tile += tstride) {
         Tile tc = at(tile);
-        place(tc, ring, p.hmax > 256);
+        place<TWO>(tc, ring);
         // a lane per block
         const uint32_t mine = (((1u << (tc.nn0 >> 5)) - 1) << tc.col0) | (((1u << (tc.nn1 >> 5)) - 1) << tc.col1);
         const bool held = lane < kCols && (mine & used) >> lane & 1;
@@ -462,7 +481,7 @@ __global__ void __launch_bounds__(kThreads, 1) qmm_pair_kernel(const __grid_cons
     bool ok = true;
     for (int tile = tile0; tile < ntiles && ok; tile += tstride) {
       Tile tc = at(tile);
-      place(tc, ring, p.hmax > 256);
+      place<TWO>(tc, ring);
       const int n = tc.n0 + rank * 128 + q * 32 + lane;
       for (int j = 0; j < tc.units; ++j) {
         const int col = j ? tc.col1 : tc.col0;
@@ -472,15 +491,34 @@ __global__ void __launch_bounds__(kThreads, 1) qmm_pair_kernel(const __grid_cons
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const int t0 = tc.row0 + (j ? tc.nn0 : 0), nt = j ? tc.nn1 : tc.nn0;
         const uint32_t freed = full0 + (uint32_t)((unsigned char*)&acc_empty[col] - (unsigned char*)full);
+        const uint32_t acc = tmem + ((uint32_t)(q * 32) << 16) + col * 32;
+        if constexpr (TWO) {
+          if (n - lane < tc.nend) {   // (a branch around the stores inside the loop, or around the arrival: 150 cycles more a block)
 #pragma unroll 1
-        for (int c0 = 0; c0 < nt; c0 += 32) {
-          uint32_t v[32];
-          tmem_ld32(tmem + ((uint32_t)(q * 32) << 16) + col * 32 + c0, v);
-          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+            for (int c0 = 0; c0 < nt; c0 += 32) {
+              uint32_t v[32];
+              tmem_ld32(acc + c0, v);
+              asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+              asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+              arrive_if(freed + (uint32_t)c0 / 4, lane == 0);    // the block may be overwritten
+              store_cols32(p.y + (int64_t)(t0 + c0) * p.ldy, p.ldy, v, tc.row_end - (t0 + c0), n, tc.nend, p.y_vec != 0, lane);
+            }
+          } else {
+            arrive_if(freed + 8 * (uint32_t)lane, lane < nt >> 5);
+          }
+        } else {               // tiles short enough that the next one does not wait for a block: all of them given back at the end
+          if (n - lane < tc.nend) {
+#pragma unroll 1
+            for (int c0 = 0; c0 < nt; c0 += 32) {
+              uint32_t v[32];
+              tmem_ld32(acc + c0, v);
+              asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+              store_cols32(p.y + (int64_t)(t0 + c0) * p.ldy, p.ldy, v, tc.row_end - (t0 + c0), n, tc.nend, p.y_vec != 0, lane);
+            }
+          }
           asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
           __syncwarp();
-          if (lane == 0) arrive_addr(freed + (uint32_t)c0 / 4);   // the block may be overwritten
-          if (n - lane < tc.nend) store_cols32(p.y + (int64_t)(t0 + c0) * p.ldy, p.ldy, v, tc.row_end - (t0 + c0), n, tc.nend, p.y_vec != 0, lane);
+          arrive_if(freed + 8 * (uint32_t)lane, lane < nt >> 5);
         }
       }
     }
@@ -492,9 +530,9 @@ __global__ void __launch_bounds__(kThreads, 1) qmm_pair_kernel(const __grid_cons
   if (warp == kMmaWarp) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u));
 }
 
-template <int BITS, bool GROUPED>
+template <int BITS, bool GROUPED, bool TWO>
 cudaError_t launch_inst(const CUtensorMap& xmap, const CUtensorMap& wmap, const PairK& p, int pairs, cudaStream_t st) {
-  auto kern = qmm_pair_kernel<BITS, GROUPED>;
+  auto kern = qmm_pair_kernel<BITS, GROUPED, TWO>;
   static bool done[64] = {};
   int dev = 0;
   cudaGetDevice(&dev);
@@ -526,8 +564,11 @@ cudaError_t launch_pair(PairK& p, const void* x, int64_t ldx, const uint32_t* w,
   p.sb_vec = p.K % (512 << p.gshift) == 0 && p.lds % 8 == 0 && ((((uintptr_t)p.s) | ((uintptr_t)p.b)) & 15) == 0;
   p.y_vec = p.ldy % 2 == 0 && ((uintptr_t)p.y & 3) == 0;
   p.stages = p.hmax == 512 ? 4 : (grouped && p.E > kMaxE ? 5 : 6);
-  if (grouped) return bits == 4 ? launch_inst<4, true>(xmap, wmap, p, pairs, st) : launch_inst<8, true>(xmap, wmap, p, pairs, st);
-  return bits == 4 ? launch_inst<4, false>(xmap, wmap, p, pairs, st) : launch_inst<8, false>(xmap, wmap, p, pairs, st);
+  const auto launch = p.hmax == 512 ? (grouped ? (bits == 4 ? launch_inst<4, true, true> : launch_inst<8, true, true>)
+                                               : (bits == 4 ? launch_inst<4, false, true> : launch_inst<8, false, true>))
+                                    : (grouped ? (bits == 4 ? launch_inst<4, true, false> : launch_inst<8, true, false>)
+                                               : (bits == 4 ? launch_inst<4, false, false> : launch_inst<8, false, false>));
+  return launch(xmap, wmap, p, pairs, st);
 }
 
 }  // namespace
@@ -545,15 +586,18 @@ cudaError_t launch_qmm_pair(const QmmArgs& a, cudaStream_t st) {
   p.lds = a.lds; p.ldy = a.ldy; p.M = (int)a.M; p.N = (int)a.N; p.K = (int)a.K; p.gshift = a.gs == 128 ? 1 : 0;
   const int pairs = sm_count() / 2;
   const int64_t nb = (a.N + 255) / 256;
-  // Waves x time of a tile, in us: its k-blocks, and what of the epilogue the next tile's do not hide.  Fitted to 48 shapes (300 to 4096
-  // tokens, K 2048 to 14336, every height from 96): the height taken is 0.3 % slower than the best of a shape on average, 3.5 % at
-  // worst.  The fit before, whose steps at 256 tokens favoured one unit, was 4 % and 33 % off (2048 tokens, 9728 x 2560: 94 us at 256,
-  // 80 at 416; 6144 x 2048: 54 at 256, 43 at 352).
+  // Waves x time of a tile, in us: its k-blocks, and what of the epilogue the next tile's do not hide -- more of it in two units where K is
+  // short, and where the rows of y are off 4 bytes and stored value by value.  Fitted to 48 shapes (300 to 4096 tokens, K 2048 to 14336,
+  // every height from 96): the height taken is 0.3 % slower than the best of a shape on average, 3.5 % at worst.  Below K = 2048 and for odd
+  // rows (74 shapes) 1.1 % and 9.5 %.
+  const bool y_vec = p.ldy % 2 == 0 && ((uintptr_t)p.y & 3) == 0;
+  const int nkb = p.K / BK;
   double best = -1.0;
   for (int h = 512; h >= 128; h -= 32) {
     const int64_t tiles = ((a.M + h - 1) / h) * nb;
-    const double kb = 0.375 + h * 0.00016 + (h > 352 ? (h - 352) * 0.00067 : 0.0), epi = 1.25 + (h > 256 ? (h - 256) * 0.0207 : 0.0);
-    const double cost = (double)((tiles + pairs - 1) / pairs) * ((double)(a.K / BK) * kb + epi);
+    const double kb = 0.375 + h * 0.00016 + (h > 352 ? (h - 352) * 0.00067 : 0.0);
+    const double epi = 1.25 + (h > 256 ? (h - 256) * 0.0207 + 7.0 / nkb : 0.0) + (y_vec ? 0.0 : h / 32 * (h > 256 ? 1.05 : 0.7));
+    const double cost = (double)((tiles + pairs - 1) / pairs) * (nkb * kb + epi);
     if (best < 0 || cost < best - 1e-9) { best = cost; p.h = h; }
   }
   p.hmax = p.h > 256 ? 512 : 256;
