@@ -633,7 +633,10 @@ cudaError_t clusters_of(int cluster, int* n) {
   return cudaSuccess;
 }
 
-// The cluster size: waves of tiles x (units of a tile's share + hand-over of its sums), in units of about 0.65 us
+// The cluster size: tiles x units of a tile's share, and the hand-over of the sums, which the first tile of a cluster hides better than those
+// behind it (its last CTA then waits for the peers' epilogues and the start of its own next tile).  In units of about 0.65 us; by times of
+// every size over 1618 shapes (9 - 64 tokens, 1 - 625 tiles, K 256 - 14336).  With 0.4 a tile it took clusters of many short tiles: 4-bit 18945
+// x 1280 at 9 tokens, six tiles of one unit a cluster of five, 21.7 us, now two of five units a CTA, 10.6; 28672 x 4096 26.1 -> 24.0.
 struct Plan { int cluster, ncl, per, ku; };                // CTAs that split K, clusters, tiles and units of K of one at most
 template <int BITS>
 cudaError_t plan(const TmK& p, int most, Plan* out) {
@@ -644,7 +647,7 @@ cudaError_t plan(const TmK& p, int most, Plan* out) {
     if (e != cudaSuccess) return e;
     if (n < 1) continue;
     const int t = (ntiles + n - 1) / n, ku = (p.spb + c - 1) / c;
-    const double cost = t * (ku + (c > 1 ? 0.4 : 0.0)) + (c > 1 ? 1.0 : 0.0);
+    const double cost = t * ku + (c > 1 ? 1.4 + 1.6 * (t - 1) : 0.0);
     if (best < 0 || cost < best - 1e-9) { best = cost; *out = {c, n < ntiles ? n : ntiles, t, ku}; }
   }
   return best < 0 ? cudaErrorInvalidConfiguration : cudaSuccess;

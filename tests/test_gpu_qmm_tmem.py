@@ -97,8 +97,8 @@ def _gate_exact(y, x, w, gs, bits, what):
 # (on 148 SMs: tiles of 128 rows, the CTAs that share a row tile, units of K of one)
 @pytest.mark.parametrize("bits,gs,M,N,K", [
     (8, 64, 9, 19500, 256), (8, 64, 32, 40000, 256), (8, 64, 17, 40000, 256), (4, 128, 64, 40000, 256),    # 1 CTA, 1 unit: the second group's first one is in the second tile
-    (4, 64, 16, 40000, 768), (8, 128, 32, 19500, 1280), (4, 64, 25, 11264, 2560),                          # odd shares: units change groups from tile to tile
-    (4, 64, 9, 19500, 256), (4, 64, 32, 40000, 256)])                                                      # the wide streaming kernel
+    (4, 64, 16, 40000, 768), (8, 128, 32, 19500, 1280), (4, 64, 25, 10000, 8192),                          # odd shares: units change groups from tile to tile
+    (4, 64, 9, 19500, 256), (4, 64, 32, 40000, 256), (4, 64, 25, 11264, 2560)])                            # the wide streaming kernel; a tile a CTA
 def test_activations_of_the_kernel_before(bits, gs, M, N, K):
     """Two linears in a graph, the first one's output the second one's activations: the second is let in early and converts its weights
     meanwhile, and has to wait for every unit of x."""
@@ -128,8 +128,9 @@ def test_activations_of_the_kernel_before(bits, gs, M, N, K):
 
 @pytest.mark.parametrize("M", [16, 32, 64])
 @pytest.mark.parametrize("bits,gs,N,K", [
-    (4, 64, 28672, 4096), (8, 64, 13000, 4096),     # clusters of four, seven and three tiles each
-    (4, 128, 11648, 2560), (4, 64, 12000, 2304)])   # clusters of three, two tiles each: shares of 3, 3, 4 units and of 3
+    (4, 64, 28672, 4096), (8, 64, 13000, 4096), (4, 128, 11648, 2560), (4, 64, 12000, 2304),   # CTAs by themselves
+    (4, 64, 19200, 8192),                                                                      # clusters of four, five tiles each
+    (4, 128, 10000, 8192), (8, 64, 10000, 8192)])                                              # of three, two tiles: shares of 10, 11, 11 units
 def test_several_tiles_a_cluster(bits, gs, N, K, M):
     import qb200
     g = torch.Generator(device="cuda").manual_seed(N + K + M)
@@ -187,8 +188,8 @@ def test_rows_that_no_tensor_map_takes(M):
 
 
 @pytest.mark.parametrize("bits,M,N,K", [
-    (4, 16, 28672, 4096), (4, 64, 11648, 2560),      # clusters with several tiles
-    (4, 13, 40000, 768), (8, 64, 300, 8192)])        # CTAs by themselves; x in a ring
+    (4, 16, 10000, 8192), (4, 64, 19200, 8192),      # clusters with several tiles
+    (4, 16, 28672, 4096), (4, 64, 11648, 2560), (4, 13, 40000, 768), (8, 64, 300, 8192)])   # CTAs by themselves; x in a ring
 def test_waits_that_run_out(bits, M, N, K):
     """A wait that gives up ends the launch: its status is set, nothing is stored behind it, and the next launch is as ever."""
     import qb200
