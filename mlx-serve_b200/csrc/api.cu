@@ -314,20 +314,12 @@ static int prepare_qmm(qb200_tensor* res, const qb200_tensor* x, const qb200_ten
 // Routing by token count.  Up to 8 tokens: the narrow streaming kernel (one launch).  9 .. 64 (bf16 activations that a tensor map takes): the
 // kernel that streams weights through tensor memory (us, before -> there, a layer of Llama-3-8B's projections 85 -> 58 at 16 tokens;
 // 4-bit 4096 x 4096 16.8 -> 8.8 at 32, 26.6 -> 10.3 at 64; 512 x 512 7.8 -> 3.4, 6.9 -> 4.9; 128 x 256, the smallest, 3.3 -> 3.3 at 9,
-// 4.0 -> 3.4, 5.9 -> 4.7).  9 .. 32 of other activations, and the shortest contraction at 4 bits over many rows: the wide streaming kernel.
-// Above, the tensor-core kernel, whose time does not depend on the token count up to 128.
+// 4.0 -> 3.4, 5.9 -> 4.7).  9 .. 32 of other activations: the wide streaming kernel.  Above, the tensor-core kernel, whose time does not
+// depend on the token count up to 128.
 constexpr int64_t kWideMax = 32;
 static bool takes_wide(const QmmArgs& a) { return a.M > 8 && a.M <= kWideMax && qmv_wide_supported(a); }
-// Up to 32 tokens, what the wide kernel does not serve -- a contraction above 16384 -- keeps the narrow one's weights in fp32.  Of what it does,
-// K = 256 at 4 bits stays with it over many rows (of all matrices of a call): a tile of the other then has one unit to convert, less than its
-// epilogue takes.  us, wide / there: 9 tokens, 12288 rows 4.5 / 4.7, 14336 4.5 / 5.0, 28672 4.6 / 6.8, 128256 13.0 / 16.6; 32 tokens, 14336 rows
-// 6.0 / 5.4, 22000 6.0 / 6.5, 28672 6.1 / 7.3, 128256 18.4 / 18.5; K = 512, 9 tokens, 28672 rows 12.3 / 6.9.
-static bool takes_tmem(const QmmArgs& a, int64_t rows) {
-  if (!qmv_tmem_supported(a)) return false;
-  if (a.M > kWideMax) return true;
-  if (!qmv_wide_supported(a)) return !qmv_stream_supported(a);
-  return a.K > 256 || a.bits != 4 || rows <= (a.M <= 16 ? 12288 : 16384);
-}
+// (up to 32 tokens, what the wide kernel does not serve -- a contraction above 16384 -- keeps the narrow one's weights in fp32)
+static bool takes_tmem(const QmmArgs& a) { return qmv_tmem_supported(a) && (a.M > kWideMax || qmv_wide_supported(a) || !qmv_stream_supported(a)); }
 
 // What the tuned kernels decline -- K no multiple of 256, group size 32, group size 128 at 8 bits -- goes to one of four kernels,
 // by times of each over M 1 - 64, N 100 - 12000, K 128 - 4416 (us a call, replayed):
@@ -362,7 +354,7 @@ static bool launched(cudaError_t e) {
 static cudaError_t dispatch_qmm(const QmmArgs& a, cudaStream_t s) {
   if (!a.transpose) return qmv_rows_supported(a) ? launch_qmv_rows(a, s) : launch_qmm_generic(a, s);
   if (a.nbatch > 1 && qmv_shortk_supported(a)) return launch_qmv_shortk(a, s);   // one W per batch element, short K: q @ K^T
-  if (takes_tmem(a, a.N) && launched(launch_qmv_tmem(a, s))) return cudaSuccess;
+  if (takes_tmem(a) && launched(launch_qmv_tmem(a, s))) return cudaSuccess;
   if (takes_wide(a)) return launch_qmv_wide(a, s);
   if (qmm_pair_supported(a) && launched(launch_qmm_pair(a, s))) return cudaSuccess;
   if (a.M > kWideMax && qmm_tc_supported(a)) return launch_qmm_tc(a, s);
@@ -407,19 +399,16 @@ QB200_API int qb200_quantized_matmul_batch(qb200_tensor* const* res, const qb200
     QmmArgs a[kChunk];
     bool empty[kChunk];
     bool fuse = n > 1, tmem = n > 1, wide = n > 1, f16 = n > 1;
-    int64_t rows = 0;
     for (int i = 0; i < n; ++i) {
       int st = prepare_qmm(res[i0 + i], x, w[i0 + i], scales[i0 + i], biases[i0 + i], transpose_w, group_size, bits,
                            mode, &a[i], &empty[i]);
       if (st) return st;
       // the matrices share a launch where the single call would take a streaming kernel (same rule as dispatch_qmm)
       f16 = f16 && !empty[i] && a[i].K == a[0].K && ragged_kernel(a[i]) == Ragged::f16;
-      rows += a[i].N;
-      tmem = tmem && !empty[i] && a[i].K == a[0].K;
+      tmem = tmem && !empty[i] && takes_tmem(a[i]) && a[i].K == a[0].K;
       wide = wide && !empty[i] && takes_wide(a[i]) && a[i].K == a[0].K;
       fuse = fuse && !empty[i] && a[i].M <= 8 && qmv_stream_supported(a[i]) && a[i].K == a[0].K;
     }
-    for (int i = 0; i < n; ++i) tmem = tmem && takes_tmem(a[i], rows);
     // beyond the streaming kernels' widths, up to 256 tokens: one launch of the tensor-core kernel over all matrices
     auto takes_tc = [&] {
       for (int i = 0; i < n; ++i)

@@ -96,9 +96,9 @@ def _gate_exact(y, x, w, gs, bits, what):
 
 # (on 148 SMs: tiles of 128 rows, the CTAs that share a row tile, units of K of one)
 @pytest.mark.parametrize("bits,gs,M,N,K", [
-    (8, 64, 9, 19500, 256), (8, 64, 32, 40000, 256), (8, 64, 17, 40000, 256), (4, 128, 64, 40000, 256),    # 1 CTA, 1 unit: the second group's first one is in the second tile
+    (4, 64, 9, 19500, 256), (4, 64, 32, 40000, 256), (8, 64, 17, 40000, 256), (4, 128, 64, 40000, 256),    # 1 CTA, 1 unit: the second group's first one is in the second tile
     (4, 64, 16, 40000, 768), (8, 128, 32, 19500, 1280), (4, 64, 25, 10000, 8192),                          # odd shares: units change groups from tile to tile
-    (4, 64, 9, 19500, 256), (4, 64, 32, 40000, 256), (4, 64, 25, 11264, 2560)])                            # the wide streaming kernel; a tile a CTA
+    (4, 64, 25, 11264, 2560)])                                                                             # a tile a CTA
 def test_activations_of_the_kernel_before(bits, gs, M, N, K):
     """Two linears in a graph, the first one's output the second one's activations: the second is let in early and converts its weights
     meanwhile, and has to wait for every unit of x."""
@@ -215,20 +215,3 @@ def test_waits_that_run_out(bits, M, N, K):
         L.qb200_debug_tc_reset()
     assert torch.equal(qb200.quantized_matmul(x, *w, True, 64, bits), good)
     assert L.qb200_debug_tc_status() == 0
-
-
-@pytest.mark.parametrize("gs", [64, 128])
-@pytest.mark.parametrize("M,rows", [
-    (9, (12288,)), (9, (12289,)), (16, (12160, 129)), (17, (16384,)), (32, (16385,)), (32, (16128, 256)), (20, (9000, 9000, 3)), (33, (20000,))])
-def test_shortest_contraction(M, rows, gs):
-    """K = 256 at 4 bits on both sides of the rows, of all matrices of a call, from which the wide streaming kernel takes it."""
-    import qb200
-    g = torch.Generator(device="cuda").manual_seed(M + sum(rows))
-    ws = [_weight(n, 256, gs, 4, g) for n in rows]
-    x = torch.randn((M, 256), device="cuda", generator=g).to(torch.bfloat16)
-    outs = [torch.empty((M, n), dtype=torch.bfloat16, device="cuda") for n in rows]
-    qb200.quantized_matmul_batch(x, ws, outs, True, gs, 4)
-    for w, y in zip(ws, outs):
-        _gate_exact(y, x, w, gs, 4, "a call")
-        _gate_exact(qb200.quantized_matmul(x, *w, True, gs, 4), x, w, gs, 4, "alone")
-    assert qb200.lib().qb200_debug_tc_status() == 0
