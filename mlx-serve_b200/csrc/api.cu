@@ -4,6 +4,7 @@
 // on the host before any CUDA call, so bad input never reaches a kernel.
 #include <cstdarg>
 #include <cstdio>
+#include <cstdlib>
 #include <cstring>
 #include <mutex>
 #include <string>
@@ -316,10 +317,22 @@ static int prepare_qmm(qb200_tensor* res, const qb200_tensor* x, const qb200_ten
 // 4-bit 4096 x 4096 16.8 -> 8.8 at 32, 26.6 -> 10.3 at 64; 512 x 512 7.8 -> 3.4, 6.9 -> 4.9; 128 x 256, the smallest, 3.3 -> 3.3 at 9,
 // 4.0 -> 3.4, 5.9 -> 4.7).  9 .. 32 of other activations: the wide streaming kernel.  Above, the tensor-core kernel, whose time does not
 // depend on the token count up to 128.
-constexpr int64_t kWideMax = 32;
-static bool takes_wide(const QmmArgs& a) { return a.M > 8 && a.M <= kWideMax && qmv_wide_supported(a); }
+// QB200_WIDE_MAX_TOKENS in the environment, read once, sends all that the wide kernel serves of 9 up to so many tokens (64 at most; 0: nothing)
+// there: a diagnostic, to measure the others against it.
+static int64_t wide_switch() {
+  static const int64_t v = [] {
+    const char* e = getenv("QB200_WIDE_MAX_TOKENS");
+    return e ? (int64_t)atoll(e) : (int64_t)-1;
+  }();
+  return v;
+}
+static int64_t wide_max_tokens() { return wide_switch() < 0 ? 32 : wide_switch(); }
+static bool takes_wide(const QmmArgs& a) { return a.M > 8 && a.M <= wide_max_tokens() && qmv_wide_supported(a); }
 // (up to 32 tokens, what the wide kernel does not serve -- a contraction above 16384 -- keeps the narrow one's weights in fp32)
-static bool takes_tmem(const QmmArgs& a) { return qmv_tmem_supported(a) && (a.M > kWideMax || qmv_wide_supported(a) || !qmv_stream_supported(a)); }
+static bool takes_tmem(const QmmArgs& a) {
+  if (!qmv_tmem_supported(a) || (wide_switch() >= 0 && takes_wide(a))) return false;
+  return a.M > 32 || qmv_wide_supported(a) || !qmv_stream_supported(a);
+}
 
 // What the tuned kernels decline -- K no multiple of 256, group size 32, group size 128 at 8 bits -- goes to one of four kernels,
 // by times of each over M 1 - 64, N 100 - 12000, K 128 - 4416 (us a call, replayed):
@@ -357,7 +370,7 @@ static cudaError_t dispatch_qmm(const QmmArgs& a, cudaStream_t s) {
   if (takes_tmem(a) && launched(launch_qmv_tmem(a, s))) return cudaSuccess;
   if (takes_wide(a)) return launch_qmv_wide(a, s);
   if (qmm_pair_supported(a) && launched(launch_qmm_pair(a, s))) return cudaSuccess;
-  if (a.M > kWideMax && qmm_tc_supported(a)) return launch_qmm_tc(a, s);
+  if (a.M > wide_max_tokens() && a.M > 8 && qmm_tc_supported(a)) return launch_qmm_tc(a, s);
   if (a.M > 8 && !qmv_stream_supported(a) && qmm_tc_supported(a)) return launch_qmm_tc(a, s);
   if (qmv_stream_supported(a)) return launch_qmv_stream(a, s);
   switch (ragged_kernel(a)) {
@@ -412,7 +425,7 @@ QB200_API int qb200_quantized_matmul_batch(qb200_tensor* const* res, const qb200
     // beyond the streaming kernels' widths, up to 256 tokens: one launch of the tensor-core kernel over all matrices
     auto takes_tc = [&] {
       for (int i = 0; i < n; ++i)
-        if (empty[i] || a[i].M <= kWideMax || qmm_pair_supported(a[i])) return false;
+        if (empty[i] || a[i].M <= wide_max_tokens() || a[i].M <= 8 || qmm_pair_supported(a[i])) return false;
       return qmm_tc_multi_supported(a, n);
     };
     cudaError_t e = cudaSuccess;

@@ -148,7 +148,7 @@ bool qmv_stream_supported(const QmmArgs& a);
 cudaError_t launch_qmv_stream(const QmmArgs& a, cudaStream_t st);
 cudaError_t launch_qmv_stream_multi(const QmmArgs* a, int count, cudaStream_t st);  // same x, <= 4 matrices
 
-// ---- qmv_wide.cu : 9..32 tokens per pass of activations that TMA does not take, every packed word read once (stream-K over a persistent grid) ----
+// ---- qmv_wide.cu : 9..32 tokens of activations that no tensor map takes (64 by a switch), every packed word read once (stream-K over a persistent grid) ----
 bool qmv_wide_supported(const QmmArgs& a);
 cudaError_t launch_qmv_wide(const QmmArgs& a, cudaStream_t st);
 cudaError_t launch_qmv_wide_multi(const QmmArgs* a, int count, cudaStream_t st);   // same x, <= 4 matrices

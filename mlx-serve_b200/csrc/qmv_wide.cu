@@ -1,6 +1,6 @@
-// Weight-streaming quantized matmul for 9..32 tokens: y[M, N] = x[M, K] . What[N, K]^T with every packed word read from HBM once for
-// all tokens, What = bf16(q*s + b).  It serves the activations whose rows no tensor map takes (off 16 bytes, broadcast, overlapping); the
-// others go to qmv_tmem.
+// Weight-streaming quantized matmul for 9..64 tokens per pass: y[M, N] = x[M, K] . What[N, K]^T with every
+// packed word read from HBM once for all tokens, What = bf16(q*s + b).  It serves 9..32 tokens whose rows no tensor map takes (off 16 bytes,
+// broadcast, overlapping) and, by the switch in the dispatch, others that qmv_tmem would.
 //
 // Replaces mlx_quantized_matmul(transpose=true) as called by qmatmulBits (mlx-serve
 // src/transformer.zig:20894-20983) at the widths its scheduler batches (up to 32 slots,
@@ -18,7 +18,7 @@
 //
 // Organisation:
 //  * A small kernel rewrites the activations once into B-fragment order in a scratch buffer in global
-//    memory (it stays in L2), cut into slices of 512 K values.  CTAs fetch slices with one bulk
+//    memory (it stays in L2), cut into slices of 512 (or 256) K values.  CTAs fetch slices with one bulk
 //    copy each (cp.async.bulk + mbarrier, double buffered) instead of every CTA re-staging all of x.
 //  * Work is cut stream-K style.  A *step* is one ring stage (16 rows x 128 bytes) per warp for the 16
 //    warps of a CTA: 16 consecutive row tiles at the same K offset, so the warps of a step share one
@@ -49,13 +49,13 @@ constexpr int kMaxMat = 4;
 constexpr int kMaxK = 16384;                // longest contraction the activation scratch holds
 constexpr int kMaxTileBlocks = 8192;
 constexpr int kMaxGrid = 160;               // CTAs (one per SM)
-constexpr int kMaxNT = 4;                   // n8 token tiles (32 tokens)
+constexpr int kMaxNT = 8;                   // n8 token tiles per pass (64 tokens)
 constexpr uint32_t kSpinLimit = 1u << 22;
 
-// K values per activation slice: 64 bytes per K value at 32 tokens -- two slices must fit beside the ring.
-constexpr int kSliceK = 512;
+// K values per activation slice: 64 bytes per K value at 32 tokens, 128 at 64 -- two slices must fit beside the ring.
+__host__ __device__ constexpr int slice_k(int nt) { return nt <= 4 ? 512 : 256; }
 // One slice: [64-group][n8 tile][MMA pair][lane][16 B] bf16 B fragments = 1 KiB per (group, tile).
-__host__ __device__ constexpr int slice_bytes(int nt) { return (kSliceK / 64) * nt * 1024; }
+__host__ __device__ constexpr int slice_bytes(int nt) { return (slice_k(nt) / 64) * nt * 1024; }
 
 constexpr size_t kPrepBytes = (size_t)kMaxK * kMaxNT * 16;                                   // 16 bytes per K value and n8 tile
 constexpr size_t kPartSlotFloats = (size_t)kWarps * kMaxNT * 4 * 32;                         // one tile block of partial sums
@@ -139,7 +139,7 @@ __global__ void __launch_bounds__(256) wide_prep_kernel(PrepK p) {
   if (p.early) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  const int NT = p.NT, SK = kSliceK, kpad = (p.K + SK - 1) / SK * SK;
+  const int NT = p.NT, SK = slice_k(NT), kpad = (p.K + SK - 1) / SK * SK;
   const int ppt = kpad >> 4;                                   // 16-value pieces per token
   const int idx = blockIdx.x * 256 + threadIdx.x;
   if (idx >= NT * 8 * ppt) return;
@@ -187,7 +187,7 @@ __global__ void __launch_bounds__(kThreads, 1) qmv_wide_kernel(const __grid_cons
   constexpr int U = BITS == 4 ? 4 : 2;        // 64-wide groups per unit
   constexpr int CK = 64 * U;                  // K values per unit (128 bytes per row)
   constexpr int SB = slice_bytes(NT);
-  constexpr int UPS = kSliceK / CK;       // units (= steps) per activation slice, a power of two
+  constexpr int UPS = slice_k(NT) / CK;       // units (= steps) per activation slice, a power of two
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
   unsigned char* ring = smem;
@@ -521,7 +521,7 @@ cudaError_t wide_scratch(unsigned char** out) {
 }
 
 constexpr size_t smem_wide(int nt) { return (size_t)kWarps * kStages * kStageBytes + (size_t)2 * slice_bytes(nt) + 64; }
-static_assert(smem_wide(kMaxNT) <= 227 * 1024, "shared memory");
+static_assert(smem_wide(4) <= 227 * 1024 && smem_wide(8) <= 227 * 1024, "shared memory");
 
 template <int BITS, int NT>
 cudaError_t launch_wide_inst(const WideK& p, int grid, cudaStream_t st) {
@@ -558,7 +558,7 @@ bool qmv_wide_supported(const QmmArgs& a) {
   if (!((a.bits == 4 && (a.gs == 64 || a.gs == 128)) || (a.bits == 8 && a.gs == 64))) return false;
   if (a.x_dtype != QB200_BFLOAT16) return false;
   if (a.K % 256 != 0 || a.K <= 0 || a.K > kMaxK) return false;
-  if (a.N <= 0 || a.N > (int64_t)kMaxTileBlocks * kWarps * 16 || a.M <= 8 || a.M > 8 * kMaxNT) return false;
+  if (a.N <= 0 || a.N > (int64_t)kMaxTileBlocks * kWarps * 16 || a.M <= 8) return false;
   if ((((uintptr_t)a.w) & 15) != 0 || (a.ldw * 4) % 16 != 0) return false;
   if ((((uintptr_t)a.s) & 7) != 0 || (((uintptr_t)a.b) & 7) != 0) return false;
   if (a.gs == 64 && a.lds % 4 != 0) return false;
@@ -566,7 +566,7 @@ bool qmv_wide_supported(const QmmArgs& a) {
   return true;
 }
 
-// `count` (<= 4) weight matrices on the same activations
+// `count` (<= 4) weight matrices on the same activations; more than 64 tokens run in passes of 64.
 cudaError_t launch_qmv_wide_multi(const QmmArgs* a, int count, cudaStream_t st) {
   unsigned char* scratch = nullptr;
   cudaError_t e = wide_scratch(&scratch);
@@ -599,31 +599,37 @@ cudaError_t launch_qmv_wide_multi(const QmmArgs* a, int count, cudaStream_t st) 
   p.spb = p.K / CK;
   p.total_steps = ntb * p.spb;
   const int grid = p.total_steps < nsm ? p.total_steps : nsm;
-  const int M = (int)a[0].M, NT = M <= 16 ? 2 : 4;
-  PrepK pk;
-  pk.x = (const uint16_t*)a[0].x + a[0].xb.offset(0);
-  pk.out = scratch;
-  pk.M = M; pk.K = p.K; pk.NT = NT; pk.ldx = a[0].ldx;
-  pk.early = weights_settled(st);
-  const int kpad = (p.K + kSliceK - 1) / kSliceK * kSliceK;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)((NT * 8 * (kpad / 16) + 255) / 256));
-  cfg.blockDim = dim3(256);
-  cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  e = bits == 4 ? cudaLaunchKernelEx(&cfg, wide_prep_kernel<4>, pk) : cudaLaunchKernelEx(&cfg, wide_prep_kernel<8>, pk);
-  if (e != cudaSuccess) return e;
-  for (int i = 0; i < kMaxMat; ++i) {
-    const QmmArgs& q = a[i < count ? i : 0];
-    p.y[i] = (uint16_t*)q.y + q.yb.offset(0);
+  for (int64_t m0 = 0; m0 < a[0].M; m0 += 64) {
+    const int M = (int)((a[0].M - m0) < 64 ? (a[0].M - m0) : 64);
+    const int NT = M <= 16 ? 2 : (M <= 32 ? 4 : 8);
+    PrepK pk;
+    pk.x = (const uint16_t*)a[0].x + (a[0].xb.offset(0) + m0 * a[0].ldx);
+    pk.out = scratch;
+    pk.M = M; pk.K = p.K; pk.NT = NT; pk.ldx = a[0].ldx;
+    pk.early = m0 > 0 || weights_settled(st);   // (behind the first pass: that pass's launch is what comes before)
+    const int sk = slice_k(NT), kpad = (p.K + sk - 1) / sk * sk;
+    const int pblocks = (NT * 8 * (kpad / 16) + 255) / 256;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(pblocks);
+    cfg.blockDim = dim3(256);
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    e = bits == 4 ? cudaLaunchKernelEx(&cfg, wide_prep_kernel<4>, pk) : cudaLaunchKernelEx(&cfg, wide_prep_kernel<8>, pk);
+    if (e != cudaSuccess) return e;
+    for (int i = 0; i < kMaxMat; ++i) {
+      const QmmArgs& q = a[i < count ? i : 0];
+      p.y[i] = (uint16_t*)q.y + (q.yb.offset(0) + m0 * q.ldy);
+    }
+    p.M = M;
+    if (bits == 4) e = NT == 2 ? launch_wide_inst<4, 2>(p, grid, st) : (NT == 4 ? launch_wide_inst<4, 4>(p, grid, st) : launch_wide_inst<4, 8>(p, grid, st));
+    else e = NT == 2 ? launch_wide_inst<8, 2>(p, grid, st) : (NT == 4 ? launch_wide_inst<8, 4>(p, grid, st) : launch_wide_inst<8, 8>(p, grid, st));
+    if (e != cudaSuccess) return e;
   }
-  p.M = M;
-  if (bits == 4) return NT == 2 ? launch_wide_inst<4, 2>(p, grid, st) : launch_wide_inst<4, 4>(p, grid, st);
-  return NT == 2 ? launch_wide_inst<8, 2>(p, grid, st) : launch_wide_inst<8, 4>(p, grid, st);
+  return cudaSuccess;
 }
 
 cudaError_t launch_qmv_wide(const QmmArgs& a, cudaStream_t st) { return launch_qmv_wide_multi(&a, 1, st); }

@@ -79,6 +79,36 @@ def test_nine_to_sixty_four_tokens(bits, gs, M, N, K):
     _run(rand_bf16(rng, (M, K)), q, s, b, gs, bits)
 
 
+_WIDE64_CHILD = r"""
+import sys, numpy as np, torch
+sys.path.insert(0, sys.argv[1]); sys.path.insert(0, sys.argv[2]); sys.path.insert(0, sys.argv[3])
+from oracle import qoracle as qo
+import qb200
+from util import make_weight, rand_bf16, dev_triple, to_dev_bf16, gate_bf16
+for (M, N, K, bits, gs) in [(64, 640, 4096, 4, 64), (40, 1000, 2048, 8, 64), (57, 4096, 1024, 4, 128), (33, 16, 512, 4, 64)]:
+    rng = np.random.default_rng(M + N + K)
+    q, s, b = make_weight(rng, (N, K), gs, bits)
+    xh = qo.f32_to_bf16(rand_bf16(rng, (M, K)))
+    y = qb200.quantized_matmul(to_dev_bf16(xh), *dev_triple(q, s, b), True, gs, bits)
+    ref = qo.qmm(qo.bf16_to_f32(xh), q, s, b, gs, bits, True, bf16_weights=True)
+    gate_bf16(y.float().cpu().numpy(), ref, f"64-token form {M}x{N}x{K}")
+assert qb200.lib().qb200_debug_tc_status() == 0
+print("ok")
+"""
+
+
+def test_wide_kernel_64_token_form_behind_the_environment_switch():
+    """QB200_WIDE_MAX_TOKENS=64 (read once per process, hence a child process) sends 33..64 tokens to the wide streaming
+    kernel's 64-token form, which the default routing no longer reaches."""
+    import os, subprocess, sys
+    here = os.path.dirname(os.path.abspath(__file__))
+    root = os.path.dirname(here)
+    env = dict(os.environ, QB200_WIDE_MAX_TOKENS="64")
+    out = subprocess.run([sys.executable, "-c", _WIDE64_CHILD, root, os.path.join(root, "mlx-serve_b200"), here],
+                         env=env, capture_output=True, text=True, timeout=600)
+    assert out.returncode == 0 and out.stdout.strip().endswith("ok"), out.stdout[-2000:] + out.stderr[-2000:]
+
+
 def test_config2_m128():
     rng = np.random.default_rng(0xC2 + 128)
     q, s, b = make_weight(rng, (4096, 4096), 64, 4)
