@@ -88,8 +88,22 @@ def test_where_no_cluster_can_be_placed(no_clusters):
     (4, (288, 256, 512, 1, 224, 481, 320, 96)), (8, (510, 290, 33, 300)), (4, (270,) * 8)])
 def test_accumulators_in_turn(bits, counts):
     """Several tiles a pair, of one and two units, whose accumulators go round the ring of tensor memory in many ways: cut at its end,
-    moved to its start, beside those of the tile before."""
-    sorted_rows_exact(bits, counts, 11264)                  # 44 tiles and more of 256 weight rows an expert
+    moved to its start, beside those of the tile before.  One expert's weights against the exact sum over all its rows."""
+    import qb200
+    N, K, E = 11264, 256, len(counts)                       # 44 tiles and more of 256 weight rows an expert
+    g = torch.Generator(device="cuda").manual_seed(bits + E)
+    w = qb200.quantize(torch.randn(E, N, K, device="cuda", generator=g).to(torch.bfloat16) * 0.05, 64, bits)
+    x = torch.randn(sum(counts), 1, K, device="cuda", generator=g).to(torch.bfloat16)
+    idx = torch.repeat_interleave(torch.arange(E), torch.tensor(counts)).int().cuda()
+    y = qb200.gather_qmm(x, *w, None, idx, True, 64, bits, sorted_indices=True)
+    assert qb200.lib().qb200_debug_tc_status() == 0
+    for e in range(E):
+        m = idx == e
+        wd = qb200.dequantize(*(t[e].contiguous() for t in w), 64, bits, dtype=torch.bfloat16).double()
+        ref = x[m, 0].double() @ wd.t()
+        # bf16 rounding of the result (2^-8), and fp32 sums of 256 products in any order (2^-23 a step)
+        tol = 2.0 ** -8 * ref.abs() + 256 * 2.0 ** -23 * (x[m, 0].double().abs() @ wd.abs().t())
+        assert bool(((y[m, 0].double() - ref).abs() <= tol).all()), f"expert {e}"
 
 
 @pytest.mark.parametrize("bits,counts,N", [
@@ -106,7 +120,7 @@ def test_dense_short_contractions(M, N, K):
 
 
 def sorted_rows_exact(bits, counts, N, K=256):
-    """One expert's weights against the exact sum over all its rows; a single one is a dense product."""
+    """The same with any number of weight rows and any contraction; a single expert is a dense product."""
     import qb200
     E = len(counts)
     g = torch.Generator(device="cuda").manual_seed(bits + E)
