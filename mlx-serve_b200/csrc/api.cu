@@ -313,7 +313,7 @@ static int prepare_qmm(qb200_tensor* res, const qb200_tensor* x, const qb200_ten
 }
 
 // Routing by token count.  Up to 8 tokens: the narrow streaming kernel (one launch).  9 .. 64 (bf16 activations that a tensor map takes): the
-// kernel that streams weights through tensor memory (us, before -> there, a layer of Llama-3-8B's projections 85 -> 58 at 16 tokens;
+// kernel that streams weights through tensor memory (us, before -> there, a layer of Llama-3-8B's projections 85 -> 55 at 16 tokens;
 // 4-bit 4096 x 4096 16.8 -> 8.8 at 32, 26.6 -> 10.3 at 64; 512 x 512 7.8 -> 3.4, 6.9 -> 4.9; 128 x 256, the smallest, 3.3 -> 3.3 at 9,
 // 4.0 -> 3.4, 5.9 -> 4.7).  9 .. 32 of other activations: the wide streaming kernel.  Above, the tensor-core kernel, whose time does not
 // depend on the token count up to 128.

@@ -14,8 +14,8 @@
 //    has read it, and so works beside the next tile except for the blocks that two tiles have in common (two tiles of 288 tokens: 64
 //    of 512 columns).  With two slots of 256 columns a tile of two units began after the whole epilogue of the one before, 6800 of
 //    16800 cycles at K = 768 (128 experts, us, before -> after: 256 rows an expert 768 x 2048 123 -> 117, 2048 x 768 134 -> 115; 290
-//    rows 132 -> 124, 148 -> 126).  Launches of one-unit tiles are a form of their own, without the arithmetic of cut tiles, whose epilogue
-//    gives its blocks back at the end of a tile: with one form for both they took 150 cycles a block and 0.2 us a tile more (us, two slots,
+//    rows 132 -> 124, 148 -> 126).  Launches of one-unit tiles are a form of their own, without the arithmetic of cut tiles, which take
+//    the two halves in turn and give one back at the end of a tile: with one form for both they took 150 cycles a block and 0.2 us a tile more (us, two slots,
 //    one form, two forms: 2048 tokens, 14336 x 256 25.6, 29.0, 25.2; 1138 tokens, 14147 x 768 53.3, 59.1, 53.7).
 //  * Roles per CTA: twelve warps convert weights (three groups of four that take k-blocks in turn, a thread per weight row), four
 //    are the epilogue, and one each loads x, loads packed codes, issues the MMAs (CTA 0 only: its instructions read both CTAs'

@@ -2,10 +2,10 @@
 // word read once, What = bf16(q*s + b) as the dense route that it stands for has it (mlx-serve src/transformer.zig:20987-21011; the
 // widths its scheduler batches, src/scheduler.zig:5147, and prompts of a few dozen tokens).
 //
-// Bound: what a unit of 128 rows x 256 K costs.  At 27 tokens (57344 x 4096, ncu) it takes 852 issue slots of a scheduler over all roles and
-// 1535 cycles, with four warps a scheduler to fill them; its 18 KB would take 820 at the copy bandwidth, the tensor pipe is busy for 14 %.
+// Bound: what a unit of 128 rows x 256 K costs.  At 27 tokens (57344 x 4096, ncu) it takes 781 issue slots of a scheduler over all roles and
+// 1403 cycles, with four warps a scheduler to fill them; its 18 KB would take 820 at the copy bandwidth, the tensor pipe is busy for 18 %.
 // us a layer of Llama-3-8B's projections (218 M weights, four launches, each replayed), before -> after: 16 tokens
-// 85 -> 58, 27 tokens 110 -> 61 (a streaming kernel on mma.sync before), 64 tokens 143 -> 75 (tcgen05 with the weights through shared
+// 85 -> 55, 27 tokens 110 -> 58 (a streaming kernel on mma.sync before), 64 tokens 143 -> 67 (tcgen05 with the weights through shared
 // memory); 4096 x 4096 alone 16.8 -> 8.8 at 32, 26.6 -> 10.3 at 64; 512 x 512 7.8 -> 3.4, 6.9 -> 4.9.
 //  * A thread converts a weight row.  Its codes lie in a lane of registers and go to the same lane of tensor memory, the A operand of
 //    the MMA: no shuffles, no shared-memory tile, scale and bias one register each.
