@@ -467,9 +467,14 @@ __global__ void __launch_bounds__(kThreads, 1) qmv_tmem_kernel(const __grid_cons
             else *(uint4*)(rx + b * rx_buf + (rank * gpc + g - a) * 2048 + r * 16) = make_uint4(o4[0], o4[1], o4[2], o4[3]);
           }
         } else {
+          uint16_t* to_y = y + (int64_t)c * ldy;                              // (with a product for every address tiles of few units waited for this: 1.7 us a tile at K = 256 and 512, now 1.3)
+          const int left = row_ok ? p.M - c : 0;
 #pragma unroll
-          for (int i = 0; i < 32; ++i)
-            if (row_ok && c + i < p.M) y[(int64_t)(c + i) * ldy] = f32_to_bf16_bits(__uint_as_float(v[i]));
+          for (int i = 0; i < 32; ++i) {
+            if (i % 8 == 0 && c + i >= p.M) break;
+            if (i < left) *to_y = f32_to_bf16_bits(__uint_as_float(v[i]));
+            to_y += ldy;
+          }
         }
       }
       if (C > 1 && g1 > g0) {
