@@ -314,9 +314,10 @@ static int prepare_qmm(qb200_tensor* res, const qb200_tensor* x, const qb200_ten
 
 // Routing by token count.  Up to 8 tokens: the narrow streaming kernel (one launch).  9 .. 64 (bf16 activations that a tensor map takes): the
 // kernel that streams weights through tensor memory (us, before -> there, a layer of Llama-3-8B's projections 85 -> 55 at 16 tokens;
-// 4-bit 4096 x 4096 16.8 -> 8.8 at 32, 26.6 -> 10.3 at 64; 512 x 512 7.8 -> 3.4, 6.9 -> 4.9; 128 x 256, the smallest, 3.3 -> 3.3 at 9,
-// 4.0 -> 3.4, 5.9 -> 4.7).  9 .. 32 of other activations: the wide streaming kernel.  Above, the tensor-core kernel, whose time does not
-// depend on the token count up to 128.
+// 4-bit 4096 x 4096 17.2 -> 9.2 at 32, 26.9 -> 10.6 at 64; 512 x 512 8.1 -> 3.5, 7.2 -> 4.1; 128 x 256 3.7 -> 3.3 at 9, 4.3 -> 3.4, 6.1 -> 3.8;
+// slower only at K = 256 and 4 bits over 16,000 to 40,000 rows, 28672 x 256 4.6 -> 5.8 at 9; the kernel before has one scratch array for all
+// streams, which these calls no longer share).  9 .. 32 of other activations: the wide streaming kernel.  Above, the tensor-core kernel, whose
+// time does not depend on the token count up to 128.
 // QB200_WIDE_MAX_TOKENS in the environment, read once, sends all that the wide kernel serves of 9 up to so many tokens (64 at most; 0: nothing)
 // there: a diagnostic, to measure the others against it.
 static int64_t wide_switch() {

@@ -2,11 +2,11 @@
 // word read once, What = bf16(q*s + b) as the dense route that it stands for has it (mlx-serve src/transformer.zig:20987-21011; the
 // widths its scheduler batches, src/scheduler.zig:5147, and prompts of a few dozen tokens).
 //
-// Bound: what a unit of 128 rows x 256 K costs.  At 27 tokens (57344 x 4096, ncu) it takes 781 issue slots of a scheduler over all roles and
-// 1403 cycles, with four warps a scheduler to fill them; its 18 KB would take 820 at the copy bandwidth, the tensor pipe is busy for 18 %.
+// Bound: what a unit of 128 rows x 256 K costs.  At 27 tokens (57344 x 4096, ncu) it takes 770 issue slots of a scheduler over all roles and
+// 1359 cycles, with four warps a scheduler to fill them; its 18 KB would take 820 at the copy bandwidth, the tensor pipe is busy for 19 %.
 // us a layer of Llama-3-8B's projections (218 M weights, four launches, each replayed), before -> after: 16 tokens
-// 85 -> 55, 27 tokens 110 -> 58 (a streaming kernel on mma.sync before), 64 tokens 143 -> 67 (tcgen05 with the weights through shared
-// memory); 4096 x 4096 alone 16.8 -> 8.8 at 32, 26.6 -> 10.3 at 64; 512 x 512 7.8 -> 3.4, 6.9 -> 4.9.
+// 85 -> 55, 27 tokens 110 -> 57 (a streaming kernel on mma.sync before), 64 tokens 143 -> 66 (tcgen05 with the weights through shared
+// memory); 4096 x 4096 alone 17.2 -> 9.2 at 32, 26.9 -> 10.6 at 64; 512 x 512 8.1 -> 3.5, 7.2 -> 4.1.
 //  * A thread converts a weight row.  Its codes lie in a lane of registers and go to the same lane of tensor memory, the A operand of
 //    the MMA: no shuffles, no shared-memory tile, scale and bias one register each.
 //  * A group of four warps takes units in turn, half a unit (64 columns of tensor memory) at a time, and meets its issuer at a named barrier
@@ -641,7 +641,7 @@ cudaError_t clusters_of(int cluster, int* n) {
 // The cluster size: tiles x units of a tile's share, and the hand-over of the sums, which the first tile of a cluster hides better than those
 // behind it (its last CTA then waits for the peers' epilogues and the start of its own next tile).  In units of about 0.65 us; by times of
 // every size over 1618 shapes (9 - 64 tokens, 1 - 625 tiles, K 256 - 14336).  With 0.4 a tile it took clusters of many short tiles: 4-bit 18945
-// x 1280 at 9 tokens, six tiles of one unit a cluster of five, 21.7 us, now two of five units a CTA, 10.6; 28672 x 4096 26.1 -> 24.0.
+// x 1280 at 9 tokens, six tiles of one unit a cluster of five, 21.7 us, now two of five units a CTA, 9.8; 28672 x 4096 26.1 -> 22.9.
 struct Plan { int cluster, ncl, per, ku; };                // CTAs that split K, clusters, tiles and units of K of one at most
 template <int BITS>
 cudaError_t plan(const TmK& p, int most, Plan* out) {
